@@ -253,9 +253,9 @@ rt_status rt_mesh_upload(rt_ctx *ctx, const rt_mesh_desc *mesh);
 rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const int32_t *cellIJK);
 
 /* Options.  RT_OPT_SWEEP: 0 auto (systolic when structured), 1 level-scheduled
- * sweeps, 2 structured systolic sweeps.  RT_OPT_SWEEP_PLANES: planes per
- * thread-block cluster of the systolic sweeps, one CTA per plane (1 .. 16;
- * default 16, or 8 where a cluster of 16 cannot be scheduled).
+ * sweeps, 2 structured systolic sweeps.  RT_OPT_SWEEP_PLANES (1 .. 16, on a
+ * structured mesh) is kept for callers of the sweeps that ran in thread-block
+ * clusters of planes; it has no effect.
  * RT_OPT_PRECISION: RT_PREC_FP64 or RT_PREC_MIXED for rt_ldu_solve (the time
  * step takes its precision from rt_case_ctl). */
 #define RT_OPT_SWEEP 1
@@ -271,27 +271,25 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
  * FP64 solve differs from the exact solution, so the mixed form iterates a
  * little further to keep its fields within 1e-6 of the FP64 form. */
 #define RT_OPT_MIXED_TIGHTEN 5
-/* RT_OPT_SWEEP_TUNE: schedule of the one-component systolic sweeps (chunk of
- * P steps, NB chunks staged ahead): 0 (default) times the candidates on the
- * first application per structured mesh and precision and keeps the fastest;
- * 1 .. 5 forces one (P, NB) of (8,3) (8,5) (16,3) (16,4) (4,6). */
+/* RT_OPT_SWEEP_TUNE: schedule of the systolic sweeps (chunk of P steps, NB
+ * chunks staged ahead): 0 (default) the library's choice by precision, size
+ * and components; 1 .. 5 forces one (P, NB) of (8,3) (8,5) (16,3) (16,4) (4,6).
+ * All give the same bits. */
 #define RT_OPT_SWEEP_TUNE 6
-/* RT_OPT_SWEEP_RING: deepest plane-to-plane ring of the systolic sweeps, in
- * steps (a power of two, 8 .. 128; 0 = default 128).  Each launch takes the
- * deepest ring up to this cap that fits the shared memory. */
+/* RT_OPT_SWEEP_RING: kept for callers of the sweeps that handed planes over
+ * through rings of that depth (0, or a power of two 8 .. 128); no effect. */
 #define RT_OPT_SWEEP_RING 7
 /* RT_OPT_WAIT_LIMIT: spins a bounded device-side wait of the systolic sweeps
  * makes before it gives up (sets the sweep's error flag; the call returns
  * RT_ETIMEOUT and the context stays usable).  Default 2^24 (about a second
- * for a wait between thread-block clusters, which polls 16x less often);
- * 64 .. 2^40. */
+ * for a wait between CTAs, whose spins are L2 round trips, eight counted as
+ * one); 64 .. 2^40. */
 #define RT_OPT_WAIT_LIMIT 8
 /* RT_OPT_STALL_TEST: failure-detection tests only.  value > 0: in the next
- * `value` systolic sweep launches, the first plane of every thread-block
- * cluster after the first waits for a hand-off word that no plane writes, so
- * its bounded wait runs out and the call returns RT_ETIMEOUT (meshes with
- * more planes than one cluster holds; see RT_OPT_SWEEP_PLANES).  0 (default)
- * clears it. */
+ * `value` systolic sweep launches, every CTA that waits for the hand-off words
+ * of another takes them as never written, so its bounded wait runs out and the
+ * call returns RT_ETIMEOUT (meshes of more rows or planes than one CTA holds: at
+ * most 16 rows and 8 planes, or 128 rows in one plane).  0 (default) clears it. */
 #define RT_OPT_STALL_TEST 9
 /* RT_OPT_MIXED_PRECOND: the preconditioner of the mixed form's pressure
  * solve (DIC selected).  -2 (default): on structured meshes without coupled
@@ -315,11 +313,9 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
  * decisions; the persistent form sums each case's reductions in one pass of
  * its CTA, so the iterates agree to round-off, not bit for bit. */
 #define RT_OPT_BATCH_PERSISTENT 11
-/* RT_OPT_SWEEP_COMPONENTS: the systolic sweeps of a solve of two or three
- * components (the momentum solve).  1 (default): the components side by
- * side, one one-component sweep each in a single launch (each thread-block
- * cluster takes a plane group of one component); 0: one sweep carrying all
- * the components lane by lane.  Both give the same bits. */
+/* RT_OPT_SWEEP_COMPONENTS (0 or 1): kept for callers that chose between the
+ * components of a solve lane by lane and side by side; they always go side by
+ * side in one launch, with the same bits. */
 #define RT_OPT_SWEEP_COMPONENTS 12
 /* RT_OPT_MIXED_PRECOND_U: the preconditioner of the mixed form's momentum
  * solve (DILU selected, up to three components).  -2 (default): on

@@ -391,20 +391,26 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
             lo[(size_t)dir * N + n] = f;
         }
         s.nx = nx; s.ny = ny; s.nz = nz;
-        s.nJB = (ny + 31) / 32;
-        s.T = ((nx + 31 + 15) / 16) * 16;   // steps per block, padded to whole chunks (P <= 16)
-        s.nSkew = (long long)nz * s.nJB * s.T * 32;
+        // the sweeps' tiles: 8 x 4 rows (j, k), or 32 x 1 in one plane
+        s.TJ = nz == 1 ? 32 : 8;
+        const int TJ = s.TJ, TK = 32 / TJ;
+        s.nTJ = (ny + TJ - 1) / TJ;
+        s.nTK = (nz + TK - 1) / TK;
+        // steps per tile, padded to whole chunks (P <= 16)
+        s.T = (nx + kSkewJ * (TJ - 1) + kSkewK * (TK - 1) + 15) / 16 * 16;
+        s.nSkew = (long long)s.nTJ * s.nTK * s.T * 32;
         std::vector<int> cellOf((size_t)s.nSkew, -1);
         for (int k = 0; k < nz; ++k)
-            for (int jb = 0; jb < s.nJB; ++jb)
-                for (int t = 0; t < s.T; ++t)
-                    for (int l = 0; l < 32; ++l) {
-                        int i = t - l, j = jb * 32 + l;
-                        if (i < 0 || i >= nx || j >= ny) continue;
-                        // quad layout: one lane's four consecutive steps are adjacent
-                        long long e = ((long long)k * s.nJB + jb) * s.T * 32 + (long long)(t >> 2) * 128 + l * 4 + (t & 3);
-                        cellOf[(size_t)e] = at[((size_t)k * ny + j) * nx + i];
-                    }
+            for (int j = 0; j < ny; ++j) {
+                const int l = (k % TK) * TJ + j % TJ;
+                const long long tile = (long long)(k / TK) * s.nTJ + j / TJ;
+                for (int i = 0; i < nx; ++i) {
+                    const int t = i + kSkewJ * (j % TJ) + kSkewK * (k % TK);
+                    // one lane's two consecutive steps are adjacent
+                    cellOf[(size_t)(tile * s.T * 32 + (long long)(t >> 1) * 64 + l * 2 + (t & 1))] =
+                        at[((size_t)k * ny + j) * nx + i];
+                }
+            }
         upload_vec(ctx, cellOf, s.cellOf);
         upload_vec(ctx, lo, s.faceLo);
         upload_vec(ctx, hi, s.faceHi);
@@ -418,11 +424,9 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
             for (MgGraph &g : s.mgGraph) g.reset();
             s.mgNext = 0;
         }
-        RT_REQUIRE(s.nJB <= 8 && skew_fits(s.nJB), RT_EINVAL, "structured sweeps need ny <= 256");
-        // planes (CTAs) per thread-block cluster: 16 (the non-portable maximum;
-        // fewer hand-offs through global memory), 8 where 16 cannot be scheduled
-        s.KC = std::max(1, std::min(nz, 16));
-        s.sync.alloc(SYNC_PROGRESS + (size_t)nz * s.nJB);
+        RT_REQUIRE(ny <= 256, RT_EINVAL, "structured sweeps need ny <= 256");
+        s.sync.alloc(SYNC_WORDS);
+        for (auto &x : s.xfer) x.release();   // laid out anew on the next sweep
         s.sync.zero(ctx->stream);
         s.data.alloc((size_t)(12 + 6 + 6) * s.nSkew);
         s.data.zero(ctx->stream);
@@ -455,21 +459,17 @@ rt_status rt_set_option(rt_ctx *ctx, int32_t option, int64_t value) {
             StructMesh &s = ctx->mesh.sm;
             RT_REQUIRE(s.on, RT_ENOTREADY, "mesh is not structured");
             RT_REQUIRE(value >= 1 && value <= 16, RT_EINVAL, "planes per cluster: 1 .. 16");
-            s.KC = (int)std::min<int64_t>(value, s.nz);
-            s.tune[0] = s.tune[1] = -1;
-            return RT_OK;
+            return RT_OK;   // the sweeps' tiles need no clusters
         }
         case RT_OPT_SWEEP_TUNE:
-            RT_REQUIRE(value >= 0 && value <= 5, RT_EINVAL, "RT_OPT_SWEEP_TUNE: 0 autotune, 1 .. 5 a schedule");
+            RT_REQUIRE(value >= 0 && value <= 5, RT_EINVAL, "RT_OPT_SWEEP_TUNE: 0 default, 1 .. 5 a schedule");
             ctx->sweepTune = (int)value;
             ctx->mesh.sm.tune[0] = ctx->mesh.sm.tune[1] = -1;
             return RT_OK;
         case RT_OPT_SWEEP_RING:
             RT_REQUIRE(value == 0 || (value >= 8 && value <= 128 && (value & (value - 1)) == 0), RT_EINVAL,
                        "RT_OPT_SWEEP_RING: 0, or a power of two 8 .. 128");
-            ctx->sweepRing = (int)value;
-            ctx->mesh.sm.tune[0] = ctx->mesh.sm.tune[1] = -1;
-            return RT_OK;
+            return RT_OK;   // the tiles hand their words over through whole rows, not rings
         case RT_OPT_WAIT_LIMIT:
             RT_REQUIRE(value >= 64 && value <= (1ll << 40), RT_EINVAL, "RT_OPT_WAIT_LIMIT: 64 .. 2^40 spins");
             ctx->waitLimit = value;
@@ -495,8 +495,7 @@ rt_status rt_set_option(rt_ctx *ctx, int32_t option, int64_t value) {
             return RT_OK;
         case RT_OPT_SWEEP_COMPONENTS:
             RT_REQUIRE(value == 0 || value == 1, RT_EINVAL, "RT_OPT_SWEEP_COMPONENTS: 0 or 1");
-            ctx->sweepComponents = (int)value;
-            return RT_OK;
+            return RT_OK;   // always side by side
         case RT_OPT_BATCH_PERSISTENT:
             RT_REQUIRE(value >= 0 && value <= 2, RT_EINVAL, "RT_OPT_BATCH_PERSISTENT: 0 never, 1 auto, 2 always");
             ctx->batchPersistent = (int)value;

@@ -92,13 +92,17 @@ struct DBuf {
     operator T *() const { return p; }
 };
 
-constexpr int SYNC_WORK = 0, SYNC_ERROR = 1, SYNC_PROGRESS = 2;
+constexpr int SYNC_WORK = 0, SYNC_ERROR = 1, SYNC_DONE = 2, SYNC_WORDS = 4;
+
+// steps by which a row of the structured sweeps' tiles lags the row before it
+// in j and in k (sweep.cu)
+constexpr int kSkewJ = 1, kSkewK = 2;
 
 // raw view passed to the kernels; every array has nSkew entries in the
-// skewed (block, step / 4, lane, step % 4) layout, wS has 6 components of nSkew
+// skewed (tile, step / 2, lane, step % 2) layout, wS has 6 components of nSkew
 template <class Real>
 struct SkewT {
-    int nx, ny, nz, nJB, T;
+    int nTJ, nTK, T;
     long long nSkew;
     const int *cellOf;
     Real *D, *Pz, *Py, *Px, *rDraw;   // rD recurrence inputs / output (FP64 only)
@@ -137,16 +141,14 @@ constexpr int kMgGraphs = 8;   // captured V-cycles kept per mesh
 
 struct StructMesh {
     bool on = false;
-    int nx = 0, ny = 0, nz = 0, nJB = 0, T = 0;
-    int KC = 1;                // planes per CTA of the systolic sweeps
+    int nx = 0, ny = 0, nz = 0, T = 0;
+    int TJ = 8, nTJ = 0, nTK = 0;   // the sweeps' tiles: TJ x 32 / TJ rows (j, k) each, nTJ x nTK of them
     long long nSkew = 0;
     DBuf<int> cellOf;          // nSkew: cell of each skewed entry, -1 outside the mesh
     DBuf<int> faceLo, faceHi;  // 3*N: face to the (z, y, x) lower / upper neighbour, -1 if none
-    DBuf<int> sync;            // work counter, error flag
-    DBuf<unsigned long long> xfer;   // tagged hand-off words between clusters
-    unsigned epoch = 0;        // tag of the current launch's hand-off words
-    int tune[2] = {-1, -1};    // schedule of the one-component sweeps (FP64, FP32), -1 until tuned
-    float tuneMs[2] = {0, 0};  // its time per application
+    DBuf<int> sync;            // tickets taken, error flag, tiles finished
+    DBuf<unsigned long long> xfer[2];   // hand-off words between tiles (FP64, FP32)
+    int tune[2] = {-1, -1};    // schedule of the sweeps (FP64, FP32), -1 before the first application
     DBuf<double> data;         // 12 + 6 + 6 arrays of nSkew doubles
     bool pendingCheck = false;
     // the box: the cell of each box position (-1 outside the mesh) and the
@@ -159,7 +161,7 @@ struct StructMesh {
 
     SkewView view() {
         SkewView v;
-        v.nx = nx; v.ny = ny; v.nz = nz; v.nJB = nJB; v.T = T; v.nSkew = nSkew;
+        v.nTJ = nTJ; v.nTK = nTK; v.T = T; v.nSkew = nSkew;
         v.cellOf = cellOf.p;
         double *p = data.p;
         double **slots[] = {&v.D, &v.Pz, &v.Py, &v.Px, &v.rDraw, &v.rDinv, &v.Az, &v.Ay, &v.Ax,
@@ -191,7 +193,7 @@ struct StructMesh {
     SkewView32 view32() {
         if (data32.n != (size_t)19 * nSkew) data32.alloc((size_t)19 * nSkew);
         SkewView32 v;
-        v.nx = nx; v.ny = ny; v.nz = nz; v.nJB = nJB; v.T = T; v.nSkew = nSkew;
+        v.nTJ = nTJ; v.nTK = nTK; v.T = T; v.nSkew = nSkew;
         v.cellOf = cellOf.p;
         v.D = v.Pz = v.Py = v.Px = v.rDraw = nullptr;
         float *p = data32.p;

@@ -10,34 +10,46 @@
 // FMA contraction).  The same kernel runs in FP32 for the mixed-precision
 // solvers (coefficients rounded from the FP64 factorisation).
 //
-// Work decomposition: rows (j,k) are grouped in blocks of 32 consecutive j in
-// one plane k.  A warp owns a block; at step t lane l updates cell i = t - l of
-// row j = 32 jb + l.  The i-1 value is the lane's own previous result
-// (register) and the j-1 value lane l-1's previous result (shuffle).  Lane 0
-// reads j-1 from the j-block below (step t + 31) and every lane reads k-1 from
-// the block of the previous plane (same step).  The steps are taken in chunks
-// of P: a chunk stages its coefficients and exchanges the j-block words once,
-// and takes the previous plane's words and publishes its own to the next
-// plane quad by quad (four steps), so the planes lag one another by a quad.
+// Work decomposition: the rows (j, k) are grouped in tiles of TJ x TK = 32 (8 x
+// 4, or 32 x 1 on a mesh of one plane), a tile a warp and a row a lane, and WJ
+// x WK neighbouring tiles in a CTA.  At step t the lane of row (j, k) of its
+// tile updates cell i = t - kSkewJ j - kSkewK k.  The i-1 value is the lane's own
+// last result; the j-1 and k-1 values are results that other lanes formed, read
+// from a ring of the last steps' results of all the CTA's tiles in shared
+// memory; those of the tiles of other CTAs (the ghosts) lie in the same ring.  So
+// a lane reads its two neighbours at addresses fixed but for the step, and a
+// step is two reads, three products and one write, without a branch.
 //
-// One CTA owns one plane (warp = j-block); a thread-block cluster owns CS
-// consecutive planes.  Values handed to another warp (plane to plane through
-// distributed shared memory, j-block to j-block through shared memory,
-// cluster to cluster through global memory) travel as tagged 64-bit words, so
-// a consumer waits on the data itself and no fence or release/acquire pair
-// sits on the dependency chain.  Clusters take plane groups in dependency
-// order from an atomic counter, so a cluster only waits on groups owned by
-// running clusters: no deadlock.  Every wait is bounded; a timeout sets an
-// error flag, every other wait gives up on seeing it, and the host reports
-// RT_ETIMEOUT.
+// What bounds it: latency.  Measured on GB300: a dependent FP64 fused
+// multiply-add takes a warp 64 cycles and an independent one 48 (one FP64 unit
+// a quarter of an SM, whatever the lanes in use), an FP32 one 4, a value
+// through shared memory 35, through L2 to another SM 480 to 860.  An FP64 step
+// cannot take less than about 150 cycles and an FP32 one 45; the longest chain
+// has nx + kSkewJ ny + kSkewK nz steps.  So four tiles of a CTA (one a quarter
+// of the SM) hand over in shared memory, only every second tile boundary
+// goes through L2, and all else is kept off the tiles' warps: other warps of
+// the CTA fetch the ghosts, hand results to the next CTAs, stage coefficients
+// and write results out.  With kSkewK = 2 the k product is formed a step ahead,
+// off the chain of a step.
 //
-// Per-entry data live in a "skewed" layout of (block, step, lane) in which one
-// lane's four consecutive steps are adjacent (a quad), so a lane reads and
-// writes its coefficients, results and hand-off words as 16-byte vectors.
-// The backward sweep walks the same layout in reverse (lanes mirrored).
+// A value handed to another CTA is its own flag: the hand-off words hold the
+// pattern of all ones until the producer writes the value (a result with that
+// pattern, a NaN, is written as another NaN), and the consumer puts the
+// pattern back once it has read the word.  So a consumer waits on the data
+// itself, one L2 round trip after the store; no fence, tag or release/acquire
+// pair sits on the dependency chain.  Groups of tiles are taken in dependency
+// order from an atomic counter, so a CTA only waits on CTAs already running: no
+// deadlock.  Every wait is bounded; a timeout sets an error flag, every other
+// wait gives up on seeing it, and the host reports RT_ETIMEOUT and clears the
+// hand-off words.
+//
+// Per-entry data live in a "skewed" layout of (tile, step, lane) in which one
+// lane's two consecutive steps are adjacent (a pair), so a lane reads and
+// writes its coefficients and results as 16-byte vectors without bank
+// conflicts, and a chunk of P steps of one array is one contiguous block,
+// staged by one bulk copy NB chunks ahead.  The backward sweep walks the
+// same layout in reverse (lanes mirrored).
 #include <algorithm>
-
-#include <cooperative_groups.h>
 
 #include "real_ops.cuh"
 #include "rt_internal.h"
@@ -45,583 +57,520 @@
 
 namespace rt {
 
-namespace cg = cooperative_groups;
-
-// ---- tagged hand-off words ------------------------------------------------
-// A value handed to another warp travels with the step it belongs to, packed
-// into one 64-bit word (32-bit payload in the low half, 32-bit tag in the
-// high half) that is written and read with single-copy-atomic 64-bit
-// accesses: a reader sees either the old word (wrong tag) or the new one
-// (value and tag together), so no fence, release or acquire is needed.  An
-// FP64 value travels as two words (its high and low halves), each tagged.
-// Ring slots inside a launch carry tag = step + 1 (the rings are cleared at
-// launch); the global hand-off between clusters carries the launch's epoch,
-// so words left by an earlier launch never match.
 typedef unsigned long long u64;
-template <class Real> struct Words;
-template <> struct Words<float> { static constexpr int W = 1; };
-template <> struct Words<double> { static constexpr int W = 2; };
 
-__device__ __forceinline__ bool get(const volatile u64 *p, unsigned tag, float &v) {
-    const u64 a = *p;
-    if ((unsigned)(a >> 32) != tag) return false;
-    v = __uint_as_float((unsigned)a);
-    return true;
+// ---- hand-off words ---------------------------------------------------------
+template <class Real> struct Word;
+template <> struct Word<double> {
+    typedef u64 T;
+    static __device__ __forceinline__ T of(double v) { return (T)__double_as_longlong(v); }
+    static __device__ __forceinline__ double value(T w) { return __longlong_as_double((long long)w); }
+    static constexpr T kOtherNaN = 0x7ff8000000000000ull;
+};
+template <> struct Word<float> {
+    typedef unsigned T;
+    static __device__ __forceinline__ T of(float v) { return __float_as_uint(v); }
+    static __device__ __forceinline__ float value(T w) { return __uint_as_float(w); }
+    static constexpr T kOtherNaN = 0x7fc00000u;
+};
+__device__ __forceinline__ u64 ld_word(const u64 *p) {
+    u64 v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+    return v;
 }
-__device__ __forceinline__ bool get(const volatile u64 *p, unsigned tag, double &v) {
-    const u64 a = p[0], b = p[1];
-    if ((unsigned)(a >> 32) != tag || (unsigned)(b >> 32) != tag) return false;
-    v = __hiloint2double((int)(unsigned)a, (int)(unsigned)b);
-    return true;
+__device__ __forceinline__ unsigned ld_word(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_word(u64 *p, u64 v) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v));
+}
+__device__ __forceinline__ void st_word(unsigned *p, unsigned v) {
+    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v));
 }
 
+// ---- staging: bulk copies into shared memory, one mbarrier a buffer ------------
+__device__ __forceinline__ void bar_init(unsigned bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool bar_test(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void ld2(const double *p, double &x, double &y) {
+    const double2 a = *reinterpret_cast<const double2 *>(p);
+    x = a.x; y = a.y;
+}
+__device__ __forceinline__ void ld2(const float *p, float &x, float &y) {
+    const float2 a = *reinterpret_cast<const float2 *>(p);
+    x = a.x; y = a.y;
+}
+__device__ __forceinline__ void ld2(const int *p, int &x, int &y) {
+    const int2 a = *reinterpret_cast<const int2 *>(p);
+    x = a.x; y = a.y;
+}
+__device__ __forceinline__ void st2(double *p, double x, double y) {
+    *reinterpret_cast<double2 *>(p) = make_double2(x, y);
+}
+__device__ __forceinline__ void st2(float *p, float x, float y) { *reinterpret_cast<float2 *>(p) = make_float2(x, y); }
 
-// the value of a word pair, and whether it carries the tag (no branch)
-__device__ __forceinline__ bool peek(const u64 *w, unsigned tag, float &v) {
-    v = __uint_as_float((unsigned)w[0]);
-    return (unsigned)(w[0] >> 32) == tag;
+template <int N> struct IntC { static constexpr int v = N; };
+
+// x, not before v is known (zero: a zero that the compiler does not know)
+__device__ __forceinline__ double after(double x, double v, int zero) {
+    return __hiloint2double(__double2hiint(x), __double2loint(x) | (__double2loint(v) & zero));
 }
-__device__ __forceinline__ bool peek(const u64 *w, unsigned tag, double &v) {
-    v = __hiloint2double((int)(unsigned)w[0], (int)(unsigned)w[1]);
-    return ((unsigned)(w[0] >> 32) == tag) & ((unsigned)(w[1] >> 32) == tag);
-}
-// bounded wait of one lane for a tagged value; false after a timeout or when
-// another warp has failed (the error flag is then set)
+__device__ __forceinline__ float after(float x, float, int) { return x; }
+
+// one launch's tiles, components and hand-off words
 template <class Real>
-__device__ __forceinline__ bool wait_get(const volatile u64 *p, unsigned tag, Real &v, int *sync, long long maxSpin,
-                                         bool sleep) {
-    long long spins = 0;
-    while (!get(p, tag, v)) {
-        if ((++spins & 63) == 0 && (spins > maxSpin || *(volatile int *)(sync + SYNC_ERROR))) {
-            atomicExch(sync + SYNC_ERROR, 1);
-            return false;
-        }
-        if (sleep) __nanosleep(64);
-    }
-    return true;
+struct TileRun {
+    SkewT<Real> g;
+    unsigned mask;                  // the components of the launch
+    Real *w;                        // the backward sweep's result (cell order), or null (g.w64)
+    int N, ncc;                     // cells; components launched side by side (one bit of mask each)
+    int *sync;
+    typename Word<Real>::T *xfer;   // hand-off words: per component xstride of them
+    long long xstride;
+    long long maxSpin;
+    int stall;                      // failure-detection test: the hand-off words never arrive
+};
+
+// staged arrays a chunk: MODE 2: D, Pz, Py, Px; MODE 0/1: the z, y, x
+// coefficients and the right-hand side
+constexpr int kStaged = 4;
+constexpr int kWindow = 16;   // steps of hand-off words looked at together
+
+// a CTA's shape and its ring: kRing steps of every tile's 32 results, then the
+// ghosts: the last plane's results (TJ a tile) of the tiles before in k, and the
+// last row's (TK a tile) of the tiles before in j.  A slot holds one step of
+// the tile that formed the value.  A tile lags its producers by kSkewJ TJ or
+// kSkewK TK steps, so the ring is deeper than that.
+template <int TJ, int WJ, int WK>
+struct Group {
+    static constexpr int TK = 32 / TJ, W = WJ * WK;
+    static constexpr int nK = TK > 1 ? WJ : 0, nJ = WK;   // streams of ghosts, and of results handed on
+    static constexpr int ringSteps = TJ >= 32 ? 64 : 32;
+    static constexpr int ghostK = 32 * W, ghostJ = ghostK + nK * TJ;
+    static constexpr int pitch = (ghostJ + nJ * TK + 3) / 4 * 4;
+    static constexpr int warps = 2 * W + 2 * (nK + nJ) + 1;
+};
+
+template <class Real, int P>
+__host__ __device__ constexpr int stage_bytes() { return P * 32 * kStaged * (int)sizeof(Real); }
+template <class Real, class G, int P, int NB>
+__host__ __device__ constexpr int group_smem() {
+    return G::W * NB * stage_bytes<Real, P>() + G::ringSteps * G::pitch * (int)sizeof(Real);
 }
 
-// bounded wait of lane 0 on a progress counter; -1 after a timeout
-__device__ __forceinline__ int wait_count(const volatile int *c, int need, int *sync, long long maxSpin) {
+// counters shared by a CTA's warps (steps of a tile): computed and written out
+// by each tile; ghosts that have arrived and results handed on by each stream;
+// steps staged for each tile
+enum { C_COMPUTED = 0, C_WRITTEN = 8, C_GHOST_K = 16, C_GHOST_J = 20, C_HANDED_K = 24, C_HANDED_J = 28, C_STAGED = 32, C_ABORT = 40,
+       C_TICKET, C_COUNT };
+
+// bounded wait until a counter reaches `need`, by all lanes; -1 when a wait ran out
+template <int NS>
+__device__ __forceinline__ int wait_steps(const volatile int *c, int need, volatile int *cnt, long long maxSpin) {
     long long spins = 0;
-    int v = *c;
-    while (v < need) {
-        if ((++spins & 255) == 0 && (spins > maxSpin || *(volatile int *)(sync + SYNC_ERROR))) {
-            atomicExch(sync + SYNC_ERROR, 1);
+    int v;
+    while ((v = __shfl_sync(0xffffffffu, *c, 0)) < need) {
+        if ((++spins & 63) == 0 && (spins > maxSpin || cnt[C_ABORT])) {
+            cnt[C_ABORT] = 1;
             return -1;
         }
-        v = *c;
+        __nanosleep(NS);   // leaves the issue slots and the shared memory to the recurrence
     }
     return v;
 }
-
-// Ring depths (steps, powers of two) of the hand-offs for chunk size P.  The
-// plane ring is chosen per launch (at least R, at most kMaxRing): a producer
-// may run at most one ring ahead of its consumer, and with a ring of only two
-// chunks it waits one round trip (data forward, progress back) every chunk,
-// so the launch takes the deepest ring that fits the shared memory.
-template <int P> struct Ring {
-    static constexpr int R = (P >= 16) ? 32 : (P >= 4) ? 16 : 8;   // plane ring: at least two chunks
-    static constexpr int RJ = (P >= 8) ? 128 : 64;    // j-block ring: the consumer lags ~32 + P steps
-};
-constexpr int kMaxRing = 128;
-
-// Per-warp staging of a chunk's coefficients (cp.async, NB buffers): NA
-// arrays of P steps x 32 lanes (MODE 2: D, Pz, Py, Px; MODE 0/1: the z, y, x
-// coefficients and the NC right-hand sides), plus the cells of the backward
-// sweep.
-template <int MODE, int NC> struct Stage { static constexpr int NA = (MODE == 2) ? 4 : 3 + NC; };
-
-constexpr size_t kMaxSmem = 227 * 1024 - 1024;   // dynamic shared memory per CTA (static part kept free)
-
-template <class Real, int MODE, int NC, int P, int NB = 3>
-size_t sweep_smem_bytes(int nJB, int R = Ring<P>::R) {
-    constexpr int VW = NC * Words<Real>::W;
-    const size_t rings = (size_t)nJB * ((size_t)R * 32 + Ring<P>::RJ) * VW * sizeof(u64);
-    const size_t stage =
-        (size_t)nJB * NB * P * 32 * (Stage<MODE, NC>::NA * sizeof(Real) + (MODE == 1 ? sizeof(int) : 0));
-    return rings + stage;
+// the lanes' counters until each has reached its need (the rare case, out of
+// line: inlined it slows the recurrence's fast path down); the last values seen
+__device__ __noinline__ int wait_watched(const volatile int *watch, int need, volatile int *cnt, long long maxSpin) {
+    long long spins = 0;
+    for (;;) {
+        const int seen = *watch;
+        if (__all_sync(0xffffffffu, seen >= need)) return seen;
+        if ((++spins & 63) == 0 && (spins > maxSpin || cnt[C_ABORT])) {
+            cnt[C_ABORT] = 1;
+            return seen;
+        }
+    }
 }
-
-// the deepest plane ring (a power of two from Ring<P>::R up to cap, and no
-// deeper than the sweep) that fits the shared memory
-template <class Real, int MODE, int NC, int P, int NB = 3>
-int ring_depth(int nJB, int T, int cap) {
-    int R = Ring<P>::R;
-    while (2 * R <= cap && R < T && sweep_smem_bytes<Real, MODE, NC, P, NB>(nJB, 2 * R) <= kMaxSmem) R *= 2;
-    return R;
-}
-
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void *smem, const void *gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(gmem), "n"(BYTES));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// ---- pairs of tagged words (16-byte vector accesses; each 64-bit element is
-// single-copy atomic on its own, which is all the tag protocol needs)
-__device__ __forceinline__ void ld2_shared(unsigned a, u64 &x, u64 &y) {
-    asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory");
-}
-__device__ __forceinline__ void st2_shared(unsigned a, u64 x, u64 y) {
-    asm volatile("st.volatile.shared.v2.u64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
-}
-__device__ __forceinline__ void st2_cluster(unsigned a, u64 x, u64 y) {
-    asm volatile("st.volatile.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory");
-}
-__device__ __forceinline__ void ld2_global(const u64 *p, u64 &x, u64 &y) {
-    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void st2_global(u64 *p, u64 x, u64 y) {
-    asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x), "l"(y) : "memory");
-}
-__device__ __forceinline__ unsigned map_cluster(unsigned a, unsigned rank) {
-    unsigned m;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(a), "r"(rank));
-    return m;
-}
-__device__ __forceinline__ void pack(float v, unsigned tag, u64 *w) { w[0] = ((u64)tag << 32) | __float_as_uint(v); }
-__device__ __forceinline__ void pack(double v, unsigned tag, u64 *w) {
-    w[0] = ((u64)tag << 32) | (unsigned)__double2hiint(v);
-    w[1] = ((u64)tag << 32) | (unsigned)__double2loint(v);
-}
-
-// ---- four consecutive steps of one lane (one quad of the skewed layout)
-__device__ __forceinline__ void ld4(const float *p, float *v) {
-    const float4 a = *reinterpret_cast<const float4 *>(p);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void ld4(const double *p, double *v) {
-    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
-    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-__device__ __forceinline__ void ld4(const int *p, int *v) {
-    const int4 a = *reinterpret_cast<const int4 *>(p);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void st4(float *p, const float *v) {
-    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
-}
-__device__ __forceinline__ void st4(double *p, const double *v) {
-    reinterpret_cast<double2 *>(p)[0] = make_double2(v[0], v[1]);
-    reinterpret_cast<double2 *>(p)[1] = make_double2(v[2], v[3]);
-}
+// lanes in step, without a barrier on the compiler's other memory accesses
+__device__ __forceinline__ void warp_sync() { asm volatile("bar.warp.sync 0xffffffff;"); }
 
 // MODE 0: forward application, 1: backward application, 2: rD recurrence
-// (FP64 only).
-//
-// Skewed layout: the entry of (block, step t, lane l) is
-// block * 32 T + (t / 4) * 128 + l * 4 + t % 4, so one lane's four
-// consecutive steps are one 16-byte (FP32) or 32-byte (FP64) vector and one
-// chunk of P steps is one contiguous range of P x 32 entries.  The hand-off
-// rings use the same quad order, so a chunk's words are written and read
-// with 16-byte vector accesses.
-//
-// The producer CTA of a plane writes each quad (four steps) of its 32 lanes,
-// tagged, straight into the consumer CTA's ring as soon as the quad is
-// computed (distributed shared memory: remote stores do not wait, and the
-// consumer's local loads are cheap); each consumer lane checks its own words
-// quad by quad, so a plane lags the previous one by about a quad.  The consumer reports its progress back into the
-// producer's shared memory after each chunk, which bounds how far the
-// producer may run ahead (so a slot is never overwritten before it is read;
-// the two waits can never close a cycle).  The j-block hand-off stays inside
-// the CTA (lane 31 of the block below, through a tagged shared ring).  The
-// first plane of a cluster reads the previous cluster's last plane from a
-// tagged global array (one entry per boundary, block, step and lane, written
-// once per launch).  All CTAs of a cluster are co-scheduled, and none leaves
-// before the final cluster barrier, so no CTA ever touches the shared memory
-// of a CTA that has exited.
-//
-// Latency: a chunk's coefficients are staged into shared memory with cp.async
-// NB - 1 chunks ahead and read, with the j-block words, before the wait for
-// the previous plane; the terms of a step that do not depend on the previous
-// step are formed quad by quad ahead of the recurrence, so only the j and i
-// terms stay on the dependent chain.  Invalid entries (outside the mesh, padding) have
-// zero coefficients and zero right-hand sides, so every lane runs the same
-// branch-free recurrence.
-template <class Real, int MODE, int NC, int P, int NB>
-__global__ void __launch_bounds__(256, 1) k_systolic(SkewT<Real> g, unsigned mask, Real *__restrict__ w, int N,
-                                                  int *sync, u64 *__restrict__ xfer, unsigned epoch,
-                                                  unsigned cepoch, long long maxSpin, int R, int ncc,
-                                                  long long xstride) {
-    static_assert(P % 4 == 0 && P <= 32, "a chunk is whole quads");
+// (FP64 only).  The entry of (tile, step t, lane l) is tile * 32 T + (t / 2) *
+// 64 + l * 2 + t % 2.  Entries outside the mesh have zero coefficients and
+// right-hand sides, so every lane runs the same branch-free recurrence.
+// The hand-off words of a tile: for each of its T steps the TJ results of its
+// last plane, for the tile next in k, and the TK results of its last row, for
+// the tile next in j.  Its step s is step s - offK (s - offJ) of that tile.
+template <class Real, int MODE, int TJ, int WJ, int WK, int P, int NB>
+__global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep(TileRun<Real> a) {
+    typedef Group<TJ, WJ, WK> G;
+    typedef Word<Real> Wd;
+    typedef typename Wd::T W;
+    constexpr int TK = 32 / TJ, PITCH = G::pitch, R = G::ringSteps;
+    constexpr int offJ = kSkewJ * (TJ - 1), offK = kSkewK * (TK - 1);   // a producer's lead in steps
+        constexpr int GS = sizeof(Real) == 8 ? 2 : 4;   // steps between two looks at the counters
+    constexpr int B = P < 8 ? P : 8;   // steps that share their slots' addresses
+    static_assert(B % GS == 0 && P % B == 0 && P <= 16 && R % P == 0, "groups fill blocks, blocks chunks, chunks the ring");
+    static_assert(kSkewJ * TJ % B == 0 && (TK == 1 || kSkewK * TK % B == 0), "a block of another tile's slots does not wrap");
+    static_assert(kSkewJ == 1 && kSkewK == 2, "the k product is formed one step ahead, the j product is not");
+    constexpr W kNone = ~W(0);
+    const Real zk = (MODE == 2) ? Real(1) : Real(0);
+    SkewT<Real> &g = a.g;
     // every component of the launch has stopped iterating (the same word for
     // every CTA, written by an earlier kernel): nothing to do
-    if (g.dmask) {
-        mask &= *g.dmask;
-        if (!mask) return;
+    const unsigned live = g.dmask ? a.mask & *g.dmask : a.mask;
+    if (!live) return;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) u64 bars[G::W * NB];
+    __shared__ int s_cnt[C_COUNT];
+    volatile int *cnt = s_cnt;
+    volatile Real *ring = reinterpret_cast<Real *>(smem + G::W * NB * stage_bytes<Real, P>());
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const unsigned bar0 = (unsigned)__cvta_generic_to_shared(bars);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < C_COUNT; ++i) s_cnt[i] = 0;
+        s_cnt[C_TICKET] = atomicAdd(a.sync + SYNC_WORK, 1);
+        for (int b = 0; b < G::W * NB; ++b) bar_init(bar0 + 8 * b);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    constexpr int RJ = Ring<P>::RJ, NA = Stage<MODE, NC>::NA, W = Words<Real>::W;
-    constexpr int VW = NC * W;   // words per (step, lane)
-    constexpr int QW = 4 * VW;   // words per (quad, lane)
-    constexpr int PQ = P / 4;    // quads per chunk
-    cg::cluster_group cluster = cg::this_cluster();
-    const int CS = (int)cluster.num_blocks(), r = (int)cluster.block_rank();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int s_grp;
-    __shared__ int kBack[16], jProg[16];
-    const int lane = threadIdx.x & 31, jo = threadIdx.x >> 5;
-    const int nJB = g.nJB;
-    u64 *ringK = reinterpret_cast<u64 *>(smem_raw);                 // [nJB][R/4][32][4][VW], written by the k-producer
-    u64 *ringJ = ringK + (size_t)nJB * R * 32 * VW;                  // [nJB][RJ][VW]
-    Real *stage = reinterpret_cast<Real *>(ringJ + (size_t)nJB * RJ * VW);   // [nJB][NB][NA][P * 32]
-    int *cstage = (int *)(stage + (size_t)nJB * NB * P * NA * 32);   // [nJB][NB][P * 32] (MODE 1)
-    Real *myStage = stage + (size_t)jo * NB * P * NA * 32;
-    int *myCStage = cstage + (size_t)jo * NB * P * 32;
-    for (size_t i = threadIdx.x; i < (size_t)nJB * (R * 32 + RJ) * VW; i += blockDim.x) ringK[i] = 0ull;
-    if (threadIdx.x < 16) { kBack[threadIdx.x] = 0; jProg[threadIdx.x] = 0; }
-    if (r == 0 && threadIdx.x == 0) s_grp = atomicAdd(sync + SYNC_WORK, 1);
-    cluster.sync();
-    // ncc > 1 (one-component kernels only): the launch sweeps ncc components
-    // side by side; ticket t is plane group t / ncc of component t % ncc, so
-    // every component's groups are taken in dependency order
-    const int ticket = *cluster.map_shared_rank(&s_grp, 0);
-    const int comp = ticket % ncc;
-    const int grp = ticket / ncc;
-    if (ncc > 1) {
-        g.rS += (long long)comp * g.nSkew;
-        g.wS += (long long)comp * g.nSkew;
-        if (w) w += (long long)comp * N;
-        if (g.w64) g.w64 += (long long)comp * N;
-        xfer += (long long)comp * xstride;
-        mask = (mask >> comp) & 1u;
-    }
-    const int nGroups = (g.nz + CS - 1) / CS;
-    const int T = g.T;
-    const int gi = (MODE == 1) ? nGroups - 1 - grp : grp;
-    const int k = (MODE == 1) ? gi * CS + (CS - 1 - r) : gi * CS + r;
-    const bool exists = grp < nGroups && k >= 0 && k < g.nz && mask != 0u;
-    if (exists) {
-        const int jb = (MODE == 1) ? nJB - 1 - jo : jo;
-        const int lf = (MODE == 1) ? 31 - lane : lane;   // the lane's entry column in the forward layout
-        const long long BS = (long long)T * 32;
-        const int blk = k * nJB + jb;
-        const long long blk0 = (long long)blk * BS;
-        const bool hasK = (MODE == 1) ? (k + 1 < g.nz) : (k > 0);
-        const bool kLocalProd = hasK && r > 0;
-        const bool kGlob = hasK && r == 0;
-        const bool consExists = (MODE == 1) ? (k - 1 >= 0) : (k + 1 < g.nz);
-        const bool kLocalCons = consExists && r + 1 < CS;
-        const bool crossProducer = consExists && r == CS - 1;
-        // cluster boundaries: b separates plane groups b and b + 1
-        const int bIn = (MODE == 1) ? gi : gi - 1, bOut = (MODE == 1) ? gi - 1 : gi;
-        const int depJ = (jo > 0) ? jo - 1 : -1;
-        const int consJ = (jo + 1 < nJB) ? jo + 1 : -1;
-        const unsigned ringKs = (unsigned)__cvta_generic_to_shared(ringK);
-        const unsigned ringJs = (unsigned)__cvta_generic_to_shared(ringJ);
-        // the consumer plane's ring, written through distributed shared memory
-        const unsigned consRing = kLocalCons ? map_cluster(ringKs, (unsigned)(r + 1)) : 0u;
-        int *prodBack = kLocalProd ? cluster.map_shared_rank(kBack, r - 1) : nullptr;
-        // word index, in this warp's plane ring, of the quad holding step t of this lane
-        auto kword = [&](int t) -> unsigned {
-            return ((unsigned)(jo * (R >> 2) + ((t & (R - 1)) >> 2)) * 32u + (unsigned)lane) * QW;
-        };
-        // the same in the global hand-off at cluster boundary b
-        auto xword = [&](int b, int t) -> u64 * {
-            return xfer + ((((size_t)b * nJB + jb) * (T >> 2) + (t >> 2)) * 32 + lane) * QW;
-        };
-        // stage the coefficients of the chunk starting at step tc into buffer
-        // b: the chunk's entries of one array are one contiguous block of
-        // P x 32 (the backward sweep walks it mirrored), copied in 16-byte
-        // pieces spread over the lanes; smem layout [buffer][array][P * 32]
-        constexpr int EPC = 16 / (int)sizeof(Real);   // entries per 16-byte piece
-        constexpr int PIECES = P * 32 / EPC;
-        auto copy_block = [&](Real *dst, const Real *src) {
-#pragma unroll
-            for (int i = lane; i < PIECES; i += 32) cp_async<16>(dst + i * EPC, src + i * EPC);
-        };
-        auto stage_chunk = [&](int tc, int b) {
-            const long long lo = (MODE == 1) ? blk0 + (long long)(T - tc - P) * 32 : blk0 + (long long)tc * 32;
-            Real *dst = myStage + (size_t)b * NA * P * 32;
-            if (MODE == 2) {
-                copy_block(dst + 0 * P * 32, g.D + lo); copy_block(dst + 1 * P * 32, g.Pz + lo);
-                copy_block(dst + 2 * P * 32, g.Py + lo); copy_block(dst + 3 * P * 32, g.Px + lo);
-            } else {
-                copy_block(dst + 0 * P * 32, (MODE == 0 ? g.Az : g.Bz) + lo);
-                copy_block(dst + 1 * P * 32, (MODE == 0 ? g.Ay : g.By) + lo);
-                copy_block(dst + 2 * P * 32, (MODE == 0 ? g.Ax : g.Bx) + lo);
-#pragma unroll
-                for (int q = 0; q < NC; ++q)
-                    copy_block(dst + (size_t)(3 + q) * P * 32, (MODE == 0 ? g.rS : g.wS) + (long long)q * g.nSkew + lo);
-                if (MODE == 1) {
-#pragma unroll
-                    for (int i = lane; i < P * 8; i += 32)
-                        cp_async<16>(myCStage + b * P * 32 + i * 4, g.cellOf + lo + i * 4);
-                }
+    for (int i = threadIdx.x; i < R * PITCH; i += blockDim.x) ring[i] = zk;
+    __syncthreads();
+    const int ticket = s_cnt[C_TICKET];
+    // ticket t is group t / ncc of the (t % ncc)-th component, so every
+    // component's groups are taken in dependency order
+    unsigned m = a.mask;
+    for (int q = ticket % a.ncc; q > 0; --q) m &= m - 1;
+    const int comp = __ffs(m) - 1;
+    if ((live >> comp) & 1u) {
+        const int nTJ = g.nTJ, nTK = g.nTK, T = g.T;
+        const int nGJ = (nTJ + WJ - 1) / WJ, grp = ticket / a.ncc;
+        const int J0 = grp % nGJ * WJ, K0 = grp / nGJ * WK;   // the group's first tile, in the direction of the sweep
+        // the role of this warp and its tile (or the tile at its stream's edge)
+        int role, wj, wk;
+        if (wid < 2 * G::W) {
+            role = wid / G::W;   // 0 the recurrence, 1 results
+            wj = wid % G::W % WJ;
+            wk = wid % G::W / WJ;
+        } else {
+            const int q = wid - 2 * G::W;
+            role = 2 + q / (G::nK + G::nJ);   // 2 ghosts, 3 results handed on, 4 staging
+            const int st = q % (G::nK + G::nJ);
+            const bool alongK = st < G::nK;
+            if (role < 4) role += alongK ? 0 : 3;   // 5, 6: the same along j
+            wj = alongK ? st : (role == 6 ? min(WJ, nTJ - J0) - 1 : 0);
+            wk = alongK ? (role == 3 ? min(WK, nTK - K0) - 1 : 0) : st - G::nK;
+            if (role == 4) {   // a lane a tile and array
+                wj = lane / kStaged % WJ;
+                wk = lane / kStaged / WJ % WK;
             }
-        };
-        int seenCK = 0, seenCJ = 0, fail = 0;
-        Real yprev[NC];
-#pragma unroll
-        for (int q = 0; q < NC; ++q) yprev[q] = (MODE == 2) ? Real(1) : Real(0);
-        // NB staging buffers: chunk c is staged NB - 1 chunks ahead
-#pragma unroll
-        for (int c = 0; c < NB - 1; ++c) {
-            if (c * P < T) stage_chunk(c * P, c);
-            cp_async_commit();
         }
-
-        for (int t0 = 0; t0 < T; t0 += P) {
-            const int te = t0 + P;   // T is a multiple of P
-            const int buf = (t0 / P) % NB;
-            cp_async_wait<NB - 2>();   // this chunk's group is complete
-            // ---- back-pressure: consumers have read what this chunk overwrites
-            if (kLocalCons && seenCK < te - R) {
-                int v = 0;
-                if (lane == 0) v = wait_count(kBack + jo, te - R, sync, maxSpin);
-                v = __shfl_sync(0xffffffffu, v, 0);
-                if (v < 0) { fail = 1; break; }
-                seenCK = v;
+        const int w = wk * WJ + wj, J = J0 + wj, K = K0 + wk;
+        const int here = K * nTJ + J;
+        const int tile = (MODE == 1) ? (nTK - 1 - K) * nTJ + (nTJ - 1 - J) : here;
+        const long long e0 = (long long)tile * T * 32;
+        const int lf = (MODE == 1) ? 31 - lane : lane;   // the lane's column in the forward layout
+        const bool there = J < nTJ && K < nTK && !(role == 4 && lane >= kStaged * G::W), exists = there || role == 4;
+        // hand-off words: [tile][T][TJ] along k, then [tile][T][TK] along j
+        W *xk = a.xfer + (long long)comp * a.xstride, *xj = xk + (long long)nTJ * nTK * T * TJ;
+        const long long maxLocal = a.maxSpin << 7;   // spins on shared memory: shorter, and never the first to run out
+        const unsigned myBars = bar0 + 8 * w * NB;
+        unsigned char *myStage = smem + (size_t)w * NB * stage_bytes<Real, P>();
+        if (!exists) {
+        } else if (role == 0) {
+            // ---- the recurrence -------------------------------------------------
+            const int lj = lane % TJ, lk = lane / TJ;
+            // where this lane's neighbours' values are in a slot, and whether they
+            // are another tile's (a slot kSkew? * T? steps on)
+            // (in one plane the k coefficients are zero: any value serves)
+            const bool farK = TK > 1 && lk == 0, farJ = lj == 0;
+            const int iK = TK == 1 ? w * 32 + lane
+                           : !farK ? w * 32 + lane - TJ
+                           : wk > 0 ? (w - WJ) * 32 + (TK - 1) * TJ + lj
+                                    : G::ghostK + wj * TJ + lj;
+            const int iJ = !farJ ? w * 32 + lane - 1
+                           : wj > 0 ? (w - 1) * 32 + lk * TJ + TJ - 1
+                                    : G::ghostJ + wk * TK + lk;
+            const int leadK = farK ? kSkewK * TK : 0, leadJ = farJ ? kSkewJ * TJ : 0;
+            // what must have happened before a group of steps t .. t + GS - 1:
+            // lanes 0 .. 4 each watch a counter that must reach min(t + off, T)
+            const volatile int *watch = cnt + C_COMPUTED + w;
+            int off = -(1 << 29);
+            if (lane == 0 && (wj > 0 || J > 0)) {   // the j producer's steps
+                watch = wj > 0 ? cnt + C_COMPUTED + w - 1 : cnt + C_GHOST_J + wk;
+                off = GS + offJ;
+            } else if (lane == 1 && (wk > 0 || (TK > 1 && K > 0))) {   // the k producer's (one step ahead)
+                watch = wk > 0 ? cnt + C_COMPUTED + w - WJ : cnt + C_GHOST_K + wj;
+                off = GS + offK + 1;
+            } else if (lane == 2 && J + 1 < nTJ) {   // the j consumer has read what these steps overwrite
+                watch = wj + 1 < WJ ? cnt + C_COMPUTED + w + 1 : cnt + C_HANDED_J + wk;
+                off = GS - R;
+            } else if (lane == 3 && TK > 1 && K + 1 < nTK) {
+                watch = wk + 1 < WK ? cnt + C_COMPUTED + w + WJ : cnt + C_HANDED_K + wj;
+                off = GS - R;
+            } else if (lane == 4) {
+                watch = cnt + C_WRITTEN + w;
+                off = GS - R;
+            } else if (lane == 5) {   // the coefficients (a chunk arrives whole)
+                watch = cnt + C_STAGED + w;
+                off = GS;
             }
-            if (consJ >= 0 && seenCJ < te - RJ - 31) {
-                int v = 0;
-                if (lane == 0) v = wait_count(jProg + consJ, te - RJ - 31, sync, maxSpin);
-                v = __shfl_sync(0xffffffffu, v, 0);
-                if (v < 0) { fail = 1; break; }
-                seenCJ = v;
-            }
-            // ---- the chunk's inputs, in the order of their readiness: the
-            // j-block words (the block below runs ahead) and the staged
-            // coefficients first, then, quad by quad, the previous plane's
-            // words, which the pipeline waits on
-            Real wkv[P][NC], wjv[P][NC];
-            bool ok = true;
-            const Real zk = (MODE == 2) ? Real(1) : Real(0);
+            const int zero = a.N >> 31;   // 0
+            int seen = 0;
+            Real y1 = zk, pre = zk;
+            // looks at the counters until the steps from t on may be taken
+            auto until_ready = [&](int t) {
+                const int need = min(t + off, T);
+                if (!__all_sync(0xffffffffu, seen >= need)) seen = wait_watched(watch, need, cnt, maxLocal);
+            };
+            int buf = 0;
+            for (int t0 = 0; t0 < T; t0 += P) {
+                until_ready(t0);
+                const Real *db = reinterpret_cast<const Real *>(myStage + (size_t)buf * stage_bytes<Real, P>());
+                Real va[kStaged][P];
 #pragma unroll
-            for (int s = 0; s < P; ++s)
+                for (int i = 0; i < kStaged; ++i)
 #pragma unroll
-                for (int q = 0; q < NC; ++q) wjv[s][q] = zk;
-            if (depJ >= 0) {
-                // lane s < P fetches and checks the words of step t0 + 31 + s
-                // of the block below (lanes past P repeat the last one), all
-                // in parallel; lane 0 gathers them by shuffles
-                const int ts = t0 + 31 + min(lane, P - 1);
-                const bool live = ts < T;   // steps past the row end read as zero
-                const volatile u64 *src = ringJ + ((size_t)depJ * RJ + (ts & (RJ - 1))) * VW;
-                u64 jw[VW];
+                    for (int s = 0; s < P; s += 2) ld2(db + i * P * 32 + s * 32 + lf * 2, va[i][s], va[i][s + 1]);
 #pragma unroll
-                for (int j = 0; j < VW; ++j) jw[j] = src[j];
-                Real jv[NC];
-                bool hit = true;
+                for (int b0 = 0; b0 < P; b0 += B) {
+                    const int tb = t0 + b0;
+                    volatile Real *cur = ring + (tb & (R - 1)) * PITCH + w * 32 + lane;
+                    // the neighbours' slots of steps tb - 2, tb - 1 and from tb on
+                    const volatile Real *kPast = ring + ((tb - 2 + leadK) & (R - 1)) * PITCH + iK;
+                    const volatile Real *kNow = ring + ((tb + leadK) & (R - 1)) * PITCH + iK;
+                    const volatile Real *jPast = ring + ((tb - 1 + leadJ) & (R - 1)) * PITCH + iJ;
+                    const volatile Real *jNow = ring + ((tb + leadJ) & (R - 1)) * PITCH + iJ;
+                    auto product_k = [&](int s, Real xz) {   // D - Pz / rD(k-1), or r - a_z w(k-1)
+                        const int sf = (MODE == 1) ? P - 1 - b0 - s : b0 + s;
+                        return MODE == 2 ? r_sub(va[0][sf], r_div(va[1][sf], xz)) : r_fma(-va[0][sf], xz, va[3][sf]);
+                    };
 #pragma unroll
-                for (int q = 0; q < NC; ++q) hit &= peek(&jw[q * W], (unsigned)(ts + 1), jv[q]);
-                if (__any_sync(0xffffffffu, live && !hit)) {
-                    if (live) {
-#pragma unroll
-                        for (int q = 0; q < NC; ++q)
-                            ok &= wait_get(src + q * W, (unsigned)(ts + 1), jv[q], sync, maxSpin, false);
-                    }
-                    if (__any_sync(0xffffffffu, !ok)) { fail = 1; break; }
-                }
-#pragma unroll
-                for (int q = 0; q < NC; ++q) jv[q] = live ? jv[q] : zk;
-#pragma unroll
-                for (int s = 0; s < P; ++s)
-#pragma unroll
-                    for (int q = 0; q < NC; ++q) {
-                        const Real v = __shfl_sync(0xffffffffu, jv[q], s);
-                        if (lane == 0) wjv[s][q] = v;
-                    }
-            }
-            // ---- the terms that do not depend on the previous step (the
-            // staged quads of this lane, indexed by forward step offset)
-            Real out[P][NC];
-            int cell[P];   // MODE 1: the cells, by forward step offset
-            Real pre[P][NC], cy[P], cx[P];
-            const Real *db = myStage + (size_t)buf * NA * P * 32;
-            Real va[NA][P];
-#pragma unroll
-            for (int a = 0; a < NA; ++a)
-#pragma unroll
-                for (int qd = 0; qd < PQ; ++qd) ld4(db + (size_t)a * P * 32 + qd * 128 + lf * 4, &va[a][4 * qd]);
-            if (MODE == 1) {
-#pragma unroll
-                for (int qd = 0; qd < PQ; ++qd) ld4(myCStage + buf * P * 32 + qd * 128 + lf * 4, &cell[4 * qd]);
-            }
-            // ---- quad by quad: the previous plane's words of four steps, the
-            // terms that wait on them, the recurrence and the publication of
-            // the quad's results to the next plane.  The next plane starts on a
-            // quad as soon as it is published, so a plane lags the previous
-            // one by about one quad of work plus the hand-off, not a chunk.
-            // (Each word is checked in registers; one warp-uniform branch
-            // leads to the rare bounded waits for words not there yet.  A
-            // ring never wraps inside a chunk: R is a multiple of P.)
-            // (cepoch, the tag a cluster's first plane expects from the
-            // previous cluster, is the launch's epoch except in a
-            // failure-detection test, where no producer writes it)
-            const unsigned ktag = kLocalProd ? (unsigned)(t0 + 1) : cepoch;
-            bool qfail = false;
-            // across a cluster boundary the words come from global memory: the
-            // whole chunk's words are loaded at once (one memory round trip),
-            // and checked quad by quad
-            u64 kwg[PQ][QW];
-            if (kGlob) {
-#pragma unroll
-                for (int qd = 0; qd < PQ; ++qd)
-#pragma unroll
-                    for (int h = 0; h < QW / 2; ++h) ld2_global(xword(bIn, t0 + 4 * qd) + 2 * h, kwg[qd][2 * h], kwg[qd][2 * h + 1]);
-            }
-#pragma unroll
-            for (int qd = 0; qd < PQ; ++qd) {
-                if (kLocalProd || kGlob) {
-                    u64 kw[QW];
-#pragma unroll
-                    for (int h = 0; h < QW / 2; ++h) {
-                        if (kLocalProd) ld2_shared(ringKs + 8u * (kword(t0 + 4 * qd) + 2 * h), kw[2 * h], kw[2 * h + 1]);
-                        else { kw[2 * h] = kwg[qd][2 * h]; kw[2 * h + 1] = kwg[qd][2 * h + 1]; }
-                    }
-                    bool hit = true;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-#pragma unroll
-                        for (int q = 0; q < NC; ++q)
-                            hit &= peek(&kw[e * VW + q * W], kLocalProd ? ktag + 4 * qd + e : ktag, wkv[4 * qd + e][q]);
-                    if (__any_sync(0xffffffffu, !hit)) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-#pragma unroll
-                            for (int q = 0; q < NC; ++q) {
-                                const int s = 4 * qd + e;
-                                const int wi = e * VW + q * W;
-                                const unsigned tag = kLocalProd ? ktag + s : ktag;
-                                const volatile u64 *src = kLocalProd ? ringK + kword(t0 + s) + wi : xword(bIn, t0 + s) + wi;
-                                ok &= wait_get(src, tag, wkv[s][q], sync, kLocalProd ? maxSpin : maxSpin >> 4, kGlob);
-                            }
-                        if (__any_sync(0xffffffffu, !ok)) { qfail = true; break; }
-                    }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-#pragma unroll
-                        for (int q = 0; q < NC; ++q) wkv[4 * qd + e][q] = zk;
-                }
-                // the terms of the quad's steps that do not depend on the previous step
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int s = 4 * qd + e;
-                    const int sf = (MODE == 1) ? P - 1 - s : s;
-                    if (MODE == 2) {
-                        cy[s] = va[2][sf];
-                        cx[s] = va[3][sf];
-                        pre[s][0] = r_sub(va[0][sf], r_div(va[1][sf], wkv[s][0]));   // D - Pz / rD(k-1)
-                    } else {
-                        const Real c0 = va[0][sf];
-                        cy[s] = va[1][sf];
-                        cx[s] = va[2][sf];
-                        // MODE 0: rk = rD r (premultiplied by the gather, the
-                        // sequential sweep's first product); MODE 1: rk = w
-#pragma unroll
-                        for (int q = 0; q < NC; ++q) pre[s][q] = r_fma(-c0, wkv[s][q], va[3 + q][sf]);
-                    }
-                }
-                // the recurrence (order of operations of the sequential sweep)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int s = 4 * qd + e;
-#pragma unroll
-                    for (int q = 0; q < NC; ++q) {
-                        const Real yup = __shfl_up_sync(0xffffffffu, yprev[q], 1);
-                        const Real yj = (lane > 0) ? yup : wjv[s][q];
+                    for (int s = 0; s < B; ++s) {
+                        if (s % GS == 0) {
+                            if (b0 + s > 0) until_ready(tb + s);
+                            seen = *watch;   // for the next group
+                            if (b0 + s == 0) pre = product_k(0, kPast[0]);
+                        }
+                        const int sf = (MODE == 1) ? P - 1 - b0 - s : b0 + s;
+                        const Real xy = s >= 1 ? jNow[(s - 1) * PITCH] : jPast[0];
+                        const Real xzNext = s + 1 >= 2 ? kNow[(s - 1) * PITCH] : kPast[(s + 1) * PITCH];
                         Real v;
                         if (MODE == 2) {
-                            v = r_sub(pre[s][q], r_div(cy[s], yj));
-                            v = r_sub(v, r_div(cx[s], yprev[q]));
+                            v = r_sub(pre, r_div(va[2][sf], xy));
+                            v = r_sub(v, r_div(va[3][sf], y1));
                         } else if (sizeof(Real) == 4) {
-                            // FP32: the i term first, so only one product waits on the shuffle
-                            v = r_fma(-cx[s], yprev[q], pre[s][q]);
-                            v = r_fma(-cy[s], yj, v);
+                            // FP32: the i term before the j term
+                            v = r_fma(-va[2][sf], y1, pre);
+                            v = r_fma(-va[1][sf], xy, v);
                         } else {
-                            v = r_fma(-cy[s], yj, pre[s][q]);
-                            v = r_fma(-cx[s], yprev[q], v);
+                            v = r_fma(-va[1][sf], xy, pre);
+                            v = r_fma(-va[2][sf], y1, v);
                         }
-                        out[s][q] = v;
-                        yprev[q] = v;
+                        // the next step's k product after this step's (FP64: one
+                        // product at a time; before them it would delay them), in
+                        // the shadow of the result's way through the ring
+                        if (b0 + s + 1 < P) pre = product_k(s + 1, after(xzNext, v, zero));
+                        cur[s * PITCH] = v;
+                        y1 = v;
+                        warp_sync();
+                        if (s % 2 == 1) cnt[C_COMPUTED + w] = tb + s + 1;   // (every lane the same word)
                     }
                 }
-                // publish the quad to the next plane
-                if (kLocalCons || crossProducer) {
-                    u64 wd[QW];
+                if (cnt[C_ABORT]) break;
+                if (++buf == NB) buf = 0;
+            }
+        } else if (role == 1) {
+            // ---- results out -----------------------------------------------------
+            auto first = [&](int tc) { return e0 + (long long)((MODE == 1) ? T - tc - P : tc) * 32; };
+            int cell[MODE == 1 ? P : 2], next[MODE == 1 ? P : 2];
+            auto cells = [&](int at) {   // of the chunk from step at on
+                if (MODE == 1 && at < T) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-#pragma unroll
-                        for (int q = 0; q < NC; ++q)
-                            pack(out[4 * qd + e][q], kLocalCons ? (unsigned)(t0 + 4 * qd + e + 1) : epoch,
-                                 &wd[e * VW + q * W]);
-#pragma unroll
-                    for (int h = 0; h < QW / 2; ++h) {
-                        if (kLocalCons) st2_cluster(consRing + 8u * (kword(t0 + 4 * qd) + 2 * h), wd[2 * h], wd[2 * h + 1]);
-                        else st2_global(xword(bOut, t0 + 4 * qd) + 2 * h, wd[2 * h], wd[2 * h + 1]);
-                    }
+                    for (int s = 0; s < P; s += 2) ld2(g.cellOf + first(at) + s * 32 + lf * 2, next[s], next[s + 1]);
                 }
-            }
-            if (qfail) { fail = 1; break; }
-            // ---- the j-block hand-off words of the whole chunk (the block
-            // above lags by more than a chunk)
-            if (consJ >= 0 && lane == 31) {
-                u64 wd[P * VW];
+            };
+            cells(0);
+            for (int at = 0; at < T; at += P) {
+                if (MODE == 1) {
 #pragma unroll
-                for (int s = 0; s < P; ++s)
+                    for (int s = 0; s < P; ++s) cell[s] = next[s];
+                    cells(at + P);   // before the wait
+                }
+                if (wait_steps<100>(cnt + C_COMPUTED + w, at + P, cnt, maxLocal) < 0) break;
+                const volatile Real *res = ring + (at & (R - 1)) * PITCH + w * 32 + lane;
+                Real out[P];
 #pragma unroll
-                    for (int q = 0; q < NC; ++q) pack(out[s][q], (unsigned)(t0 + s + 1), &wd[s * VW + q * W]);
-                const unsigned base = ringJs + 8u * (unsigned)(((jo * RJ) + (t0 & (RJ - 1))) * VW);
+                for (int s = 0; s < P; ++s) out[s] = res[s * PITCH];
+                __syncwarp();
+                cnt[C_WRITTEN + w] = at + P;   // (read: the ring may take the next steps)
+                if (MODE == 1) {
+                    if (g.w64) {
 #pragma unroll
-                for (int h = 0; h < P * VW / 2; ++h) st2_shared(base + 16u * h, wd[2 * h], wd[2 * h + 1]);
-            }
-            // ---- progress for the producers' back-pressure (after every lane
-            // has consumed its hand-off values of this chunk)
-            __syncwarp();
-            if (lane == 0) {
-                if (kLocalProd) *(volatile int *)(prodBack + jo) = te;
-                if (depJ >= 0) *(volatile int *)(jProg + jo) = te;
-            }
-            // ---- stage chunk c + NB - 1 (always commit a group, possibly empty)
-            if (te + (NB - 2) * P < T) stage_chunk(te + (NB - 2) * P, ((t0 / P) + NB - 1) % NB);
-            cp_async_commit();
-            // ---- this chunk's results: the forward sweeps write whole quads
-            // of the skewed layout, the backward sweep scatters to the cells
-            if (MODE == 1) {
-                if (g.w64) {
+                        for (int s = 0; s < P; ++s)
+                            if (cell[P - 1 - s] >= 0) g.w64[(long long)comp * a.N + cell[P - 1 - s]] = (double)out[s];
+                    } else {
 #pragma unroll
-                    for (int s = 0; s < P; ++s)
-#pragma unroll
-                        for (int q = 0; q < NC; ++q)
-                            if (((mask >> q) & 1u) && cell[P - 1 - s] >= 0)
-                                g.w64[(long long)q * N + cell[P - 1 - s]] = (double)out[s][q];
+                        for (int s = 0; s < P; ++s)
+                            if (cell[P - 1 - s] >= 0) a.w[(long long)comp * a.N + cell[P - 1 - s]] = out[s];
+                    }
                 } else {
+                    Real *dst = ((MODE == 2) ? g.rDraw : g.wS + (long long)comp * g.nSkew) + first(at) + lane * 2;
 #pragma unroll
-                    for (int s = 0; s < P; ++s)
-#pragma unroll
-                        for (int q = 0; q < NC; ++q)
-                            if (((mask >> q) & 1u) && cell[P - 1 - s] >= 0) w[(long long)q * N + cell[P - 1 - s]] = out[s][q];
-                }
-            } else {
-                const long long e = blk0 + (long long)(t0 >> 2) * 128 + lane * 4;
-#pragma unroll
-                for (int q = 0; q < NC; ++q) {
-                    if (MODE == 0 && !((mask >> q) & 1u)) continue;
-                    Real *dst = (MODE == 2) ? g.rDraw + e : g.wS + (long long)q * g.nSkew + e;
-#pragma unroll
-                    for (int qd = 0; qd < PQ; ++qd) {
-                        Real v4[4];
-#pragma unroll
-                        for (int x = 0; x < 4; ++x) v4[x] = out[4 * qd + x][q];
-                        st4(dst + qd * 128, v4);
-                    }
+                    for (int s = 0; s < P; s += 2) st2(dst + s * 32, out[s], out[s + 1]);
                 }
             }
-        }
-        cp_async_wait<0>();
-        // a failed warp lets the producers that wait on its progress go
-        if (fail && lane == 0) {
-            if (kLocalProd) *(volatile int *)(prodBack + jo) = T;
-            if (depJ >= 0) *(volatile int *)(jProg + jo) = T;
+        } else if (role == 4) {
+            // ---- coefficients in: a lane a tile and array ---------------------------
+            const int array = lane % kStaged;
+            const Real *src;
+            if (MODE == 2) {
+                src = array == 0 ? g.D : array == 1 ? g.Pz : array == 2 ? g.Py : g.Px;
+            } else {
+                src = array == 0   ? (MODE == 0 ? g.Az : g.Bz)
+                      : array == 1 ? (MODE == 0 ? g.Ay : g.By)
+                      : array == 2 ? (MODE == 0 ? g.Ax : g.Bx)
+                                   : (MODE == 0 ? g.rS : g.wS) + (long long)comp * g.nSkew;
+            }
+            const unsigned dst = (unsigned)__cvta_generic_to_shared(myStage) + array * P * 32 * (int)sizeof(Real);
+            const bool leads = array == 0;
+            // steps in flight, in order, and told to the recurrence as they arrive
+            int staged = there ? 0 : T, told = staged;
+            long long spins = 0;
+            while (__any_sync(0xffffffffu, told < T)) {
+                // (a buffer is free once its last chunk has been computed)
+                bool go = staged < T && !cnt[C_ABORT] && cnt[C_COMPUTED + w] >= staged - (NB - 1) * P;
+                go = __shfl_sync(0xffffffffu, go, lane & ~(kStaged - 1));
+                const int b = staged / P % NB;
+                if (go && leads) bar_expect(myBars + 8 * b, stage_bytes<Real, P>());
+                __syncwarp();
+                if (go) {
+                    const long long lo = e0 + (long long)((MODE == 1) ? T - staged - P : staged) * 32;
+                    bulk_load(dst + b * stage_bytes<Real, P>(), src + lo, P * 32 * sizeof(Real), myBars + 8 * b);
+                    staged += P;
+                }
+                if (told < staged && bar_test(myBars + 8 * (told / P % NB), (told / P / NB) & 1)) {
+                    told += P;
+                    if (leads) cnt[C_STAGED + w] = told;
+                    spins = 0;
+                }
+                if ((++spins & 63) == 0 && (spins > maxLocal || cnt[C_ABORT])) {
+                    cnt[C_ABORT] = 1;
+                    if (told == staged) told = staged = T;   // given up, with no copy in flight
+                }
+            }
+        } else if (role == 2 || role == 5) {
+            // ---- ghosts: one stream, from the tile before in k (j) to tile w -------
+            auto ghosts = [&](auto nConst, int off, W *src, int ringAt, volatile int *arrived, bool any) {
+                constexpr int n = decltype(nConst)::v;            // words a step
+                constexpr int L = (kWindow * n + 31) / 32;        // and words a lane
+                int pos = any ? off : T;                          // the producer's step
+                if (!any) return;
+                long long spins = 0;
+                while (pos < T) {
+                    // the ring holds the producer's steps before `room`
+                    const int room = min(T, __shfl_sync(0xffffffffu, cnt[C_COMPUTED + w], 0) + R);
+                    W v[L];
+#pragma unroll
+                    for (int i = 0; i < L; ++i) {
+                        const int q = i * 32 + lane, st = pos + q / n;
+                        v[i] = q < kWindow * n && st < room ? ld_word(src + (long long)st * n + q % n) : kNone;
+                    }
+                    // whole steps that have arrived
+                    int k = kWindow * n;
+#pragma unroll
+                    for (int i = L - 1; i >= 0; --i) {
+                        const unsigned no = __ballot_sync(0xffffffffu, v[i] == kNone);
+                        if (no) k = i * 32 + __ffs(no) - 1;
+                    }
+                    k = a.stall ? 0 : min(k, kWindow * n) / n;
+                    if (k == 0) {
+                        if ((++spins & 63) == 0 &&
+                            (spins > a.maxSpin || cnt[C_ABORT] || *(volatile int *)(a.sync + SYNC_ERROR))) {
+                            cnt[C_ABORT] = 1;
+                            break;
+                        }
+                        continue;
+                    }
+                    spins = 0;
+#pragma unroll
+                    for (int i = 0; i < L; ++i) {
+                        const int q = i * 32 + lane, st = pos + q / n;
+                        if (st < pos + k) ring[(st & (R - 1)) * PITCH + ringAt + q % n] = Wd::value(v[i]);
+                    }
+                    __syncwarp();
+                    *arrived = pos + k;
+#pragma unroll
+                    for (int i = 0; i < L; ++i) {
+                        const int q = i * 32 + lane, st = pos + q / n;
+                        if (st < pos + k) st_word(src + (long long)st * n + q % n, kNone);
+                    }
+                    pos += k;
+                }
+            };
+            if (role == 2)
+                ghosts(IntC<TJ>{}, offK, xk + (long long)(here - nTJ) * T * TJ, G::ghostK + wj * TJ, cnt + C_GHOST_K + wj,
+                       K > 0);
+            else
+                ghosts(IntC<TK>{}, offJ, xj + (long long)(here - 1) * T * TK, G::ghostJ + wk * TK, cnt + C_GHOST_J + wk,
+                       J > 0);
+        } else {
+            // ---- one stream of results handed on, from tile w ----------------------
+            auto hand_on = [&](auto nConst, W *dst, int ringAt, int stride, volatile int *handed, bool any) {
+                constexpr int n = decltype(nConst)::v;
+                constexpr int L = (kWindow * n + 31) / 32;
+                if (!any) return;
+                int pos = 0;
+                while (pos < T) {
+                    const int c = wait_steps<20>(cnt + C_COMPUTED + w, pos + 1, cnt, maxLocal);
+                    if (c < 0) break;
+                    const int k = min(c - pos, kWindow);
+#pragma unroll
+                    for (int i = 0; i < L; ++i) {
+                        const int q = i * 32 + lane, st = pos + q / n;
+                        if (st < pos + k) {
+                            const W v = Wd::of(ring[(st & (R - 1)) * PITCH + ringAt + q % n * stride]);
+                            st_word(dst + (long long)st * n + q % n, v == kNone ? Wd::kOtherNaN : v);
+                        }
+                    }
+                    pos += k;
+                    __syncwarp();
+                    *handed = pos;
+                }
+            };
+            if (role == 3)
+                hand_on(IntC<TJ>{}, xk + (long long)here * T * TJ, w * 32 + 32 - TJ, 1, cnt + C_HANDED_K + wj, K + 1 < nTK);
+            else
+                hand_on(IntC<TK>{}, xj + (long long)here * T * TK, w * 32 + TJ - 1, TJ, cnt + C_HANDED_J + wk, J + 1 < nTJ);
         }
     }
-    // no CTA may leave while a neighbour can still access its shared memory
-    cluster.sync();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (cnt[C_ABORT]) atomicExch(a.sync + SYNC_ERROR, 1);
+        // the last CTA to finish re-arms the counters for the next launch
+        const int n = atomicAdd(a.sync + SYNC_DONE, 1);
+        if (n == (int)gridDim.x - 1) {
+            a.sync[SYNC_WORK] = 0;
+            a.sync[SYNC_DONE] = 0;
+        }
+    }
 }
 
 // rS = rD r gathered into the skewed layout (0 outside the mesh): the first
@@ -693,184 +642,88 @@ __global__ void k_skew_to32(SkewView g, SkewView32 h) {
 
 namespace {
 
-template <class Real, int MODE, int NC, int P, int NB = 3>
-void launch_one(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w, int CS, int ncc = 1) {
+// the hand-off words of ncomp components, all ones, kept per precision (the
+// words that no consumer reads keep old values, at the same places in every
+// launch of that precision)
+template <class Real>
+typename Word<Real>::T *hand_off_words(rt_ctx *ctx, long long perComp, int ncomp) {
     StructMesh &s = ctx->mesh.sm;
-    const int R = ring_depth<Real, MODE, NC, P, NB>(g.nJB, g.T, ctx->sweepRing > 0 ? ctx->sweepRing : kMaxRing);
-    const size_t shm = sweep_smem_bytes<Real, MODE, NC, P, NB>(g.nJB, R);
-    static size_t attr = 0;   // per instantiation: dynamic shared memory opted in so far
-    if (shm > attr) {
-        RT_CUDA(cudaFuncSetAttribute(k_systolic<Real, MODE, NC, P, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)shm));
-        RT_CUDA(cudaFuncSetAttribute(k_systolic<Real, MODE, NC, P, NB>, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                     1));
-        attr = shm;
+    DBuf<u64> &buf = s.xfer[sizeof(Real) == 4 ? 1 : 0];
+    const size_t need = ((size_t)perComp * ncomp * sizeof(Real) + 7) / 8;
+    if (buf.n < need) {
+        buf.alloc(need);
+        RT_CUDA(cudaMemsetAsync(buf.p, 0xff, buf.n * 8, ctx->stream));
     }
-    // a cluster of more than 8 CTAs (non-portable) must fit one GPC with this
-    // launch's shared memory; otherwise the portable 8 (checked once per
-    // instantiation and cluster size)
-    static int fits16 = -1;
-    if (CS > 8) {
-        if (fits16 < 0) {
-            cudaLaunchConfig_t q = {};
-            q.gridDim = dim3(CS);
-            q.blockDim = dim3(32 * g.nJB);
-            q.dynamicSmemBytes = shm;
-            cudaLaunchAttribute qa[1];
-            qa[0].id = cudaLaunchAttributeClusterDimension;
-            qa[0].val.clusterDim.x = CS;
-            qa[0].val.clusterDim.y = 1;
-            qa[0].val.clusterDim.z = 1;
-            q.attrs = qa;
-            q.numAttrs = 1;
-            int n = 0;
-            cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_systolic<Real, MODE, NC, P, NB>, &q);
-            if (e != cudaSuccess) (void)cudaGetLastError();
-            fits16 = (e == cudaSuccess && n >= 1) ? 1 : 0;
-        }
-        if (!fits16) CS = 8;
-    }
-    const int nGroups = (g.nz + CS - 1) / CS;
-    // tagged hand-off between clusters: (boundaries) x blocks x steps x lanes x words
-    const size_t words = (size_t)std::max(1, nGroups - 1) * g.nJB * g.T * 32 * NC * Words<Real>::W;
-    if (s.xfer.n < words * ncc) {
-        s.xfer.alloc(words * ncc);
-        s.xfer.zero(ctx->stream);
-    }
-    if (++s.epoch == 0) s.epoch = 1;   // 0 marks a cleared word
-    // failure-detection test (RT_OPT_STALL_TEST): this launch's consumers of
-    // the cluster-to-cluster hand-off wait for a tag that no launch writes
-    // (epochs stay far below 2^31), so their bounded waits run out
-    unsigned cepoch = s.epoch;
-    if (ctx->stallTest > 0) {
-        cepoch = s.epoch ^ 0x80000000u;
-        --ctx->stallTest;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nGroups * CS * ncc);
-    cfg.blockDim = dim3(32 * g.nJB);
-    cfg.dynamicSmemBytes = shm;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CS;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    RT_CUDA(cudaLaunchKernelEx(&cfg, k_systolic<Real, MODE, NC, P, NB>, g, mask, w, ctx->mesh.N, s.sync.p, s.xfer.p,
-                               s.epoch, cepoch, ctx->waitLimit, R, ncc, (long long)words));
+    return reinterpret_cast<typename Word<Real>::T *>(buf.p);
 }
 
-// Schedules of the one-component sweeps (the pressure solve): chunk size P
-// (steps per wait) and staging depth NB (chunks in flight); the autotuner
-// times the candidates that fit on the first application per mesh and
-// precision and keeps the fastest.
+template <class Real, int MODE, int TJ, int WJ, int WK, int P, int NB>
+void launch_one(rt_ctx *ctx, const TileRun<Real> &run) {
+    typedef Group<TJ, WJ, WK> G;
+    constexpr int shm = group_smem<Real, G, P, NB>();
+    static_assert(shm <= 226 * 1024, "one CTA's shared memory");
+    static bool opted = false;   // per instantiation
+    if (!opted) {
+        RT_CUDA(cudaFuncSetAttribute(k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+        opted = true;
+    }
+    const int groups = (run.g.nTJ + WJ - 1) / WJ * ((run.g.nTK + WK - 1) / WK);
+    k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB><<<groups * run.ncc, 32 * G::warps, shm, ctx->stream>>>(run);
+}
+
+// Schedules of the sweeps: chunk size P (steps per staged block), staging depth
+// NB (blocks in flight) and with them the CTA's tiles: chunks of 16 steps leave
+// an FP64 CTA room for two.  RT_OPT_SWEEP_TUNE takes one of them; the default is
+// two tiles and (16, 3), as fewer warps share the SM's issue slots (1M cells,
+// one component: FP64 248 us an application against 260 with four tiles and
+// (8, 5), FP32 133 against 163), but four in FP64 when the groups of two would
+// not all run at once, one an SM (three components: 271 us against 331).
 constexpr int kTuneN = 5;
 constexpr int kTuneP[kTuneN] = {8, 8, 16, 16, 4};
 constexpr int kTuneNB[kTuneN] = {3, 5, 3, 4, 6};
+constexpr int kNarrow = 2, kWide = 1;
 
-template <class Real, int MODE, int K>
-bool tune_fits(int nJB) {
-    return sweep_smem_bytes<Real, MODE, 1, kTuneP[K], kTuneNB[K]>(nJB) <= kMaxSmem;
-}
-template <class Real, int MODE>
-bool tune_fits_any(int k, int nJB) {
+template <class Real, int MODE, int TJ>
+void launch_tuned(rt_ctx *ctx, const TileRun<Real> &run, int k) {
+    constexpr int WJ = TJ == 32 ? 4 : 2, WK = TJ == 32 ? 1 : 2;
+    if (k < 0) {
+        const int two = (run.g.nTJ + 1) / 2 * run.g.nTK * run.ncc;
+        k = sizeof(Real) == 8 && two > ctx->numSMs ? kWide : kNarrow;
+    }
     switch (k) {
-    case 0: return tune_fits<Real, MODE, 0>(nJB);
-    case 1: return tune_fits<Real, MODE, 1>(nJB);
-    case 2: return tune_fits<Real, MODE, 2>(nJB);
-    case 3: return tune_fits<Real, MODE, 3>(nJB);
-    default: return tune_fits<Real, MODE, 4>(nJB);
-    }
-}
-template <class Real, int MODE>
-void launch_tuned(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w, int CS, int k, int ncc = 1) {
-    switch (k) {
-    case 0: launch_one<Real, MODE, 1, kTuneP[0], kTuneNB[0]>(ctx, g, mask, w, CS, ncc); break;
-    case 1: launch_one<Real, MODE, 1, kTuneP[1], kTuneNB[1]>(ctx, g, mask, w, CS, ncc); break;
-    case 2: launch_one<Real, MODE, 1, kTuneP[2], kTuneNB[2]>(ctx, g, mask, w, CS, ncc); break;
-    case 3: launch_one<Real, MODE, 1, kTuneP[3], kTuneNB[3]>(ctx, g, mask, w, CS, ncc); break;
-    default: launch_one<Real, MODE, 1, kTuneP[4], kTuneNB[4]>(ctx, g, mask, w, CS, ncc); break;
+    case 0: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[0], kTuneNB[0]>(ctx, run); break;
+    case 1: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[1], kTuneNB[1]>(ctx, run); break;
+    case 2: launch_one<Real, MODE, TJ, 2, 1, kTuneP[2], kTuneNB[2]>(ctx, run); break;
+    case 3: launch_one<Real, MODE, TJ, 2, 1, kTuneP[3], kTuneNB[3]>(ctx, run); break;
+    default: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[4], kTuneNB[4]>(ctx, run); break;
     }
 }
 
-// the chunk schedule of an NC-component sweep: the tuned one (one
-// component), else chunks of 8 (one component) or 4 steps with three staging
-// buffers, else 4 steps with two; false when none fits
-template <class Real, int MODE, int NC>
-bool launch_fit(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w, int CS, int ncc = 1) {
-    if constexpr (NC == 1 && MODE != 2) {
-        const int k = ctx->mesh.sm.tune[sizeof(Real) == 4 ? 1 : 0];
-        if (k >= 0 && tune_fits_any<Real, MODE>(k, g.nJB)) {
-            launch_tuned<Real, MODE>(ctx, g, mask, w, CS, k, ncc);
-            return true;
-        }
-    }
-    if constexpr (NC == 1) {
-        if (sweep_smem_bytes<Real, MODE, NC, 8>(g.nJB) <= kMaxSmem) {
-            launch_one<Real, MODE, NC, 8>(ctx, g, mask, w, CS, ncc);
-            return true;
-        }
-        if (ncc > 1) return false;
-    }
-    if (sweep_smem_bytes<Real, MODE, NC, 4>(g.nJB) <= kMaxSmem) {
-        launch_one<Real, MODE, NC, 4>(ctx, g, mask, w, CS);
-        return true;
-    }
-    if (sweep_smem_bytes<Real, MODE, NC, 4, 2>(g.nJB) <= kMaxSmem) {
-        launch_one<Real, MODE, NC, 4, 2>(ctx, g, mask, w, CS);
-        return true;
-    }
-    return false;
-}
-
-// the nc components of one sweep, in launches of as many components as fit
-// one CTA's shared memory (six in FP32, three, or one), on shifted views
+// one sweep of the masked components, side by side in one launch
 template <class Real, int MODE>
-void launch_mode(rt_ctx *ctx, const SkewT<Real> &g, int nc, unsigned mask, Real *w) {
+void launch_mode(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w) {
     StructMesh &s = ctx->mesh.sm;
-    const int CS = s.KC;   // planes (CTAs) per cluster
-    // components c0 .. c0 + n - 1 in one launch; false (nothing launched)
-    // when they do not fit
-    auto part = [&](int c0, int n) -> bool {
-        const unsigned mc = (mask >> c0) & ((1u << n) - 1u);
-        if (!mc) return true;
-        SkewT<Real> h = g;
-        h.rS += (size_t)c0 * g.nSkew;
-        h.wS += (size_t)c0 * g.nSkew;
-        if (h.w64) h.w64 += (size_t)c0 * ctx->mesh.N;
-        Real *wc = w ? w + (size_t)c0 * ctx->mesh.N : w;
-        // the group counter restarts; the error flag stays until skew_check reads it
-        RT_CUDA(cudaMemsetAsync(s.sync.p + SYNC_WORK, 0, sizeof(int), ctx->stream));
-        bool ok = false;
-        if (n == 1) {
-            ok = launch_fit<Real, MODE, 1>(ctx, h, mc, wc, CS);
-        } else if (n <= 3 && ctx->sweepComponents == 1) {
-            // the components side by side: one-component sweeps, one launch
-            const int ncc = 32 - __builtin_clz(mc);
-            ok = launch_fit<Real, MODE, 1>(ctx, h, mc, wc, CS, ncc);
-        }
-        if constexpr (MODE != 2) {
-            if (!ok && n == 3) ok = launch_fit<Real, MODE, 3>(ctx, h, mc, wc, CS);
-            else if (!ok && n == 6) {
-                if constexpr (sizeof(Real) == 4) ok = launch_fit<Real, MODE, 6>(ctx, h, mc, wc, CS);
-            }
-        }
-        if (ok) launch_count(ctx, 2);
-        return ok;
-    };
-    auto singles = [&](int c0, int n) -> bool {
-        bool ok = true;
-        for (int c = c0; c < c0 + n && ok; ++c) ok = part(c, 1);
-        return ok;
-    };
-    bool ok;
-    if (MODE == 2 || nc == 1) ok = part(0, 1);
-    else if (nc <= 3) ok = part(0, 3) || singles(0, nc);
-    else ok = part(0, 6) || ((part(0, 3) || singles(0, 3)) && (part(3, 3) || singles(3, nc - 3)));
-    RT_REQUIRE(ok, RT_EINVAL, "the systolic sweep does not fit one CTA's shared memory");
+    if (!mask) return;
+    const int k = ctx->sweepTune - 1;   // -1: the default
+    s.tune[sizeof(Real) == 4 ? 1 : 0] = k >= 0 ? k : kNarrow;
+    TileRun<Real> run;
+    run.g = g;
+    run.mask = mask;
+    run.w = w;
+    run.N = ctx->mesh.N;
+    run.ncc = __builtin_popcount(mask);
+    run.sync = s.sync.p;
+    run.xstride = (long long)s.nTJ * s.nTK * (s.TJ + 32 / s.TJ) * s.T;
+    run.xfer = hand_off_words<Real>(ctx, run.xstride, 32 - __builtin_clz(mask));
+    // a spin is an L2 round trip: 2^24 / 8 of them are about a second
+    run.maxSpin = std::max(64ll, ctx->waitLimit >> 3);
+    run.stall = ctx->stallTest > 0 ? 1 : 0;
+    if (run.stall) --ctx->stallTest;
+    if (s.TJ == 32) launch_tuned<Real, MODE, 32>(ctx, run, k);
+    else launch_tuned<Real, MODE, 8>(ctx, run, k);
     RT_CHECK_LAUNCH();
+    launch_count(ctx);
     s.pendingCheck = true;
 }
 
@@ -883,54 +736,11 @@ void skew_prepare(rt_ctx *ctx, const double *diag, const double *upper, const do
     k_skew_setup<<<nb, RT_BLOCK, 0, ctx->stream>>>(g, s.faceLo.p, ctx->mesh.N, diag, upper, lower);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
-    launch_mode<double, 2>(ctx, g, 1, 1u, (double *)nullptr);
+    launch_mode<double, 2>(ctx, g, 1u, (double *)nullptr);
     k_skew_premul<<<nb, RT_BLOCK, 0, ctx->stream>>>(g, s.faceLo.p, s.faceHi.p, ctx->mesh.N, upper, lower);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
 }
-
-namespace {
-
-// time every fitting schedule of the one-component sweeps on the current
-// right-hand side (two applications each, CUDA events) and keep the fastest
-template <class Real>
-void autotune(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w) {
-    StructMesh &s = ctx->mesh.sm;
-    int &choice = s.tune[sizeof(Real) == 4 ? 1 : 0];
-    if (choice >= 0) return;
-    if (ctx->sweepTune > 0) {   // forced (RT_OPT_SWEEP_TUNE)
-        choice = ctx->sweepTune - 1;
-        return;
-    }
-    cudaEvent_t a, b;
-    RT_CUDA(cudaEventCreate(&a));
-    RT_CUDA(cudaEventCreate(&b));
-    float best = 1e30f;
-    int bestK = 0;
-    for (int k = 0; k < kTuneN; ++k) {
-        if (!tune_fits_any<Real, 0>(k, g.nJB) || !tune_fits_any<Real, 1>(k, g.nJB)) continue;
-        choice = k;
-        for (int rep = 0; rep < 3; ++rep) {
-            if (rep == 1) RT_CUDA(cudaEventRecord(a, ctx->stream));
-            launch_mode<Real, 0>(ctx, g, 1, mask, w);
-            launch_mode<Real, 1>(ctx, g, 1, mask, w);
-        }
-        RT_CUDA(cudaEventRecord(b, ctx->stream));
-        RT_CUDA(cudaEventSynchronize(b));
-        float ms = 0.f;
-        RT_CUDA(cudaEventElapsedTime(&ms, a, b));
-        if (ms < best) {
-            best = ms;
-            bestK = k;
-        }
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    choice = bestK;
-    s.tuneMs[sizeof(Real) == 4 ? 1 : 0] = best / 2;
-}
-
-}  // namespace
 
 void skew_precondition(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w, const unsigned *dmask) {
     SkewView g = ctx->mesh.sm.view();
@@ -938,9 +748,8 @@ void skew_precondition(rt_ctx *ctx, int nc, unsigned mask, const double *r, doub
     k_skew_gather<double, double><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
-    if (nc == 1) autotune<double>(ctx, g, mask, w);
-    launch_mode<double, 0>(ctx, g, nc, mask, w);
-    launch_mode<double, 1>(ctx, g, nc, mask, w);
+    launch_mode<double, 0>(ctx, g, mask, w);
+    launch_mode<double, 1>(ctx, g, mask, w);
 }
 
 // 1/rD of the last skew_prepare, in cell order
@@ -974,9 +783,8 @@ void skew_precondition_T(rt_ctx *ctx, int nc, unsigned mask, const double *r, do
     k_skew_gather<double, double><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
-    if (nc == 1) autotune<double>(ctx, g, mask, w);
-    launch_mode<double, 0>(ctx, g, nc, mask, w);
-    launch_mode<double, 1>(ctx, g, nc, mask, w);
+    launch_mode<double, 0>(ctx, g, mask, w);
+    launch_mode<double, 1>(ctx, g, mask, w);
 }
 
 void skew_prepare32(rt_ctx *ctx, const double *diag, const double *upper, const double *lower) {
@@ -994,14 +802,8 @@ void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, flo
     k_skew_gather<float, float><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
-    if (nc == 1) autotune<float>(ctx, g, mask, w);
-    launch_mode<float, 0>(ctx, g, nc, mask, w);
-    launch_mode<float, 1>(ctx, g, nc, mask, w);
-}
-
-bool skew_fits(int nJB) {
-    return nJB >= 1 && nJB <= 16 && sweep_smem_bytes<double, 2, 1, 4, 2>(nJB) <= kMaxSmem &&
-           sweep_smem_bytes<double, 0, 1, 4, 2>(nJB) <= kMaxSmem && sweep_smem_bytes<double, 1, 1, 4, 2>(nJB) <= kMaxSmem;
+    launch_mode<float, 0>(ctx, g, mask, w);
+    launch_mode<float, 1>(ctx, g, mask, w);
 }
 
 void skew_precondition32d(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w, const unsigned *dmask) {
@@ -1011,9 +813,8 @@ void skew_precondition32d(rt_ctx *ctx, int nc, unsigned mask, const double *r, d
     k_skew_gather<float, double><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
-    if (nc == 1) autotune<float>(ctx, g, mask, (float *)nullptr);
-    launch_mode<float, 0>(ctx, g, nc, mask, (float *)nullptr);
-    launch_mode<float, 1>(ctx, g, nc, mask, (float *)nullptr);
+    launch_mode<float, 0>(ctx, g, mask, (float *)nullptr);
+    launch_mode<float, 1>(ctx, g, mask, (float *)nullptr);
 }
 
 rt_status skew_check(rt_ctx *ctx) {
@@ -1023,7 +824,11 @@ rt_status skew_check(rt_ctx *ctx) {
     RT_CUDA(cudaMemcpyAsync(&err, s.sync.p + SYNC_ERROR, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     RT_CUDA(cudaStreamSynchronize(ctx->stream));
     s.pendingCheck = false;
-    if (err) RT_CUDA(cudaMemsetAsync(s.sync.p + SYNC_ERROR, 0, sizeof(int), ctx->stream));
+    if (err) {   // words were left behind and unread: clear them all
+        RT_CUDA(cudaMemsetAsync(s.sync.p, 0, sizeof(int) * SYNC_WORDS, ctx->stream));
+        for (DBuf<u64> &x : s.xfer)
+            if (x.p) RT_CUDA(cudaMemsetAsync(x.p, 0xff, x.n * 8, ctx->stream));
+    }
     return err ? RT_ETIMEOUT : RT_OK;
 }
 

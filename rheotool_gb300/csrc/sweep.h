@@ -34,8 +34,6 @@ bool mg_available(rt_ctx *ctx);
 void mg_prepare(rt_ctx *ctx, const double *diag, const double *upper, const double *lower, bool sym);
 void mg_apply(rt_ctx *ctx, const double *r, double *w, const unsigned *dm = nullptr);
 void mg_apply32(rt_ctx *ctx, unsigned mask, const float *r, float *w);
-// whether the sweeps of a structured mesh with nJB j-blocks fit one CTA's shared memory
-bool skew_fits(int nJB);
 // RT_ETIMEOUT if a bounded wait of the last sweeps ran out
 rt_status skew_check(rt_ctx *ctx);
 

@@ -12,7 +12,7 @@ import pytest
 
 from rheotool_gb300 import abi
 from rheotool_gb300.case import Fields, SolverControl, cavity_case, channel_case, contraction_case
-from rheotool_gb300.mesh import cavity_mesh, contraction_mesh
+from rheotool_gb300.mesh import cavity_mesh, channel_mesh, contraction_mesh
 
 pytestmark = pytest.mark.gpu
 
@@ -271,6 +271,34 @@ def test_systolic_sweeps_equal_level_sweeps(ctx, mesh_name, solver, pre, asym, n
     diag, upper, lower = laplacian_system(mesh, rng, asym=asym)
     b = rng.normal(size=(nc, mesh.nCells)) * mesh.V
     ctl = SolverControl(solver, pre, 1e-12, 0.0, 0, 500)
+    ctx.upload_mesh(mesh)
+    out = {}
+    try:
+        for mode in (abi.SWEEP_LEVELS, abi.SWEEP_SYSTOLIC):
+            ctx.set_sweep(mode)
+            x = np.zeros((nc, mesh.nCells))
+            perf = ctx.ldu_solve(diag, upper, lower, b, x, ctl)
+            out[mode] = (x, [p.nIterations for p in perf])
+    finally:
+        ctx.set_sweep(abi.SWEEP_AUTO)
+    assert out[abi.SWEEP_LEVELS][1] == out[abi.SWEEP_SYSTOLIC][1]
+    assert np.array_equal(out[abi.SWEEP_LEVELS][0], out[abi.SWEEP_SYSTOLIC][0])
+
+
+@pytest.mark.parametrize("nc", [1, 3, 6])
+@pytest.mark.parametrize("dims", [(3, 1, 1), (5, 8, 4), (7, 9, 5), (19, 16, 8), (12, 17, 9), (33, 15, 3), (2, 40, 13),
+                                  (6, 31, 1), (40, 32, 1), (9, 65, 1), (3, 129, 1)])
+def test_systolic_sweeps_at_tile_edges(ctx, dims, nc):
+    """The structured sweeps on boxes at the edges of their tiles (8 x 4 rows,
+    32 x 1 in one plane) and of the CTAs' groups of tiles, one to six
+    components: the level-scheduled sweeps' bits and iteration counts."""
+    nx, ny, nz = dims
+    mesh = cavity_mesh(nx, ny) if nz == 1 else channel_mesh(nx, ny, nz)
+    assert mesh.shape == dims
+    rng = np.random.default_rng(23)
+    diag, upper, lower = laplacian_system(mesh, rng, asym=1.0)
+    b = rng.normal(size=(nc, mesh.nCells)) * mesh.V
+    ctl = SolverControl("PBiCGStab", "DILU", 1e-12, 0.0, 0, 200)
     ctx.upload_mesh(mesh)
     out = {}
     try:
