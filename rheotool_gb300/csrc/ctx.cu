@@ -340,6 +340,7 @@ rt_status rt_mesh_upload(rt_ctx *ctx, const rt_mesh_desc *md) {
         std::vector<int> lc(N), pos(m.levelStartH.begin(), m.levelStartH.end() - 1);
         for (int c = 0; c < N; ++c) lc[pos[lev[c]]++] = c;
         upload_vec(ctx, lc, m.levelCells);
+        m.lev.ready = false;
         // ---- scratch ---------------------------------------------------------
         size_t need = (size_t)N * 160 + (size_t)F * 24 + (size_t)NB * 96 + 4096;
         ctx->work.a.alloc(need);

@@ -13,8 +13,8 @@
 //     applied as w = rD r, forward w_u -= rD_u a_ul w_l (faces ascending),
 //     backward w_l -= rD_l a_lu w_u (faces descending).
 //
-// The triangular recurrences are exact: cells are processed level by level
-// (level = 1 + max level of the lower neighbours), and inside a cell the
+// The triangular recurrences are exact: cells are processed in tiles along the
+// box (sweep.cu) or level by level (levels.cu), and inside a cell the
 // neighbour contributions are accumulated in face order, which reproduces the
 // sequential sweep's arithmetic.  Reductions are two-stage block trees in a
 // fixed order, so every solve is run-to-run bit-reproducible.
@@ -201,84 +201,9 @@ __global__ void k_dot(int N, unsigned mask, const double *__restrict__ a, const 
     }
 }
 
-// --------------------------------------------------------------------------
-// D-ILU / DIC, level scheduled
-// --------------------------------------------------------------------------
-__global__ void k_rd_level(Ell e, int l0, int l1, const int *__restrict__ cells,
-                           const double *__restrict__ diag, const double *__restrict__ upper,
-                           const double *__restrict__ lower, double *__restrict__ rD) {
-    int t = l0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= l1) return;
-    int c = cells[t];
-    double r = diag[c];
-    for (int s = 0; s < e.nSlots; ++s) {
-        int nb = e.nbr[s * e.N + c];
-        if (nb < 0 || nb > c) break;          // lower neighbours come first
-        int f = e.face[s * e.N + c];
-        r = __dsub_rn(r, __ddiv_rn(__dmul_rn(upper[f], lower[f]), rD[nb]));
-    }
-    rD[c] = r;
-}
-
-__global__ void k_recip(int N, double *rD) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < N) rD[c] = 1.0 / rD[c];
-}
-
 __global__ void k_recip_diag(int N, const double *diag, double *rD) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < N) rD[c] = 1.0 / diag[c];
-}
-
-// (templated on the real type: FP64 for the plain solvers, FP32 inside the
-// mixed-precision ones)
-template <class Real>
-__global__ void k_fwd_level(Ell e, int l0, int l1, const int *__restrict__ cells, unsigned mask,
-                            const Real *__restrict__ rD, const Real *__restrict__ lower,
-                            const Real *__restrict__ r, Real *__restrict__ w) {
-    int t = l0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= l1) return;
-    int c = cells[t];
-    const int N = e.N;
-    const Real rd = rD[c];
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        size_t o = (size_t)k * N;
-        Real acc = r_mul(rd, r[o + c]);
-        for (int s = 0; s < e.nSlots; ++s) {
-            int nb = e.nbr[s * N + c];
-            if (nb < 0 || nb > c) break;
-            int f = e.face[s * N + c];
-            acc = r_fma(-r_mul(rd, lower[f]), w[o + nb], acc);
-        }
-        w[o + c] = acc;
-    }
-}
-
-template <class Real>
-__global__ void k_bwd_level(Ell e, int l0, int l1, const int *__restrict__ cells, unsigned mask,
-                            const Real *__restrict__ rD, const Real *__restrict__ upper,
-                            Real *__restrict__ w) {
-    int t = l0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= l1) return;
-    int c = cells[t];
-    const int N = e.N;
-    const Real rd = rD[c];
-    // number of used slots
-    int ns = 0;
-    while (ns < e.nSlots && e.nbr[ns * N + c] >= 0) ++ns;
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        size_t o = (size_t)k * N;
-        Real acc = w[o + c];
-        for (int s = ns - 1; s >= 0; --s) {
-            int nb = e.nbr[s * N + c];
-            if (nb < c) break;                // upper neighbours are the last slots
-            int f = e.face[s * N + c];
-            acc = r_fma(-r_mul(rd, upper[f]), w[o + nb], acc);
-        }
-        w[o + c] = acc;
-    }
 }
 
 __global__ void k_diag_apply(int N, unsigned mask, const double *__restrict__ rD,
@@ -753,21 +678,21 @@ struct Solver {
         } else if (pre == RT_PRECOND_DIC || pre == RT_PRECOND_DILU) {
             const double fpc = (double)m.F / N;
             ProfScope ps(ctx, "dilu_rD", (double)N * (16.0 + fpc * 28.0));
-            for (int l = 0; l < m.nLevels; ++l) {
-                int l0 = m.levelStartH[l], l1 = m.levelStartH[l + 1];
-                k_rd_level<<<nblocks(l1 - l0), RT_BLOCK, 0, st>>>(pe, l0, l1, m.levelCells.p, a.diag,
-                                                                  a.upper, a.lower, rD);
-            }
-            RT_CHECK_LAUNCH();
-            launch_count(ctx, m.nLevels);
-            k_recip<<<nblocks(N), RT_BLOCK, 0, st>>>(N, rD);
-            RT_CHECK_LAUNCH();
-            launch_count(ctx);
+            level_factor(ctx, a.diag, a.upper, a.lower, rD);
         } else if (pre == RT_PRECOND_DIAGONAL) {
             k_recip_diag<<<nblocks(N), RT_BLOCK, 0, st>>>(N, a.diag, rD);
             RT_CHECK_LAUNCH();
             launch_count(ctx);
         }
+    }
+
+    bool levels() const {
+        const int pre = a.ctl.preconditioner;
+        return !systolic() && (pre == RT_PRECOND_DIC || pre == RT_PRECOND_DILU);
+    }
+    // the level-scheduled sweeps' coefficients from 1 / rD (T: of the transposed factorisation)
+    void sweep_coefs(const double *rD, bool T = false) {
+        if (levels()) level_coefs(ctx, rD, a.lower, a.upper, T);
     }
 
     // w = M^-1 r, or with T the transposed preconditioner M^-T r (the same rD,
@@ -778,7 +703,6 @@ struct Solver {
                       const unsigned *dmask = nullptr) {
         const DevMesh &m = ctx->mesh;
         int pre = a.ctl.preconditioner;
-        const double *lower = T ? a.upper : a.lower, *upper = T ? a.lower : a.upper;
         if (pre == RT_PRECOND_NONE) {
             k_copy<<<nblocks(N), RT_BLOCK, 0, st>>>(N, mask, r, w);
             launch_count(ctx);
@@ -797,17 +721,7 @@ struct Solver {
             // 2*(F/N)*8, addressing 2*(F/N)*8, r 8 + w 8 + w 16 per component
             const double fpc = (double)m.F / N;
             ProfScope ps(ctx, "dilu_precondition", (double)N * (16.0 + fpc * 32.0 + 32.0 * pop(mask)));
-            for (int l = 0; l < m.nLevels; ++l) {
-                int l0 = m.levelStartH[l], l1 = m.levelStartH[l + 1];
-                k_fwd_level<<<nblocks(l1 - l0), RT_BLOCK, 0, st>>>(pe, l0, l1, m.levelCells.p, mask, rD,
-                                                                   lower, r, w);
-            }
-            for (int l = m.nLevels - 1; l >= 0; --l) {
-                int l0 = m.levelStartH[l], l1 = m.levelStartH[l + 1];
-                k_bwd_level<<<nblocks(l1 - l0), RT_BLOCK, 0, st>>>(pe, l0, l1, m.levelCells.p, mask, rD,
-                                                                   upper, w);
-            }
-            launch_count(ctx, 2 * m.nLevels);
+            level_precondition(ctx, mask, r, w, T, dmask);
         }
         RT_CHECK_LAUNCH();
     }
@@ -915,6 +829,7 @@ rt_status run_pcg(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
     Solver sv(ctx, a);
     double *rD = ctx->kws.p + 48 * (size_t)sv.N;
     sv.compute_rd(rD);
+    sv.sweep_coefs(rD);
     sv.prologue(a.validMask, ctx->kws.p, ctx->kws.p + 6 * (size_t)sv.N);
     return pcg_device_loop<false>(ctx, sv, a, perf, [&](unsigned act, const double *r, double *w, const unsigned *dm) {
         sv.precondition(act, rD, r, w, false, dm);
@@ -989,7 +904,9 @@ rt_status run_pbicg(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
            *rD = ws + 48 * (size_t)N;
     const unsigned mask = a.validMask;
     sv.compute_rd(rD);
+    sv.sweep_coefs(rD);
     if (sv.systolic()) skew_prepare_T(ctx, a.upper, a.lower);
+    else sv.sweep_coefs(rD, true);
     sv.prologue(mask, wA, rA);
     sv.amul(mask, a.psi, wT, true);
     k_sub<<<nblocks(N), RT_BLOCK, 0, sv.st>>>(N, mask, a.source, wT, rT);
@@ -1057,6 +974,7 @@ rt_status run_pbicgstab(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
            *zA = ws + 5 * V6, *tA = ws + 6 * V6, *rA0 = ws + 7 * V6, *rD = ws + 8 * V6;
     unsigned mask = a.validMask;
     sv.compute_rd(rD);
+    sv.sweep_coefs(rD);
     sv.prologue(mask, yA, rA);
     RT_CUDA(cudaMemcpyAsync(ctx->red.hostResult, sv.S, sizeof(double) * 3 * 8, cudaMemcpyDeviceToHost, sv.st));
     RT_CUDA(cudaStreamSynchronize(sv.st));
@@ -1608,6 +1526,7 @@ struct Mixed : Solver {
             k_mx_to32<<<nblocks(N), RT_BLOCK, 0, st>>>(N, rD64, rD32);
             RT_CHECK_LAUNCH();
             launch_count(ctx);
+            if (levels()) level_coefs32(ctx, rD32, l32, u32);
         }
     }
 
@@ -1735,17 +1654,7 @@ struct Mixed : Solver {
             skew_precondition32(ctx, a.nc, mask, r, w);
         } else {
             ProfScope ps(ctx, "dilu_precondition32", (double)N * (8.0 + fpc * 24.0 + 16.0 * pop(mask)));
-            for (int l = 0; l < m.nLevels; ++l) {
-                int l0 = m.levelStartH[l], l1 = m.levelStartH[l + 1];
-                k_fwd_level<float><<<nblocks(l1 - l0), RT_BLOCK, 0, st>>>(pe, l0, l1, m.levelCells.p, mask, rD32,
-                                                                          l32, r, w);
-            }
-            for (int l = m.nLevels - 1; l >= 0; --l) {
-                int l0 = m.levelStartH[l], l1 = m.levelStartH[l + 1];
-                k_bwd_level<float><<<nblocks(l1 - l0), RT_BLOCK, 0, st>>>(pe, l0, l1, m.levelCells.p, mask, rD32,
-                                                                          u32, w);
-            }
-            launch_count(ctx, 2 * m.nLevels);
+            level_precondition32(ctx, mask, r, w);
         }
         RT_CHECK_LAUNCH();
     }

@@ -261,6 +261,15 @@ struct Batch {
     std::vector<int> hostSegI;
 };
 
+// the level-scheduled sweeps' positions and coefficients (levels.cu), on first use
+struct LevelMesh {
+    bool ready = false;
+    int width = 0;             // cells of the widest level
+    DBuf<int> maps, start;
+    DBuf<double> coef, coefT, scratch;
+    DBuf<float> coef32;
+};
+
 // ---------------------------------------------------------------------------
 // mesh: LDU addressing + geometry + cell-centric adjacency
 // ---------------------------------------------------------------------------
@@ -314,6 +323,7 @@ struct DevMesh {
     int nLevels = 0;
     std::vector<int> levelStartH;
     DBuf<int> levelCells;
+    LevelMesh lev;
     // host copies needed by the host-side orchestration
     std::vector<int> patchStartH, patchSizeH;
     Batch batch;

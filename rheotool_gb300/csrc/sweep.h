@@ -24,6 +24,14 @@ void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, flo
 // the same with an FP64 right-hand side and result (rounded on the way in and out)
 void skew_precondition32d(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w,
                           const unsigned *dmask = nullptr);
+// levels.cu, any mesh: the factorisation (rD: 1 / rD in cell order), the
+// premultiplied coefficients of its sweeps (T: of the transposed one), and w =
+// M^-1 r (M^-T r) with them
+void level_factor(rt_ctx *ctx, const double *diag, const double *upper, const double *lower, double *rD);
+void level_coefs(rt_ctx *ctx, const double *rD, const double *lower, const double *upper, bool T);
+void level_coefs32(rt_ctx *ctx, const float *rD, const float *lower, const float *upper);
+void level_precondition(rt_ctx *ctx, unsigned mask, const double *r, double *w, bool T, const unsigned *dmask);
+void level_precondition32(rt_ctx *ctx, unsigned mask, const float *r, float *w);
 // mg.cu: the aggregation multigrid V-cycle of the mixed pressure and
 // momentum solves (FP32): the hierarchy of a matrix (sym: a symmetric one,
 // its lower coefficients only), then w = V-cycle(r): mg_apply for the
