@@ -31,7 +31,7 @@ namespace rt {
 // scalar slots (device array ctx->scal, [slot*8 + comp])
 enum {
     S_NF = 0, S_INIT, S_FIN, S_XBAR, S_A, S_B, S_AOLD, S_ALPHA, S_OMEGA,
-    S_R0R, S_R0ROLD, S_SING, S_T1, S_T2, S_RST, S_ITER, S_NSLOT
+    S_R0R, S_R0ROLD, S_SING, S_TRUE, S_RST, S_ITER, S_NSLOT
 };
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -112,6 +112,21 @@ __device__ __forceinline__ double row_mul(const Ell &e, int c, const double *__r
 #pragma unroll
         for (int j = 0; j < kSG; ++j)
             if (nb[j] >= 0) acc += a[j] * xn[j];
+    }
+    return acc;
+}
+
+// y_c = rowsum_c x_c + sum_f a_f (x_nb - x_c)   (differences form, see k_mx_mat32)
+__device__ __forceinline__ float row_mul32(const Ell &e, int c, const float *__restrict__ rowsum,
+                                           const float *__restrict__ upper, const float *__restrict__ lower,
+                                           const float *__restrict__ x) {
+    const float xc = x[c];
+    float acc = rowsum[c] * xc;
+    for (int s = 0; s < e.nSlots; ++s) {
+        int nb = e.nbr[s * e.N + c];
+        if (nb < 0) break;
+        int f = e.face[s * e.N + c];
+        acc = fmaf(nb > c ? upper[f] : lower[f], x[nb] - xc, acc);
     }
     return acc;
 }
@@ -269,31 +284,6 @@ __global__ void k_sc_fin(unsigned mask, const double *res, double *S) {
     int k = threadIdx.x;
     if (k < 6 && ((mask >> k) & 1u)) S[S_FIN * 8 + k] = res[k] / S[S_NF * 8 + k];
 }
-// BiCGStab: rA0rAold = rA0rA; rA0rA = res; singularity tests, beta in S_B
-__global__ void k_sc_bicg_r0r(unsigned mask, int iter, const double *res, double *S) {
-    int k = threadIdx.x;
-    if (k < 6 && ((mask >> k) & 1u)) {
-        double old = S[S_R0R * 8 + k];
-        double r0r = res[k];
-        S[S_R0ROLD * 8 + k] = old;
-        S[S_R0R * 8 + k] = r0r;
-        if (fabs(r0r) < 1e-300) { S[S_SING * 8 + k] = 1.0; return; }
-        if (iter > 0) {
-            double om = S[S_OMEGA * 8 + k];
-            if (fabs(om) < 1e-300) { S[S_SING * 8 + k] = 1.0; return; }
-            S[S_B * 8 + k] = (r0r / old) * (S[S_ALPHA * 8 + k] / om);
-        }
-    }
-}
-__global__ void k_sc_bicg_alpha(unsigned mask, const double *res, double *S) {
-    int k = threadIdx.x;
-    if (k < 6 && ((mask >> k) & 1u)) S[S_ALPHA * 8 + k] = S[S_R0R * 8 + k] / res[k];
-}
-__global__ void k_sc_bicg_omega(unsigned mask, const double *res, double *S) {
-    int k = threadIdx.x;
-    if (k < 6 && ((mask >> k) & 1u)) S[S_OMEGA * 8 + k] = res[6 + k] / res[k];
-}
-
 // --------------------------------------------------------------------------
 // vector update kernels
 // --------------------------------------------------------------------------
@@ -333,67 +323,6 @@ __global__ void k_pcg_update(int N, unsigned mask, const double *__restrict__ S,
         store_partial(partial, nB, 0, k, v);
     }
 }
-// BiCGStab: pA = rA (first) or rA + beta (pA - omega AyA)
-__global__ void k_bicg_p(int N, unsigned mask, int first, const double *__restrict__ S,
-                         const double *__restrict__ rA, const double *__restrict__ AyA,
-                         double *__restrict__ pA) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        if (S[S_SING * 8 + k] != 0.0) continue;
-        size_t i = (size_t)k * N + c;
-        if (first) pA[i] = rA[i];
-        else pA[i] = rA[i] + S[S_B * 8 + k] * (pA[i] - S[S_OMEGA * 8 + k] * AyA[i]);
-    }
-}
-// BiCGStab: sA = rA - alpha AyA; partial |sA|
-__global__ void k_bicg_s(int N, unsigned mask, const double *__restrict__ S,
-                         const double *__restrict__ rA, const double *__restrict__ AyA,
-                         double *__restrict__ sA, double *partial, int nB) {
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        const double alpha = S[S_ALPHA * 8 + k];
-        double v = 0.0;
-        size_t o = (size_t)k * N;
-        #pragma unroll 4
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
-            double s = rA[o + c] - alpha * AyA[o + c];
-            sA[o + c] = s;
-            v += fabs(s);
-        }
-        store_partial(partial, nB, 0, k, v);
-    }
-}
-// psi += alpha yA
-__global__ void k_axpy_alpha(int N, unsigned mask, const double *__restrict__ S,
-                             const double *__restrict__ yA, double *__restrict__ psi) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    for (int k = 0; k < 6; ++k)
-        if ((mask >> k) & 1u) psi[(size_t)k * N + c] += S[S_ALPHA * 8 + k] * yA[(size_t)k * N + c];
-}
-// psi += alpha yA + omega zA; rA = sA - omega tA; partial |rA|
-__global__ void k_bicg_update(int N, unsigned mask, const double *__restrict__ S,
-                              const double *__restrict__ yA, const double *__restrict__ zA,
-                              const double *__restrict__ sA, const double *__restrict__ tA,
-                              double *__restrict__ psi, double *__restrict__ rA, double *partial, int nB) {
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        const double alpha = S[S_ALPHA * 8 + k], omega = S[S_OMEGA * 8 + k];
-        double v = 0.0;
-        size_t o = (size_t)k * N;
-        #pragma unroll 4
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
-            psi[o + c] += alpha * yA[o + c] + omega * zA[o + c];
-            double r = sA[o + c] - omega * tA[o + c];
-            rA[o + c] = r;
-            v += fabs(r);
-        }
-        store_partial(partial, nB, 0, k, v);
-    }
-}
-
 // --------------------------------------------------------------------------
 // host orchestration
 // --------------------------------------------------------------------------
@@ -405,7 +334,7 @@ void reduce_init(rt_ctx *ctx) {
     RT_CUDA(cudaMallocHost(&r.hostResult, sizeof(double) * 32 * 8));   // one copy of ctx->scal
     ctx->scal.alloc(32 * 8);
     ctx->scal.zero(ctx->stream);
-    r.active.alloc(1);
+    r.active.alloc(4);
     r.active.zero(ctx->stream);
     r.counter.alloc(1);
     r.counter.zero(ctx->stream);
@@ -609,6 +538,338 @@ __global__ void k_pcg_arm(unsigned act, unsigned *active, double *S) {
     if (k == 0) *active = act;
 }
 
+// ==========================================================================
+// PBiCGStab stopping on the device, in FP64 (V = double) and for the mixed form
+// (V = float: FP32 vectors and matrix copy, FP64 scalars and accumulations).  One
+// iteration is, beside the two preconditioner applications, k_bicg_p (p), k_bicg_Ay
+// (A y, r0.Ay: alpha), k_bicg_s (s = r - alpha Ay, |s|: the half-step test), k_bicg_t
+// (t = A z, t.t, t.s: omega) and k_bicg_update (psi, r, |r|, and r0.r of the next
+// iteration: the test, beta and the singularity tests); in the mixed form also
+// k_mx_fold and k_mx_true for the components whose residual is replaced.  As in
+// the PCG loop the last block of each reduction does the scalar work, in the order
+// of operations of k_finalize, and the host follows a few kernels behind through
+// the mapped flag: an iteration had 24 launches and two host synchronisations.
+// The masks of an iteration are device words (red.active): [0] the components at
+// its start, [1] those that go on after the half step, [2] those that met the
+// tolerance there, [3] (mixed) those whose residual is replaced.
+// ==========================================================================
+enum { M_ACTIVE = 0, M_CONT, M_HALF, M_REPL, M_COUNT };
+
+struct LoopCtl {
+    rt_solver_ctl ctl;
+    unsigned *m;        // the masks
+    int *hostFlag;
+    int iter;           // iterations before this one
+};
+
+__device__ __forceinline__ bool converged(const rt_solver_ctl &c, double fin, double init) {
+    return fin < c.tolerance || (c.relTol > 1e-20 && fin < c.relTol * init);
+}
+
+// one thread, component k, with r0.r of the iteration about to start (its number
+// is iter): rA0rAold, rA0rA, beta; false: singular, the component stops
+__device__ bool bicg_rho(double *S, int k, int iter, double r0r) {
+    const double old = S[S_R0R * 8 + k];
+    S[S_R0ROLD * 8 + k] = old;
+    S[S_R0R * 8 + k] = r0r;
+    if (fabs(r0r) < 1e-300) { S[S_SING * 8 + k] = 1.0; return false; }
+    if (iter > 0) {
+        const double om = S[S_OMEGA * 8 + k];
+        if (fabs(om) < 1e-300) { S[S_SING * 8 + k] = 1.0; return false; }
+        S[S_B * 8 + k] = (r0r / old) * (S[S_ALPHA * 8 + k] / om);
+    }
+    return true;
+}
+
+// r0.r before the first iteration
+template <class V>
+__global__ void k_bicg_first(int N, LoopCtl L, const V *__restrict__ r0, const V *__restrict__ r, double *S,
+                             double *partial, int nB, unsigned *counter) {
+    const unsigned mask = L.m[M_ACTIVE];
+    if (!mask) return;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        double v0 = 0.0;
+        size_t o = (size_t)k * N;
+        #pragma unroll 4
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x)
+            v0 += (double)r0[o + c] * (double)r[o + c];
+        store_partial(partial, nB, 0, k, v0);
+    }
+    if (!last_block(counter)) return;
+    unsigned next = mask;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double r0r = partials_sum(partial, nB, 0, k);
+        if (threadIdx.x == 0 && !bicg_rho(S, k, 0, r0r)) next &= ~(1u << k);
+    }
+    if (threadIdx.x == 0) {
+        L.m[M_ACTIVE] = next;
+        if (!next) {
+            L.m[M_CONT] = 0u;
+            *(volatile int *)L.hostFlag = 0;
+            __threadfence_system();
+        }
+    }
+}
+
+// pA = rA (first, or a restart in the mixed form) or rA + beta (pA - omega AyA)
+__global__ void k_bicg_p(int N, LoopCtl L, const double *__restrict__ S, const double *__restrict__ rA,
+                         const double *__restrict__ AyA, double *__restrict__ pA) {
+    const unsigned mask = L.m[M_ACTIVE];
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= N) return;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        size_t i = (size_t)k * N + c;
+        if (L.iter == 0) pA[i] = rA[i];
+        else pA[i] = rA[i] + S[S_B * 8 + k] * (pA[i] - S[S_OMEGA * 8 + k] * AyA[i]);
+    }
+}
+__global__ void k_bicg_p(int N, LoopCtl L, const double *__restrict__ S, const float *__restrict__ r,
+                         const float *__restrict__ Ay, float *__restrict__ p) {
+    const unsigned mask = L.m[M_ACTIVE];
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= N) return;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        size_t i = (size_t)k * N + c;
+        if (L.iter == 0 || S[S_RST * 8 + k] != 0.0) p[i] = r[i];
+        else {
+            const float beta = (float)S[S_B * 8 + k], omega = (float)S[S_OMEGA * 8 + k];
+            p[i] = fmaf(beta, fmaf(-omega, Ay[i], p[i]), r[i]);
+        }
+    }
+}
+
+// the rows c of A x for the components in mask (the coefficients and indices read
+// once for them all), as row_mul (FP64) or in the differences form (FP32, see
+// k_mx_mat32); f(k, value)
+template <class F>
+__device__ __forceinline__ void rows(const Ell &e, int c, unsigned mask, const double *__restrict__ diag,
+                                     const double *__restrict__ upper, const double *__restrict__ lower,
+                                     const double *__restrict__ x, F &&f) {
+    const double d = diag[c];
+    if (e.nSlots <= kSG) {
+        int nb[kSG], fc[kSG];
+        slot_group(e, c, 0, nb, fc);
+        double a[kSG];
+#pragma unroll
+        for (int j = 0; j < kSG; ++j) a[j] = nb[j] >= 0 ? (nb[j] > c ? upper[fc[j]] : lower[fc[j]]) : 0.0;
+        for (int k = 0; k < 6; ++k) {
+            if (!((mask >> k) & 1u)) continue;
+            const double *xk = x + (size_t)k * e.N;
+            double acc = d * xk[c], xn[kSG];
+#pragma unroll
+            for (int j = 0; j < kSG; ++j) xn[j] = nb[j] >= 0 ? xk[nb[j]] : 0.0;
+#pragma unroll
+            for (int j = 0; j < kSG; ++j)
+                if (nb[j] >= 0) acc += a[j] * xn[j];
+            f(k, acc);
+        }
+        return;
+    }
+    for (int k = 0; k < 6; ++k)
+        if ((mask >> k) & 1u) f(k, row_mul(e, c, diag, upper, lower, x + (size_t)k * e.N));
+}
+template <class F>
+__device__ __forceinline__ void rows(const Ell &e, int c, unsigned mask, const float *__restrict__ rowsum,
+                                     const float *__restrict__ upper, const float *__restrict__ lower,
+                                     const float *__restrict__ x, F &&f) {
+    const float d = rowsum[c];
+    if (e.nSlots <= kSG) {
+        int nb[kSG], fc[kSG];
+        slot_group(e, c, 0, nb, fc);
+        float a[kSG];
+#pragma unroll
+        for (int j = 0; j < kSG; ++j) a[j] = nb[j] >= 0 ? (nb[j] > c ? upper[fc[j]] : lower[fc[j]]) : 0.0f;
+        for (int k = 0; k < 6; ++k) {
+            if (!((mask >> k) & 1u)) continue;
+            const float *xk = x + (size_t)k * e.N;
+            const float xc = xk[c];
+            float acc = d * xc, xn[kSG];
+#pragma unroll
+            for (int j = 0; j < kSG; ++j) xn[j] = nb[j] >= 0 ? xk[nb[j]] : 0.0f;
+#pragma unroll
+            for (int j = 0; j < kSG; ++j)
+                if (nb[j] >= 0) acc = fmaf(a[j], xn[j] - xc, acc);
+            f(k, acc);
+        }
+        return;
+    }
+    for (int k = 0; k < 6; ++k)
+        if ((mask >> k) & 1u) f(k, row_mul32(e, c, rowsum, upper, lower, x + (size_t)k * e.N));
+}
+
+// AyA = A yA; r0.AyA; the last block: alpha (and a pending restart is consumed)
+template <class V>
+__global__ void k_bicg_Ay(Ell e, LoopCtl L, const V *__restrict__ diag, const V *__restrict__ upper,
+                          const V *__restrict__ lower, const V *__restrict__ y, const V *__restrict__ r0,
+                          V *__restrict__ Ay, double *S, double *partial, int nB, unsigned *counter) {
+    const unsigned mask = L.m[M_ACTIVE];
+    if (!mask) return;
+    const int N = e.N;
+    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x)
+        rows(e, c, mask, diag, upper, lower, y, [&](int k, V a) {
+            const size_t i = (size_t)k * N + c;
+            Ay[i] = a;
+#pragma unroll
+            for (int q = 0; q < 6; ++q)   // (v in registers: no dynamic index)
+                if (q == k) v[q] = fma((double)r0[i], (double)a, v[q]);
+        });
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        if ((mask >> k) & 1u) store_partial(partial, nB, 0, k, v[k]);
+    if (!last_block(counter)) return;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double r0Ay = partials_sum(partial, nB, 0, k);
+        if (threadIdx.x == 0) {
+            S[S_ALPHA * 8 + k] = S[S_R0R * 8 + k] / r0Ay;
+            S[S_RST * 8 + k] = 0.0;
+        }
+    }
+}
+
+// s = r - alpha Ay and |s| of one element, in the vector's type
+__device__ __forceinline__ double bicg_s(double r, double alpha, double Ay) { return r - alpha * Ay; }
+__device__ __forceinline__ float bicg_s(float r, double alpha, float Ay) { return fmaf(-(float)alpha, Ay, r); }
+
+// sA = rA - alpha AyA; |sA|; the last block: the half-step test
+template <class V>
+__global__ void k_bicg_s(int N, LoopCtl L, const V *__restrict__ r, const V *__restrict__ Ay, V *__restrict__ s,
+                         double *S, double *partial, int nB, unsigned *counter) {
+    const unsigned mask = L.m[M_ACTIVE];
+    if (!mask) return;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double alpha = S[S_ALPHA * 8 + k];
+        double v = 0.0;
+        size_t o = (size_t)k * N;
+        #pragma unroll 4
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+            const V sv = bicg_s(r[o + c], alpha, Ay[o + c]);
+            s[o + c] = sv;
+            v += fabs((double)sv);
+        }
+        store_partial(partial, nB, 0, k, v);
+    }
+    if (!last_block(counter)) return;
+    unsigned half = 0, cont = 0;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double res = partials_sum(partial, nB, 0, k);
+        if (threadIdx.x == 0) {
+            const double fin = res / S[S_NF * 8 + k];
+            const bool conv = converged(L.ctl, fin, S[S_INIT * 8 + k]);
+            if (conv) half |= 1u << k;
+            // (FP64: a residual that is no number stops the component; the mixed
+            // form goes on to its FP64 residual)
+            else if (sizeof(V) == 4 || isfinite(fin)) cont |= 1u << k;
+            if (sizeof(V) == 8) {
+                S[S_FIN * 8 + k] = fin;
+                if (!((cont >> k) & 1u)) S[S_ITER * 8 + k] = L.iter + 1;
+            }
+        }
+    }
+    if (threadIdx.x == 0) {
+        L.m[M_HALF] = half;
+        L.m[M_CONT] = cont;
+    }
+}
+
+// tA = A zA; t.t (slot 0), t.s (slot 1); the last block: omega
+template <class V>
+__global__ void k_bicg_t(Ell e, LoopCtl L, const V *__restrict__ diag, const V *__restrict__ upper,
+                         const V *__restrict__ lower, const V *__restrict__ z, const V *__restrict__ s,
+                         V *__restrict__ t, double *S, double *partial, int nB, unsigned *counter) {
+    if (!L.m[M_ACTIVE]) return;
+    const unsigned mask = L.m[M_CONT];
+    if (!mask) return;
+    const int N = e.N;
+    double v0[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, v1[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x)
+        rows(e, c, mask, diag, upper, lower, z, [&](int k, V a) {
+            const size_t i = (size_t)k * N + c;
+            t[i] = a;
+            const double d = (double)a, sv = (double)s[i];
+#pragma unroll
+            for (int q = 0; q < 6; ++q)
+                if (q == k) {
+                    v0[q] = fma(d, d, v0[q]);
+                    v1[q] = fma(d, sv, v1[q]);
+                }
+        });
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        if ((mask >> k) & 1u) {
+            store_partial(partial, nB, 0, k, v0[k]);
+            store_partial(partial, nB, 1, k, v1[k]);
+        }
+    if (!last_block(counter)) return;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double tt = partials_sum(partial, nB, 0, k), ts = partials_sum(partial, nB, 1, k);
+        if (threadIdx.x == 0) S[S_OMEGA * 8 + k] = ts / tt;
+    }
+}
+
+// the components that end this iteration at their tolerance: psi += alpha yA;
+// the others: psi += alpha yA + omega zA, rA = sA - omega tA, |rA| (slot 0) and
+// r0.rA (slot 1); the last block: lduMatrix's stopping rules, and beta
+__global__ void k_bicg_update(int N, LoopCtl L, const double *__restrict__ yA, const double *__restrict__ zA,
+                              const double *__restrict__ sA, const double *__restrict__ tA,
+                              const double *__restrict__ r0, double *__restrict__ psi, double *__restrict__ rA, double *S,
+                              double *partial, int nB, unsigned *counter) {
+    if (!L.m[M_ACTIVE]) return;
+    const unsigned mask = L.m[M_CONT], half = L.m[M_HALF];
+    for (int k = 0; k < 6; ++k) {
+        size_t o = (size_t)k * N;
+        const double alpha = S[S_ALPHA * 8 + k];
+        if ((half >> k) & 1u) {
+            for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x)
+                psi[o + c] += alpha * yA[o + c];
+            continue;
+        }
+        if (!((mask >> k) & 1u)) continue;
+        const double omega = S[S_OMEGA * 8 + k];
+        double v = 0.0, v1 = 0.0;
+        #pragma unroll 4
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+            psi[o + c] += alpha * yA[o + c] + omega * zA[o + c];
+            double r = sA[o + c] - omega * tA[o + c];
+            rA[o + c] = r;
+            v += fabs(r);
+            v1 = fma(r0[o + c], r, v1);
+        }
+        store_partial(partial, nB, 0, k, v);
+        store_partial(partial, nB, 1, k, v1);
+    }
+    if (!last_block(counter)) return;
+    unsigned next = 0;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double res = partials_sum(partial, nB, 0, k), r0r = partials_sum(partial, nB, 1, k);
+        if (threadIdx.x == 0) {
+            const double fin = res / S[S_NF * 8 + k];
+            const int it = L.iter + 1;
+            S[S_FIN * 8 + k] = fin;
+            S[S_ITER * 8 + k] = it;
+            const bool more = (it < L.ctl.maxIter && !converged(L.ctl, fin, S[S_INIT * 8 + k])) || it < L.ctl.minIter;
+            if (more && isfinite(fin) && bicg_rho(S, k, it, r0r)) next |= 1u << k;
+        }
+    }
+    if (threadIdx.x == 0) {
+        L.m[M_ACTIVE] = next;
+        if (!next) {
+            L.m[M_CONT] = 0u;
+            *(volatile int *)L.hostFlag = 0;
+            __threadfence_system();
+        }
+    }
+}
+
 namespace {
 
 struct Solver {
@@ -628,7 +889,9 @@ struct Solver {
         pe = m.hasCoupled ? Ell{m.N, m.pnSlots, m.pellFace.p, m.pellNbr.p} : e;
         st = ctx->stream;
         S = ctx->scal.p;
-        nB = ctx->red.nBlocks;
+        // the reductions' blocks: four an SM, or as many as have cells (the other
+        // blocks' partial sums are zeros)
+        nB = std::min(ctx->red.nBlocks, nblocks(N));
     }
 
     // finalize nSlots reduction slots of the masked comps into red.result
@@ -965,9 +1228,50 @@ rt_status run_pbicg(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
     return RT_OK;
 }
 
+// the loop's masks, zero iterations
+__global__ void k_bicg_arm(unsigned act, unsigned *m, double *S) {
+    const int k = threadIdx.x;
+    if (k < 6) {
+        S[S_ITER * 8 + k] = 0.0;
+        S[S_SING * 8 + k] = 0.0;
+        S[S_TRUE * 8 + k] = S[S_FIN * 8 + k];   // (mixed: the residual at the last replacement)
+    }
+    if (k < M_COUNT) m[k] = k == M_ACTIVE ? act : 0u;
+}
+
+// runs `iteration(LoopCtl)` until no component is left: the host launches
+// iterations ahead, at most two, and reads the mapped flag
+template <class It>
+void bicg_loop(rt_ctx *ctx, Solver &sv, const SolveArgs &a, It &&iteration) {
+    Reduce &red = ctx->red;
+    const int maxIt = std::max(a.ctl.maxIter, a.ctl.minIter);
+    for (int it = 0; it < maxIt; ++it) {
+        iteration(LoopCtl{a.ctl, red.active.p, red.devFlag, it});
+        RT_CUDA(cudaEventRecord(red.poll[it & 1], sv.st));
+        if (it > 0) {
+            RT_CUDA(cudaEventSynchronize(red.poll[(it - 1) & 1]));
+            if (red.hostFlag[0] == 0) break;
+        }
+    }
+}
+
+// the records of the components that iterated, from the device scalars
+void bicg_records(rt_ctx *ctx, Solver &sv, unsigned act, rt_solver_perf *perf) {
+    Reduce &red = ctx->red;
+    RT_CUDA(cudaMemcpyAsync(red.hostResult, sv.S, sizeof(double) * (S_ITER + 1) * 8, cudaMemcpyDeviceToHost, sv.st));
+    RT_CUDA(cudaStreamSynchronize(sv.st));
+    const double *H = red.hostResult;
+    for (int k = 0; k < 6; ++k) {
+        if (!((act >> k) & 1u)) continue;
+        perf[k].finalResidual = H[S_FIN * 8 + k];
+        perf[k].nIterations = (int)H[S_ITER * 8 + k];
+        perf[k].singular = H[S_SING * 8 + k] != 0.0 ? 1 : 0;
+    }
+}
+
 rt_status run_pbicgstab(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
     Solver sv(ctx, a);
-    const int N = sv.N;
+    const int N = sv.N, nB = sv.nB;
     const size_t V6 = 6 * (size_t)N;
     double *ws = ctx->kws.p;
     double *yA = ws, *rA = ws + V6, *pA = ws + 2 * V6, *AyA = ws + 3 * V6, *sA = ws + 4 * V6,
@@ -985,81 +1289,42 @@ rt_status run_pbicgstab(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
         perf[k].nIterations = 0;
         perf[k].singular = 0;
     }
-    unsigned active = 0;
+    unsigned act = 0;
     for (int k = 0; k < 6; ++k)
         if (((mask >> k) & 1u) && (a.ctl.minIter > 0 || !sv.conv(perf[k].finalResidual, perf[k].initialResidual)))
-            active |= 1u << k;
-    if (!active) return RT_OK;
+            act |= 1u << k;
+    if (!act) return RT_OK;
+    Reduce &red = ctx->red;
     RT_CUDA(cudaMemcpyAsync(rA0, rA, sizeof(double) * V6, cudaMemcpyDeviceToDevice, sv.st));
-    int iter = 0;
-    while (active) {
-        sv.dot(active, rA0, rA);
-        k_sc_bicg_r0r<<<1, 32, 0, sv.st>>>(active, iter, ctx->red.result.p, sv.S);
-        k_bicg_p<<<nblocks(N), RT_BLOCK, 0, sv.st>>>(N, active, iter == 0, sv.S, rA, AyA, pA);
-        sv.precondition(active, rD, pA, yA);
-        sv.amul(active, yA, AyA);
-        sv.dot(active, rA0, AyA);
-        k_sc_bicg_alpha<<<1, 32, 0, sv.st>>>(active, ctx->red.result.p, sv.S);
-        k_bicg_s<<<sv.nB, RT_BLOCK, 0, sv.st>>>(N, active, sv.S, rA, AyA, sA, ctx->red.partial.p, sv.nB);
-        RT_CHECK_LAUNCH();
-        sv.finalize(1, active);
-        k_sc_fin<<<1, 32, 0, sv.st>>>(active, ctx->red.result.p, sv.S);
+    red.hostFlag[0] = 1;
+    k_bicg_arm<<<1, 32, 0, sv.st>>>(act, red.active.p, sv.S);
+    k_bicg_first<double><<<nB, RT_BLOCK, 0, sv.st>>>(N, LoopCtl{a.ctl, red.active.p, red.devFlag, 0}, rA0, rA, sv.S,
+                                                    red.partial.p, nB, red.counter.p);
+    RT_CHECK_LAUNCH();
+    launch_count(ctx, 2);
+    const double fpc = (double)ctx->mesh.F / N, nc = sv.pop(act);
+    const double amulBytes = (double)N * (8.0 + fpc * 24.0 + 24.0 * nc);
+    bicg_loop(ctx, sv, a, [&](const LoopCtl &L) {
+        k_bicg_p<<<nblocks(N), RT_BLOCK, 0, sv.st>>>(N, L, sv.S, rA, AyA, pA);
+        sv.precondition(act, rD, pA, yA, false, L.m + M_ACTIVE);
+        {
+            ProfScope ps(ctx, "amul", amulBytes);
+            k_bicg_Ay<double><<<nB, RT_BLOCK, 0, sv.st>>>(sv.e, L, a.diag, a.upper, a.lower, yA, rA0, AyA, sv.S,
+                                                         red.partial.p, nB, red.counter.p);
+        }
+        k_bicg_s<double><<<nB, RT_BLOCK, 0, sv.st>>>(N, L, rA, AyA, sA, sv.S, red.partial.p, nB, red.counter.p);
+        sv.precondition(act, rD, sA, zA, false, L.m + M_CONT);
+        {
+            ProfScope ps(ctx, "amul", amulBytes);
+            k_bicg_t<double><<<nB, RT_BLOCK, 0, sv.st>>>(sv.e, L, a.diag, a.upper, a.lower, zA, sA, tA, sv.S,
+                                                        red.partial.p, nB, red.counter.p);
+        }
+        k_bicg_update<<<nB, RT_BLOCK, 0, sv.st>>>(N, L, yA, zA, sA, tA, rA0, a.psi, rA, sv.S, red.partial.p, nB,
+                                                  red.counter.p);
         RT_CHECK_LAUNCH();
         launch_count(ctx, 5);
-        RT_CUDA(cudaMemcpyAsync(ctx->red.hostResult, sv.S, sizeof(double) * (S_SING + 1) * 8,
-                                cudaMemcpyDeviceToHost, sv.st));
-        RT_CUDA(cudaStreamSynchronize(sv.st));
-        double H[(S_SING + 1) * 8];
-        memcpy(H, ctx->red.hostResult, sizeof H);
-        unsigned finish = 0, cont = 0;
-        for (int k = 0; k < 6; ++k) {
-            if (!((active >> k) & 1u)) continue;
-            if (H[S_SING * 8 + k] != 0.0) {
-                perf[k].singular = 1;
-                continue;     // stops without an update
-            }
-            perf[k].finalResidual = H[S_FIN * 8 + k];
-            if (sv.conv(perf[k].finalResidual, perf[k].initialResidual)) {
-                finish |= 1u << k;
-                perf[k].nIterations = iter + 1;
-            } else if (!std::isfinite(perf[k].finalResidual)) {
-                perf[k].nIterations = iter + 1;   // stops (RT_ENAN follows)
-            } else {
-                cont |= 1u << k;
-            }
-        }
-        if (finish) {
-            k_axpy_alpha<<<nblocks(N), RT_BLOCK, 0, sv.st>>>(N, finish, sv.S, yA, a.psi);
-            RT_CHECK_LAUNCH();
-            launch_count(ctx);
-        }
-        active = cont;
-        if (!active) break;
-        sv.precondition(active, rD, sA, zA);
-        sv.amul(active, zA, tA);
-        sv.dot(active, tA, tA, tA, sA);
-        k_sc_bicg_omega<<<1, 32, 0, sv.st>>>(active, ctx->red.result.p, sv.S);
-        k_bicg_update<<<sv.nB, RT_BLOCK, 0, sv.st>>>(N, active, sv.S, yA, zA, sA, tA, a.psi, rA,
-                                                     ctx->red.partial.p, sv.nB);
-        RT_CHECK_LAUNCH();
-        sv.finalize(1, active);
-        k_sc_fin<<<1, 32, 0, sv.st>>>(active, ctx->red.result.p, sv.S);
-        RT_CHECK_LAUNCH();
-        launch_count(ctx, 3);
-        RT_CUDA(cudaMemcpyAsync(ctx->red.hostResult, sv.S, sizeof(double) * (S_SING + 1) * 8,
-                                cudaMemcpyDeviceToHost, sv.st));
-        RT_CUDA(cudaStreamSynchronize(sv.st));
-        const double *H2 = ctx->red.hostResult;
-        ++iter;
-        for (int k = 0; k < 6; ++k) {
-            if (!((active >> k) & 1u)) continue;
-            perf[k].finalResidual = H2[S_FIN * 8 + k];
-            perf[k].nIterations = iter;
-            bool more = (iter < a.ctl.maxIter && !sv.conv(perf[k].finalResidual, perf[k].initialResidual)) ||
-                        iter < a.ctl.minIter;
-            if (!more || !std::isfinite(perf[k].finalResidual)) active &= ~(1u << k);
-        }
-    }
+    });
+    bicg_records(ctx, sv, act, perf);
     return RT_OK;
 }
 
@@ -1117,47 +1382,6 @@ __global__ void k_mx_start(int N, unsigned mask, const double *__restrict__ rA, 
     }
 }
 
-// y_c = rowsum_c x_c + sum_f a_f (x_nb - x_c)   (differences form, see k_mx_mat32)
-__device__ __forceinline__ float row_mul32(const Ell &e, int c, const float *__restrict__ rowsum,
-                                           const float *__restrict__ upper, const float *__restrict__ lower,
-                                           const float *__restrict__ x) {
-    const float xc = x[c];
-    float acc = rowsum[c] * xc;
-    for (int s = 0; s < e.nSlots; ++s) {
-        int nb = e.nbr[s * e.N + c];
-        if (nb < 0) break;
-        int f = e.face[s * e.N + c];
-        acc = fmaf(nb > c ? upper[f] : lower[f], x[nb] - xc, acc);
-    }
-    return acc;
-}
-
-__global__ void k_mx_amul(Ell e, unsigned mask, const float *__restrict__ diag, const float *__restrict__ upper,
-                          const float *__restrict__ lower, const float *__restrict__ x, float *__restrict__ y) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= e.N) return;
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        y[(size_t)k * e.N + c] = row_mul32(e, c, diag, upper, lower, x + (size_t)k * e.N);
-    }
-}
-
-// dot products of FP32 vectors accumulated in FP64: slot0 = a.b, slot1 = c.d
-__global__ void k_mx_dot(int N, unsigned mask, const float *__restrict__ a, const float *__restrict__ b,
-                         const float *__restrict__ c2, const float *__restrict__ d2, double *partial, int nB) {
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        double v0 = 0.0, v1 = 0.0;
-        size_t o = (size_t)k * N;
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
-            v0 += (double)a[o + c] * (double)b[o + c];
-            if (c2) v1 += (double)c2[o + c] * (double)d2[o + c];
-        }
-        store_partial(partial, nB, 0, k, v0);
-        if (c2) store_partial(partial, nB, 1, k, v1);
-    }
-}
-
 __global__ void k_mx_copy(int N, unsigned mask, const float *__restrict__ r, float *__restrict__ w) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
@@ -1171,32 +1395,6 @@ __global__ void k_mx_diag_apply(int N, unsigned mask, const float *__restrict__ 
     if (c >= N) return;
     for (int k = 0; k < 6; ++k)
         if ((mask >> k) & 1u) w[(size_t)k * N + c] = rD[c] * r[(size_t)k * N + c];
-}
-
-// flexible PCG scalars: wArAold = wArA; wArA = w.r; beta = w.(r - r_old) /
-// wArAold = -alpha_old w.q_old / wArAold, since r - r_old = -alpha_old q_old
-// (Polak-Ribiere form; equal to wArA / wArAold in exact arithmetic, robust to
-// the FP32 preconditioner, which is not exactly the same operator twice)
-__global__ void k_mx_sc_pcg_a(unsigned mask, int first, const double *res, double *S) {
-    int k = threadIdx.x;
-    if (k < 6 && ((mask >> k) & 1u)) {
-        const double aold = S[S_A * 8 + k];
-        S[S_AOLD * 8 + k] = aold;
-        S[S_A * 8 + k] = res[k];
-        if (!first) S[S_B * 8 + k] = -S[S_ALPHA * 8 + k] * res[6 + k] / aold;
-    }
-}
-
-// flexible PCG: p = z (+ beta p), beta from k_mx_sc_pcg_a
-__global__ void k_pcg_p_flex(int N, unsigned mask, int first, const double *__restrict__ S,
-                             const double *__restrict__ z, double *__restrict__ p) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        size_t i = (size_t)k * N + c;
-        p[i] = first ? z[i] : fma(S[S_B * 8 + k], p[i], z[i]);
-    }
 }
 
 // FP64 <-> FP32 copies of the masked components
@@ -1213,8 +1411,10 @@ __global__ void k_mx_f2d(int N, unsigned mask, const float *__restrict__ a, doub
         if ((mask >> k) & 1u) b[(size_t)k * N + c] = (double)a[(size_t)k * N + c];
 }
 
-// psi += x32; x32 = 0
-__global__ void k_mx_fold(int N, unsigned mask, float *__restrict__ x32, double *__restrict__ psi) {
+// psi += x32; x32 = 0 on the components of mask, or of the device word *m
+__global__ void k_mx_fold(int N, unsigned mask, const unsigned *__restrict__ m, float *__restrict__ x32,
+                          double *__restrict__ psi) {
+    if (m) mask = *m;
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
     for (int k = 0; k < 6; ++k) {
@@ -1225,101 +1425,119 @@ __global__ void k_mx_fold(int N, unsigned mask, float *__restrict__ x32, double 
     }
 }
 
-// r32 = b - A psi from the FP64 matrix; partial |b - A psi| (slot 0)
-__global__ void k_mx_true_res(Ell e, unsigned mask, const double *__restrict__ diag,
-                              const double *__restrict__ upper, const double *__restrict__ lower,
-                              const double *__restrict__ b, const double *__restrict__ psi,
-                              float *__restrict__ r32, double *partial, int nB) {
-    const int N = e.N;
+// the end of an iteration before any replacement: the components at the half
+// step: x32 += alpha y; the others: x32 += alpha y + omega z, r = s - omega t, |r|
+// and r0.r.  The last block: the components whose residual is replaced (dropped
+// by kReplace since the last time, converged, at the end of the budget, or no
+// number), and beta of those that go on as they are
+__global__ void k_mx_update(int N, LoopCtl L, double replace, const float *__restrict__ y, const float *__restrict__ z,
+                            const float *__restrict__ s, const float *__restrict__ t, const float *__restrict__ r0,
+                            float *__restrict__ x, float *__restrict__ r, double *S, double *partial, int nB,
+                            unsigned *counter) {
+    if (!L.m[M_ACTIVE]) return;
+    const unsigned mask = L.m[M_CONT], half = L.m[M_HALF];
     for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        double v = 0.0;
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
-            const double r = b[(size_t)k * N + c] - row_mul(e, c, diag, upper, lower, psi + (size_t)k * N);
-            r32[(size_t)k * N + c] = (float)r;
-            v += fabs(r);
-        }
-        store_partial(partial, nB, 0, k, v);
-    }
-}
-
-// BiCGStab: p = r (first iteration or restart) or r + beta (p - omega Ay)
-__global__ void k_mx_bicg_p(int N, unsigned mask, int first, const double *__restrict__ S,
-                            const float *__restrict__ r, const float *__restrict__ Ay, float *__restrict__ p) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        if (S[S_SING * 8 + k] != 0.0) continue;
-        size_t i = (size_t)k * N + c;
-        if (first || S[S_RST * 8 + k] != 0.0) p[i] = r[i];
-        else {
-            const float beta = (float)S[S_B * 8 + k], omega = (float)S[S_OMEGA * 8 + k];
-            p[i] = fmaf(beta, fmaf(-omega, Ay[i], p[i]), r[i]);
-        }
-    }
-}
-
-// BiCGStab: alpha = r0r / (r0 . Ay); a pending restart is consumed
-__global__ void k_mx_sc_bicg_alpha(unsigned mask, const double *res, double *S) {
-    int k = threadIdx.x;
-    if (k < 6 && ((mask >> k) & 1u)) {
-        S[S_ALPHA * 8 + k] = S[S_R0R * 8 + k] / res[k];
-        S[S_RST * 8 + k] = 0.0;
-    }
-}
-
-__global__ void k_mx_set_rst(unsigned mask, double *S) {
-    int k = threadIdx.x;
-    if (k < 6 && ((mask >> k) & 1u)) S[S_RST * 8 + k] = 1.0;
-}
-
-// BiCGStab: s = r - alpha Ay; partial |s|
-__global__ void k_mx_bicg_s(int N, unsigned mask, const double *__restrict__ S, const float *__restrict__ r,
-                            const float *__restrict__ Ay, float *__restrict__ s, double *partial, int nB) {
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        const float alpha = (float)S[S_ALPHA * 8 + k];
-        double v = 0.0;
         size_t o = (size_t)k * N;
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
-            const float sv = fmaf(-alpha, Ay[o + c], r[o + c]);
-            s[o + c] = sv;
-            v += fabs((double)sv);
-        }
-        store_partial(partial, nB, 0, k, v);
-    }
-}
-
-// x32 += alpha y
-__global__ void k_mx_axpy_alpha(int N, unsigned mask, const double *__restrict__ S, const float *__restrict__ y,
-                                float *__restrict__ x) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    for (int k = 0; k < 6; ++k)
-        if ((mask >> k) & 1u) {
-            size_t i = (size_t)k * N + c;
-            x[i] = fmaf((float)S[S_ALPHA * 8 + k], y[i], x[i]);
-        }
-}
-
-// x32 += alpha y + omega z; r = s - omega t; partial |r|
-__global__ void k_mx_bicg_update(int N, unsigned mask, const double *__restrict__ S, const float *__restrict__ y,
-                                 const float *__restrict__ z, const float *__restrict__ s,
-                                 const float *__restrict__ t, float *__restrict__ x, float *__restrict__ r,
-                                 double *partial, int nB) {
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
         const float alpha = (float)S[S_ALPHA * 8 + k], omega = (float)S[S_OMEGA * 8 + k];
-        double v = 0.0;
-        size_t o = (size_t)k * N;
+        if ((half >> k) & 1u) {
+            for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x)
+                x[o + c] = fmaf(alpha, y[o + c], x[o + c]);
+            continue;
+        }
+        if (!((mask >> k) & 1u)) continue;
+        double v = 0.0, v1 = 0.0;
+        #pragma unroll 4
         for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
             x[o + c] = fmaf(alpha, y[o + c], fmaf(omega, z[o + c], x[o + c]));
             const float rv = fmaf(-omega, t[o + c], s[o + c]);
             r[o + c] = rv;
             v += fabs((double)rv);
+            v1 = fma((double)r0[o + c], (double)rv, v1);
         }
         store_partial(partial, nB, 0, k, v);
+        store_partial(partial, nB, 1, k, v1);
+    }
+    if (!last_block(counter)) return;
+    unsigned next = 0, repl = half;
+    const int it = L.iter + 1;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double res = partials_sum(partial, nB, 0, k), r0r = partials_sum(partial, nB, 1, k);
+        if (threadIdx.x == 0) {
+            const double fin = res / S[S_NF * 8 + k];
+            S[S_FIN * 8 + k] = fin;
+            S[S_ITER * 8 + k] = it;
+            if (fin < replace * S[S_TRUE * 8 + k] || converged(L.ctl, fin, S[S_INIT * 8 + k]) || it >= L.ctl.maxIter ||
+                !isfinite(fin))
+                repl |= 1u << k;
+            else if (bicg_rho(S, k, it, r0r))
+                next |= 1u << k;
+        }
+    }
+    if (threadIdx.x == 0) {
+        L.m[M_ACTIVE] = next;
+        L.m[M_REPL] = repl;
+        if (!next && !repl) {
+            L.m[M_CONT] = 0u;
+            *(volatile int *)L.hostFlag = 0;
+            __threadfence_system();
+        }
+    }
+}
+
+// the components in M_REPL, their x32 folded into psi: r32 = b - A psi from the
+// FP64 matrix, |b - A psi| and r0.r32; the last block: the stopping rules on that
+// residual, the restart of those that stopped at the half step, and beta
+__global__ void k_mx_true(Ell e, LoopCtl L, const double *__restrict__ diag, const double *__restrict__ upper,
+                          const double *__restrict__ lower, const double *__restrict__ b,
+                          const double *__restrict__ psi, const float *__restrict__ r0, float *__restrict__ r32,
+                          double *S, double *partial, int nB, unsigned *counter) {
+    const unsigned mask = L.m[M_REPL];
+    if (!mask) return;
+    const unsigned half = L.m[M_HALF] & mask;
+    const int N = e.N;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        double v = 0.0, v1 = 0.0;
+        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
+            const double r = b[(size_t)k * N + c] - row_mul(e, c, diag, upper, lower, psi + (size_t)k * N);
+            const float rv = (float)r;
+            r32[(size_t)k * N + c] = rv;
+            v += fabs(r);
+            v1 = fma((double)r0[(size_t)k * N + c], (double)rv, v1);
+        }
+        store_partial(partial, nB, 0, k, v);
+        store_partial(partial, nB, 1, k, v1);
+    }
+    if (!last_block(counter)) return;
+    unsigned next = 0;
+    const int it = L.iter + 1;
+    for (int k = 0; k < 6; ++k) {
+        if (!((mask >> k) & 1u)) continue;
+        const double res = partials_sum(partial, nB, 0, k), r0r = partials_sum(partial, nB, 1, k);
+        if (threadIdx.x == 0) {
+            const double fin = res / S[S_NF * 8 + k];
+            S[S_FIN * 8 + k] = fin;
+            S[S_TRUE * 8 + k] = fin;
+            S[S_ITER * 8 + k] = it;
+            const bool conv = converged(L.ctl, fin, S[S_INIT * 8 + k]), isHalf = (half >> k) & 1u;
+            const bool more = isHalf ? (!conv || it < L.ctl.minIter) && it < L.ctl.maxIter
+                                     : (it < L.ctl.maxIter && !conv) || it < L.ctl.minIter;
+            if (more && isfinite(fin)) {
+                if (isHalf) S[S_RST * 8 + k] = 1.0;
+                if (bicg_rho(S, k, it, r0r)) next |= 1u << k;
+            }
+        }
+    }
+    if (threadIdx.x == 0) {
+        next |= L.m[M_ACTIVE];
+        L.m[M_ACTIVE] = next;
+        L.m[M_REPL] = 0u;
+        if (!next) {
+            L.m[M_CONT] = 0u;
+            *(volatile int *)L.hostFlag = 0;
+            __threadfence_system();
+        }
     }
 }
 
@@ -1630,7 +1848,8 @@ struct Mixed : Solver {
         launch_count(ctx, 2);
     }
 
-    void precondition32(unsigned mask, const float *r, float *w) {
+    // (dmask: the device word of the components still iterating, or null)
+    void precondition32(unsigned mask, const float *r, float *w, const unsigned *dmask = nullptr) {
         const DevMesh &m = ctx->mesh;
         const int pre = a.ctl.preconditioner;
         const double fpc = (double)m.F / N;
@@ -1640,7 +1859,7 @@ struct Mixed : Solver {
             // add about 1/7
             const double nc = pop(mask);
             ProfScope ps(ctx, "mg_vcycle32", (double)N * (8.0 * nc + 5.0 * (28.0 + 12.0 * nc)) * 8.0 / 7.0);
-            mg_apply32(ctx, mask, r, w);
+            mg_apply32(ctx, mask, r, w, dmask);
             return;
         }
         if (pre == RT_PRECOND_NONE) {
@@ -1651,57 +1870,18 @@ struct Mixed : Solver {
             launch_count(ctx);
         } else if (systolic()) {
             ProfScope ps(ctx, "dilu_precondition32", (double)N * (4.0 + fpc * 8.0 + 16.0 * pop(mask)));
-            skew_precondition32(ctx, a.nc, mask, r, w);
+            skew_precondition32(ctx, a.nc, mask, r, w, dmask);
         } else {
             ProfScope ps(ctx, "dilu_precondition32", (double)N * (8.0 + fpc * 24.0 + 16.0 * pop(mask)));
-            level_precondition32(ctx, mask, r, w);
+            level_precondition32(ctx, mask, r, w, dmask);
         }
         RT_CHECK_LAUNCH();
     }
 
-    void amul32(unsigned mask, const float *x, float *y) {
-        const double fpc = (double)ctx->mesh.F / N;
-        ProfScope ps(ctx, "amul32", (double)N * (4.0 + fpc * 16.0 + 8.0 * pop(mask)));
-        k_mx_amul<<<nblocks(N), RT_BLOCK, 0, st>>>(e, mask, d32, u32, l32, x, y);
-        RT_CHECK_LAUNCH();
-        launch_count(ctx);
-    }
-
-    void dot32(unsigned mask, const float *x, const float *y, const float *x2 = nullptr,
-               const float *y2 = nullptr) {
-        ProfScope ps(ctx, "dot32", (double)N * 4.0 * (x2 ? 4 : 2) * pop(mask));
-        k_mx_dot<<<nB, RT_BLOCK, 0, st>>>(N, mask, x, y, x2, y2, ctx->red.partial.p, nB);
-        RT_CHECK_LAUNCH();
-        launch_count(ctx);
-        finalize(x2 ? 2 : 1, mask);
-    }
-
-    void sync_scalars() {
-        RT_CUDA(cudaMemcpyAsync(ctx->red.hostResult, S, sizeof(double) * (S_SING + 1) * 8, cudaMemcpyDeviceToHost,
-                                st));
-        RT_CUDA(cudaStreamSynchronize(st));
-    }
-
-    // fold x32 into psi and replace r32 by b - A psi; S_FIN gets the
-    // normalised FP64 residual of the masked components
-    void replace(unsigned mask, float *x32, float *r32) {
-        if (!mask) return;
-        const double fpc = (double)ctx->mesh.F / N;
-        ProfScope ps(ctx, "residual_replace", (double)N * (8.0 + fpc * 24.0 + 44.0 * pop(mask)));
-        k_mx_fold<<<nblocks(N), RT_BLOCK, 0, st>>>(N, mask, x32, a.psi);
-        k_mx_true_res<<<nB, RT_BLOCK, 0, st>>>(e, mask, a.diag, a.upper, a.lower, a.source, a.psi, r32,
-                                               ctx->red.partial.p, nB);
-        RT_CHECK_LAUNCH();
-        finalize(1, mask);
-        k_sc_fin<<<1, 32, 0, st>>>(mask, ctx->red.result.p, S);
-        RT_CHECK_LAUNCH();
-        launch_count(ctx, 3);
-    }
 };
 
 // prologue shared by the mixed solvers; returns the components to iterate
-unsigned mixed_begin(Mixed &mx, const SolveArgs &a, rt_solver_perf *perf, float *r32, float *x32,
-                     double *lastTrue) {
+unsigned mixed_begin(Mixed &mx, const SolveArgs &a, rt_solver_perf *perf, float *r32, float *x32) {
     rt_ctx *ctx = mx.ctx;
     const int N = mx.N;
     double *wA = ctx->kws.p, *rA = ctx->kws.p + 6 * (size_t)N;
@@ -1720,24 +1900,9 @@ unsigned mixed_begin(Mixed &mx, const SolveArgs &a, rt_solver_perf *perf, float 
         perf[k].finalResidual = ctx->red.hostResult[S_FIN * 8 + k];
         perf[k].nIterations = 0;
         perf[k].singular = 0;
-        lastTrue[k] = perf[k].finalResidual;
         if (a.ctl.minIter > 0 || !mx.conv(perf[k].finalResidual, perf[k].initialResidual)) active |= 1u << k;
     }
     return active;
-}
-
-// after an iteration: which components need a residual replacement
-unsigned mixed_replace_set(const Mixed &mx, const SolveArgs &a, unsigned cand, const double *H, int iter,
-                           const rt_solver_perf *perf, const double *lastTrue) {
-    unsigned R = 0;
-    for (int k = 0; k < 6; ++k) {
-        if (!((cand >> k) & 1u)) continue;
-        const double fin = H[S_FIN * 8 + k];
-        if (fin < kReplace * lastTrue[k] || mx.conv(fin, perf[k].initialResidual) || iter >= a.ctl.maxIter ||
-            !std::isfinite(fin))
-            R |= 1u << k;
-    }
-    return R;
 }
 
 // Mixed form of the pressure solve: PCG with FP64 vectors and scalars and
@@ -1758,104 +1923,51 @@ rt_status run_pcg_flex32(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) 
 
 rt_status run_pbicgstab_mixed(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
     Mixed mx(ctx, a, 9);
-    const int N = mx.N;
+    const int N = mx.N, nB = mx.nB;
     float *r = mx.v(0), *r0 = mx.v(1), *p = mx.v(2), *y = mx.v(3), *Ay = mx.v(4), *s = mx.v(5), *z = mx.v(6),
           *t = mx.v(7), *x = mx.v(8);
-    double lastTrue[6] = {};
-    unsigned active = mixed_begin(mx, a, perf, r, x, lastTrue);
-    if (!active) return RT_OK;
+    const unsigned act = mixed_begin(mx, a, perf, r, x);
+    if (!act) return RT_OK;
+    Reduce &red = ctx->red;
     RT_CUDA(cudaMemcpyAsync(r0, r, sizeof(float) * 6 * (size_t)N, cudaMemcpyDeviceToDevice, mx.st));
-    int iter = 0;
-    double H[(S_SING + 1) * 8];
-    while (active) {
-        mx.dot32(active, r0, r);
-        k_sc_bicg_r0r<<<1, 32, 0, mx.st>>>(active, iter, ctx->red.result.p, mx.S);
-        k_mx_bicg_p<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, active, iter == 0, mx.S, r, Ay, p);
-        mx.precondition32(active, p, y);
-        mx.amul32(active, y, Ay);
-        mx.dot32(active, r0, Ay);
-        k_mx_sc_bicg_alpha<<<1, 32, 0, mx.st>>>(active, ctx->red.result.p, mx.S);
-        k_mx_bicg_s<<<mx.nB, RT_BLOCK, 0, mx.st>>>(N, active, mx.S, r, Ay, s, ctx->red.partial.p, mx.nB);
+    red.hostFlag[0] = 1;
+    k_bicg_arm<<<1, 32, 0, mx.st>>>(act, red.active.p, mx.S);
+    k_bicg_first<float><<<nB, RT_BLOCK, 0, mx.st>>>(N, LoopCtl{a.ctl, red.active.p, red.devFlag, 0}, r0, r, mx.S,
+                                                   red.partial.p, nB, red.counter.p);
+    RT_CHECK_LAUNCH();
+    launch_count(ctx, 2);
+    const double fpc = (double)ctx->mesh.F / N, nc = mx.pop(act);
+    const double amulBytes = (double)N * (4.0 + fpc * 16.0 + 12.0 * nc);
+    bicg_loop(ctx, mx, a, [&](const LoopCtl &L) {
+        k_bicg_p<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, L, mx.S, r, Ay, p);
+        mx.precondition32(act, p, y, L.m + M_ACTIVE);
+        {
+            ProfScope ps(ctx, "amul32", amulBytes);
+            k_bicg_Ay<float><<<nB, RT_BLOCK, 0, mx.st>>>(mx.e, L, mx.d32, mx.u32, mx.l32, y, r0, Ay, mx.S,
+                                                        red.partial.p, nB, red.counter.p);
+        }
+        k_bicg_s<float><<<nB, RT_BLOCK, 0, mx.st>>>(N, L, r, Ay, s, mx.S, red.partial.p, nB, red.counter.p);
+        mx.precondition32(act, s, z, L.m + M_CONT);
+        {
+            ProfScope ps(ctx, "amul32", amulBytes);
+            k_bicg_t<float><<<nB, RT_BLOCK, 0, mx.st>>>(mx.e, L, mx.d32, mx.u32, mx.l32, z, s, t, mx.S, red.partial.p,
+                                                       nB, red.counter.p);
+        }
+        k_mx_update<<<nB, RT_BLOCK, 0, mx.st>>>(N, L, kReplace, y, z, s, t, r0, x, r, mx.S, red.partial.p, nB,
+                                                red.counter.p);
+        {
+            ProfScope ps(ctx, "residual_replace", (double)N * (8.0 + fpc * 24.0 + 44.0 * nc));
+            k_mx_fold<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, 0u, L.m + M_REPL, x, a.psi);
+            k_mx_true<<<nB, RT_BLOCK, 0, mx.st>>>(mx.e, L, a.diag, a.upper, a.lower, a.source, a.psi, r0, r, mx.S,
+                                                  red.partial.p, nB, red.counter.p);
+        }
         RT_CHECK_LAUNCH();
-        mx.finalize(1, active);
-        k_sc_fin<<<1, 32, 0, mx.st>>>(active, ctx->red.result.p, mx.S);
-        RT_CHECK_LAUNCH();
-        launch_count(ctx, 5);
-        mx.sync_scalars();
-        memcpy(H, ctx->red.hostResult, sizeof H);
-        // the half-step test: components whose s meets the tolerance take
-        // x += alpha y and have their residual replaced; the FP64 residual
-        // decides whether they stop or restart
-        unsigned half = 0, cont = 0;
-        for (int k = 0; k < 6; ++k) {
-            if (!((active >> k) & 1u)) continue;
-            if (H[S_SING * 8 + k] != 0.0) {
-                perf[k].singular = 1;
-                continue;
-            }
-            if (mx.conv(H[S_FIN * 8 + k], perf[k].initialResidual)) half |= 1u << k;
-            else cont |= 1u << k;
-        }
-        unsigned restart = 0;
-        if (half) {
-            k_mx_axpy_alpha<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, half, mx.S, y, x);
-            RT_CHECK_LAUNCH();
-            launch_count(ctx);
-            mx.replace(half, x, r);
-            mx.sync_scalars();
-            for (int k = 0; k < 6; ++k) {
-                if (!((half >> k) & 1u)) continue;
-                perf[k].finalResidual = ctx->red.hostResult[S_FIN * 8 + k];
-                perf[k].nIterations = iter + 1;
-                lastTrue[k] = perf[k].finalResidual;
-                const bool conv = mx.conv(perf[k].finalResidual, perf[k].initialResidual);
-                if ((!conv || iter + 1 < a.ctl.minIter) && iter + 1 < a.ctl.maxIter &&
-                    std::isfinite(perf[k].finalResidual))
-                    restart |= 1u << k;
-            }
-            if (restart) {
-                k_mx_set_rst<<<1, 32, 0, mx.st>>>(restart, mx.S);
-                RT_CHECK_LAUNCH();
-                launch_count(ctx);
-            }
-        }
-        unsigned next = restart;
-        if (cont) {
-            mx.precondition32(cont, s, z);
-            mx.amul32(cont, z, t);
-            mx.dot32(cont, t, t, t, s);
-            k_sc_bicg_omega<<<1, 32, 0, mx.st>>>(cont, ctx->red.result.p, mx.S);
-            k_mx_bicg_update<<<mx.nB, RT_BLOCK, 0, mx.st>>>(N, cont, mx.S, y, z, s, t, x, r, ctx->red.partial.p,
-                                                            mx.nB);
-            RT_CHECK_LAUNCH();
-            mx.finalize(1, cont);
-            k_sc_fin<<<1, 32, 0, mx.st>>>(cont, ctx->red.result.p, mx.S);
-            RT_CHECK_LAUNCH();
-            launch_count(ctx, 3);
-            mx.sync_scalars();
-            memcpy(H, ctx->red.hostResult, sizeof H);
-            const unsigned R = mixed_replace_set(mx, a, cont, H, iter + 1, perf, lastTrue);
-            mx.replace(R, x, r);
-            if (R) {
-                mx.sync_scalars();
-                memcpy(H, ctx->red.hostResult, sizeof H);
-            }
-            for (int k = 0; k < 6; ++k) {
-                if (!((cont >> k) & 1u)) continue;
-                perf[k].finalResidual = H[S_FIN * 8 + k];
-                perf[k].nIterations = iter + 1;
-                if ((R >> k) & 1u) lastTrue[k] = perf[k].finalResidual;
-                const bool conv = ((R >> k) & 1u) && mx.conv(perf[k].finalResidual, perf[k].initialResidual);
-                const bool more = (iter + 1 < a.ctl.maxIter && !conv) || iter + 1 < a.ctl.minIter;
-                if (more && std::isfinite(perf[k].finalResidual)) next |= 1u << k;
-            }
-        }
-        ++iter;
-        active = next;
-    }
-    k_mx_fold<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, a.validMask, x, a.psi);
+        launch_count(ctx, 7);
+    });
+    k_mx_fold<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, a.validMask, nullptr, x, a.psi);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
+    bicg_records(ctx, mx, act, perf);
     return RT_OK;
 }
 

@@ -370,8 +370,8 @@ void level_precondition(rt_ctx *ctx, unsigned mask, const double *r, double *w, 
     apply<double>(ctx, T ? l.coefT : l.coef, mask, r, w, dmask);
 }
 
-void level_precondition32(rt_ctx *ctx, unsigned mask, const float *r, float *w) {
-    apply<float>(ctx, ctx->mesh.lev.coef32, mask, r, w, nullptr);
+void level_precondition32(rt_ctx *ctx, unsigned mask, const float *r, float *w, const unsigned *dmask) {
+    apply<float>(ctx, ctx->mesh.lev.coef32, mask, r, w, dmask);
 }
 
 }  // namespace rt

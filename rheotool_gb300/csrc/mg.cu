@@ -116,7 +116,8 @@ __device__ __forceinline__ float nb_sum(const float (&c)[7], const Nb6 &n, const
     return s;
 }
 
-__device__ __forceinline__ bool skip(const unsigned *dm) { return dm && !(*dm & 1u); }
+// the components of m that still iterate (dm: a device word, or null)
+__device__ __forceinline__ unsigned live(unsigned m, const unsigned *dm) { return dm ? m & *dm : m; }
 
 // The passes of a V-cycle are launched to start while the pass before still runs
 // (programmatic dependent launch): a thread loads its cell's coefficients, which
@@ -233,7 +234,8 @@ __global__ void k_mg_first(MgLev L, const int *__restrict__ cellAt, int N, unsig
                            const unsigned *__restrict__ dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L.nh || skip(dm)) return;
+    m = live(m, dm);
+    if (t >= L.nh || !m) return;
     const At a = at_of(L.nx, L.ny, L.hx, 0, t);   // (o: the red cell's place in the pair)
     const int b0 = 2 * a.ii + L.nx * (a.j + L.ny * a.k);
     const int c0 = cellAt[b0], c1 = 2 * a.ii + 1 < L.nx ? cellAt[b0 + 1] : -1;
@@ -254,7 +256,8 @@ __global__ void k_mg_first(MgLev L, const int *__restrict__ cellAt, int N, unsig
 __global__ void k_mg_smooth(MgLev L, int colour, unsigned m, const unsigned *__restrict__ dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L.nh || skip(dm)) return;
+    m = live(m, dm);
+    if (t >= L.nh || !m) return;
     float c[7];
     coeffs(L, colour, t, c);
     const Nb6 n = neighbours(L.ny, L.nz, L.hx, at_of(L.nx, L.ny, L.hx, colour, t), t);
@@ -273,7 +276,8 @@ __global__ void k_mg_last(MgLev L, int colour, unsigned m, const int *__restrict
                           const unsigned *__restrict__ dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L.nh || skip(dm)) return;
+    m = live(m, dm);
+    if (t >= L.nh || !m) return;
     const At a = at_of(L.nx, L.ny, L.hx, colour, t);
     const int b0 = 2 * a.ii + L.nx * (a.j + L.ny * a.k);
     const int c0 = cellAt[b0], c1 = 2 * a.ii + 1 < L.nx ? cellAt[b0 + 1] : -1;
@@ -297,7 +301,8 @@ __global__ void k_mg_last(MgLev L, int colour, unsigned m, const int *__restrict
 __global__ void k_mg_correct(MgLev F, MgLev C, unsigned m, const unsigned *__restrict__ dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= F.nh || skip(dm)) return;
+    m = live(m, dm);
+    if (t >= F.nh || !m) return;
     float c[7];
     coeffs(F, 1, t, c);
     const At a = at_of(F.nx, F.ny, F.hx, 1, t);
@@ -335,7 +340,8 @@ __global__ void k_mg_correct(MgLev F, MgLev C, unsigned m, const unsigned *__res
 __global__ void k_mg_restrict(MgLev F, MgLev C, unsigned m, const unsigned *__restrict__ dm) {
     next_may_start();
     const int B = blockIdx.x * blockDim.x + threadIdx.x;
-    if (B >= C.n || skip(dm)) return;
+    m = live(m, dm);
+    if (B >= C.n || !m) return;
     int I, J, K;
     box_ijk(C, B, I, J, K);
     const int fx = F.nx == C.nx ? 1 : 2, fy = F.ny == C.ny ? 1 : 2, fz = F.nz == C.nz ? 1 : 2;
@@ -448,7 +454,7 @@ template <int NQ>
 __global__ void __launch_bounds__(tail_threads(NQ), 1) k_mg_tail(MgTail T, int sweeps, unsigned m,
                                                             const unsigned *__restrict__ dm) {
     next_may_start();
-    if (skip(dm)) return;
+    if (!live(m, dm)) return;
     const int nt = blockDim.x;
     extern __shared__ __align__(16) float sh[];
     __shared__ TailLev lev[kMaxLevels];
@@ -832,8 +838,8 @@ void mg_apply(rt_ctx *ctx, const double *r, double *w, const unsigned *dm) {
     apply<double>(ctx, true, 1u, r, w, dm);
 }
 
-void mg_apply32(rt_ctx *ctx, unsigned mask, const float *r, float *w) {
-    apply<float>(ctx, false, mask, r, w, nullptr);
+void mg_apply32(rt_ctx *ctx, unsigned mask, const float *r, float *w, const unsigned *dm) {
+    apply<float>(ctx, false, mask, r, w, dm);
 }
 
 }  // namespace rt

@@ -797,8 +797,9 @@ void skew_prepare32(rt_ctx *ctx, const double *diag, const double *upper, const 
     launch_count(ctx);
 }
 
-void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w) {
+void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w, const unsigned *dmask) {
     SkewView32 g = ctx->mesh.sm.view32();
+    g.dmask = dmask;
     k_skew_gather<float, float><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);

@@ -20,7 +20,8 @@ void skew_rdinv_cells(rt_ctx *ctx, double *rDc);
 // mixed precision: skew_prepare, then FP32 copies of the sweep coefficients
 void skew_prepare32(rt_ctx *ctx, const double *diag, const double *upper, const double *lower);
 // FP32 w = M^-1 r with the coefficients of the last skew_prepare32
-void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w);
+void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w,
+                         const unsigned *dmask = nullptr);
 // the same with an FP64 right-hand side and result (rounded on the way in and out)
 void skew_precondition32d(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w,
                           const unsigned *dmask = nullptr);
@@ -31,17 +32,16 @@ void level_factor(rt_ctx *ctx, const double *diag, const double *upper, const do
 void level_coefs(rt_ctx *ctx, const double *rD, const double *lower, const double *upper, bool T);
 void level_coefs32(rt_ctx *ctx, const float *rD, const float *lower, const float *upper);
 void level_precondition(rt_ctx *ctx, unsigned mask, const double *r, double *w, bool T, const unsigned *dmask);
-void level_precondition32(rt_ctx *ctx, unsigned mask, const float *r, float *w);
+void level_precondition32(rt_ctx *ctx, unsigned mask, const float *r, float *w, const unsigned *dmask);
 // mg.cu: the aggregation multigrid V-cycle of the mixed pressure and
 // momentum solves (FP32): the hierarchy of a matrix (sym: a symmetric one,
 // its lower coefficients only), then w = V-cycle(r): mg_apply for the
-// pressure (FP64 vectors; dm, device or null: component 0 still iterating),
-// mg_apply32 for the momentum components in mask (FP32 vectors, component k
-// at k N)
+// pressure (FP64 vectors), mg_apply32 for the momentum components in mask (FP32
+// vectors, component k at k N); dm, device or null: the components still iterating
 bool mg_available(rt_ctx *ctx);
 void mg_prepare(rt_ctx *ctx, const double *diag, const double *upper, const double *lower, bool sym);
 void mg_apply(rt_ctx *ctx, const double *r, double *w, const unsigned *dm = nullptr);
-void mg_apply32(rt_ctx *ctx, unsigned mask, const float *r, float *w);
+void mg_apply32(rt_ctx *ctx, unsigned mask, const float *r, float *w, const unsigned *dm = nullptr);
 // RT_ETIMEOUT if a bounded wait of the last sweeps ran out
 rt_status skew_check(rt_ctx *ctx);
 
