@@ -96,7 +96,7 @@ constexpr int SYNC_WORK = 0, SYNC_ERROR = 1, SYNC_DONE = 2, SYNC_WORDS = 4;
 
 // steps by which a row of the structured sweeps' tiles lags the row before it
 // in j and in k (sweep.cu)
-constexpr int kSkewJ = 1, kSkewK = 2;
+constexpr int kSkewJ = 1, kSkewK = 1;
 
 // raw view passed to the kernels; every array has nSkew entries in the
 // skewed (tile, step / 2, lane, step % 2) layout, wS has 6 components of nSkew

@@ -22,15 +22,17 @@
 //
 // What bounds it: latency.  Measured on GB300: a dependent FP64 fused
 // multiply-add takes a warp 64 cycles and an independent one 48 (one FP64 unit
-// a quarter of an SM, whatever the lanes in use), an FP32 one 4, a value
-// through shared memory 35, through L2 to another SM 480 to 860.  An FP64 step
-// cannot take less than about 150 cycles and an FP32 one 45; the longest chain
-// has nx + kSkewJ ny + kSkewK nz steps.  So four tiles of a CTA (one a quarter
+// a quarter of an SM, whatever the lanes in use), an FP32 one 4; an FP64 result
+// reaches shared memory 105 cycles after its product; a value takes 35 through
+// shared memory and 480 to 860 through L2 to another SM.  So an FP64 step cannot
+// take less than about 245 cycles and an FP32 one 45; the longest chain has nx +
+// kSkewJ ny + kSkewK nz steps.  So four tiles of a CTA (one a quarter
 // of the SM) hand over in shared memory, only every second tile boundary
 // goes through L2, and all else is kept off the tiles' warps: other warps of
 // the CTA fetch the ghosts, hand results to the next CTAs, stage coefficients
-// and write results out.  With kSkewK = 2 the k product is formed a step ahead,
-// off the chain of a step.
+// and write results out.  (A skew of two in k would take the k product off a
+// step's chain, but a warp issues its FP64 products in order: a step was no shorter,
+// and there were nz more of them.)
 //
 // A value handed to another CTA is its own flag: the hand-off words hold the
 // pattern of all ones until the producer writes the value (a result with that
@@ -128,12 +130,6 @@ __device__ __forceinline__ void st2(float *p, float x, float y) { *reinterpret_c
 
 template <int N> struct IntC { static constexpr int v = N; };
 
-// x, not before v is known (zero: a zero that the compiler does not know)
-__device__ __forceinline__ double after(double x, double v, int zero) {
-    return __hiloint2double(__double2hiint(x), __double2loint(x) | (__double2loint(v) & zero));
-}
-__device__ __forceinline__ float after(float x, float, int) { return x; }
-
 // one launch's tiles, components and hand-off words
 template <class Real>
 struct TileRun {
@@ -226,10 +222,10 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
     constexpr int TK = 32 / TJ, PITCH = G::pitch, R = G::ringSteps;
     constexpr int offJ = kSkewJ * (TJ - 1), offK = kSkewK * (TK - 1);   // a producer's lead in steps
         constexpr int GS = sizeof(Real) == 8 ? 2 : 4;   // steps between two looks at the counters
-    constexpr int B = P < 8 ? P : 8;   // steps that share their slots' addresses
+    constexpr int B = 4;   // steps that share their slots' addresses
     static_assert(B % GS == 0 && P % B == 0 && P <= 16 && R % P == 0, "groups fill blocks, blocks chunks, chunks the ring");
     static_assert(kSkewJ * TJ % B == 0 && (TK == 1 || kSkewK * TK % B == 0), "a block of another tile's slots does not wrap");
-    static_assert(kSkewJ == 1 && kSkewK == 2, "the k product is formed one step ahead, the j product is not");
+    static_assert(kSkewJ == 1 && kSkewK == 1, "a step reads the values of the step before");
     constexpr W kNone = ~W(0);
     const Real zk = (MODE == 2) ? Real(1) : Real(0);
     SkewT<Real> &g = a.g;
@@ -316,9 +312,9 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
             if (lane == 0 && (wj > 0 || J > 0)) {   // the j producer's steps
                 watch = wj > 0 ? cnt + C_COMPUTED + w - 1 : cnt + C_GHOST_J + wk;
                 off = GS + offJ;
-            } else if (lane == 1 && (wk > 0 || (TK > 1 && K > 0))) {   // the k producer's (one step ahead)
+            } else if (lane == 1 && (wk > 0 || (TK > 1 && K > 0))) {   // the k producer's
                 watch = wk > 0 ? cnt + C_COMPUTED + w - WJ : cnt + C_GHOST_K + wj;
-                off = GS + offK + 1;
+                off = GS + offK;
             } else if (lane == 2 && J + 1 < nTJ) {   // the j consumer has read what these steps overwrite
                 watch = wj + 1 < WJ ? cnt + C_COMPUTED + w + 1 : cnt + C_HANDED_J + wk;
                 off = GS - R;
@@ -332,9 +328,8 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
                 watch = cnt + C_STAGED + w;
                 off = GS;
             }
-            const int zero = a.N >> 31;   // 0
             int seen = 0;
-            Real y1 = zk, pre = zk;
+            Real y1 = zk;
             // looks at the counters until the steps from t on may be taken
             auto until_ready = [&](int t) {
                 const int need = min(t + off, T);
@@ -353,41 +348,36 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
                 for (int b0 = 0; b0 < P; b0 += B) {
                     const int tb = t0 + b0;
                     volatile Real *cur = ring + (tb & (R - 1)) * PITCH + w * 32 + lane;
-                    // the neighbours' slots of steps tb - 2, tb - 1 and from tb on
-                    const volatile Real *kPast = ring + ((tb - 2 + leadK) & (R - 1)) * PITCH + iK;
+                    // the neighbours' slots of step tb - 1 and from tb on
+                    const volatile Real *kPast = ring + ((tb - 1 + leadK) & (R - 1)) * PITCH + iK;
                     const volatile Real *kNow = ring + ((tb + leadK) & (R - 1)) * PITCH + iK;
                     const volatile Real *jPast = ring + ((tb - 1 + leadJ) & (R - 1)) * PITCH + iJ;
                     const volatile Real *jNow = ring + ((tb + leadJ) & (R - 1)) * PITCH + iJ;
-                    auto product_k = [&](int s, Real xz) {   // D - Pz / rD(k-1), or r - a_z w(k-1)
-                        const int sf = (MODE == 1) ? P - 1 - b0 - s : b0 + s;
-                        return MODE == 2 ? r_sub(va[0][sf], r_div(va[1][sf], xz)) : r_fma(-va[0][sf], xz, va[3][sf]);
-                    };
 #pragma unroll
                     for (int s = 0; s < B; ++s) {
                         if (s % GS == 0) {
                             if (b0 + s > 0) until_ready(tb + s);
                             seen = *watch;   // for the next group
-                            if (b0 + s == 0) pre = product_k(0, kPast[0]);
                         }
                         const int sf = (MODE == 1) ? P - 1 - b0 - s : b0 + s;
+                        const Real xz = s >= 1 ? kNow[(s - 1) * PITCH] : kPast[0];
                         const Real xy = s >= 1 ? jNow[(s - 1) * PITCH] : jPast[0];
-                        const Real xzNext = s + 1 >= 2 ? kNow[(s - 1) * PITCH] : kPast[(s + 1) * PITCH];
                         Real v;
                         if (MODE == 2) {
-                            v = r_sub(pre, r_div(va[2][sf], xy));
+                            v = r_sub(va[0][sf], r_div(va[1][sf], xz));   // D - Pz / rD(k-1) - ...
+                            v = r_sub(v, r_div(va[2][sf], xy));
                             v = r_sub(v, r_div(va[3][sf], y1));
-                        } else if (sizeof(Real) == 4) {
-                            // FP32: the i term before the j term
-                            v = r_fma(-va[2][sf], y1, pre);
-                            v = r_fma(-va[1][sf], xy, v);
                         } else {
-                            v = r_fma(-va[1][sf], xy, pre);
-                            v = r_fma(-va[2][sf], y1, v);
+                            v = r_fma(-va[0][sf], xz, va[3][sf]);
+                            if (sizeof(Real) == 4) {
+                                // FP32: the i term before the j term
+                                v = r_fma(-va[2][sf], y1, v);
+                                v = r_fma(-va[1][sf], xy, v);
+                            } else {
+                                v = r_fma(-va[1][sf], xy, v);
+                                v = r_fma(-va[2][sf], y1, v);
+                            }
                         }
-                        // the next step's k product after this step's (FP64: one
-                        // product at a time; before them it would delay them), in
-                        // the shadow of the result's way through the ring
-                        if (b0 + s + 1 < P) pre = product_k(s + 1, after(xzNext, v, zero));
                         cur[s * PITCH] = v;
                         y1 = v;
                         warp_sync();
@@ -676,9 +666,10 @@ void launch_one(rt_ctx *ctx, const TileRun<Real> &run) {
 // NB (blocks in flight) and with them the CTA's tiles: chunks of 16 steps leave
 // an FP64 CTA room for two.  RT_OPT_SWEEP_TUNE takes one of them; the default is
 // two tiles and (16, 3), as fewer warps share the SM's issue slots (1M cells,
-// one component: FP64 248 us an application against 260 with four tiles and
-// (8, 5), FP32 133 against 163), but four in FP64 when the groups of two would
-// not all run at once, one an SM (three components: 271 us against 331).
+// one component: FP64 235 us an application against 248 with four tiles and
+// (8, 5), FP32 132 against 154), but four when the groups of two would not all
+// run at once, one an SM (three components: FP64 258 us against 330, FP32 162
+// against 169).
 constexpr int kTuneN = 5;
 constexpr int kTuneP[kTuneN] = {8, 8, 16, 16, 4};
 constexpr int kTuneNB[kTuneN] = {3, 5, 3, 4, 6};
@@ -689,7 +680,7 @@ void launch_tuned(rt_ctx *ctx, const TileRun<Real> &run, int k) {
     constexpr int WJ = TJ == 32 ? 4 : 2, WK = TJ == 32 ? 1 : 2;
     if (k < 0) {
         const int two = (run.g.nTJ + 1) / 2 * run.g.nTK * run.ncc;
-        k = sizeof(Real) == 8 && two > ctx->numSMs ? kWide : kNarrow;
+        k = two > ctx->numSMs ? kWide : kNarrow;
     }
     switch (k) {
     case 0: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[0], kTuneNB[0]>(ctx, run); break;
