@@ -387,9 +387,10 @@ __device__ double partials_sum(const double *partial, int nB, int slot, int k) {
 // rho = w.r (slot 0) and, in the flexible form after the first iteration,
 // w.q_old (slot 1); the last block: wArAold = wArA, wArA = rho, flexible beta
 template <bool FLEX>
-__global__ void k_pcg_rho(int N, unsigned mask0, const unsigned *__restrict__ active, int first,
-                          const double *__restrict__ w, const double *__restrict__ r, const double *__restrict__ qold,
-                          double *S, double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_pcg_rho_body(int N, unsigned mask0, const unsigned *__restrict__ active, int first,
+                                               const double *__restrict__ w, const double *__restrict__ r, const
+                                               double *__restrict__ qold, double *S, double *partial, int nB, unsigned
+                                               *counter) {
     const unsigned mask = mask0 & *active;
     if (!mask) return;
     const bool two = FLEX && !first;
@@ -418,16 +419,22 @@ __global__ void k_pcg_rho(int N, unsigned mask0, const unsigned *__restrict__ ac
         }
     }
 }
+template <bool FLEX>
+__global__ void k_pcg_rho(int N, unsigned mask0, const unsigned *active, int first, const double *w, const double *r,
+                          const double *qold, double *S, double *partial, int nB, unsigned *counter) {
+    after_previous();
+    k_pcg_rho_body<FLEX>(N, mask0, active, first, w, r, qold, S, partial, nB, counter);
+}
 
 // p_new = w (+ beta p_old); q = A p_new, the neighbours' p_new formed from
 // their w and p_old exactly as the cell's own; p.q; the last block: alpha =
 // wArA / wApA or the singularity test
 template <bool FLEX>
-__global__ void k_pcg_pq(Ell e, unsigned mask0, const unsigned *__restrict__ active, int first,
-                         const double *__restrict__ diag, const double *__restrict__ upper,
-                         const double *__restrict__ lower, const double *__restrict__ w,
-                         const double *__restrict__ pold, double *__restrict__ pnew, double *__restrict__ q, double *S,
-                         double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_pcg_pq_body(Ell e, unsigned mask0, const unsigned *__restrict__ active, int first,
+                                              const double *__restrict__ diag, const double *__restrict__ upper, const
+                                              double *__restrict__ lower, const double *__restrict__ w, const double
+                                              *__restrict__ pold, double *__restrict__ pnew, double *__restrict__ q,
+                                              double *S, double *partial, int nB, unsigned *counter) {
     const unsigned mask = mask0 & *active;
     if (!mask) return;
     const int N = e.N;
@@ -475,13 +482,21 @@ __global__ void k_pcg_pq(Ell e, unsigned mask0, const unsigned *__restrict__ act
         }
     }
 }
+template <bool FLEX>
+__global__ void k_pcg_pq(Ell e, unsigned mask0, const unsigned *active, int first, const double *diag, const double
+                         *upper, const double *lower, const double *w, const double *pold, double *pnew, double *q,
+                         double *S, double *partial, int nB, unsigned *counter) {
+    after_previous();
+    k_pcg_pq_body<FLEX>(e, mask0, active, first, diag, upper, lower, w, pold, pnew, q, S, partial, nB, counter);
+}
 
 // psi += alpha p; r -= alpha q; |r|; the last block: residual, iteration
 // count and lduMatrix's stopping rules per component (a singular component
 // stops without an update, keeping its last residual and count)
-__global__ void k_pcg_step(int N, unsigned mask0, unsigned *active, rt_solver_ctl ctl, const double *__restrict__ p,
-                           const double *__restrict__ q, double *__restrict__ psi, double *__restrict__ r, double *S,
-                           double *partial, int nB, unsigned *counter, int *hostFlag) {
+__device__ __forceinline__ void k_pcg_step_body(int N, unsigned mask0, unsigned *active, rt_solver_ctl ctl, const
+                                                double *__restrict__ p, const double *__restrict__ q, double
+                                                *__restrict__ psi, double *__restrict__ r, double *S, double *partial,
+                                                int nB, unsigned *counter, int *hostFlag) {
     const unsigned mask = mask0 & *active;
     if (!mask) return;
     for (int k = 0; k < 6; ++k) {
@@ -526,6 +541,12 @@ __global__ void k_pcg_step(int N, unsigned mask0, unsigned *active, rt_solver_ct
             __threadfence_system();
         }
     }
+}
+__global__ void k_pcg_step(int N, unsigned mask0, unsigned *active, rt_solver_ctl ctl, const double *p, const double
+                           *q, double *psi, double *r, double *S, double *partial, int nB, unsigned *counter, int
+                           *hostFlag) {
+    after_previous();
+    k_pcg_step_body(N, mask0, active, ctl, p, q, psi, r, S, partial, nB, counter, hostFlag);
 }
 
 // the loop's starting state: the components to iterate, zero iterations
@@ -583,8 +604,8 @@ __device__ bool bicg_rho(double *S, int k, int iter, double r0r) {
 
 // r0.r before the first iteration
 template <class V>
-__global__ void k_bicg_first(int N, LoopCtl L, const V *__restrict__ r0, const V *__restrict__ r, double *S,
-                             double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_bicg_first_body(int N, LoopCtl L, const V *__restrict__ r0, const V *__restrict__ r,
+                                                  double *S, double *partial, int nB, unsigned *counter) {
     const unsigned mask = L.m[M_ACTIVE];
     if (!mask) return;
     for (int k = 0; k < 6; ++k) {
@@ -612,10 +633,17 @@ __global__ void k_bicg_first(int N, LoopCtl L, const V *__restrict__ r0, const V
         }
     }
 }
+template <class V>
+__global__ void k_bicg_first(int N, LoopCtl L, const V *r0, const V *r, double *S, double *partial, int nB, unsigned
+                             *counter) {
+    after_previous();
+    k_bicg_first_body<V>(N, L, r0, r, S, partial, nB, counter);
+}
 
 // pA = rA (first, or a restart in the mixed form) or rA + beta (pA - omega AyA)
-__global__ void k_bicg_p(int N, LoopCtl L, const double *__restrict__ S, const double *__restrict__ rA,
-                         const double *__restrict__ AyA, double *__restrict__ pA) {
+__device__ __forceinline__ void k_bicg_p_body(int N, LoopCtl L, const double *__restrict__ S, const double
+                                              *__restrict__ rA, const double *__restrict__ AyA, double *__restrict__
+                                              pA) {
     const unsigned mask = L.m[M_ACTIVE];
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
@@ -626,8 +654,12 @@ __global__ void k_bicg_p(int N, LoopCtl L, const double *__restrict__ S, const d
         else pA[i] = rA[i] + S[S_B * 8 + k] * (pA[i] - S[S_OMEGA * 8 + k] * AyA[i]);
     }
 }
-__global__ void k_bicg_p(int N, LoopCtl L, const double *__restrict__ S, const float *__restrict__ r,
-                         const float *__restrict__ Ay, float *__restrict__ p) {
+__global__ void k_bicg_p(int N, LoopCtl L, const double *S, const double *rA, const double *AyA, double *pA) {
+    after_previous();
+    k_bicg_p_body(N, L, S, rA, AyA, pA);
+}
+__device__ __forceinline__ void k_bicg_p_body(int N, LoopCtl L, const double *__restrict__ S, const float
+                                              *__restrict__ r, const float *__restrict__ Ay, float *__restrict__ p) {
     const unsigned mask = L.m[M_ACTIVE];
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
@@ -640,6 +672,10 @@ __global__ void k_bicg_p(int N, LoopCtl L, const double *__restrict__ S, const f
             p[i] = fmaf(beta, fmaf(-omega, Ay[i], p[i]), r[i]);
         }
     }
+}
+__global__ void k_bicg_p(int N, LoopCtl L, const double *S, const float *r, const float *Ay, float *p) {
+    after_previous();
+    k_bicg_p_body(N, L, S, r, Ay, p);
 }
 
 // the rows c of A x for the components in mask (the coefficients and indices read
@@ -703,9 +739,10 @@ __device__ __forceinline__ void rows(const Ell &e, int c, unsigned mask, const f
 
 // AyA = A yA; r0.AyA; the last block: alpha (and a pending restart is consumed)
 template <class V>
-__global__ void k_bicg_Ay(Ell e, LoopCtl L, const V *__restrict__ diag, const V *__restrict__ upper,
-                          const V *__restrict__ lower, const V *__restrict__ y, const V *__restrict__ r0,
-                          V *__restrict__ Ay, double *S, double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_bicg_Ay_body(Ell e, LoopCtl L, const V *__restrict__ diag, const V *__restrict__
+                                               upper, const V *__restrict__ lower, const V *__restrict__ y, const V
+                                               *__restrict__ r0, V *__restrict__ Ay, double *S, double *partial, int
+                                               nB, unsigned *counter) {
     const unsigned mask = L.m[M_ACTIVE];
     if (!mask) return;
     const int N = e.N;
@@ -731,6 +768,12 @@ __global__ void k_bicg_Ay(Ell e, LoopCtl L, const V *__restrict__ diag, const V 
         }
     }
 }
+template <class V>
+__global__ void k_bicg_Ay(Ell e, LoopCtl L, const V *diag, const V *upper, const V *lower, const V *y, const V *r0, V
+                          *Ay, double *S, double *partial, int nB, unsigned *counter) {
+    after_previous();
+    k_bicg_Ay_body<V>(e, L, diag, upper, lower, y, r0, Ay, S, partial, nB, counter);
+}
 
 // s = r - alpha Ay and |s| of one element, in the vector's type
 __device__ __forceinline__ double bicg_s(double r, double alpha, double Ay) { return r - alpha * Ay; }
@@ -738,8 +781,9 @@ __device__ __forceinline__ float bicg_s(float r, double alpha, float Ay) { retur
 
 // sA = rA - alpha AyA; |sA|; the last block: the half-step test
 template <class V>
-__global__ void k_bicg_s(int N, LoopCtl L, const V *__restrict__ r, const V *__restrict__ Ay, V *__restrict__ s,
-                         double *S, double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_bicg_s_body(int N, LoopCtl L, const V *__restrict__ r, const V *__restrict__ Ay, V
+                                              *__restrict__ s, double *S, double *partial, int nB, unsigned *counter)
+                                              {
     const unsigned mask = L.m[M_ACTIVE];
     if (!mask) return;
     for (int k = 0; k < 6; ++k) {
@@ -778,12 +822,19 @@ __global__ void k_bicg_s(int N, LoopCtl L, const V *__restrict__ r, const V *__r
         L.m[M_CONT] = cont;
     }
 }
+template <class V>
+__global__ void k_bicg_s(int N, LoopCtl L, const V *r, const V *Ay, V *s, double *S, double *partial, int nB, unsigned
+                         *counter) {
+    after_previous();
+    k_bicg_s_body<V>(N, L, r, Ay, s, S, partial, nB, counter);
+}
 
 // tA = A zA; t.t (slot 0), t.s (slot 1); the last block: omega
 template <class V>
-__global__ void k_bicg_t(Ell e, LoopCtl L, const V *__restrict__ diag, const V *__restrict__ upper,
-                         const V *__restrict__ lower, const V *__restrict__ z, const V *__restrict__ s,
-                         V *__restrict__ t, double *S, double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_bicg_t_body(Ell e, LoopCtl L, const V *__restrict__ diag, const V *__restrict__
+                                              upper, const V *__restrict__ lower, const V *__restrict__ z, const V
+                                              *__restrict__ s, V *__restrict__ t, double *S, double *partial, int nB,
+                                              unsigned *counter) {
     if (!L.m[M_ACTIVE]) return;
     const unsigned mask = L.m[M_CONT];
     if (!mask) return;
@@ -814,14 +865,21 @@ __global__ void k_bicg_t(Ell e, LoopCtl L, const V *__restrict__ diag, const V *
         if (threadIdx.x == 0) S[S_OMEGA * 8 + k] = ts / tt;
     }
 }
+template <class V>
+__global__ void k_bicg_t(Ell e, LoopCtl L, const V *diag, const V *upper, const V *lower, const V *z, const V *s, V
+                         *t, double *S, double *partial, int nB, unsigned *counter) {
+    after_previous();
+    k_bicg_t_body<V>(e, L, diag, upper, lower, z, s, t, S, partial, nB, counter);
+}
 
 // the components that end this iteration at their tolerance: psi += alpha yA;
 // the others: psi += alpha yA + omega zA, rA = sA - omega tA, |rA| (slot 0) and
 // r0.rA (slot 1); the last block: lduMatrix's stopping rules, and beta
-__global__ void k_bicg_update(int N, LoopCtl L, const double *__restrict__ yA, const double *__restrict__ zA,
-                              const double *__restrict__ sA, const double *__restrict__ tA,
-                              const double *__restrict__ r0, double *__restrict__ psi, double *__restrict__ rA, double *S,
-                              double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_bicg_update_body(int N, LoopCtl L, const double *__restrict__ yA, const double
+                                                  *__restrict__ zA, const double *__restrict__ sA, const double
+                                                  *__restrict__ tA, const double *__restrict__ r0, double
+                                                  *__restrict__ psi, double *__restrict__ rA, double *S, double
+                                                  *partial, int nB, unsigned *counter) {
     if (!L.m[M_ACTIVE]) return;
     const unsigned mask = L.m[M_CONT], half = L.m[M_HALF];
     for (int k = 0; k < 6; ++k) {
@@ -868,6 +926,12 @@ __global__ void k_bicg_update(int N, LoopCtl L, const double *__restrict__ yA, c
             __threadfence_system();
         }
     }
+}
+__global__ void k_bicg_update(int N, LoopCtl L, const double *yA, const double *zA, const double *sA, const double
+                              *tA, const double *r0, double *psi, double *rA, double *S, double *partial, int nB,
+                              unsigned *counter) {
+    after_previous();
+    k_bicg_update_body(N, L, yA, zA, sA, tA, r0, psi, rA, S, partial, nB, counter);
 }
 
 namespace {
@@ -1049,20 +1113,20 @@ rt_status pcg_device_loop(rt_ctx *ctx, Solver &sv, const SolveArgs &a, rt_solver
         precondition(act, rA, z, red.active.p);
         {
             ProfScope ps(ctx, "dot", (double)N * 8.0 * ((FLEX && !first) ? 3 : 2) * sv.pop(act));
-            k_pcg_rho<FLEX><<<sv.nB, RT_BLOCK, 0, sv.st>>>(N, act, red.active.p, first, z, rA, q, sv.S,
+            launch_next(k_pcg_rho<FLEX>, sv.nB, RT_BLOCK, 0, sv.st, N, act, red.active.p, first, z, rA, q, sv.S,
                                                              red.partial.p, sv.nB, red.counter.p);
             RT_CHECK_LAUNCH();
         }
         {
             // the amul's bytes, plus w and p_old read and p written per component
             ProfScope ps(ctx, "amul", (double)N * (8.0 + fpc * 24.0 + 40.0 * sv.pop(act)));
-            k_pcg_pq<FLEX><<<sv.nB, RT_BLOCK, 0, sv.st>>>(sv.e, act, red.active.p, first, a.diag, a.upper, a.lower, z,
+            launch_next(k_pcg_pq<FLEX>, sv.nB, RT_BLOCK, 0, sv.st, sv.e, act, red.active.p, first, a.diag, a.upper, a.lower, z,
                                                             pold, pnew, q, sv.S, red.partial.p, sv.nB, red.counter.p);
             RT_CHECK_LAUNCH();
         }
         {
             ProfScope ps(ctx, "pcg_update", (double)N * 40.0 * sv.pop(act));
-            k_pcg_step<<<sv.nB, RT_BLOCK, 0, sv.st>>>(N, act, red.active.p, a.ctl, pnew, q, a.psi, rA, sv.S,
+            launch_next(k_pcg_step, sv.nB, RT_BLOCK, 0, sv.st, N, act, red.active.p, a.ctl, pnew, q, a.psi, rA, sv.S,
                                                       red.partial.p, sv.nB, red.counter.p, red.devFlag);
             RT_CHECK_LAUNCH();
         }
@@ -1298,28 +1362,29 @@ rt_status run_pbicgstab(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
     RT_CUDA(cudaMemcpyAsync(rA0, rA, sizeof(double) * V6, cudaMemcpyDeviceToDevice, sv.st));
     red.hostFlag[0] = 1;
     k_bicg_arm<<<1, 32, 0, sv.st>>>(act, red.active.p, sv.S);
-    k_bicg_first<double><<<nB, RT_BLOCK, 0, sv.st>>>(N, LoopCtl{a.ctl, red.active.p, red.devFlag, 0}, rA0, rA, sv.S,
+    launch_next(k_bicg_first<double>, nB, RT_BLOCK, 0, sv.st, N, LoopCtl{a.ctl, red.active.p, red.devFlag, 0}, rA0, rA, sv.S,
                                                     red.partial.p, nB, red.counter.p);
     RT_CHECK_LAUNCH();
     launch_count(ctx, 2);
     const double fpc = (double)ctx->mesh.F / N, nc = sv.pop(act);
     const double amulBytes = (double)N * (8.0 + fpc * 24.0 + 24.0 * nc);
     bicg_loop(ctx, sv, a, [&](const LoopCtl &L) {
-        k_bicg_p<<<nblocks(N), RT_BLOCK, 0, sv.st>>>(N, L, sv.S, rA, AyA, pA);
+        launch_next<int, LoopCtl, const double *, const double *, const double *, double *>(
+            k_bicg_p, nblocks(N), RT_BLOCK, 0, sv.st, N, L, sv.S, rA, AyA, pA);
         sv.precondition(act, rD, pA, yA, false, L.m + M_ACTIVE);
         {
             ProfScope ps(ctx, "amul", amulBytes);
-            k_bicg_Ay<double><<<nB, RT_BLOCK, 0, sv.st>>>(sv.e, L, a.diag, a.upper, a.lower, yA, rA0, AyA, sv.S,
+            launch_next(k_bicg_Ay<double>, nB, RT_BLOCK, 0, sv.st, sv.e, L, a.diag, a.upper, a.lower, yA, rA0, AyA, sv.S,
                                                          red.partial.p, nB, red.counter.p);
         }
-        k_bicg_s<double><<<nB, RT_BLOCK, 0, sv.st>>>(N, L, rA, AyA, sA, sv.S, red.partial.p, nB, red.counter.p);
+        launch_next(k_bicg_s<double>, nB, RT_BLOCK, 0, sv.st, N, L, rA, AyA, sA, sv.S, red.partial.p, nB, red.counter.p);
         sv.precondition(act, rD, sA, zA, false, L.m + M_CONT);
         {
             ProfScope ps(ctx, "amul", amulBytes);
-            k_bicg_t<double><<<nB, RT_BLOCK, 0, sv.st>>>(sv.e, L, a.diag, a.upper, a.lower, zA, sA, tA, sv.S,
+            launch_next(k_bicg_t<double>, nB, RT_BLOCK, 0, sv.st, sv.e, L, a.diag, a.upper, a.lower, zA, sA, tA, sv.S,
                                                         red.partial.p, nB, red.counter.p);
         }
-        k_bicg_update<<<nB, RT_BLOCK, 0, sv.st>>>(N, L, yA, zA, sA, tA, rA0, a.psi, rA, sv.S, red.partial.p, nB,
+        launch_next(k_bicg_update, nB, RT_BLOCK, 0, sv.st, N, L, yA, zA, sA, tA, rA0, a.psi, rA, sv.S, red.partial.p, nB,
                                                   red.counter.p);
         RT_CHECK_LAUNCH();
         launch_count(ctx, 5);
@@ -1412,8 +1477,8 @@ __global__ void k_mx_f2d(int N, unsigned mask, const float *__restrict__ a, doub
 }
 
 // psi += x32; x32 = 0 on the components of mask, or of the device word *m
-__global__ void k_mx_fold(int N, unsigned mask, const unsigned *__restrict__ m, float *__restrict__ x32,
-                          double *__restrict__ psi) {
+__device__ __forceinline__ void k_mx_fold_body(int N, unsigned mask, const unsigned *__restrict__ m, float
+                                               *__restrict__ x32, double *__restrict__ psi) {
     if (m) mask = *m;
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
@@ -1424,16 +1489,21 @@ __global__ void k_mx_fold(int N, unsigned mask, const unsigned *__restrict__ m, 
         x32[i] = 0.0f;
     }
 }
+__global__ void k_mx_fold(int N, unsigned mask, const unsigned *m, float *x32, double *psi) {
+    after_previous();
+    k_mx_fold_body(N, mask, m, x32, psi);
+}
 
 // the end of an iteration before any replacement: the components at the half
 // step: x32 += alpha y; the others: x32 += alpha y + omega z, r = s - omega t, |r|
 // and r0.r.  The last block: the components whose residual is replaced (dropped
 // by kReplace since the last time, converged, at the end of the budget, or no
 // number), and beta of those that go on as they are
-__global__ void k_mx_update(int N, LoopCtl L, double replace, const float *__restrict__ y, const float *__restrict__ z,
-                            const float *__restrict__ s, const float *__restrict__ t, const float *__restrict__ r0,
-                            float *__restrict__ x, float *__restrict__ r, double *S, double *partial, int nB,
-                            unsigned *counter) {
+__device__ __forceinline__ void k_mx_update_body(int N, LoopCtl L, double replace, const float *__restrict__ y, const
+                                                 float *__restrict__ z, const float *__restrict__ s, const float
+                                                 *__restrict__ t, const float *__restrict__ r0, float *__restrict__ x,
+                                                 float *__restrict__ r, double *S, double *partial, int nB, unsigned
+                                                 *counter) {
     if (!L.m[M_ACTIVE]) return;
     const unsigned mask = L.m[M_CONT], half = L.m[M_HALF];
     for (int k = 0; k < 6; ++k) {
@@ -1484,14 +1554,21 @@ __global__ void k_mx_update(int N, LoopCtl L, double replace, const float *__res
         }
     }
 }
+__global__ void k_mx_update(int N, LoopCtl L, double replace, const float *y, const float *z, const float *s, const
+                            float *t, const float *r0, float *x, float *r, double *S, double *partial, int nB,
+                            unsigned *counter) {
+    after_previous();
+    k_mx_update_body(N, L, replace, y, z, s, t, r0, x, r, S, partial, nB, counter);
+}
 
 // the components in M_REPL, their x32 folded into psi: r32 = b - A psi from the
 // FP64 matrix, |b - A psi| and r0.r32; the last block: the stopping rules on that
 // residual, the restart of those that stopped at the half step, and beta
-__global__ void k_mx_true(Ell e, LoopCtl L, const double *__restrict__ diag, const double *__restrict__ upper,
-                          const double *__restrict__ lower, const double *__restrict__ b,
-                          const double *__restrict__ psi, const float *__restrict__ r0, float *__restrict__ r32,
-                          double *S, double *partial, int nB, unsigned *counter) {
+__device__ __forceinline__ void k_mx_true_body(Ell e, LoopCtl L, const double *__restrict__ diag, const double
+                                               *__restrict__ upper, const double *__restrict__ lower, const double
+                                               *__restrict__ b, const double *__restrict__ psi, const float
+                                               *__restrict__ r0, float *__restrict__ r32, double *S, double *partial,
+                                               int nB, unsigned *counter) {
     const unsigned mask = L.m[M_REPL];
     if (!mask) return;
     const unsigned half = L.m[M_HALF] & mask;
@@ -1539,6 +1616,12 @@ __global__ void k_mx_true(Ell e, LoopCtl L, const double *__restrict__ diag, con
             __threadfence_system();
         }
     }
+}
+__global__ void k_mx_true(Ell e, LoopCtl L, const double *diag, const double *upper, const double *lower, const double
+                          *b, const double *psi, const float *r0, float *r32, double *S, double *partial, int nB,
+                          unsigned *counter) {
+    after_previous();
+    k_mx_true_body(e, L, diag, upper, lower, b, psi, r0, r32, S, partial, nB, counter);
 }
 
 // --------------------------------------------------------------------------
@@ -1932,39 +2015,40 @@ rt_status run_pbicgstab_mixed(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *p
     RT_CUDA(cudaMemcpyAsync(r0, r, sizeof(float) * 6 * (size_t)N, cudaMemcpyDeviceToDevice, mx.st));
     red.hostFlag[0] = 1;
     k_bicg_arm<<<1, 32, 0, mx.st>>>(act, red.active.p, mx.S);
-    k_bicg_first<float><<<nB, RT_BLOCK, 0, mx.st>>>(N, LoopCtl{a.ctl, red.active.p, red.devFlag, 0}, r0, r, mx.S,
+    launch_next(k_bicg_first<float>, nB, RT_BLOCK, 0, mx.st, N, LoopCtl{a.ctl, red.active.p, red.devFlag, 0}, r0, r, mx.S,
                                                    red.partial.p, nB, red.counter.p);
     RT_CHECK_LAUNCH();
     launch_count(ctx, 2);
     const double fpc = (double)ctx->mesh.F / N, nc = mx.pop(act);
     const double amulBytes = (double)N * (4.0 + fpc * 16.0 + 12.0 * nc);
     bicg_loop(ctx, mx, a, [&](const LoopCtl &L) {
-        k_bicg_p<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, L, mx.S, r, Ay, p);
+        launch_next<int, LoopCtl, const double *, const float *, const float *, float *>(
+            k_bicg_p, nblocks(N), RT_BLOCK, 0, mx.st, N, L, mx.S, r, Ay, p);
         mx.precondition32(act, p, y, L.m + M_ACTIVE);
         {
             ProfScope ps(ctx, "amul32", amulBytes);
-            k_bicg_Ay<float><<<nB, RT_BLOCK, 0, mx.st>>>(mx.e, L, mx.d32, mx.u32, mx.l32, y, r0, Ay, mx.S,
+            launch_next(k_bicg_Ay<float>, nB, RT_BLOCK, 0, mx.st, mx.e, L, mx.d32, mx.u32, mx.l32, y, r0, Ay, mx.S,
                                                         red.partial.p, nB, red.counter.p);
         }
-        k_bicg_s<float><<<nB, RT_BLOCK, 0, mx.st>>>(N, L, r, Ay, s, mx.S, red.partial.p, nB, red.counter.p);
+        launch_next(k_bicg_s<float>, nB, RT_BLOCK, 0, mx.st, N, L, r, Ay, s, mx.S, red.partial.p, nB, red.counter.p);
         mx.precondition32(act, s, z, L.m + M_CONT);
         {
             ProfScope ps(ctx, "amul32", amulBytes);
-            k_bicg_t<float><<<nB, RT_BLOCK, 0, mx.st>>>(mx.e, L, mx.d32, mx.u32, mx.l32, z, s, t, mx.S, red.partial.p,
+            launch_next(k_bicg_t<float>, nB, RT_BLOCK, 0, mx.st, mx.e, L, mx.d32, mx.u32, mx.l32, z, s, t, mx.S, red.partial.p,
                                                        nB, red.counter.p);
         }
-        k_mx_update<<<nB, RT_BLOCK, 0, mx.st>>>(N, L, kReplace, y, z, s, t, r0, x, r, mx.S, red.partial.p, nB,
+        launch_next(k_mx_update, nB, RT_BLOCK, 0, mx.st, N, L, kReplace, y, z, s, t, r0, x, r, mx.S, red.partial.p, nB,
                                                 red.counter.p);
         {
             ProfScope ps(ctx, "residual_replace", (double)N * (8.0 + fpc * 24.0 + 44.0 * nc));
-            k_mx_fold<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, 0u, L.m + M_REPL, x, a.psi);
-            k_mx_true<<<nB, RT_BLOCK, 0, mx.st>>>(mx.e, L, a.diag, a.upper, a.lower, a.source, a.psi, r0, r, mx.S,
+            launch_next(k_mx_fold, nblocks(N), RT_BLOCK, 0, mx.st, N, 0u, L.m + M_REPL, x, a.psi);
+            launch_next(k_mx_true, nB, RT_BLOCK, 0, mx.st, mx.e, L, a.diag, a.upper, a.lower, a.source, a.psi, r0, r, mx.S,
                                                   red.partial.p, nB, red.counter.p);
         }
         RT_CHECK_LAUNCH();
         launch_count(ctx, 7);
     });
-    k_mx_fold<<<nblocks(N), RT_BLOCK, 0, mx.st>>>(N, a.validMask, nullptr, x, a.psi);
+    launch_next(k_mx_fold, nblocks(N), RT_BLOCK, 0, mx.st, N, a.validMask, nullptr, x, a.psi);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     bicg_records(ctx, mx, act, perf);

@@ -209,23 +209,24 @@ __device__ void level_sweep(const LevelView &v, const int *start, Real *x, const
 // they fit) or in `scratch`.
 template <class Real, int CS, int NP>
 __global__ void __launch_bounds__(kMaxThreads) k_level_apply(LevelView v, LevelCoef<Real> a, unsigned mask, int walkers,
-                                                            int inSmem, const Real *__restrict__ r,
-                                                            Real *__restrict__ w, Real *scratch,
-                                                            const unsigned *__restrict__ dmask) {
+                                                            int inSmem, const Real *r, Real *w, Real *scratch,
+                                                            const unsigned *dmask) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    int *start = reinterpret_cast<int *>(smem);
+    next_may_start();
+    for (int i = threadIdx.x; i <= v.nl; i += blockDim.x) start[i] = v.start[i];
+    wait_for_previous();
     const unsigned live = dmask ? mask & *dmask : mask;
     unsigned m = mask;
     for (int q = blockIdx.x / CS; q > 0; --q) m &= m - 1;
     const int comp = __ffs(m) - 1;
     if (!((live >> comp) & 1u)) return;   // (every CTA of the cluster alike)
-    extern __shared__ __align__(16) unsigned char smem[];
-    int *start = reinterpret_cast<int *>(smem);
     Real *x = inSmem ? reinterpret_cast<Real *>(smem + ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16)
                      : scratch + (size_t)comp * v.N;
     r += (size_t)comp * v.N;
     w += (size_t)comp * v.N;
     const int rank = CS > 1 ? blockIdx.x % CS : 0;
     const int all = CS * blockDim.x, tid = rank * blockDim.x + threadIdx.x;
-    for (int i = threadIdx.x; i <= v.nl; i += blockDim.x) start[i] = v.start[i];
     for (int p = tid; p < v.N; p += all) x[p] = r_mul(a.rd[p], r[v.cell[p]]);
     __syncthreads();
     if (CS > 1) level_barrier<CS>(0);
@@ -246,6 +247,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_level_factor(LevelView v, int w
                                                              const double *__restrict__ upper,
                                                              const double *__restrict__ lower, double *scratch,
                                                              double *__restrict__ rD) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     int *start = reinterpret_cast<int *>(smem);
     double *x = inSmem ? reinterpret_cast<double *>(smem + ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16) : scratch;
@@ -306,13 +308,15 @@ void launch_levels(rt_ctx *ctx, void (*one)(A...), void (*eight)(A...), const Le
     cfg.blockDim = dim3(q.threads);
     cfg.dynamicSmemBytes = q.smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = q.CS;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (see launch_next)
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = q.CS;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = q.CS > 1 ? 1 : 0;
+    cfg.numAttrs = q.CS > 1 ? 2 : 1;
     RT_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
     RT_CHECK_LAUNCH();
     launch_count(ctx);

@@ -122,9 +122,9 @@ __device__ __forceinline__ unsigned live(unsigned m, const unsigned *dm) { retur
 // The passes of a V-cycle are launched to start while the pass before still runs
 // (programmatic dependent launch): a thread loads its cell's coefficients, which
 // no pass writes, and then waits until the pass before has finished.  Every pass
-// waits before it touches x or b, so each starts them after all earlier ones.
-__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// waits before it touches x or b, so each starts them after all earlier ones.  The
+// first lets none of the others start until it has itself waited for what came
+// before the cycle, so the rest read the mask of components at once.
 
 // level 0 from the FP64 LDU matrix (box arrays zeroed before): the face to
 // the lower neighbour c' of cell c carries A[c][c'] = lower, A[c'][c] = upper
@@ -230,18 +230,17 @@ __device__ __forceinline__ float *split(float *a, const MgLev &L, int q, int col
 // component k at k N), then the red half-sweep (x_red = b / dg); a thread the
 // cells 2 ii and 2 ii + 1 of a row
 template <class T>
-__global__ void k_mg_first(MgLev L, const int *__restrict__ cellAt, int N, unsigned m, const T *__restrict__ r,
-                           const unsigned *__restrict__ dm) {
-    next_may_start();
+__global__ void k_mg_first(MgLev L, const int *__restrict__ cellAt, int N, unsigned m, const T *r, const unsigned *dm) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    m = live(m, dm);
-    if (t >= L.nh || !m) return;
+    if (t >= L.nh) return;
     const At a = at_of(L.nx, L.ny, L.hx, 0, t);   // (o: the red cell's place in the pair)
     const int b0 = 2 * a.ii + L.nx * (a.j + L.ny * a.k);
     const int c0 = cellAt[b0], c1 = 2 * a.ii + 1 < L.nx ? cellAt[b0 + 1] : -1;
     const int red = a.o ? c1 : c0, black = a.o ? c0 : c1;
-    const float d = L.co[t];
     wait_for_previous();
+    next_may_start();
+    m = live(m, dm);
+    const float d = L.co[t];
 #pragma unroll
     for (int q = 0; q < 3; ++q)
         if ((m >> q) & 1u) {
@@ -253,7 +252,7 @@ __global__ void k_mg_first(MgLev L, const int *__restrict__ cellAt, int N, unsig
 }
 
 // one half-sweep of red-black Gauss-Seidel (colour 0: i + j + k even)
-__global__ void k_mg_smooth(MgLev L, int colour, unsigned m, const unsigned *__restrict__ dm) {
+__global__ void k_mg_smooth(MgLev L, int colour, unsigned m, const unsigned *dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     m = live(m, dm);
@@ -273,7 +272,7 @@ __global__ void k_mg_smooth(MgLev L, int colour, unsigned m, const unsigned *__r
 // level 0's last half-sweep (red): every cell's x to w in cell order
 template <class T>
 __global__ void k_mg_last(MgLev L, int colour, unsigned m, const int *__restrict__ cellAt, int N, T *__restrict__ w,
-                          const unsigned *__restrict__ dm) {
+                          const unsigned *dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     m = live(m, dm);
@@ -298,7 +297,7 @@ __global__ void k_mg_last(MgLev L, int colour, unsigned m, const int *__restrict
 
 // the first black half-sweep after the coarse correction: the red values with
 // the correction, x + kOver x_coarse(aggregate), formed as they are read
-__global__ void k_mg_correct(MgLev F, MgLev C, unsigned m, const unsigned *__restrict__ dm) {
+__global__ void k_mg_correct(MgLev F, MgLev C, unsigned m, const unsigned *dm) {
     next_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     m = live(m, dm);
@@ -337,7 +336,7 @@ __global__ void k_mg_correct(MgLev F, MgLev C, unsigned m, const unsigned *__res
 
 // the residual b - A x of each aggregate's cells, summed into the coarse
 // right-hand side, and the coarse level's first red half-sweep from x = 0
-__global__ void k_mg_restrict(MgLev F, MgLev C, unsigned m, const unsigned *__restrict__ dm) {
+__global__ void k_mg_restrict(MgLev F, MgLev C, unsigned m, const unsigned *dm) {
     next_may_start();
     const int B = blockIdx.x * blockDim.x + threadIdx.x;
     m = live(m, dm);
@@ -452,7 +451,7 @@ __device__ __forceinline__ void tail_smooth(const TailLev &L, int colour) {
 // NQ: the components of the mask
 template <int NQ>
 __global__ void __launch_bounds__(tail_threads(NQ), 1) k_mg_tail(MgTail T, int sweeps, unsigned m,
-                                                            const unsigned *__restrict__ dm) {
+                                                            const unsigned *dm) {
     next_may_start();
     if (!live(m, dm)) return;
     const int nt = blockDim.x;
@@ -694,22 +693,6 @@ void mg_prepare(rt_ctx *ctx, const double *diag, const double *upper, const doub
 
 namespace {
 
-// a pass that may start while the one before it runs
-template <class... A>
-void launch_pass(void (*k)(A...), int blocks, int threads, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    RT_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
-}
-
 void launch_tail(const std::vector<MgLev> &L, int first, unsigned m, const unsigned *dm, cudaStream_t st) {
     MgTail tail{};
     for (size_t l = 0; l < L.size(); ++l) tail.lev[l] = L[l];
@@ -722,7 +705,7 @@ void launch_tail(const std::vector<MgLev> &L, int first, unsigned m, const unsig
     auto k = nq == 1 ? k_mg_tail<1> : nq == 2 ? k_mg_tail<2> : k_mg_tail<3>;
     RT_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem));
     const int threads = std::min(tail_threads(nq), std::max(128, (L[first].nh + 31) / 32 * 32));
-    launch_pass(k, 1, threads, bytes, st, tail, kCoarseSweeps, m, dm);
+    launch_next(k, 1, threads, bytes, st, tail, kCoarseSweeps, m, dm);
 }
 
 // one V-cycle's launches on the stream; the number of kernels
@@ -735,7 +718,7 @@ int enqueue_vcycle(rt_ctx *ctx, const std::vector<MgLev> &L, unsigned m, const T
     int launches = 0;
     auto blocks = [](int n) { return nblocks(n, kPassBlock); };
     auto smooth = [&](const MgLev &l, int colour) {
-        launch_pass(k_mg_smooth, blocks(l.nh), kPassBlock, 0, st, l, colour, m, dm);
+        launch_next(k_mg_smooth, blocks(l.nh), kPassBlock, 0, st, l, colour, m, dm);
         ++launches;
     };
     // the levels that run in one CTA: the coarsest and those above it that are
@@ -757,13 +740,13 @@ int enqueue_vcycle(rt_ctx *ctx, const std::vector<MgLev> &L, unsigned m, const T
             if (nu > 0) smooth(L[l], 0);
             smooth(L[l], 1);
         }
-        launch_pass(k_mg_restrict, blocks(L[l + 1].n), kPassBlock, 0, st, L[l], L[l + 1], m, dm);
+        launch_next(k_mg_restrict, blocks(L[l + 1].n), kPassBlock, 0, st, L[l], L[l + 1], m, dm);
         ++launches;
     }
     launch_tail(L, tf, m, dm, st);
     ++launches;
     if (nL == 1) {   // a mesh no larger than the coarsest level: its x to w, as it is
-        launch_pass(k_mg_last<T>, blocks(L[0].nh), kPassBlock, 0, st, L[0], 1, m, (const int *)s.cellAt.p, N, w, dm);
+        launch_next(k_mg_last<T>, blocks(L[0].nh), kPassBlock, 0, st, L[0], 1, m, (const int *)s.cellAt.p, N, w, dm);
         RT_CHECK_LAUNCH();
         return launches + 1;
     }
@@ -772,13 +755,13 @@ int enqueue_vcycle(rt_ctx *ctx, const std::vector<MgLev> &L, unsigned m, const T
     for (int l = tf - 1; l >= 0; --l)
         for (int nu = 0; nu < kNu; ++nu) {
             if (nu == 0) {
-                launch_pass(k_mg_correct, blocks(L[l].nh), kPassBlock, 0, st, L[l], L[l + 1], m, dm);
+                launch_next(k_mg_correct, blocks(L[l].nh), kPassBlock, 0, st, L[l], L[l + 1], m, dm);
                 ++launches;
             } else {
                 smooth(L[l], 1);
             }
             if (l == 0 && nu == kNu - 1) {
-                launch_pass(k_mg_last<T>, blocks(L[l].nh), kPassBlock, 0, st, L[l], 0, m, (const int *)s.cellAt.p, N, w, dm);
+                launch_next(k_mg_last<T>, blocks(L[l].nh), kPassBlock, 0, st, L[l], 0, m, (const int *)s.cellAt.p, N, w, dm);
                 ++launches;
             } else {
                 smooth(L[l], 0);

@@ -562,6 +562,38 @@ rt_status step_once(rt_ctx *ctx, rt_step_perf *perf);
 void ddt_begin_step(rt_ctx *ctx, bool flow);
 void init_fields(rt_ctx *ctx);
 
+// Kernels of the solver loops start while the one before them still runs
+// (programmatic dependent launch): launch_next launches such a kernel, whose
+// first act, or first before it reads what earlier kernels wrote, is
+// after_previous().  A kernel that begins so starts after every earlier one.  What
+// earlier kernels of a loop write must not reach it through a __restrict__ pointer
+// parameter: the compiler may load through one ahead of the wait (those kernels
+// have a body, a function with __restrict__ parameters, called after it).  It takes
+// about 1.5 us of launch gap off each kernel: two steps of a 32 x 32 cavity 18.1
+// -> 14.3 ms, one of a 127k-cell contraction 73.9 -> 69.3 ms.
+template <class... P, class... A>
+void launch_next(void (*k)(P...), int blocks, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    RT_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...));
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() {
+    next_may_start();
+    wait_for_previous();
+}
+#endif
+
 inline int nblocks(long long n, int b = RT_BLOCK) { return (int)((n + b - 1) / b); }
 
 // prof.cu

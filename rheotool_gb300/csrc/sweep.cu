@@ -229,10 +229,7 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
     constexpr W kNone = ~W(0);
     const Real zk = (MODE == 2) ? Real(1) : Real(0);
     SkewT<Real> &g = a.g;
-    // every component of the launch has stopped iterating (the same word for
-    // every CTA, written by an earlier kernel): nothing to do
-    const unsigned live = g.dmask ? a.mask & *g.dmask : a.mask;
-    if (!live) return;
+    next_may_start();
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) u64 bars[G::W * NB];
     __shared__ int s_cnt[C_COUNT];
@@ -242,12 +239,17 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
     const unsigned bar0 = (unsigned)__cvta_generic_to_shared(bars);
     if (threadIdx.x == 0) {
         for (int i = 0; i < C_COUNT; ++i) s_cnt[i] = 0;
-        s_cnt[C_TICKET] = atomicAdd(a.sync + SYNC_WORK, 1);
         for (int b = 0; b < G::W * NB; ++b) bar_init(bar0 + 8 * b);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     for (int i = threadIdx.x; i < R * PITCH; i += blockDim.x) ring[i] = zk;
+    wait_for_previous();
+    // every component of the launch has stopped iterating (the same word for
+    // every CTA, written by an earlier kernel): nothing to do
+    const unsigned live = g.dmask ? a.mask & *g.dmask : a.mask;
+    if (!live) return;
+    if (threadIdx.x == 0) s_cnt[C_TICKET] = atomicAdd(a.sync + SYNC_WORK, 1);
     __syncthreads();
     const int ticket = s_cnt[C_TICKET];
     // ticket t is group t / ncc of the (t % ncc)-th component, so every
@@ -567,7 +569,8 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
 // product of the forward recurrence, rounded as the sequential sweep rounds it
 // (an FP64 right-hand side of the FP32 sweeps is rounded first)
 template <class Real, class In>
-__global__ void k_skew_gather(SkewT<Real> g, unsigned mask, int nc, const In *__restrict__ r, int N) {
+__device__ __forceinline__ void k_skew_gather_body(SkewT<Real> g, unsigned mask, int nc, const In *__restrict__ r, int
+                                                  N) {
     long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (e >= g.nSkew) return;
     if (g.dmask) mask &= *g.dmask;
@@ -576,6 +579,11 @@ __global__ void k_skew_gather(SkewT<Real> g, unsigned mask, int nc, const In *__
     for (int q = 0; q < nc; ++q)
         if ((mask >> q) & 1u)
             g.rS[(long long)q * g.nSkew + e] = c >= 0 ? r_mul(rd, (Real)r[(long long)q * N + c]) : Real(0);
+}
+template <class Real, class In>
+__global__ void k_skew_gather(SkewT<Real> g, unsigned mask, int nc, const In *r, int N) {
+    after_previous();
+    k_skew_gather_body<Real, In>(g, mask, nc, r, N);
 }
 
 // gather the skewed per-entry coefficients of one matrix
@@ -659,7 +667,7 @@ void launch_one(rt_ctx *ctx, const TileRun<Real> &run) {
         opted = true;
     }
     const int groups = (run.g.nTJ + WJ - 1) / WJ * ((run.g.nTK + WK - 1) / WK);
-    k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB><<<groups * run.ncc, 32 * G::warps, shm, ctx->stream>>>(run);
+    launch_next(k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB>, groups * run.ncc, 32 * G::warps, shm, ctx->stream, run);
 }
 
 // Schedules of the sweeps: chunk size P (steps per staged block), staging depth
@@ -736,7 +744,7 @@ void skew_prepare(rt_ctx *ctx, const double *diag, const double *upper, const do
 void skew_precondition(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w, const unsigned *dmask) {
     SkewView g = ctx->mesh.sm.view();
     g.dmask = dmask;
-    k_skew_gather<double, double><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
+    launch_next(k_skew_gather<double, double>, nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream, g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     launch_mode<double, 0>(ctx, g, mask, w);
@@ -771,7 +779,7 @@ void skew_prepare_T(rt_ctx *ctx, const double *upper, const double *lower) {
 
 void skew_precondition_T(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w) {
     SkewView g = ctx->mesh.sm.viewT();
-    k_skew_gather<double, double><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
+    launch_next(k_skew_gather<double, double>, nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream, g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     launch_mode<double, 0>(ctx, g, mask, w);
@@ -791,7 +799,7 @@ void skew_prepare32(rt_ctx *ctx, const double *diag, const double *upper, const 
 void skew_precondition32(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w, const unsigned *dmask) {
     SkewView32 g = ctx->mesh.sm.view32();
     g.dmask = dmask;
-    k_skew_gather<float, float><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
+    launch_next(k_skew_gather<float, float>, nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream, g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     launch_mode<float, 0>(ctx, g, mask, w);
@@ -802,7 +810,7 @@ void skew_precondition32d(rt_ctx *ctx, int nc, unsigned mask, const double *r, d
     SkewView32 g = ctx->mesh.sm.view32();
     g.w64 = w;
     g.dmask = dmask;
-    k_skew_gather<float, double><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
+    launch_next(k_skew_gather<float, double>, nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream, g, mask, nc, r, ctx->mesh.N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     launch_mode<float, 0>(ctx, g, mask, (float *)nullptr);
