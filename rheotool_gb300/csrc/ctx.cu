@@ -1144,7 +1144,7 @@ rt_status rt_batch_layout(rt_ctx *ctx, int32_t nCases, const int32_t *cellStart,
                     mgDims[((size_t)c * kBatchMgLevels + l) * 2] = nx;
                     mgDims[((size_t)c * kBatchMgLevels + l) * 2 + 1] = ny;
                     mgOff[(size_t)c * kBatchMgLevels + l] = mgTotal;
-                    mgTotal += kBatchMgArrays * (((long long)nx * ny + 3) / 4 * 4);
+                    mgTotal += batch_mg_floats(nx, ny);
                     mgNL[c] = l + 1;
                     if ((long long)nx * ny <= kBatchMgCoarse) break;
                     nx = (nx + 1) / 2;

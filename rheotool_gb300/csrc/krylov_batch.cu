@@ -40,6 +40,7 @@ namespace rt {
 namespace {
 
 constexpr double kReplaceB = 0.1;
+constexpr int kSlots = 4;   // ELL width of the 2-D cases
 
 __device__ __forceinline__ double bsum(double v) {   // valid in thread 0
     __shared__ double sh[32];
@@ -634,22 +635,34 @@ __global__ void k_b_copy(int N, unsigned vm, const V *__restrict__ r, V *__restr
 // it: the same aggregation (2 x 2 blocks, Galerkin 5-point coarse
 // operators), red-black Gauss-Seidel smoothing (kBMgNu sweeps each way,
 // coarse correction scaled by kBMgOver) and symmetric sweeps on the
-// coarsest level, every phase a loop of the CTA over a level's box followed
-// by a barrier.  A level holds the diagonal and each cell's couplings to and
-// from its (i-1) and (j-1) neighbours: A[c][c-1] in xl, A[c-1][c] in xu (yl,
+// coarsest level, every phase a loop of the CTA over a level followed by a
+// barrier.  A momentum solve takes it component by component.
+//
+// The hierarchy is built in box order: the diagonal and each cell's couplings to
+// and from its (i-1) and (j-1) neighbours, A[c][c-1] in xl, A[c-1][c] in xu (yl,
 // yu likewise); the symmetric pressure matrix keeps one copy (xu aliases xl).
 // With piecewise-constant prolongation P and restriction P^T, the coarse
 // operator P^T A P of a non-symmetric matrix is again such a stencil, so the
-// momentum matrix (convection makes it non-symmetric) takes the same cycle,
-// its components sharing every coefficient load.
+// momentum matrix (convection makes it non-symmetric) takes the same cycle.
+//
+// The cycle itself runs on the levels split by colour: cell (i, j) is entry
+// j st + (i >> 1) of colour (i + j) & 1, rows padded to whole 16-byte vectors,
+// and a thread takes four neighbouring entries of a row at a time.  What bounds
+// it: the instructions and the shared memory of the one SM (a half-sweep of 8192
+// cells 16.5k cycles in box order out of the L2, with a division and a branch a
+// neighbour for each cell).  So as much of the hierarchy as fits lies in the CTA's
+// shared memory, the coarse levels first, then the finest level's x, b and
+// coefficients; the rest stays in the pool.  Missing neighbours have a zero
+// coupling and any finite x: entries outside the mesh stay zero, and x has a
+// margin of a row and a vector either side.  A half-sweep repeated on the same
+// colour changes nothing and is left out, the first one from x = 0 is folded
+// into the pass that writes b, and levels small enough are swept by as many
+// warps as have work.  A cycle of 128 x 128 cells takes 140k cycles of the SM
+// against 430k; what is left is the finest level's coefficients from the L2 (some 25
+// bytes a cycle to an SM when 96 of them read).
 constexpr int kBMgNu = 3;
 constexpr float kBMgOver = 1.3f;
 constexpr int kBMgCoarseSweeps = 16;
-// cells a thread smooths per round of loads: the pressure solve's one
-// component 4; the momentum solve's kernel has no registers to spare for
-// more than one cell at a time (0: the one-cell loop)
-constexpr int kMgPcgB = 4;
-constexpr int kMgBicgB = 0;
 
 struct BMg {
     const int *__restrict__ dims;       // [case][level][2]: nx, ny
@@ -659,13 +672,15 @@ struct BMg {
     const long long *__restrict__ cellOff;
     const int *__restrict__ faceLo;     // 2N: the face to the (y, x) lower neighbour
     float *pool;
+    int floats;                         // of shared memory for the levels
     int on;
 };
 
+// a level in box order (the construction)
 struct CL {
     int nx, ny, n;
-    size_t np;   // the stride of the components' x and b
-    float *dg, *xl, *yl, *xu, *yu, *x, *b;
+    float *dg, *xl, *yl, *xu, *yu;
+    float *split;   // the arrays of the split form
 };
 
 __device__ __forceinline__ CL case_level(const BMg &mg, int cb, int l, bool sym) {
@@ -674,42 +689,24 @@ __device__ __forceinline__ CL case_level(const BMg &mg, int cb, int l, bool sym)
     L.nx = mg.dims[2 * k];
     L.ny = mg.dims[2 * k + 1];
     L.n = L.nx * L.ny;
-    L.np = ((size_t)L.n + 3) / 4 * 4;
+    const size_t np = batch_mg_box(L.nx, L.ny);
     float *p = mg.pool + mg.off[k];
     L.dg = p;
-    L.xl = p + L.np;
-    L.yl = p + 2 * L.np;
-    L.xu = sym ? L.xl : p + 3 * L.np;
-    L.yu = sym ? L.yl : p + 4 * L.np;
-    L.x = p + 5 * L.np;
-    L.b = p + 8 * L.np;
+    L.xl = p + np;
+    L.yl = p + 2 * np;
+    L.xu = sym ? L.xl : p + 3 * np;
+    L.yu = sym ? L.yl : p + 4 * np;
+    L.split = p + 5 * np;
     return L;
 }
 
-// the couplings of box cell b = (i, j) to its four neighbours
-struct CNb {
-    float w, e, s, n;
+// a level split by colour: co [dg, -x, +x, -y, +y][colour][S], x [colour][X] (behind
+// the first margin), b [colour][S], each in shared memory or in the pool
+struct CSplit {
+    int ny, nq, st, S, X, items;   // nq vectors in a row of st entries
+    unsigned inv;                  // t / nq = umulhi(t, inv), or 0: divide
+    float *co[5], *x, *b;
 };
-
-__device__ __forceinline__ CNb cl_coeffs(const CL &L, int b, int i, int j) {
-    CNb a;
-    a.w = i > 0 ? L.xl[b] : 0.0f;
-    a.e = i + 1 < L.nx ? L.xu[b + 1] : 0.0f;
-    a.s = j > 0 ? L.yl[b] : 0.0f;
-    a.n = j + 1 < L.ny ? L.yu[b + L.nx] : 0.0f;
-    return a;
-}
-
-// sum over the four neighbours of a_nb x_nb (x: one component's array)
-__device__ __forceinline__ float cl_nb(const CL &L, const CNb &a, const float *__restrict__ x, int b, int i,
-                                       int j) {
-    float s = 0.0f;
-    if (i > 0) s += a.w * x[b - 1];
-    if (i + 1 < L.nx) s += a.e * x[b + 1];
-    if (j > 0) s += a.s * x[b - L.nx];
-    if (j + 1 < L.ny) s += a.n * x[b + L.nx];
-    return s;
-}
 
 // level 0 from the FP64 matrix, then the Galerkin coarse levels
 __device__ void case_mg_build(const BMg &mg, int cb, int N, bool sym, const double *__restrict__ diag,
@@ -783,175 +780,345 @@ __device__ void case_mg_build(const BMg &mg, int cb, int N, bool sym, const doub
     }
 }
 
-// one red-black half-sweep of a level (colour 0: i + j even), the
-// components in m; the CTA's threads walk the colour's cells only (row j
-// holds them at i = (colour + j) % 2, +2, ...)
-template <int KB>
-__device__ __forceinline__ void cl_smooth(const CL &L, int colour, unsigned m) {
-    const int hx = (L.nx + 1) >> 1, nh = hx * L.ny;
-    if constexpr (KB == 0) {   // one cell at a time (fewest registers)
-        for (int t = threadIdx.x; t < nh; t += blockDim.x) {
-            const int j = t / hx;
-            const int i = 2 * (t - j * hx) + ((colour + j) & 1);
-            if (i >= L.nx) continue;
-            const int b = i + L.nx * j;
-            const float d = L.dg[b];
-            if (d == 0.0f) continue;
-            const CNb a = cl_coeffs(L, b, i, j);
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if ((m >> k) & 1u) {
-                    float *x = L.x + k * L.np;
-                    x[b] = (L.b[k * L.np + b] - cl_nb(L, a, x, b, i, j)) / d;
-                }
-        }
-        __syncthreads();
-        return;
-    } else {
-        // KB cells a thread per round: every load of the round before its
-        // stores (the colour's cells read only the other colour's x, so no store
-        // of a round feeds a load of it), one memory latency a round instead of
-        // one a cell
-        for (int t0 = threadIdx.x; t0 < nh; t0 += KB * blockDim.x) {
-            int bb[KB];
-            float v[KB][3];
-#pragma unroll
-            for (int u = 0; u < KB; ++u) {
-                const int t = t0 + u * (int)blockDim.x;
-                bb[u] = -1;
-                if (t >= nh) continue;
-                const int j = t / hx;
-                const int i = 2 * (t - j * hx) + ((colour + j) & 1);
-                if (i >= L.nx) continue;
-                const int b = i + L.nx * j;
-                // the box arrays hold every position (zero outside the mesh), so
-                // the loads need not wait for the diagonal's test
-                const float d = L.dg[b];
-                const CNb a = cl_coeffs(L, b, i, j);
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    if ((m >> k) & 1u) {
-                        const float *x = L.x + k * L.np;
-                        v[u][k] = L.b[k * L.np + b] - cl_nb(L, a, x, b, i, j);
-                    }
-                if (d != 0.0f) {
-                    bb[u] = b;
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        if ((m >> k) & 1u) v[u][k] = v[u][k] / d;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < KB; ++u)
-                if (bb[u] >= 0)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        if ((m >> k) & 1u) L.x[k * L.np + bb[u]] = v[u][k];
-        }
-        __syncthreads();
-    }
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ int row_of(const CSplit &L, int t) {
+    return L.inv ? (int)__umulhi((unsigned)t, L.inv) : t / L.nq;
 }
 
-// w = V-cycle(r) on the case's cells for the components in m (FP32 vectors
-// in cell order, component k at k N); KB: cells a thread smooths per round
-template <class V, int KB>
-__device__ void case_mg_apply(const BMg &mg, int cb, int N, bool sym, unsigned m, const V *__restrict__ r,
-                              V *__restrict__ w) {
-    const int nL = mg.nl[cb];
+// the split levels of the case: their places, zero x and b, the coefficients
+// from the box-order arrays (all threads; ends with a barrier)
+__device__ void case_mg_split(const BMg &mg, int cb, bool sym, CSplit *lev, float *sh) {
+    const int nL = mg.nl[cb], nt = blockDim.x, tid = threadIdx.x;
+    if (tid == 0) {
+        int used = 0;
+        auto place = [&](float *&p, int n) {
+            if (n <= mg.floats - used) {
+                p = sh + used;
+                used += n;
+            }
+        };
+        auto place_rest = [&](CSplit &L) {
+            place(L.b, 2 * L.S);
+            for (int k = 0; k < 5; ++k) place(L.co[k], 2 * L.S);
+        };
+        for (int l = nL - 1; l >= 0; --l) {
+            const CL B = case_level(mg, cb, l, sym);
+            CSplit L;
+            L.ny = B.ny;
+            L.st = batch_mg_row(B.nx);
+            L.nq = L.st / 4;
+            L.S = batch_mg_entries(B.nx, B.ny);
+            L.X = batch_mg_x(B.nx, B.ny);
+            L.items = L.ny * L.nq;
+            // exact for t < items while items nq < 2^32
+            L.inv = L.nq > 1 && (unsigned long long)L.items * L.nq < (1ull << 32)
+                        ? (unsigned)((1ull << 32) / (unsigned)L.nq + 1) : 0u;
+            for (int k = 0; k < 5; ++k) L.co[k] = B.split + 2 * (size_t)k * L.S;
+            L.x = B.split + 10 * (size_t)L.S;
+            L.b = L.x + 2 * (size_t)L.X;
+            place(L.x, 2 * L.X);
+            lev[l] = L;
+        }
+        // x first: each half-sweep reads it; then the small levels' rest, which is
+        // little; then the rest of the levels of more than a vector a thread, and of
+        // those whose threads keep it in registers
+        for (int l = nL - 1; l >= 0; --l)
+            if (4 * lev[l].items <= nt) place_rest(lev[l]);
+        for (int l = 0; l < nL; ++l)
+            if (lev[l].items > nt) place_rest(lev[l]);
+        for (int l = 0; l < nL; ++l)
+            if (lev[l].items <= nt && 4 * lev[l].items > nt) place_rest(lev[l]);
+    }
+    __syncthreads();
+    for (int l = 0; l < nL; ++l) {
+        const CL B = case_level(mg, cb, l, sym);
+        const CSplit L = lev[l];
+        for (int i = tid; i < 2 * L.X; i += nt) L.x[i] = 0.0f;
+        for (int i = tid; i < 2 * L.S; i += nt) {
+            L.b[i] = 0.0f;
+            const int c = i >= L.S, t = i - c * L.S, j = t / L.st, ii = t - j * L.st;
+            const int x = 2 * ii + ((c + j) & 1);
+            float v[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            if (x < B.nx) {
+                const int b = x + B.nx * j;
+                v[0] = B.dg[b];
+                if (x > 0) v[1] = B.xl[b];
+                if (x + 1 < B.nx) v[2] = B.xu[b + 1];
+                if (j > 0) v[3] = B.yl[b];
+                if (j + 1 < B.ny) v[4] = B.yu[b + B.nx];
+            }
+#pragma unroll
+            for (int k = 0; k < 5; ++k) L.co[k][i] = v[k];
+        }
+    }
+    __syncthreads();
+    if (tid < nL) lev[tid].x += lev[tid].st + 4;   // behind the margin
+    __syncthreads();
+}
+
+// the couplings of four entries of a row to their -x, +x, -y, +y neighbours
+struct Co4 {
+    float4 w, a, s, n;
+};
+__device__ __forceinline__ Co4 ld_co(const CSplit &L, int i) {
+    return {ld4(L.co[1] + i), ld4(L.co[2] + i), ld4(L.co[3] + i), ld4(L.co[4] + i)};
+}
+// sum over the four neighbours of a_nb x_nb for the entries e .. e + 3 of a row:
+// xo the other colour, o the entries' place in their pairs
+__device__ __forceinline__ float4 cl_nb(const Co4 &q, const float *xo, int e, int st, int o) {
+    const float4 xc = ld4(xo + e), xs = ld4(xo + e - st), xn = ld4(xo + e + st);
+    const float xe = xo[o ? e + 4 : e - 1];
+    float4 v;
+    v.x = __fmaf_rn(q.w.x, o ? xc.x : xe, 0.0f);
+    v.y = __fmaf_rn(q.w.y, o ? xc.y : xc.x, 0.0f);
+    v.z = __fmaf_rn(q.w.z, o ? xc.z : xc.y, 0.0f);
+    v.w = __fmaf_rn(q.w.w, o ? xc.w : xc.z, 0.0f);
+    v.x = __fmaf_rn(q.a.x, o ? xc.y : xc.x, v.x);
+    v.y = __fmaf_rn(q.a.y, o ? xc.z : xc.y, v.y);
+    v.z = __fmaf_rn(q.a.z, o ? xc.w : xc.z, v.z);
+    v.w = __fmaf_rn(q.a.w, o ? xe : xc.w, v.w);
+    v.x = __fmaf_rn(q.n.x, xn.x, __fmaf_rn(q.s.x, xs.x, v.x));
+    v.y = __fmaf_rn(q.n.y, xn.y, __fmaf_rn(q.s.y, xs.y, v.y));
+    v.z = __fmaf_rn(q.n.z, xn.z, __fmaf_rn(q.s.z, xs.z, v.z));
+    v.w = __fmaf_rn(q.n.w, xn.w, __fmaf_rn(q.s.w, xs.w, v.w));
+    return v;
+}
+__device__ __forceinline__ float over(float a, float d) { return d != 0.0f ? a / d : 0.0f; }
+__device__ __forceinline__ float4 relaxed(const float4 &b, const float4 &s, const float4 &d) {
+    return make_float4(over(b.x - s.x, d.x), over(b.y - s.y, d.y), over(b.z - s.z, d.z), over(b.w - s.w, d.w));
+}
+__device__ __forceinline__ void st4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
+
+// n half-sweeps by turns, a black one first (colour 0, red: i + j
+// even); ends with a barrier.  Only the warps with entries take part; where a
+// thread has one vector of each colour it keeps their coefficients and b.
+__device__ void cl_sweeps(const CSplit &lev, int n) {
+    const CSplit L = lev;
+    const int na = min((int)blockDim.x, (L.items + 31) & ~31);
+    auto barrier = [&]() {
+        if (na == 32) __syncwarp();
+        else asm volatile("bar.sync 1, %0;" ::"r"(na) : "memory");
+    };
+    const int t0 = threadIdx.x;
+    if (t0 < na) {
+        if (L.items <= na) {
+            const bool in = t0 < L.items;
+            const int e = in ? 4 * t0 : 0, o = (1 + row_of(L, in ? t0 : 0)) & 1;   // o: of the black
+            const Co4 q1 = ld_co(L, L.S + e), q0 = ld_co(L, e);
+            const float4 d1 = ld4(L.co[0] + L.S + e), d0 = ld4(L.co[0] + e), b1 = ld4(L.b + L.S + e), b0 = ld4(L.b + e);
+            float *x0 = L.x, *x1 = L.x + L.X;
+            for (int h = 0; h < n; ++h) {
+                if (in) st4(x1 + e, relaxed(b1, cl_nb(q1, x0, e, L.st, o), d1));
+                barrier();
+                if (++h == n) break;
+                if (in) st4(x0 + e, relaxed(b0, cl_nb(q0, x1, e, L.st, 1 - o), d0));
+                barrier();
+            }
+        } else {
+            for (int h = 0; h < n; ++h) {
+                const int c = 1 - (h & 1);
+                const float *xo = L.x + (1 - c) * L.X;
+                float *x = L.x + c * L.X;
+#pragma unroll 2
+                for (int t = t0; t < L.items; t += na) {
+                    const int e = 4 * t, i = c * L.S + e, o = (c + row_of(L, t)) & 1;
+                    const Co4 q = ld_co(L, i);
+                    const float4 d = ld4(L.co[0] + i), b = ld4(L.b + i);
+                    st4(x + e, relaxed(b, cl_nb(q, xo, e, L.st, o), d));
+                }
+                barrier();
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// the residual b - A x summed over each aggregate into the coarse level's b, and
+// that level's first red half-sweep from x = 0 (all threads; ends with a barrier)
+__device__ void cl_restrict(const CSplit &fine, const CSplit &coarse) {
+    const CSplit F = fine, C = coarse;
+    for (int t = threadIdx.x; t < C.ny * F.nq; t += blockDim.x) {
+        const int J = row_of(F, t), m = t - J * F.nq;
+        float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int dj = 0; dj < 2; ++dj) {
+            const int j = 2 * J + dj;
+            if (j >= F.ny) break;
+            const int e = j * F.st + 4 * m;
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const int c = (o + dj) & 1;
+                const float4 d = ld4(F.co[0] + c * F.S + e), x = ld4(F.x + c * F.X + e), b = ld4(F.b + c * F.S + e);
+                const float4 v = cl_nb(ld_co(F, c * F.S + e), F.x + (1 - c) * F.X, e, F.st, o);
+                s.x += __fmaf_rn(-d.x, x.x, b.x) - v.x;
+                s.y += __fmaf_rn(-d.y, x.y, b.y) - v.y;
+                s.z += __fmaf_rn(-d.z, x.z, b.z) - v.z;
+                s.w += __fmaf_rn(-d.w, x.w, b.w) - v.w;
+            }
+        }
+        // coarse cells (4 m .. 4 m + 3, J): two of each colour
+        const int c = J & 1, e = J * C.st + 2 * m;
+        *reinterpret_cast<float2 *>(C.b + c * C.S + e) = make_float2(s.x, s.z);
+        *reinterpret_cast<float2 *>(C.b + (1 - c) * C.S + e) = make_float2(s.y, s.w);
+        const float2 d = *reinterpret_cast<const float2 *>(C.co[0] + e);
+        *reinterpret_cast<float2 *>(C.x + e) = c == 0 ? make_float2(over(s.x, d.x), over(s.z, d.y))
+                                                      : make_float2(over(s.y, d.x), over(s.w, d.y));
+    }
+    __syncthreads();
+}
+
+// x += kBMgOver x_coarse on the red cells (the black half-sweep that follows
+// overwrites the others; all threads, ends with a barrier)
+__device__ void cl_prolong(const CSplit &fine, const CSplit &coarse) {
+    const CSplit F = fine, C = coarse;
+    for (int t = threadIdx.x; t < F.items; t += blockDim.x) {
+        const int j = row_of(F, t), m = t - j * F.nq, J = j >> 1, c = J & 1, e = J * C.st + 2 * m;
+        const float4 d = ld4(F.co[0] + 4 * t);
+        const float2 a = *reinterpret_cast<const float2 *>(C.x + c * C.X + e);
+        const float2 b = *reinterpret_cast<const float2 *>(C.x + (1 - c) * C.X + e);
+        float4 x = ld4(F.x + 4 * t);
+        if (d.x != 0.0f) x.x = __fmaf_rn(kBMgOver, a.x, x.x);
+        if (d.y != 0.0f) x.y = __fmaf_rn(kBMgOver, b.x, x.y);
+        if (d.z != 0.0f) x.z = __fmaf_rn(kBMgOver, a.y, x.z);
+        if (d.w != 0.0f) x.w = __fmaf_rn(kBMgOver, b.y, x.w);
+        st4(F.x + 4 * t, x);
+    }
+    __syncthreads();
+}
+
+// w = V-cycle(r) on the case's cells (one component, cell order)
+template <class V>
+__device__ void case_mg_apply(const BMg &mg, int cb, const CSplit *lev, const V *__restrict__ r, V *__restrict__ w) {
+    const int nL = mg.nl[cb], nx = mg.dims[2 * (size_t)cb * kBatchMgLevels];
     const int *cell = mg.cell + mg.cellOff[cb];
-    {   // level 0 from x = 0: b, then the red half-sweep
-        const CL L = case_level(mg, cb, 0, sym);
-        for (int b = threadIdx.x; b < L.n; b += blockDim.x) {
-            const int c = cell[b];
-            const float d = L.dg[b];
-            const bool red = (((b % L.nx) + (b / L.nx)) & 1) == 0 && d != 0.0f;
+    const CSplit L0 = lev[0];
+    const int nt = blockDim.x;
+    // the cells of the pairs (2 ii, 2 ii + 1) of level 0's rows: kG pairs a thread at
+    // a time, their loads together
+    constexpr int kG = 4;
+    int row[kG], c0[kG], c1[kG];
+    auto pairs = [&](int t0) {
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if ((m >> k) & 1u) {
-                    const float rb = c >= 0 ? (float)r[(size_t)k * N + c] : 0.0f;
-                    L.b[k * L.np + b] = rb;
-                    L.x[k * L.np + b] = red ? rb / d : 0.0f;
-                }
+        for (int g = 0; g < kG; ++g) {
+            const int t = min(t0 + g * nt, L0.S - 1);
+            row[g] = row_of(L0, t >> 2);
+            const int i = 2 * (t - row[g] * L0.st), b = row[g] * nx + i;
+            c0[g] = i < nx ? __ldg(cell + b) : -1;
+            c1[g] = i + 1 < nx ? __ldg(cell + b + 1) : -1;
         }
-        __syncthreads();
+    };
+    // level 0 from x = 0: b, then the red half-sweep
+    for (int t0 = threadIdx.x; t0 < L0.S; t0 += kG * nt) {
+        pairs(t0);
+        float r0[kG], r1[kG], d[kG];
+#pragma unroll
+        for (int g = 0; g < kG; ++g) {
+            r0[g] = c0[g] >= 0 ? (float)r[c0[g]] : 0.0f;
+            r1[g] = c1[g] >= 0 ? (float)r[c1[g]] : 0.0f;
+            d[g] = L0.co[0][min(t0 + g * nt, L0.S - 1)];
+        }
+#pragma unroll
+        for (int g = 0; g < kG; ++g) {
+            const int t = t0 + g * nt;
+            if (t >= L0.S) break;
+            const float red = (row[g] & 1) ? r1[g] : r0[g];
+            L0.b[t] = red;
+            L0.b[L0.S + t] = (row[g] & 1) ? r0[g] : r1[g];
+            L0.x[t] = over(red, d[g]);
+        }
     }
+    __syncthreads();
     for (int l = 0; l + 1 < nL; ++l) {
-        const CL F = case_level(mg, cb, l, sym), C = case_level(mg, cb, l + 1, sym);
-        for (int nu = 0; nu < kBMgNu; ++nu) {
-            if (l > 0 || nu > 0) cl_smooth<KB>(F, 0, m);
-            cl_smooth<KB>(F, 1, m);
-        }
-        const int fx = F.nx == C.nx ? 1 : 2, fy = F.ny == C.ny ? 1 : 2;
-        for (int B = threadIdx.x; B < C.n; B += blockDim.x) {   // restriction
-            const int I = B % C.nx, J = B / C.nx;
-            float s[3] = {0.0f, 0.0f, 0.0f};
-            for (int dj = 0; dj < fy; ++dj)
-                for (int di = 0; di < fx; ++di) {
-                    const int i = I * fx + di, j = J * fy + dj;
-                    if (i >= F.nx || j >= F.ny) continue;
-                    const int b = i + F.nx * j;
-                    const float d = F.dg[b];
-                    if (d == 0.0f) continue;
-                    const CNb a = cl_coeffs(F, b, i, j);
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        if ((m >> k) & 1u) {
-                            const float *x = F.x + k * F.np;
-                            s[k] += F.b[k * F.np + b] - d * x[b] - cl_nb(F, a, x, b, i, j);
-                        }
-                }
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if ((m >> k) & 1u) {
-                    C.b[k * C.np + B] = s[k];
-                    C.x[k * C.np + B] = 0.0f;
-                }
-        }
-        __syncthreads();
+        cl_sweeps(lev[l], 2 * kBMgNu - 1);
+        cl_restrict(lev[l], lev[l + 1]);
     }
-    {   // the coarsest level: symmetric sweeps (red, black, black, red)
-        const CL L = case_level(mg, cb, nL - 1, sym);
-        if (nL == 1) {
-            for (int b = threadIdx.x; b < L.n; b += blockDim.x)
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    if ((m >> k) & 1u) L.x[k * L.np + b] = 0.0f;
-            __syncthreads();
-        }
-        for (int s = 0; s < kBMgCoarseSweeps; ++s) {
-            cl_smooth<KB>(L, 0, m);
-            cl_smooth<KB>(L, 1, m);
-            cl_smooth<KB>(L, 1, m);
-            cl_smooth<KB>(L, 0, m);
-        }
-    }
+    cl_sweeps(lev[nL - 1], 2 * kBMgCoarseSweeps);
     for (int l = nL - 2; l >= 0; --l) {
-        const CL F = case_level(mg, cb, l, sym), C = case_level(mg, cb, l + 1, sym);
-        for (int b = threadIdx.x; b < F.n; b += blockDim.x) {   // prolongation
-            if (F.dg[b] == 0.0f) continue;
-            const int i = b % F.nx, j = b / F.nx;
-            const int I = F.nx == C.nx ? i : i / 2, J = F.ny == C.ny ? j : j / 2;
+        cl_prolong(lev[l], lev[l + 1]);
+        cl_sweeps(lev[l], 2 * kBMgNu);
+    }
+    for (int t0 = threadIdx.x; t0 < L0.S; t0 += kG * nt) {   // level 0's result to w
+        pairs(t0);
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if ((m >> k) & 1u) F.x[k * F.np + b] += kBMgOver * C.x[k * C.np + I + C.nx * J];
-        }
-        __syncthreads();
-        for (int nu = 0; nu < kBMgNu; ++nu) {
-            cl_smooth<KB>(F, 1, m);
-            cl_smooth<KB>(F, 0, m);
+        for (int g = 0; g < kG; ++g) {
+            const int t = t0 + g * nt;
+            if (t >= L0.S) break;
+            const float red = L0.x[t], black = L0.x[L0.X + t];
+            if (c0[g] >= 0) w[c0[g]] = (V)((row[g] & 1) ? black : red);
+            if (c1[g] >= 0) w[c1[g]] = (V)((row[g] & 1) ? red : black);
         }
     }
-    {   // level 0's result to w (cell order)
-        const CL L = case_level(mg, cb, 0, sym);
-        for (int b = threadIdx.x; b < L.n; b += blockDim.x) {
-            const int c = cell[b];
-            if (c < 0) continue;
+    __syncthreads();
+}
+
+// psi += x, x = 0, r = b - A psi (FP64 matrix) on the case's cells of one
+// component; the thread's sum of |r|.  The loads of kR cells are issued together:
+// a row's neighbours, then their coefficients and values (one cell and one
+// neighbour at a time it was three memory latencies a neighbour, 170k cycles for
+// 16384 cells).
+constexpr int kR = 2;
+template <class V>
+__device__ double case_replace(const BEll &e, int N, int c0, int c1, const double *__restrict__ diag,
+                               const double *__restrict__ upper, const double *__restrict__ lower,
+                               const double *__restrict__ b, double *psi, V *x, V *r) {
+    const int nt = blockDim.x;
+    for (int i0 = c0 + (int)threadIdx.x; i0 < c1; i0 += 4 * nt) {
+        double p[4];
+        V xv[4];
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
-                if ((m >> k) & 1u) w[(size_t)k * N + c] = (V)L.x[k * L.np + b];
+        for (int k = 0; k < 4; ++k) {
+            const int c = min(i0 + k * nt, c1 - 1);
+            p[k] = psi[c];
+            xv[k] = x[c];
         }
-        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int c = i0 + k * nt;
+            if (c >= c1) break;
+            psi[c] = p[k] + (double)xv[k];
+            x[c] = V(0);
+        }
     }
+    __syncthreads();
+    double sum = 0.0;
+    for (int i0 = c0 + (int)threadIdx.x; i0 < c1; i0 += kR * nt) {
+        int nb[kR][kSlots], f[kR][kSlots];
+        double dg[kR], pc[kR], bc[kR], a[kR][kSlots], pn[kR][kSlots];
+#pragma unroll
+        for (int k = 0; k < kR; ++k) {
+            const int c = min(i0 + k * nt, c1 - 1);
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s) {
+                nb[k][s] = s < e.nSlots ? e.nbr[(size_t)s * N + c] : -1;
+                f[k][s] = s < e.nSlots ? e.face[(size_t)s * N + c] : 0;
+            }
+            dg[k] = diag[c];
+            pc[k] = psi[c];
+            bc[k] = b[c];
+        }
+#pragma unroll
+        for (int k = 0; k < kR; ++k) {
+            const int c = min(i0 + k * nt, c1 - 1);
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s) {
+                a[k][s] = nb[k][s] >= 0 ? (nb[k][s] > c ? upper : lower)[f[k][s]] : 0.0;
+                pn[k][s] = nb[k][s] >= 0 ? psi[nb[k][s]] : 0.0;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kR; ++k) {
+            const int c = i0 + k * nt;
+            if (c >= c1) break;
+            double acc = dg[k] * pc[k];
+#pragma unroll
+            for (int s = 0; s < kSlots; ++s)
+                if (nb[k][s] >= 0) acc = fma(a[k][s], pn[k][s], acc);
+            const double rr = bc[k] - acc;
+            r[c] = (V)rr;
+            sum += fabs(rr);
+        }
+    }
+    return sum;
 }
 
 // ---- the persistent per-case PCG -------------------------------------------
@@ -973,6 +1140,8 @@ template <class V>
 constexpr int kBicgP = sizeof(V) == 4 ? 8 : 4;
 template <class V>
 constexpr int kBicgNB = sizeof(V) == 4 ? 3 : 2;
+template <class V>
+constexpr int kRingBytes = s2d::kRJ * s2d::W<V>::n * (int)sizeof(s2d::u64);   // of a j-block
 template <class V, int NC, int P, int NB>
 __host__ __device__ constexpr int case_stage_bytes() {   // one warp's staging area, the larger of the two sweeps
     return s2d::stage_bytes<V, 0, NC, P, NB>() > s2d::stage_bytes<V, 1, NC, P, NB>()
@@ -981,7 +1150,6 @@ __host__ __device__ constexpr int case_stage_bytes() {   // one warp's staging a
 }
 constexpr int kU = 4;                            // cells per thread whose loads are issued together
 constexpr int kUA = 4;                           // the same for q = A p
-constexpr int kSlots = 4;                        // ELL width of the 2-D cases
 
 // 16-byte packs of a vector: four FP32 or two FP64 values, one load or store
 template <class V> struct Pack;
@@ -1060,21 +1228,27 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_pcg_case(BTab t, BEll e, 
                                                               V *__restrict__ aEll, BMg mg, int *err,
                                                               long long maxSpin, int cap) {
     using Acc = typename AccOf<V>::type;
-    __shared__ s2d::u64 ring[8 * s2d::kRJ * s2d::W<V>::n];
     __shared__ int sProg[32];
-    extern __shared__ __align__(16) unsigned char stageSmem[];   // 8 warps' sweep staging
+    __shared__ CSplit lev[kBatchMgLevels];
+    // the multigrid levels, or the sweeps' j-block ring and 8 warps' staging
+    extern __shared__ __align__(16) unsigned char smem[];
+    s2d::u64 *ring = reinterpret_cast<s2d::u64 *>(smem);
+    unsigned char *stageSmem = smem + 8 * kRingBytes<V>;
     const int cb = order[blockIdx.x], sg = cb * 8, tid = threadIdx.x, nt = blockDim.x, N = t.N;
     const int c0 = t.blkCell0[t.caseBlk[cb]], c1 = t.blkCell1[t.caseBlk[cb + 1] - 1];
     const long long e0 = g.off[cb], e1 = e0 + (long long)g.JB[cb] * g.T[cb] * 32;
     case_ell_coefficients(e, N, c0, c1, u32, l32, aEll);
     // the FP32 form may take the multigrid V-cycle in place of the DIC sweeps
     const bool useMg = sizeof(V) == 4 && mg.on;
-    if (useMg) case_mg_build(mg, cb, N, true, diag, upper, lower);
+    if (useMg) {
+        case_mg_build(mg, cb, N, true, diag, upper, lower);
+        case_mg_split(mg, cb, true, lev, reinterpret_cast<float *>(smem));
+    }
     for (int it = 0; it < cap; ++it) {
         __syncthreads();
         if (!S.active[sg]) break;
         if (useMg) {
-            case_mg_apply<V, kMgPcgB>(mg, cb, N, true, 1u, r, w);
+            case_mg_apply<V>(mg, cb, lev, r, w);
         } else {
         // ---- w = M^-1 r: gather, forward and backward sweeps of this case
         for (long long i0 = e0 + tid; i0 < e1; i0 += (long long)kU * nt) {
@@ -1263,18 +1437,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_pcg_case(BTab t, BEll e, 
         __syncthreads();
         // ---- residual replacement (mixed): psi += x, x = 0, r = b - A psi
         if (S.repl[sg]) {
-            for (int c = c0 + tid; c < c1; c += nt) {
-                psi[c] += (double)x[c];
-                x[c] = V(0);
-            }
-            __syncthreads();
-            double vt = 0.0;
-            for (int c = c0 + tid; c < c1; c += nt) {
-                const double rr = b[c] - brow_mul(e, c, diag, upper, lower, psi);
-                r[c] = (V)rr;
-                vt += fabs(rr);
-            }
-            const double rt = case_total(vt);
+            const double rt = case_total(case_replace<V>(e, N, c0, c1, diag, upper, lower, b, psi, x, r));
             if (tid == 0 && S.active[sg]) {   // k_b_after
                 const double fin = rt / S.nf[sg];
                 S.fin[sg] = fin;
@@ -1446,8 +1609,12 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
                                                               long long maxSpin, int cap) {
     using Acc = typename AccOf<V>::type;
     constexpr int PN = Pack<V>::n;
-    __shared__ s2d::u64 ring[16 * s2d::kRJ * s2d::W<V>::n];   // two halves of the CTA, 8 j-blocks each
-    extern __shared__ __align__(16) unsigned char stageSmem[];   // 16 warps' sweep staging
+    __shared__ CSplit lev[kBatchMgLevels];
+    // the multigrid levels, or the sweeps' rings (two halves of the CTA, 8 j-blocks
+    // each) and 16 warps' staging
+    extern __shared__ __align__(16) unsigned char smem[];
+    s2d::u64 *ring = reinterpret_cast<s2d::u64 *>(smem);
+    unsigned char *stageSmem = smem + 16 * kRingBytes<V>;
     __shared__ int sProg[32];
     // segment masks that thread 0 publishes, one slot per use, so that no
     // slot is rewritten in an iteration after threads have read it without a
@@ -1460,7 +1627,14 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
     case_ell_coefficients(e, N, c0, c1, u32, l32, aEll);
     // the FP32 form may take the multigrid V-cycle in place of the DILU sweeps
     const bool useMg = sizeof(V) == 4 && mg.on;
-    if (useMg) case_mg_build(mg, cb, N, false, diag, upper, lower);
+    if (useMg) {
+        case_mg_build(mg, cb, N, false, diag, upper, lower);
+        case_mg_split(mg, cb, false, lev, reinterpret_cast<float *>(smem));
+    }
+    auto vcycles = [&](const V *in, V *out) {
+        for (int k = 0; k < 3; ++k)
+            if ((vm >> k) & 1u) case_mg_apply<V>(mg, cb, lev, in + (size_t)k * N, out + (size_t)k * N);
+    };
     // the segments (components) selected by a predicate on their state
     auto seg_mask = [&](auto pred) {
         unsigned mm = 0;
@@ -1474,25 +1648,11 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
 #pragma unroll
         for (int k = 0; k < 3; ++k) tot[k] = 0.0;
         if (!mr) return;
-#pragma unroll 4
-        for (int c = c0 + tid; c < c1; c += nt)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (!((mr >> k) & 1u)) continue;
-                const size_t i = (size_t)k * N + c;
-                psi[i] += (double)x[i];
-                x[i] = V(0);
-            }
-        __syncthreads();
-#pragma unroll 4
-        for (int c = c0 + tid; c < c1; c += nt)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                if (!((mr >> k) & 1u)) continue;
+        for (int k = 0; k < 3; ++k)
+            if ((mr >> k) & 1u) {
                 const size_t o = (size_t)k * N;
-                const double rr = b[o + c] - brow_mul(e, c, diag, upper, lower, psi + o);
-                r[o + c] = (V)rr;
-                tot[k] += fabs(rr);
+                tot[k] = case_replace<V>(e, N, c0, c1, diag, upper, lower, b + o, psi + o, x + o, r + o);
             }
         case_totals(tot);
     };
@@ -1563,7 +1723,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
         __syncthreads();
         // ---- y = M^-1 p, Ay = A y, alpha = r0r / r0.Ay
         if (useMg) {
-            case_mg_apply<V, kMgBicgB>(mg, cb, N, false, vm, p, y);
+            vcycles(p, y);
         } else {
             case_precondition(g, cb, N, vm, p, y, err, maxSpin, ring, sProg, stageSmem);
             if (case_error(err)) break;
@@ -1685,7 +1845,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
         const unsigned full = sMask[3];
         // ---- z = M^-1 s, tt = A z, omega = tt.s / tt.tt
         if (useMg) {
-            case_mg_apply<V, kMgBicgB>(mg, cb, N, false, vm, sv, z);
+            vcycles(sv, z);
         } else {
             case_precondition(g, cb, N, vm, sv, z, err, maxSpin, ring, sProg, stageSmem);
             if (case_error(err)) break;
@@ -2010,6 +2170,16 @@ struct BSolver {
     }
 };
 
+// the dynamic shared memory a block of this kernel may have beside its static
+int block_smem_left(const void *kernel) {
+    int dev = 0, most = 0;
+    cudaFuncAttributes at{};
+    RT_CUDA(cudaGetDevice(&dev));
+    RT_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    RT_CUDA(cudaFuncGetAttributes(&at, kernel));
+    return (most - (int)at.sharedSizeBytes) / 16 * 16;
+}
+
 // iterations between two polls of the active count
 constexpr int kPoll = 4;
 
@@ -2047,10 +2217,14 @@ rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
         else g = sweep2d_view64(ctx);
         {
             // the multigrid V-cycle for the FP32 form (RT_OPT_MIXED_PRECOND -2, DIC)
-            BMg bmg{bt.mgDims.p, bt.mgNL.p, bt.mgOff.p, bt.mgCell.p, bt.mgCellOff.p, bt.sFaceLo.p, bt.mgPool.p,
+            BMg bmg{bt.mgDims.p, bt.mgNL.p, bt.mgOff.p, bt.mgCell.p, bt.mgCellOff.p, bt.sFaceLo.p, bt.mgPool.p, 0,
                     (sizeof(V) == 4 && ctx->mixedJacobi == -2 && pre == RT_PRECOND_DIC && bt.mgPool.p) ? 1 : 0};
             ProfScope ps(ctx, "batch_pcg_persistent");
-            const int shm = 8 * case_stage_bytes<V, 1, kCaseP<V>, kCaseNB>();
+            int shm = 8 * kRingBytes<V> + 8 * case_stage_bytes<V, 1, kCaseP<V>, kCaseNB>();
+            if (bmg.on) {   // all that a block may have goes to the levels
+                shm = block_smem_left((const void *)k_b_pcg_case<V>);
+                bmg.floats = shm / (int)sizeof(float);
+            }
             RT_CUDA(cudaFuncSetAttribute(k_b_pcg_case<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
             k_b_pcg_case<V><<<bt.n, kCaseThreads, shm, sv.st>>>(sv.t, sv.e, g, sv.S, sv.ctl, sv.mixed, sv.d32, sv.u32,
                                                               sv.l32, a.diag, a.upper, a.lower, a.source, a.psi, r,
@@ -2070,10 +2244,14 @@ rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
         else g = sweep2d_view64(ctx);
         {
             // the multigrid V-cycle for the FP32 form (RT_OPT_MIXED_PRECOND_U -2, DILU)
-            BMg bmg{bt.mgDims.p, bt.mgNL.p, bt.mgOff.p, bt.mgCell.p, bt.mgCellOff.p, bt.sFaceLo.p, bt.mgPool.p,
+            BMg bmg{bt.mgDims.p, bt.mgNL.p, bt.mgOff.p, bt.mgCell.p, bt.mgCellOff.p, bt.sFaceLo.p, bt.mgPool.p, 0,
                     (sizeof(V) == 4 && ctx->mixedPrecondU == -2 && pre == RT_PRECOND_DILU && bt.mgPool.p) ? 1 : 0};
             ProfScope ps(ctx, "batch_bicgstab_persistent");
-            const int shm = 16 * case_stage_bytes<V, 1, kBicgP<V>, kBicgNB<V>>();
+            int shm = 16 * kRingBytes<V> + 16 * case_stage_bytes<V, 1, kBicgP<V>, kBicgNB<V>>();
+            if (bmg.on) {   // all that a block may have goes to the levels
+                shm = block_smem_left((const void *)k_b_bicg_case<V>);
+                bmg.floats = shm / (int)sizeof(float);
+            }
             RT_CUDA(cudaFuncSetAttribute(k_b_bicg_case<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
             k_b_bicg_case<V><<<bt.n, kCaseThreads, shm, sv.st>>>(
                 sv.t, sv.e, g, sv.S, sv.ctl, sv.vm, sv.mixed, sv.d32, sv.u32, sv.l32, a.diag, a.upper, a.lower,

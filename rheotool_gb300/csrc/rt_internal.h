@@ -215,7 +215,16 @@ struct StructMesh {
 // ---------------------------------------------------------------------------
 constexpr int kBatchMgLevels = 8;     // levels of a batched case's multigrid hierarchy, at most
 constexpr int kBatchMgCoarse = 64;    // cells of its coarsest level, at most
-constexpr int kBatchMgArrays = 11;   // arrays of a level: dg, xl, yl, xu, yu, x[3], b[3]
+// a level of nx x ny cells in the pool: dg, xl, yl, xu, yu in box order, then its
+// colour-split form (two colours of rows padded to whole 16-byte vectors): five
+// coefficients, x with a margin of a row and a vector either side, b
+__host__ __device__ inline long long batch_mg_box(int nx, int ny) { return ((long long)nx * ny + 3) / 4 * 4; }
+__host__ __device__ inline int batch_mg_row(int nx) { return ((nx + 1) / 2 + 3) / 4 * 4; }
+__host__ __device__ inline int batch_mg_entries(int nx, int ny) { return batch_mg_row(nx) * ny; }
+__host__ __device__ inline int batch_mg_x(int nx, int ny) { return batch_mg_entries(nx, ny) + 2 * batch_mg_row(nx) + 8; }
+__host__ __device__ inline long long batch_mg_floats(int nx, int ny) {
+    return 5 * batch_mg_box(nx, ny) + 12ll * batch_mg_entries(nx, ny) + 2ll * batch_mg_x(nx, ny);
+}
 
 struct Batch {
     int n = 1;
@@ -246,7 +255,7 @@ struct Batch {
     // structured 2-D cases: each case's multigrid hierarchy (the mixed
     // pressure and momentum solves of the persistent solvers, one at a time):
     // per case and level the box (nx, ny) and its arrays' offset in mgPool
-    // (kBatchMgArrays of them, each padded to 4), the level count, and level
+    // (batch_mg_floats of them), the level count, and level
     // 0's cell of each box position
     DBuf<int> mgDims, mgNL, mgCell;
     DBuf<long long> mgOff, mgCellOff;
