@@ -2180,8 +2180,12 @@ int block_smem_left(const void *kernel) {
     return (most - (int)at.sharedSizeBytes) / 16 * 16;
 }
 
-// iterations between two polls of the active count
-constexpr int kPoll = 4;
+// iterations launched one by one, with a poll of the active count after each,
+// before the rest is captured, and iterations between two polls from then on: the
+// constitutive solves end after one to three, and a replay of four past their end
+// with the capture before it was 2.0 of the 5.1 ms they took (96 cavities of 32^2 to
+// 128^2), while a poll is some 15 us
+constexpr int kEager = 3, kPoll = 4;
 
 template <class V>
 rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
@@ -2263,12 +2267,12 @@ rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
         bt.sPending = true;
         active = 0;
     }
-    if (active) {
-        body();   // first iteration eagerly (sets kernel attributes outside any capture)
+    while (active && done < std::min(kEager, cap)) {
+        body();   // (the first one sets kernel attributes outside any capture)
         ++done;
         active = sv.poll();
     }
-    if (active) {
+    if (active && done < cap) {
         RT_CUDA(cudaStreamBeginCapture(sv.st, cudaStreamCaptureModeThreadLocal));
         try {
             body();
