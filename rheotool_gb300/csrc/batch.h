@@ -41,8 +41,8 @@ rt_status batch_solve(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf);
 
 // sweep2d.cu: rD of one matrix, then FP32 (or FP64) applications
 void sweep2d_prepare(rt_ctx *ctx, const double *diag, const double *upper, const double *lower, bool fp32);
-void sweep2d_precondition(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w);
-void sweep2d_precondition(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w);
+void sweep2d_precondition(rt_ctx *ctx, unsigned mask, const float *r, float *w);
+void sweep2d_precondition(rt_ctx *ctx, unsigned mask, const double *r, double *w);
 rt_status sweep2d_check(rt_ctx *ctx);
 // the skewed layout of the batch (for the per-case persistent solver)
 Skew2D<float> sweep2d_view32(rt_ctx *ctx);

@@ -1142,11 +1142,11 @@ template <class V>
 constexpr int kBicgNB = sizeof(V) == 4 ? 3 : 2;
 template <class V>
 constexpr int kRingBytes = s2d::kRJ * s2d::W<V>::n * (int)sizeof(s2d::u64);   // of a j-block
-template <class V, int NC, int P, int NB>
+template <class V, int P, int NB>
 __host__ __device__ constexpr int case_stage_bytes() {   // one warp's staging area, the larger of the two sweeps
-    return s2d::stage_bytes<V, 0, NC, P, NB>() > s2d::stage_bytes<V, 1, NC, P, NB>()
-               ? s2d::stage_bytes<V, 0, NC, P, NB>()
-               : s2d::stage_bytes<V, 1, NC, P, NB>();
+    return s2d::stage_bytes<V, 0, P, NB>() > s2d::stage_bytes<V, 1, P, NB>()
+               ? s2d::stage_bytes<V, 0, P, NB>()
+               : s2d::stage_bytes<V, 1, P, NB>();
 }
 constexpr int kU = 4;                            // cells per thread whose loads are issued together
 constexpr int kUA = 4;                           // the same for q = A p
@@ -1266,13 +1266,13 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_pcg_case(BTab t, BEll e, 
                 if (i0 + (long long)k * nt < e1) g.rS[i0 + (long long)k * nt] = v[k];
         }
         for (int mode = 0; mode < 2; ++mode) {
-            s2d::reset<V, 1>(ring, 8, sProg);
+            s2d::reset<V>(ring, 8, sProg);
             __syncthreads();
             if (mode == 0)
-                sweep2d_cta<V, 0, 1, kCaseP<V>, true, s2d::kRJ, kCaseNB>(g, cb, 1u, nullptr, N, err, maxSpin, ring,
+                sweep2d_cta<V, 0, kCaseP<V>, true, s2d::kRJ, kCaseNB>(g, cb, nullptr, err, maxSpin, ring,
                                                                          sProg, 0, stageSmem);
             else
-                sweep2d_cta<V, 1, 1, kCaseP<V>, true, s2d::kRJ, kCaseNB>(g, cb, 1u, w, N, err, maxSpin, ring, sProg,
+                sweep2d_cta<V, 1, kCaseP<V>, true, s2d::kRJ, kCaseNB>(g, cb, w, err, maxSpin, ring, sProg,
                                                                          0, stageSmem);
             __syncthreads();
         }
@@ -1575,16 +1575,16 @@ __device__ void case_precondition(const Skew2D<V> &g, int cb, int N, unsigned m,
             gk.wS += (long long)k * g.nSkew;
         }
         for (int mode = 0; mode < 2; ++mode) {
-            s2d::reset<V, 1>(ring, 16, sProg);
+            s2d::reset<V>(ring, 16, sProg);
             __syncthreads();
             if (k >= 0) {
                 s2d::u64 *rg = ring + grp * 8 * s2d::kRJ * s2d::W<V>::n;
-                unsigned char *sg = stage + (size_t)grp * 8 * case_stage_bytes<V, 1, kBicgP<V>, kBicgNB<V>>();
+                unsigned char *sg = stage + (size_t)grp * 8 * case_stage_bytes<V, kBicgP<V>, kBicgNB<V>>();
                 if (mode == 0)
-                    sweep2d_cta<V, 0, 1, kBicgP<V>, true, s2d::kRJ, kBicgNB<V>>(gk, cb, 1u, nullptr, N, err, maxSpin, rg,
+                    sweep2d_cta<V, 0, kBicgP<V>, true, s2d::kRJ, kBicgNB<V>>(gk, cb, nullptr, err, maxSpin, rg,
                                                                              sProg + 8 * grp, 8 * grp, sg);
                 else
-                    sweep2d_cta<V, 1, 1, kBicgP<V>, true, s2d::kRJ, kBicgNB<V>>(gk, cb, 1u, w + (size_t)k * N, N, err,
+                    sweep2d_cta<V, 1, kBicgP<V>, true, s2d::kRJ, kBicgNB<V>>(gk, cb, w + (size_t)k * N, err,
                                                                              maxSpin, rg, sProg + 8 * grp, 8 * grp, sg);
             }
             __syncthreads();
@@ -2059,7 +2059,7 @@ struct BSolver {
             k_b_copy<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, r, w, pre == RT_PRECOND_DIAGONAL ? rD : nullptr);
             launch_count(ctx);
         } else if (bt.sweep2d) {
-            sweep2d_precondition(ctx, a.nc, vm, r, w);
+            sweep2d_precondition(ctx, vm, r, w);
         } else {
             const DevMesh &m = ctx->mesh;
             for (int l = 0; l < m.nLevels; ++l) {
@@ -2224,7 +2224,7 @@ rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
             BMg bmg{bt.mgDims.p, bt.mgNL.p, bt.mgOff.p, bt.mgCell.p, bt.mgCellOff.p, bt.sFaceLo.p, bt.mgPool.p, 0,
                     (sizeof(V) == 4 && ctx->mixedJacobi == -2 && pre == RT_PRECOND_DIC && bt.mgPool.p) ? 1 : 0};
             ProfScope ps(ctx, "batch_pcg_persistent");
-            int shm = 8 * kRingBytes<V> + 8 * case_stage_bytes<V, 1, kCaseP<V>, kCaseNB>();
+            int shm = 8 * kRingBytes<V> + 8 * case_stage_bytes<V, kCaseP<V>, kCaseNB>();
             if (bmg.on) {   // all that a block may have goes to the levels
                 shm = block_smem_left((const void *)k_b_pcg_case<V>);
                 bmg.floats = shm / (int)sizeof(float);
@@ -2251,7 +2251,7 @@ rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
             BMg bmg{bt.mgDims.p, bt.mgNL.p, bt.mgOff.p, bt.mgCell.p, bt.mgCellOff.p, bt.sFaceLo.p, bt.mgPool.p, 0,
                     (sizeof(V) == 4 && ctx->mixedPrecondU == -2 && pre == RT_PRECOND_DILU && bt.mgPool.p) ? 1 : 0};
             ProfScope ps(ctx, "batch_bicgstab_persistent");
-            int shm = 16 * kRingBytes<V> + 16 * case_stage_bytes<V, 1, kBicgP<V>, kBicgNB<V>>();
+            int shm = 16 * kRingBytes<V> + 16 * case_stage_bytes<V, kBicgP<V>, kBicgNB<V>>();
             if (bmg.on) {   // all that a block may have goes to the levels
                 shm = block_smem_left((const void *)k_b_bicg_case<V>);
                 bmg.floats = shm / (int)sizeof(float);

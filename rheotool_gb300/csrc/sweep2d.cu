@@ -20,6 +20,8 @@
 // independent, so the CTAs of a launch never wait on one another.  Every wait
 // is bounded: a timeout sets the error flag, every other wait gives up on
 // seeing it, and the host reports RT_ETIMEOUT.
+#include <algorithm>
+
 #include "batch.h"
 #include "real_ops.cuh"
 #include "sweep2d_cta.cuh"
@@ -33,27 +35,60 @@ namespace {
 // memory)
 template <int MAXT>
 __host__ __device__ constexpr int ring2d() { return MAXT <= 256 ? s2d::kRJ : 64; }
-template <class Real, int MODE, int NC, int P, int MAXT>
-__global__ void __launch_bounds__(MAXT) k_sweep2d(Skew2D<Real> g, const int *__restrict__ order, unsigned mask,
-                                                  Real *__restrict__ w, int N, int *err, long long maxSpin) {
+
+// the rD recurrence of a case
+template <int P, int MAXT>
+__global__ void __launch_bounds__(MAXT) k_rd2d(Skew2D<double> g, const int *__restrict__ order, int *err,
+                                               long long maxSpin) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int sProg[32];
     constexpr int RJ = ring2d<MAXT>();
     s2d::u64 *ring = reinterpret_cast<s2d::u64 *>(smem_raw);
     const int cb = order[blockIdx.x];
-    s2d::reset<Real, NC, RJ>(ring, g.JB[cb], sProg);
+    s2d::reset<double, RJ>(ring, g.JB[cb], sProg);
     __syncthreads();
-    sweep2d_cta<Real, MODE, NC, P, (MAXT <= 256), RJ>(g, cb, mask, w, N, err, maxSpin, ring, sProg);
+    sweep2d_cta<double, 2, P, (MAXT <= 256), RJ>(g, cb, nullptr, err, maxSpin, ring, sProg);
+}
+
+// w = M^-1 r of one component of a case, r in the skewed layout: the forward and
+// the backward sweep.
+//
+// What bounds it: the chain of steps, so the components run side by side, a CTA
+// each, no launch stands between the two sweeps, and up to 8 j-blocks stage their
+// chunks three ahead in shared memory (one ahead in registers a chunk took the
+// latency of the L2, not its steps; three components in the lanes of one CTA made
+// a step 520 cycles).
+template <class Real, int P, int MAXT, int NB>
+__global__ void __launch_bounds__(MAXT) k_apply2d(Skew2D<Real> g, const int *__restrict__ order, unsigned mask, int ncc,
+                                                  Real *__restrict__ w, int N, int *err, long long maxSpin) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int sProg[32];
+    constexpr int RJ = ring2d<MAXT>();
+    s2d::u64 *ring = reinterpret_cast<s2d::u64 *>(smem_raw);
+    unsigned char *stage = smem_raw + (size_t)g.maxJB * RJ * s2d::W<Real>::n * sizeof(s2d::u64);
+    const int cb = order[blockIdx.x / ncc];
+    for (int q = blockIdx.x % ncc; q > 0; --q) mask &= mask - 1;
+    const int k = __ffs(mask) - 1;
+    g.rS += (long long)k * g.nSkew;
+    g.wS += (long long)k * g.nSkew;
+    w += (size_t)k * N;
+    s2d::reset<Real, RJ>(ring, g.JB[cb], sProg);
+    __syncthreads();
+    sweep2d_cta<Real, 0, P, false, RJ, NB>(g, cb, nullptr, err, maxSpin, ring, sProg, 0, stage);
+    __syncthreads();
+    s2d::reset<Real, RJ>(ring, g.JB[cb], sProg);
+    __syncthreads();
+    sweep2d_cta<Real, 1, P, false, RJ, NB>(g, cb, w, err, maxSpin, ring, sProg, 0, stage);
 }
 
 }  // namespace
 
 template <class Real>
-__global__ void k_s2_gather(Skew2D<Real> g, unsigned mask, int nc, const Real *__restrict__ r, int N) {
+__global__ void k_s2_gather(Skew2D<Real> g, unsigned mask, const Real *__restrict__ r, int N) {
     long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (e >= g.nSkew) return;
     int c = g.cellOf[e];
-    for (int q = 0; q < nc; ++q)
+    for (int q = 0; q < 6; ++q)
         if ((mask >> q) & 1u) g.rS[(long long)q * g.nSkew + e] = c >= 0 ? r[(long long)q * N + c] : Real(0);
 }
 
@@ -135,46 +170,38 @@ Skew2D<float> view2d<float>(Batch &b) {
     return g;
 }
 
-template <class Real, int MODE, int NC, int P, int MAXT>
-void launch2d_t(rt_ctx *ctx, const Skew2D<Real> &g, unsigned mask, Real *w) {
+// one CTA a case (and component), a warp a j-block
+template <class Real, int MAXT, class... P, class... A>
+void launch2d(rt_ctx *ctx, void (*kernel)(P...), int perCase, int stage, A... args) {
     Batch &b = ctx->mesh.batch;
-    const size_t shm = (size_t)b.maxJB * ring2d<MAXT>() * NC * s2d::W<Real>::n * sizeof(s2d::u64);
-    static size_t attr = 0;   // the dynamic shared memory this kernel was opened to
-    if (shm > attr && shm + 1024 > 48 * 1024) {   // (beside its static counters)
-        RT_CUDA(cudaFuncSetAttribute(k_sweep2d<Real, MODE, NC, P, MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)shm));
-        attr = shm;
-    }
-    k_sweep2d<Real, MODE, NC, P, MAXT><<<b.n, 32 * b.maxJB, shm, ctx->stream>>>(g, b.caseOrder.p, mask, w,
-                                                                                ctx->mesh.N, b.sErr.p, 1ll << 22);
+    const int shm = b.maxJB * (ring2d<MAXT>() * s2d::W<Real>::n * (int)sizeof(s2d::u64) + stage);
+    if (shm + 1024 > 48 * 1024)   // (beside its static counters)
+        RT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
+    kernel<<<b.n * perCase, 32 * b.maxJB, shm, ctx->stream>>>(args...);
     RT_CHECK_LAUNCH();
-}
-
-template <class Real, int MODE, int NC, int P>
-void launch2d(rt_ctx *ctx, const Skew2D<Real> &g, unsigned mask, Real *w) {
-    Batch &b = ctx->mesh.batch;
-    if (b.maxJB <= 8) launch2d_t<Real, MODE, NC, P, 256>(ctx, g, mask, w);
-    else launch2d_t<Real, MODE, NC, P, 1024>(ctx, g, mask, w);
     launch_count(ctx);
     b.sPending = true;
 }
 
-template <class Real, int MODE>
-void launch2d_nc(rt_ctx *ctx, const Skew2D<Real> &g, int nc, unsigned mask, Real *w) {
-    if (nc == 1) launch2d<Real, MODE, 1, 8>(ctx, g, mask, w);
-    else if (nc <= 3) launch2d<Real, MODE, 3, 4>(ctx, g, mask, w);
-    else launch2d<Real, MODE, 6, 2>(ctx, g, mask, w);
-}
+constexpr int kP = 8;   // steps of a chunk
+constexpr long long kMaxSpin = 1ll << 22;
 
 template <class Real>
-void precondition2d(rt_ctx *ctx, int nc, unsigned mask, const Real *r, Real *w) {
+void precondition2d(rt_ctx *ctx, unsigned mask, const Real *r, Real *w) {
+    if (!mask) return;
     Batch &b = ctx->mesh.batch;
-    Skew2D<Real> g = view2d<Real>(b);
-    k_s2_gather<Real><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, nc, r, ctx->mesh.N);
+    const Skew2D<Real> g = view2d<Real>(b);
+    const int ncc = __builtin_popcount(mask), N = ctx->mesh.N;
+    k_s2_gather<Real><<<nblocks(g.nSkew), RT_BLOCK, 0, ctx->stream>>>(g, mask, r, N);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
-    launch2d_nc<Real, 0>(ctx, g, nc, mask, w);
-    launch2d_nc<Real, 1>(ctx, g, nc, mask, w);
+    const int *order = b.caseOrder.p;
+    constexpr int PS = sizeof(Real) == 4 ? 8 : 4, NB = 4;
+    constexpr int stage = std::max(s2d::stage_bytes<Real, 0, PS, NB>(), s2d::stage_bytes<Real, 1, PS, NB>());
+    if (b.maxJB <= 8)
+        launch2d<Real, 256>(ctx, k_apply2d<Real, PS, 256, NB>, ncc, stage, g, order, mask, ncc, w, N, b.sErr.p, kMaxSpin);
+    else
+        launch2d<Real, 1024>(ctx, k_apply2d<Real, kP, 1024, 0>, ncc, 0, g, order, mask, ncc, w, N, b.sErr.p, kMaxSpin);
 }
 
 }  // namespace
@@ -189,7 +216,9 @@ void sweep2d_prepare(rt_ctx *ctx, const double *diag, const double *upper, const
     const int N = ctx->mesh.N;
     k_s2_setup<<<nb, RT_BLOCK, 0, ctx->stream>>>(g, b.sFaceLo.p, N, diag, upper, lower);
     RT_CHECK_LAUNCH();
-    launch2d<double, 2, 1, 8>(ctx, g, 1u, (double *)nullptr);
+    const int *order = b.caseOrder.p;
+    if (b.maxJB <= 8) launch2d<double, 256>(ctx, k_rd2d<kP, 256>, 1, 0, g, order, b.sErr.p, kMaxSpin);
+    else launch2d<double, 1024>(ctx, k_rd2d<kP, 1024>, 1, 0, g, order, b.sErr.p, kMaxSpin);
     k_s2_premul<<<nb, RT_BLOCK, 0, ctx->stream>>>(g, b.sFaceLo.p, b.sFaceHi.p, N, upper, lower);
     RT_CHECK_LAUNCH();
     launch_count(ctx, 2);
@@ -201,11 +230,11 @@ void sweep2d_prepare(rt_ctx *ctx, const double *diag, const double *upper, const
     }
 }
 
-void sweep2d_precondition(rt_ctx *ctx, int nc, unsigned mask, const float *r, float *w) {
-    precondition2d<float>(ctx, nc, mask, r, w);
+void sweep2d_precondition(rt_ctx *ctx, unsigned mask, const float *r, float *w) {
+    precondition2d<float>(ctx, mask, r, w);
 }
-void sweep2d_precondition(rt_ctx *ctx, int nc, unsigned mask, const double *r, double *w) {
-    precondition2d<double>(ctx, nc, mask, r, w);
+void sweep2d_precondition(rt_ctx *ctx, unsigned mask, const double *r, double *w) {
+    precondition2d<double>(ctx, mask, r, w);
 }
 
 rt_status sweep2d_check(rt_ctx *ctx) {

@@ -70,21 +70,21 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// the arrays of a staged chunk: MODE 0 rDinv, Ay, Ax, rS (NC); MODE 1 By,
-// Bx, wS (NC) and the cells; MODE 2 D, Py, Px
-template <int MODE, int NC> struct StageArrays { static constexpr int n = (MODE == 2) ? 3 : (MODE == 0 ? 3 : 2) + NC; };
+// the arrays of a staged chunk: MODE 0 rDinv, Ay, Ax, rS; MODE 1 By, Bx, wS and
+// the cells; MODE 2 D, Py, Px
+template <int MODE> struct StageArrays { static constexpr int n = MODE == 0 ? 4 : 3; };
 
 // bytes of one warp's NB staging buffers
-template <class Real, int MODE, int NC, int P, int NB>
+template <class Real, int MODE, int P, int NB>
 __host__ __device__ constexpr int stage_bytes() {
-    return NB * P * 32 * (StageArrays<MODE, NC>::n * (int)sizeof(Real) + (MODE == 1 ? 4 : 0));
+    return NB * P * 32 * (StageArrays<MODE>::n * (int)sizeof(Real) + (MODE == 1 ? 4 : 0));
 }
 
 // clears the rings and counters of a sweep (all threads of the CTA, before
 // the barrier that precedes the sweep): the tags of a sweep start from 1
-template <class Real, int NC, int RJ = kRJ>
+template <class Real, int RJ = kRJ>
 __device__ __forceinline__ void reset(u64 *ring, int nJB, int *sProg) {
-    const int n = nJB * RJ * NC * W<Real>::n;
+    const int n = nJB * RJ * W<Real>::n;
     for (int i = threadIdx.x; i < n; i += blockDim.x) ring[i] = 0ull;
     if (threadIdx.x < 32) sProg[threadIdx.x] = 0;
 }
@@ -92,19 +92,19 @@ __device__ __forceinline__ void reset(u64 *ring, int nJB, int *sProg) {
 }  // namespace s2d
 
 // the coefficients and inputs of one chunk of P steps of a lane
-template <class Real, int NC, int P>
+template <class Real, int P>
 struct S2Chunk {
     Real c0[P], cy[P], cx[P];
-    Real rk[P][NC];
+    Real rk[P];
     int cell[P];
 };
 
 // loads of the chunk starting at step t0 (independent of the recurrence):
 // coefficients and cell numbers through the read-only path, the sweep input
 // (written earlier in the same kernel by the persistent solver) plainly
-template <class Real, int MODE, int NC, int P>
+template <class Real, int MODE, int P>
 __device__ __forceinline__ void s2_load(const Skew2D<Real> &g, long long e0, long long st, int t0,
-                                        S2Chunk<Real, NC, P> &k) {
+                                        S2Chunk<Real, P> &k) {
 #pragma unroll
     for (int s = 0; s < P; ++s) {
         const long long e = e0 + (long long)(t0 + s) * st;
@@ -114,18 +114,17 @@ __device__ __forceinline__ void s2_load(const Skew2D<Real> &g, long long e0, lon
             k.c0[s] = (MODE == 0) ? __ldg(g.rDinv + e) : Real(0);
             k.cy[s] = __ldg(((MODE == 0) ? g.Ay : g.By) + e);
             k.cx[s] = __ldg(((MODE == 0) ? g.Ax : g.Bx) + e);
-#pragma unroll
-            for (int q = 0; q < NC; ++q) k.rk[s][q] = ((MODE == 0) ? g.rS : g.wS)[(long long)q * g.nSkew + e];
+            k.rk[s] = ((MODE == 0) ? g.rS : g.wS)[e];
         }
         k.cell[s] = (MODE == 1) ? __ldg(g.cellOf + e) : 0;
     }
 }
 
-// One case's sweep by the CTA that owns it (case cb; warps wbase .. wbase +
+// One component of a case's sweep by the CTA that owns it (case cb; warps wbase .. wbase +
 // nJB - 1 take the j-blocks, the others do nothing).  MODE 0: forward
 // application (rS -> wS), 1: backward application (wS -> w), 2: rD recurrence
 // (D, Py, Px -> rDraw).  ringJ: the j-block ring in shared memory
-// ([nJB][RJ][NC][W] tagged words), sProg: the consumers' progress counters;
+// ([nJB][RJ][W] tagged words), sProg: the consumers' progress counters;
 // both cleared by s2d::reset before the sweep.  At the start of a chunk of P
 // steps lanes 0 .. P-1 fetch the P words lane 0 will need from the j-block
 // below (steps t0 + 31 .. t0 + P + 30) and the warp waits until every tag
@@ -137,9 +136,9 @@ __device__ __forceinline__ void s2_load(const Skew2D<Real> &g, long long e0, lon
 // NB > 0: the chunks are staged instead into shared memory with cp.async,
 // NB - 1 chunks ahead (stage: the CTA's staging area, stage_bytes() per warp
 // of the sweep), and each chunk's values are read from there.
-template <class Real, int MODE, int NC, int P, bool PF = true, int RJ = s2d::kRJ, int NB = 0>
-__device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *__restrict__ w, int N, int *err,
-                            long long maxSpin, s2d::u64 *ringJ, int *sProg, int wbase = 0,
+template <class Real, int MODE, int P, bool PF = true, int RJ = s2d::kRJ, int NB = 0>
+__device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, Real *__restrict__ w, int *err, long long maxSpin,
+                            s2d::u64 *ringJ, int *sProg, int wbase = 0,
                             unsigned char *stage = nullptr) {
     constexpr int WN = s2d::W<Real>::n;
     const int lane = threadIdx.x & 31, jo = (int)(threadIdx.x >> 5) - wbase;
@@ -153,18 +152,16 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
     const int depJ = (jo > 0) ? jo - 1 : -1;
     const int consJ = (jo + 1 < nJB) ? jo + 1 : -1;
     const Real zk = (MODE == 2) ? Real(1) : Real(0);
-    s2d::u64 *myRing = ringJ + (size_t)jo * RJ * NC * WN;
-    const s2d::u64 *depRing = ringJ + (size_t)(depJ >= 0 ? depJ : 0) * RJ * NC * WN;
-    Real yprev[NC];
-#pragma unroll
-    for (int q = 0; q < NC; ++q) yprev[q] = zk;
+    s2d::u64 *myRing = ringJ + (size_t)jo * RJ * WN;
+    const s2d::u64 *depRing = ringJ + (size_t)(depJ >= 0 ? depJ : 0) * RJ * WN;
+    Real yprev = zk;
     int seenCJ = 0;
     bool failed = false;
-    S2Chunk<Real, NC, P> cur, nxt;
+    S2Chunk<Real, P> cur, nxt;
     // ---- staging (NB > 0): chunk c of this warp, array a, into buffer c % NB
-    constexpr int NA = s2d::StageArrays<MODE, NC>::n;
+    constexpr int NA = s2d::StageArrays<MODE>::n;
     constexpr int CH = P * 32;                                  // entries of one array in one chunk
-    constexpr int BUF = s2d::stage_bytes<Real, MODE, NC, P, NB>() / (NB > 0 ? NB : 1);
+    constexpr int BUF = s2d::stage_bytes<Real, MODE, P, NB>() / (NB > 0 ? NB : 1);
     unsigned char *myStage = stage + (size_t)jo * (NB > 0 ? NB : 1) * BUF;
     auto stage_chunk = [&](int c) {
         const int tc = c * P;
@@ -176,8 +173,8 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
         for (int a = 0; a < NA; ++a) {
             const Real *src;
             if (MODE == 2) src = a == 0 ? g.D : a == 1 ? g.Py : g.Px;
-            else if (MODE == 0) src = a == 0 ? g.rDinv : a == 1 ? g.Ay : a == 2 ? g.Ax : g.rS + (long long)(a - 3) * g.nSkew;
-            else src = a == 0 ? g.By : a == 1 ? g.Bx : g.wS + (long long)(a - 2) * g.nSkew;
+            else if (MODE == 0) src = a == 0 ? g.rDinv : a == 1 ? g.Ay : a == 2 ? g.Ax : g.rS;
+            else src = a == 0 ? g.By : a == 1 ? g.Bx : g.wS;
             for (int i = lane; i < PIECES; i += 32)
                 s2d::cp16(buf + (size_t)a * CH * sizeof(Real) + (size_t)i * 16, src + base + (long long)i * (16 / sizeof(Real)));
         }
@@ -196,12 +193,10 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
                 cur.c0[s] = arr[i]; cur.cy[s] = arr[CH + i]; cur.cx[s] = arr[2 * CH + i];
             } else if (MODE == 0) {
                 cur.c0[s] = arr[i]; cur.cy[s] = arr[CH + i]; cur.cx[s] = arr[2 * CH + i];
-#pragma unroll
-                for (int q = 0; q < NC; ++q) cur.rk[s][q] = arr[(3 + q) * CH + i];
+                cur.rk[s] = arr[3 * CH + i];
             } else {
                 cur.c0[s] = Real(0); cur.cy[s] = arr[i]; cur.cx[s] = arr[CH + i];
-#pragma unroll
-                for (int q = 0; q < NC; ++q) cur.rk[s][q] = arr[(2 + q) * CH + i];
+                cur.rk[s] = arr[2 * CH + i];
                 cur.cell[s] = cel[i];
             }
         }
@@ -213,7 +208,7 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
             s2d::cp_commit();
         }
     } else if (PF) {
-        s2_load<Real, MODE, NC, P>(g, e0, st, 0, cur);
+        s2_load<Real, MODE, P>(g, e0, st, 0, cur);
     }
     for (int t0 = 0; t0 < T; t0 += P) {
         const int te = t0 + P;   // T is a multiple of P
@@ -226,7 +221,7 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
             read_chunk(c);
             __syncwarp();   // buffer c % NB is free for chunk c + NB
         } else if (PF && te < T) {
-            s2_load<Real, MODE, NC, P>(g, e0, st, te, nxt);
+            s2_load<Real, MODE, P>(g, e0, st, te, nxt);
         }
         // the consumer has used the ring slots this chunk overwrites
         if (consJ >= 0 && seenCJ < te - RJ - 31) {
@@ -237,20 +232,14 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
             seenCJ = v;
         }
         // the words of the j-block below for this chunk's steps (lane s holds step t0 + s + 31)
-        Real jv[NC];
-#pragma unroll
-        for (int q = 0; q < NC; ++q) jv[q] = zk;
+        Real jv = zk;
         if (depJ >= 0) {
             const int tw = t0 + lane + 31;
             const bool need = lane < P && tw < T;
-            const s2d::u64 *slot = depRing + (size_t)(tw & (RJ - 1)) * NC * WN;
+            const s2d::u64 *slot = depRing + (size_t)(tw & (RJ - 1)) * WN;
             long long spins = 0;
             for (;;) {
-                bool ok = true;
-                if (need) {
-#pragma unroll
-                    for (int q = 0; q < NC; ++q) ok &= s2d::take(slot + q * WN, (unsigned)(tw + 1), jv[q]);
-                }
+                const bool ok = need ? s2d::take(slot, (unsigned)(tw + 1), jv) : true;
                 if (__all_sync(0xffffffffu, ok)) break;
                 const bool quit = (++spins > maxSpin) || *(volatile int *)err;
                 if (__any_sync(0xffffffffu, quit)) {
@@ -261,51 +250,40 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, unsigned mask, Real *
             }
             if (failed) break;
         }
-        if (NB == 0 && !PF) s2_load<Real, MODE, NC, P>(g, e0, st, t0, cur);
-        Real out[P][NC];
+        if (NB == 0 && !PF) s2_load<Real, MODE, P>(g, e0, st, t0, cur);
+        Real out[P];
 #pragma unroll
         for (int s = 0; s < P; ++s) {
             const int t = t0 + s;
-#pragma unroll
-            for (int q = 0; q < NC; ++q) {
-                const Real fromBelow = __shfl_sync(0xffffffffu, jv[q], s);
-                const Real yup = __shfl_up_sync(0xffffffffu, yprev[q], 1);
-                const Real yj = (lane > 0) ? yup : ((depJ >= 0 && t + 31 < T) ? fromBelow : zk);
-                Real v;
-                if (MODE == 2) {
-                    v = r_sub(cur.c0[s], r_div(cur.cy[s], yj));
-                    v = r_sub(v, r_div(cur.cx[s], yprev[q]));
+            const Real fromBelow = __shfl_sync(0xffffffffu, jv, s);
+            const Real yup = __shfl_up_sync(0xffffffffu, yprev, 1);
+            const Real yj = (lane > 0) ? yup : ((depJ >= 0 && t + 31 < T) ? fromBelow : zk);
+            Real v;
+            if (MODE == 2) {
+                v = r_sub(cur.c0[s], r_div(cur.cy[s], yj));
+                v = r_sub(v, r_div(cur.cx[s], yprev));
+            } else {
+                const Real pre = (MODE == 0) ? r_mul(cur.c0[s], cur.rk[s]) : cur.rk[s];
+                if (sizeof(Real) == 4) {   // FP32: the i term first (as the 3-D sweeps)
+                    v = r_fma(-cur.cx[s], yprev, pre);
+                    v = r_fma(-cur.cy[s], yj, v);
                 } else {
-                    const Real pre = (MODE == 0) ? r_mul(cur.c0[s], cur.rk[s][q]) : cur.rk[s][q];
-                    if (sizeof(Real) == 4) {   // FP32: the i term first (as the 3-D sweeps)
-                        v = r_fma(-cur.cx[s], yprev[q], pre);
-                        v = r_fma(-cur.cy[s], yj, v);
-                    } else {
-                        v = r_fma(-cur.cy[s], yj, pre);
-                        v = r_fma(-cur.cx[s], yprev[q], v);
-                    }
+                    v = r_fma(-cur.cy[s], yj, pre);
+                    v = r_fma(-cur.cx[s], yprev, v);
                 }
-                if (consJ >= 0 && lane == 31) s2d::put(myRing + ((size_t)(t & (RJ - 1)) * NC + q) * WN, v,
-                                                       (unsigned)(t + 1));
-                out[s][q] = v;
-                yprev[q] = v;
             }
+            if (consJ >= 0 && lane == 31) s2d::put(myRing + (size_t)(t & (RJ - 1)) * WN, v, (unsigned)(t + 1));
+            out[s] = v;
+            yprev = v;
         }
         // this warp has used the words of the block below through step te + 30
         if (lane == 0 && depJ >= 0) *(volatile int *)(sProg + jo) = te;
 #pragma unroll
         for (int s = 0; s < P; ++s) {
             const long long e = e0 + (long long)(t0 + s) * st;
-            if (MODE == 2) {
-                g.rDraw[e] = out[s][0];
-            } else {
-#pragma unroll
-                for (int q = 0; q < NC; ++q) {
-                    if (!((mask >> q) & 1u)) continue;
-                    if (MODE == 0) g.wS[(long long)q * g.nSkew + e] = out[s][q];
-                    else if (cur.cell[s] >= 0) w[(long long)q * N + cur.cell[s]] = out[s][q];
-                }
-            }
+            if (MODE == 2) g.rDraw[e] = out[s];
+            else if (MODE == 0) g.wS[e] = out[s];
+            else if (cur.cell[s] >= 0) w[cur.cell[s]] = out[s];
         }
         if (NB == 0 && PF) cur = nxt;
     }
