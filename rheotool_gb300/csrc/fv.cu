@@ -24,13 +24,12 @@ __global__ void k_grad(MeshView m, const double *__restrict__ x, const double *_
         bool own = nb > c;
         int o = own ? c : nb, n = own ? nb : c;
         double wf = m.w[f];
-        double S0 = m.Sf[f], S1 = m.Sf[m.F + f], S2 = m.Sf[2 * m.F + f];
+        // outward from the cell
+        double S0 = signed_by(!own, m.Sf[f]), S1 = signed_by(!own, m.Sf[m.F + f]), S2 = signed_by(!own, m.Sf[2 * m.F + f]);
 #pragma unroll
         for (int k = 0; k < NC; ++k) {
             double xf = lin_interp(wf, x[(size_t)k * m.N + o], x[(size_t)k * m.N + n]);
-            double s0 = S0 * xf, s1 = S1 * xf, s2 = S2 * xf;
-            if (own) { a[k][0] += s0; a[k][1] += s1; a[k][2] += s2; }
-            else     { a[k][0] -= s0; a[k][1] -= s1; a[k][2] -= s2; }
+            a[k][0] += __dmul_rn(S0, xf); a[k][1] += __dmul_rn(S1, xf); a[k][2] += __dmul_rn(S2, xf);
         }
     }
     for (int i = m.bStart[c]; i < m.bStart[c + 1]; ++i) {
@@ -42,11 +41,11 @@ __global__ void k_grad(MeshView m, const double *__restrict__ x, const double *_
             a[k][0] += S0 * xf; a[k][1] += S1 * xf; a[k][2] += S2 * xf;
         }
     }
-    double v = m.V[c];
+    const Divisor v = divisor(m.V[c]);
 #pragma unroll
     for (int k = 0; k < NC; ++k)
 #pragma unroll
-        for (int d = 0; d < 3; ++d) g[((size_t)d * NC + k) * m.N + c] = a[k][d] / v;
+        for (int d = 0; d < 3; ++d) g[((size_t)d * NC + k) * m.N + c] = quotient(a[k][d], v);
 }
 
 void grad_field(rt_ctx *ctx, int nc, const double *x, const double *xb, double *g) {
@@ -86,15 +85,15 @@ __global__ void k_defc_face(MeshView m, Lims L, int hr, const double *__restrict
     if (!hr) return;
     int o = m.owner[f], n = m.neighbour[f];
     double d0 = m.d[f], d1 = m.d[m.F + f], d2 = m.d[2 * m.F + f];
+    // the terms of the upwind side alone: the weights u and 1 - u of the others are
+    // zero, which adds nothing to a finite sum
+    const bool fromOwner = ph >= 0.0;
+    const int up = fromOwner ? o : n;
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-        double go0 = g[((size_t)0 * NC + k) * N + o], go1 = g[((size_t)1 * NC + k) * N + o],
-               go2 = g[((size_t)2 * NC + k) * N + o];
-        double gn0 = g[((size_t)0 * NC + k) * N + n], gn1 = g[((size_t)1 * NC + k) * N + n],
-               gn2 = g[((size_t)2 * NC + k) * N + n];
-        double gu0 = go0 * u + (1.0 - u) * gn0, gu1 = go1 * u + (1.0 - u) * gn1,
-               gu2 = go2 * u + (1.0 - u) * gn2;
-        double gud = gu0 * d0 + gu1 * d1 + gu2 * d2;
+        double g0 = g[((size_t)0 * NC + k) * N + up], g1 = g[((size_t)1 * NC + k) * N + up],
+               g2 = g[((size_t)2 * NC + k) * N + up];
+        double gud = g0 * d0 + g1 * d1 + g2 * d2;
         double xo = x[(size_t)k * N + o], xn = x[(size_t)k * N + n];
         double phitc = 1.0 - (xn - xo) / (2.0 * gud + 1e-18);
         double a, bb;
@@ -102,12 +101,9 @@ __global__ void k_defc_face(MeshView m, Lims L, int hr, const double *__restrict
         else if (phitc < L.bl[0]) { a = L.al[0]; bb = L.be[0]; }
         else if (phitc < L.bl[1]) { a = L.al[1]; bb = L.be[1]; }
         else { a = L.al[2]; bb = L.be[2]; }
-        double god = go0 * d0 + go1 * d1 + go2 * d2;
-        double gnd = gn0 * d0 + gn1 * d1 + gn2 * d2;
-        double tf = (1.0 - a - bb) * (xn - 2.0 * god) * u
-                  + (1.0 - a - bb) * (xo + 2.0 * gnd) * (1.0 - u)
-                  + ((a - 1.0) * u + bb * (1.0 - u)) * xo
-                  + (bb * u + (a - 1.0) * (1.0 - u)) * xn;
+        double am = a - 1.0;
+        double far = __dmul_rn(1.0 - a - bb, fromOwner ? xn - 2.0 * gud : xo + 2.0 * gud);
+        double tf = __fma_rn(fromOwner ? bb : am, xn, __fma_rn(fromOwner ? am : bb, xo, far));
         flux[(size_t)k * m.F + f] = tf * ph;
     }
 }
@@ -133,7 +129,7 @@ __global__ void k_defc_cell(MeshView m, int hr, const double *__restrict__ lower
 #pragma unroll
             for (int k = 0; k < NC; ++k) {
                 double fl = flux[(size_t)k * m.F + f];
-                if (own) sou[k] += fl; else sou[k] -= fl;
+                sou[k] += signed_by(!own, fl);
             }
         }
     }

@@ -73,10 +73,26 @@ void init_fields(rt_ctx *ctx) {
 // ---------------------------------------------------------------------------
 // momentum equation
 // ---------------------------------------------------------------------------
+// a cell's tau / rho (6 N) and, for coupling, kG grad U (9 N more) in `out`: the
+// faces of divTau read them twice each (formed at every face they were 72 divisions
+// and 108 products a cell: 2.1 ms of 1M cells' 2.4 ms momentum assembly)
+__global__ void k_divtau_scale(MeshView m, MomCoef mc0, const double *__restrict__ tau, const double *__restrict__ G,
+                               double *__restrict__ out) {
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= m.N) return;
+    const MomCoef mc = m.caseOf ? mom_coef(m.caseParams[m.caseOf[c]]) : mc0;
+    const Divisor rho = divisor(mc.rho);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) out[(size_t)q * m.N + c] = quotient(tau[(size_t)q * m.N + c], rho);
+    if (mc.stab == RT_STAB_COUPLING)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) out[(size_t)(6 + q) * m.N + c] = mc.kG * G[(size_t)q * m.N + c];
+}
+
 // explicit part of divTau: div(tau/rho) - div(kG grad U) (coupling) or
-// - laplacian(kG, U) (BSD), both Gauss linear
+// - laplacian(kG, U) (BSD), both Gauss linear; T: k_divtau_scale's
 __global__ void k_divtau_expl(MeshView m, MomCoef mc0,
-                              const double *__restrict__ tau, const double *__restrict__ taub,
+                              const double *__restrict__ T, const double *__restrict__ taub,
                               const double *__restrict__ G, const double *__restrict__ U,
                               const double *__restrict__ Ub, double *__restrict__ expl) {
     int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -85,6 +101,7 @@ __global__ void k_divtau_expl(MeshView m, MomCoef mc0,
     const int stab = mc.stab;
     const double rho = mc.rho, kG = mc.kG;
     const int N = m.N, NB = m.NB, F = m.F;
+    const double *__restrict__ kGG = T + (size_t)6 * N;
     double dt0 = 0.0, dt1 = 0.0, dt2 = 0.0;     // div(tau/rho) sums
     double dg0 = 0.0, dg1 = 0.0, dg2 = 0.0;     // div(kG grad U) or laplacian sums
     for (int s = 0; s < m.nSlots; ++s) {
@@ -97,19 +114,22 @@ __global__ void k_divtau_expl(MeshView m, MomCoef mc0,
         double S0 = m.Sf[f], S1 = m.Sf[F + f], S2 = m.Sf[2 * F + f];
         double Tf[6];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) Tf[q] = lin_interp(w, tau[(size_t)q * N + o] / rho, tau[(size_t)q * N + n] / rho);
+        for (int q = 0; q < 6; ++q) Tf[q] = lin_interp(w, T[(size_t)q * N + o], T[(size_t)q * N + n]);
         double v0 = S0 * Tf[0] + S1 * Tf[1] + S2 * Tf[2];
         double v1 = S0 * Tf[1] + S1 * Tf[3] + S2 * Tf[4];
         double v2 = S0 * Tf[2] + S1 * Tf[4] + S2 * Tf[5];
-        if (own) { dt0 += v0; dt1 += v1; dt2 += v2; } else { dt0 -= v0; dt1 -= v1; dt2 -= v2; }
+        dt0 += signed_by(!own, v0); dt1 += signed_by(!own, v1); dt2 += signed_by(!own, v2);
         if (stab == RT_STAB_COUPLING) {
             double Gf[9];
 #pragma unroll
-            for (int q = 0; q < 9; ++q) Gf[q] = lin_interp(w, kG * G[(size_t)q * N + o], kG * G[(size_t)q * N + n]);
+            for (int q = 0; q < 9; ++q) {   // lin_interp of kG grad U, the owner's product unrounded
+                const double gn = kGG[(size_t)q * N + n];
+                Gf[q] = __fma_rn(w, __fma_rn(kG, G[(size_t)q * N + o], -gn), gn);
+            }
             double u0 = S0 * Gf[0] + S1 * Gf[3] + S2 * Gf[6];
             double u1 = S0 * Gf[1] + S1 * Gf[4] + S2 * Gf[7];
             double u2 = S0 * Gf[2] + S1 * Gf[5] + S2 * Gf[8];
-            if (own) { dg0 += u0; dg1 += u1; dg2 += u2; } else { dg0 -= u0; dg1 -= u1; dg2 -= u2; }
+            dg0 += signed_by(!own, u0); dg1 += signed_by(!own, u1); dg2 += signed_by(!own, u2);
         } else if (stab == RT_STAB_BSD) {
             double gm = kG * m.magSf[f], dl = m.delta[f];
             double u0 = gm * (dl * (U[n] - U[o]));
@@ -154,12 +174,12 @@ __global__ void k_divtau_expl(MeshView m, MomCoef mc0,
             dg2 += gm * (dl * (Ub[2 * NB + b] - U[2 * N + c]));
         }
     }
-    double v = m.V[c];
-    double e0 = dt0 / v, e1 = dt1 / v, e2 = dt2 / v;
+    const Divisor v = divisor(m.V[c]);
+    double e0 = quotient(dt0, v), e1 = quotient(dt1, v), e2 = quotient(dt2, v);
     if (stab != RT_STAB_NONE) {
-        e0 -= dg0 / v;
-        e1 -= dg1 / v;
-        e2 -= dg2 / v;
+        e0 -= quotient(dg0, v);
+        e1 -= quotient(dg1, v);
+        e2 -= quotient(dg2, v);
     }
     expl[c] = e0;
     expl[(size_t)N + c] = e1;
@@ -286,13 +306,13 @@ __global__ void k_AH(MeshView m, const double *__restrict__ diag, const double *
 #pragma unroll
         for (int k = 0; k < 3; ++k) H[k] += bouC[(size_t)k * NB + b];
     }
-    double v = m.V[c];
-    double r = 1.0 / (A / v);
-    H1 /= v;
+    const Divisor v = divisor(m.V[c]);
+    double r = 1.0 / quotient(A, v);
+    H1 = quotient(H1, v);
     rAU[c] = r;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        double h = H[k] / v;
+        double h = quotient(H[k], v);
         Hout[(size_t)k * N + c] = h;
         HbyA[(size_t)k * N + c] = r * h;
     }
@@ -593,8 +613,12 @@ static rt_status step_inner(rt_ctx *ctx, rt_step_perf *perf, const double *U0, c
     const double gam = mc.gam;
     double *expl = W.take(3 * (size_t)N);
     ProfScope psMom(ctx, "mom_assembly", (double)N * (48.0 + 72.0 + 24.0 + 24.0 + 8.0 + 24.0 + 24.0 + 24.0 + 8.0 + 24.0) + F * 32.0);
-    k_divtau_expl<<<gN, RT_BLOCK, 0, s>>>(m, mc, multi ? cs.tauTot.p : cs.tau.p, multi ? cs.taubTot.p : cs.taub.p, G,
-                                          cs.U.p, cs.Ub.p, expl);
+    {
+        WorkMark mark(W);
+        double *scaled = W.take(15 * (size_t)N);
+        k_divtau_scale<<<gN, RT_BLOCK, 0, s>>>(m, mc, multi ? cs.tauTot.p : cs.tau.p, G, scaled);
+        k_divtau_expl<<<gN, RT_BLOCK, 0, s>>>(m, mc, scaled, multi ? cs.taubTot.p : cs.taub.p, G, cs.U.p, cs.Ub.p, expl);
+    }
     double *diag = W.take(N), *src = W.take(3 * (size_t)N);
     const double3 body = make_double3(ctl.bodyForce[0], ctl.bodyForce[1], ctl.bodyForce[2]);
     // Crank-Nicolson: the step's ddt coefficient c/dt and the old-time derivatives
@@ -605,7 +629,7 @@ static rt_status step_inner(rt_ctx *ctx, rt_step_perf *perf, const double *U0, c
     if (F) k_sub_lap<<<gF, RT_BLOCK, 0, s>>>(m, gam, lower, upper);
     if (NB) k_mom_bnd<<<gB, RT_BLOCK, 0, s>>>(m, gam, cs.bkU.p, cs.Ub.p, intC, bouC);
     RT_CHECK_LAUNCH();
-    launch_count(ctx, 4);
+    launch_count(ctx, 5);
     double *gp = W.take(3 * (size_t)N);
     grad_field(ctx, 1, cs.p.p, cs.pb.p, gp);
     double *dS = W.take(N), *bS = W.take(3 * (size_t)N);
