@@ -8,6 +8,7 @@
 // cell, so the gather is deterministic and free of atomics.
 #pragma once
 
+#include "real_ops.cuh"
 #include "rt_internal.h"
 
 namespace rt {
@@ -85,28 +86,6 @@ __device__ __forceinline__ double lin_interp(double w, double vP, double vN) {
 // -x where neg, in the integer pipe
 __device__ __forceinline__ double signed_by(bool neg, double x) {
     return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
-}
-
-// a / v for several a: the correctly rounded quotient from y = 1 / v rounded to
-// nearest.  a y is within two units in the last place, one correction makes it a
-// faithful rounding and the next the correct one (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
-// 34 (1990), theorem on q' = q + r y), as long as nothing under- or overflows:
-// exponents outside +-400 take the division itself.  Five instructions against some
-// twelve, and no branch taken.
-struct Divisor {
-    double v, y;
-    bool fast;
-};
-__device__ __forceinline__ bool mid_exponent(double x) {
-    return (unsigned)(((__double2hiint(x) >> 20) & 0x7ff) - (1023 - 400)) <= 800u;
-}
-__device__ __forceinline__ Divisor divisor(double v) { return {v, __drcp_rn(v), mid_exponent(v)}; }
-__device__ __forceinline__ double quotient(double a, const Divisor &d) {
-    if (!(d.fast && mid_exponent(a))) return a == 0.0 && d.fast && d.v > 0.0 ? a : a / d.v;
-    const double q0 = __dmul_rn(a, d.y);
-    const double q1 = __fma_rn(__fma_rn(-d.v, q0, a), d.y, q0);
-    return __fma_rn(__fma_rn(-d.v, q1, a), d.y, q1);
 }
 
 // Gauss linear gradient of one scalar (stride-N SoA component) at cell c

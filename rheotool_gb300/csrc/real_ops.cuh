@@ -12,8 +12,37 @@ __device__ __forceinline__ double r_fma(double a, double b, double c) { return _
 __device__ __forceinline__ float r_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double r_sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ float r_sub(float a, float b) { return __fsub_rn(a, b); }
-__device__ __forceinline__ double r_div(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ float r_div(float a, float b) { return __fdiv_rn(a, b); }
+
+// a / v for several a: the correctly rounded quotient from y = 1 / v rounded to
+// nearest.  a y is within two units in the last place, one correction makes it a
+// faithful rounding and the next the correct one (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev.
+// 34 (1990), theorem on q' = q + r y), as long as nothing under- or overflows:
+// exponents outside +-400 take the division itself.  Five FP64 instructions against
+// some twelve, and no call.
+struct Divisor {
+    double v, y;
+    bool fast;
+};
+__device__ __forceinline__ bool mid_exponent(double x) {
+    return (unsigned)(((__double2hiint(x) >> 20) & 0x7ff) - (1023 - 400)) <= 800u;
+}
+__device__ __forceinline__ Divisor divisor(double v, double y) { return {v, y, mid_exponent(v)}; }
+__device__ __forceinline__ Divisor divisor(double v) { return divisor(v, __drcp_rn(v)); }
+__device__ __forceinline__ bool plain_zero(double a) { return ((__double2hiint(a) << 1) | __double2loint(a)) == 0; }
+// whether corrected() is the quotient
+__device__ __forceinline__ bool correctable(double a, const Divisor &d) {
+    return d.fast && (plain_zero(a) || mid_exponent(a));
+}
+__device__ __forceinline__ double corrected(double a, const Divisor &d) {
+    const double q0 = __dmul_rn(a, d.y);
+    const double q1 = __fma_rn(__fma_rn(-d.v, q0, a), d.y, q0);
+    const double q2 = __fma_rn(__fma_rn(-d.v, q1, a), d.y, q1);
+    return plain_zero(a) ? q0 : q2;   // (a zero keeps its sign)
+}
+__device__ __forceinline__ double quotient(double a, const Divisor &d) {
+    return correctable(a, d) ? corrected(a, d) : __ddiv_rn(a, d.v);
+}
 
 // Sums of FP32 vectors kept as an unevaluated pair hi + lo of FP32 numbers:
 // each product split exactly by an FMA, each addition by Knuth's two-sum

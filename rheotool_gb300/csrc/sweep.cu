@@ -32,7 +32,9 @@
 // the CTA fetch the ghosts, hand results to the next CTAs, stage coefficients
 // and write results out.  (A skew of two in k would take the k product off a
 // step's chain, but a warp issues its FP64 products in order: a step was no shorter,
-// and there were nz more of them.)
+// and there were nz more of them.  The rD recurrence, three quotients a step, hands
+// each value on with its reciprocal, which leaves five products of a quotient: 616 us
+// for 1M cells against 1370 with three divisions, 287 against 667 for 127k.)
 //
 // A value handed to another CTA is its own flag: the hand-off words hold the
 // pattern of all ones until the producer writes the value (a result with that
@@ -166,9 +168,9 @@ struct Group {
 
 template <class Real, int P>
 __host__ __device__ constexpr int stage_bytes() { return P * 32 * kStaged * (int)sizeof(Real); }
-template <class Real, class G, int P, int NB>
-__host__ __device__ constexpr int group_smem() {
-    return G::W * NB * stage_bytes<Real, P>() + G::ringSteps * G::pitch * (int)sizeof(Real);
+template <class Real, class G, int MODE, int P, int NB>
+__host__ __device__ constexpr int group_smem() {   // (rD: a second ring, of the values' reciprocals)
+    return G::W * NB * stage_bytes<Real, P>() + (MODE == 2 ? 2 : 1) * G::ringSteps * G::pitch * (int)sizeof(Real);
 }
 
 // counters shared by a CTA's warps (steps of a tile): computed and written out
@@ -227,6 +229,7 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
     static_assert(kSkewJ * TJ % B == 0 && (TK == 1 || kSkewK * TK % B == 0), "a block of another tile's slots does not wrap");
     static_assert(kSkewJ == 1 && kSkewK == 1, "a step reads the values of the step before");
     constexpr W kNone = ~W(0);
+    constexpr int RINV = R * PITCH;   // rD: a value's reciprocal in the second ring
     const Real zk = (MODE == 2) ? Real(1) : Real(0);
     SkewT<Real> &g = a.g;
     next_may_start();
@@ -243,7 +246,7 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    for (int i = threadIdx.x; i < R * PITCH; i += blockDim.x) ring[i] = zk;
+    for (int i = threadIdx.x; i < (MODE == 2 ? 2 : 1) * R * PITCH; i += blockDim.x) ring[i] = zk;
     wait_for_previous();
     // every component of the launch has stopped iterating (the same word for
     // every CTA, written by an earlier kernel): nothing to do
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
                 off = GS;
             }
             int seen = 0;
-            Real y1 = zk;
+            Real y1 = zk, inv1 = zk;
             // looks at the counters until the steps from t on may be taken
             auto until_ready = [&](int t) {
                 const int need = min(t + off, T);
@@ -365,10 +368,14 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
                         const Real xz = s >= 1 ? kNow[(s - 1) * PITCH] : kPast[0];
                         const Real xy = s >= 1 ? jNow[(s - 1) * PITCH] : jPast[0];
                         Real v;
-                        if (MODE == 2) {
-                            v = r_sub(va[0][sf], r_div(va[1][sf], xz));   // D - Pz / rD(k-1) - ...
-                            v = r_sub(v, r_div(va[2][sf], xy));
-                            v = r_sub(v, r_div(va[3][sf], y1));
+                        if constexpr (MODE == 2) {   // D - Pz / rD(k-1) - Py / rD(j-1) - Px / rD(i-1)
+                            const Real iz = s >= 1 ? kNow[RINV + (s - 1) * PITCH] : kPast[RINV];
+                            const Real iy = s >= 1 ? jNow[RINV + (s - 1) * PITCH] : jPast[RINV];
+                            v = r_sub(va[0][sf], quotient(va[1][sf], divisor(xz, iz)));
+                            v = r_sub(v, quotient(va[2][sf], divisor(xy, iy)));
+                            v = r_sub(v, quotient(va[3][sf], divisor(y1, inv1)));
+                            inv1 = __drcp_rn(v);
+                            cur[RINV + s * PITCH] = inv1;
                         } else {
                             v = r_fma(-va[0][sf], xz, va[3][sf]);
                             if (sizeof(Real) == 4) {
@@ -505,7 +512,11 @@ __global__ void __launch_bounds__(32 * Group<TJ, WJ, WK>::warps, 1) k_tile_sweep
 #pragma unroll
                     for (int i = 0; i < L; ++i) {
                         const int q = i * 32 + lane, st = pos + q / n;
-                        if (st < pos + k) ring[(st & (R - 1)) * PITCH + ringAt + q % n] = Wd::value(v[i]);
+                        if (st < pos + k) {
+                            volatile Real *to = ring + (st & (R - 1)) * PITCH + ringAt + q % n;
+                            to[0] = Wd::value(v[i]);
+                            if constexpr (MODE == 2) to[RINV] = __drcp_rn(Wd::value(v[i]));
+                        }
                     }
                     __syncwarp();
                     *arrived = pos + k;
@@ -658,7 +669,7 @@ typename Word<Real>::T *hand_off_words(rt_ctx *ctx, long long perComp, int ncomp
 template <class Real, int MODE, int TJ, int WJ, int WK, int P, int NB>
 void launch_one(rt_ctx *ctx, const TileRun<Real> &run) {
     typedef Group<TJ, WJ, WK> G;
-    constexpr int shm = group_smem<Real, G, P, NB>();
+    constexpr int shm = group_smem<Real, G, MODE, P, NB>();
     static_assert(shm <= 226 * 1024, "one CTA's shared memory");
     static bool opted = false;   // per instantiation
     if (!opted) {
@@ -685,17 +696,22 @@ constexpr int kNarrow = 2, kWide = 1;
 
 template <class Real, int MODE, int TJ>
 void launch_tuned(rt_ctx *ctx, const TileRun<Real> &run, int k) {
-    constexpr int WJ = TJ == 32 ? 4 : 2, WK = TJ == 32 ? 1 : 2;
-    if (k < 0) {
-        const int two = (run.g.nTJ + 1) / 2 * run.g.nTK * run.ncc;
-        k = two > ctx->numSMs ? kWide : kNarrow;
-    }
-    switch (k) {
-    case 0: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[0], kTuneNB[0]>(ctx, run); break;
-    case 1: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[1], kTuneNB[1]>(ctx, run); break;
-    case 2: launch_one<Real, MODE, TJ, 2, 1, kTuneP[2], kTuneNB[2]>(ctx, run); break;
-    case 3: launch_one<Real, MODE, TJ, 2, 1, kTuneP[3], kTuneNB[3]>(ctx, run); break;
-    default: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[4], kTuneNB[4]>(ctx, run); break;
+    const bool all = (run.g.nTJ + 1) / 2 * run.g.nTK * run.ncc <= ctx->numSMs;   // groups of two tiles, one an SM
+    if constexpr (MODE == 2) {   // its two rings leave room for these
+        if constexpr (TJ == 8) {
+            if (!all) return launch_one<Real, MODE, TJ, 2, 2, 8, 3>(ctx, run);
+        }
+        launch_one<Real, MODE, TJ, 2, 1, 16, 3>(ctx, run);
+    } else {
+        constexpr int WJ = TJ == 32 ? 4 : 2, WK = TJ == 32 ? 1 : 2;
+        if (k < 0) k = all ? kNarrow : kWide;
+        switch (k) {
+        case 0: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[0], kTuneNB[0]>(ctx, run); break;
+        case 1: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[1], kTuneNB[1]>(ctx, run); break;
+        case 2: launch_one<Real, MODE, TJ, 2, 1, kTuneP[2], kTuneNB[2]>(ctx, run); break;
+        case 3: launch_one<Real, MODE, TJ, 2, 1, kTuneP[3], kTuneNB[3]>(ctx, run); break;
+        default: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[4], kTuneNB[4]>(ctx, run); break;
+        }
     }
 }
 

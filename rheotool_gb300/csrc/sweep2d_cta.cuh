@@ -154,7 +154,7 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, Real *__restrict__ w,
     const Real zk = (MODE == 2) ? Real(1) : Real(0);
     s2d::u64 *myRing = ringJ + (size_t)jo * RJ * WN;
     const s2d::u64 *depRing = ringJ + (size_t)(depJ >= 0 ? depJ : 0) * RJ * WN;
-    Real yprev = zk;
+    Real yprev = zk, rprev = zk;   // (rD: with its reciprocal)
     int seenCJ = 0;
     bool failed = false;
     S2Chunk<Real, P> cur, nxt;
@@ -250,6 +250,8 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, Real *__restrict__ w,
             }
             if (failed) break;
         }
+        Real jr = zk;   // rD: the reciprocals of the words
+        if constexpr (MODE == 2) jr = __drcp_rn(jv);
         if (NB == 0 && !PF) s2_load<Real, MODE, P>(g, e0, st, t0, cur);
         Real out[P];
 #pragma unroll
@@ -259,9 +261,13 @@ __device__ void sweep2d_cta(const Skew2D<Real> &g, int cb, Real *__restrict__ w,
             const Real yup = __shfl_up_sync(0xffffffffu, yprev, 1);
             const Real yj = (lane > 0) ? yup : ((depJ >= 0 && t + 31 < T) ? fromBelow : zk);
             Real v;
-            if (MODE == 2) {
-                v = r_sub(cur.c0[s], r_div(cur.cy[s], yj));
-                v = r_sub(v, r_div(cur.cx[s], yprev));
+            if constexpr (MODE == 2) {
+                const Real rBelow = __shfl_sync(0xffffffffu, jr, s);
+                const Real rup = __shfl_up_sync(0xffffffffu, rprev, 1);
+                const Real rj = (lane > 0) ? rup : ((depJ >= 0 && t + 31 < T) ? rBelow : zk);
+                v = r_sub(cur.c0[s], quotient(cur.cy[s], divisor(yj, rj)));
+                v = r_sub(v, quotient(cur.cx[s], divisor(yprev, rprev)));
+                rprev = __drcp_rn(v);
             } else {
                 const Real pre = (MODE == 0) ? r_mul(cur.c0[s], cur.rk[s]) : cur.rk[s];
                 if (sizeof(Real) == 4) {   // FP32: the i term first (as the 3-D sweeps)

@@ -313,6 +313,35 @@ def test_systolic_sweeps_at_tile_edges(ctx, dims, nc):
     assert np.array_equal(out[abi.SWEEP_LEVELS][0], out[abi.SWEEP_SYSTOLIC][0])
 
 
+@pytest.mark.parametrize("exponent", [-450, -420, -210, 0, 210, 450])
+@pytest.mark.parametrize("dims", [(12, 17, 9), (9, 65, 1)])
+def test_systolic_factorisation_at_all_scales(ctx, dims, exponent):
+    """The structured factorisation's quotients, by corrections of a product with
+    the divisor's reciprocal and by division where the exponents are far from 0,
+    with and without zero numerators: the level-scheduled factorisation, which
+    divides, gives the same bits."""
+    nx, ny, nz = dims
+    mesh = cavity_mesh(nx, ny) if nz == 1 else channel_mesh(nx, ny, nz)
+    rng = np.random.default_rng(29)
+    diag, upper, lower = laplacian_system(mesh, rng)
+    cut = rng.random(upper.size) < 0.1
+    upper, lower = np.where(cut, 0.0, upper), np.where(cut, 0.0, lower)
+    scale = 2.0 ** exponent
+    diag, upper, lower, b = diag * scale, upper * scale, lower * scale, rng.normal(size=(1, mesh.nCells)) * scale
+    ctx.upload_mesh(mesh)
+    out = {}
+    try:
+        for mode in (abi.SWEEP_LEVELS, abi.SWEEP_SYSTOLIC):
+            ctx.set_sweep(mode)
+            x = np.zeros((1, mesh.nCells))
+            perf = ctx.ldu_solve(diag, upper, lower, b, x, SolverControl("PCG", "DIC", 1e-300, 0.0, 0, 4))
+            assert perf[0].nIterations == 4 and np.all(np.isfinite(x)) and np.any(x)
+            out[mode] = x
+    finally:
+        ctx.set_sweep(abi.SWEEP_AUTO)
+    assert np.array_equal(out[abi.SWEEP_LEVELS], out[abi.SWEEP_SYSTOLIC])
+
+
 def test_solver_reports_non_convergence(ctx):
     mesh = small_contraction()
     rng = np.random.default_rng(13)
