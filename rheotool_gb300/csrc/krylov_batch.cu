@@ -95,20 +95,6 @@ __device__ __forceinline__ bool bconv(const Ctl &c, double fin, double init) {
 }
 
 // ---- reductions ---------------------------------------------------------
-// partial[(slot * 6 + k) * nBlk + blk]; res[slot * nSeg + case * 8 + k]
-__global__ void k_b_fin(int nSlots, unsigned vm, BTab t, const double *__restrict__ partial, double *__restrict__ res) {
-    const int cb = blockIdx.x, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (k >= 6 || !((vm >> k) & 1u)) return;
-    const int b0 = t.caseBlk[cb], b1 = t.caseBlk[cb + 1];
-    const int nSeg = 8 * t.nCases;
-    for (int slot = 0; slot < nSlots; ++slot) {
-        double v = 0.0;
-        for (int i = b0 + lane; i < b1; i += 32) v += partial[(slot * 6 + k) * t.nBlk + i];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) res[slot * nSeg + cb * 8 + k] = v;
-    }
-}
-
 __global__ void k_b_sumx(BTab t, unsigned vm, const double *__restrict__ x, double *partial) {
     const int blk = blockIdx.x, c = t.blkCell0[blk] + threadIdx.x;
     const bool in = c < t.blkCell1[blk];
@@ -394,56 +380,50 @@ __global__ void k_b_start(int nCases, unsigned vm, Ctl ctl, BSeg S, const double
 
 // PCG scalars; FP32 vectors use the flexible (Polak-Ribiere) beta
 // w.(r - r_old) / w_old.r_old = -alpha_old w.q_old / w_old.r_old
-__global__ void k_b_pcg_a(int nSeg, BSeg S, const double *__restrict__ res, int mixed) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg]) continue;
-        const double aold = S.A[sg];
-        S.Aold[sg] = aold;
-        S.A[sg] = res[sg];
-        S.beta[sg] = mixed ? -S.alpha[sg] * res[nSeg + sg] / aold : res[sg] / aold;
-    }
+__device__ __forceinline__ void seg_pcg_a(int nSeg, const BSeg &S, const double *res, int sg, int mixed) {
+    if (!S.active[sg]) return;
+    const double aold = S.A[sg];
+    S.Aold[sg] = aold;
+    S.A[sg] = res[sg];
+    S.beta[sg] = mixed ? -S.alpha[sg] * res[nSeg + sg] / aold : res[sg] / aold;
 }
 
-__global__ void k_b_pcg_alpha(int nSeg, BSeg S, const double *__restrict__ res) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg]) continue;
-        const double wApA = res[sg];
-        if (fabs(wApA) / S.nf[sg] < 1e-300) {
-            S.sing[sg] = 1;
-            S.alpha[sg] = 0.0;
-        } else {
-            S.alpha[sg] = S.A[sg] / wApA;
-        }
+__device__ __forceinline__ void seg_pcg_alpha(int nSeg, const BSeg &S, const double *res, int sg) {
+    if (!S.active[sg]) return;
+    const double wApA = res[sg];
+    if (fabs(wApA) / S.nf[sg] < 1e-300) {
+        S.sing[sg] = 1;
+        S.alpha[sg] = 0.0;
+    } else {
+        S.alpha[sg] = S.A[sg] / wApA;
     }
 }
 
 // after an iteration's residual: count the iteration, stop singular
 // segments; mixed precision flags the residual replacements, FP64 applies the
 // stopping test of the plain solvers to the iterated residual
-__global__ void k_b_iter_fin(int nSeg, Ctl ctl, BSeg S, const double *__restrict__ res, int skipHalf, int mixed) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg]) continue;
-        if (skipHalf && S.conv[sg] == 2) {   // restarted at the half step: counted, no update
-            S.iter[sg] += 1;
-            S.conv[sg] = 0;
-            continue;
-        }
-        if (S.sing[sg]) {
-            S.active[sg] = 0;
-            continue;
-        }
-        const double fin = res[sg] / S.nf[sg];
-        S.fin[sg] = fin;
+__device__ __forceinline__ void seg_iter_fin(int nSeg, const BSeg &S, const double *res, int sg, const Ctl &ctl, int skipHalf, int mixed) {
+    if (!S.active[sg]) return;
+    if (skipHalf && S.conv[sg] == 2) {   // restarted at the half step: counted, no update
         S.iter[sg] += 1;
-        if (mixed) {
-            S.repl[sg] = (fin < kReplaceB * S.last[sg] || bconv(ctl, fin, S.init[sg]) || S.iter[sg] >= ctl.maxIter ||
-                          !isfinite(fin)) ? 1 : 0;
-        } else {
-            const bool c = bconv(ctl, fin, S.init[sg]);
-            const bool more = (S.iter[sg] < ctl.maxIter && !c) || S.iter[sg] < ctl.minIter;
-            S.conv[sg] = c ? 1 : 0;
-            if (!more || !isfinite(fin)) S.active[sg] = 0;
-        }
+        S.conv[sg] = 0;
+        return;
+    }
+    if (S.sing[sg]) {
+        S.active[sg] = 0;
+        return;
+    }
+    const double fin = res[sg] / S.nf[sg];
+    S.fin[sg] = fin;
+    S.iter[sg] += 1;
+    if (mixed) {
+        S.repl[sg] = (fin < kReplaceB * S.last[sg] || bconv(ctl, fin, S.init[sg]) || S.iter[sg] >= ctl.maxIter ||
+                      !isfinite(fin)) ? 1 : 0;
+    } else {
+        const bool c = bconv(ctl, fin, S.init[sg]);
+        const bool more = (S.iter[sg] < ctl.maxIter && !c) || S.iter[sg] < ctl.minIter;
+        S.conv[sg] = c ? 1 : 0;
+        if (!more || !isfinite(fin)) S.active[sg] = 0;
     }
 }
 
@@ -476,74 +456,94 @@ __global__ void k_b_after(int nCases, Ctl ctl, BSeg S, const double *__restrict_
 }
 
 // BiCGStab scalars
-__global__ void k_b_bicg_r0r(int nSeg, BSeg S, const double *__restrict__ res) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg]) continue;
-        const double old = S.r0r[sg], r0r = res[sg];
-        S.r0rOld[sg] = old;
-        S.r0r[sg] = r0r;
-        if (fabs(r0r) < 1e-300) { S.sing[sg] = 1; continue; }
-        if (S.iter[sg] > 0 && !S.rst[sg]) {
-            const double om = S.omega[sg];
-            if (fabs(om) < 1e-300) { S.sing[sg] = 1; continue; }
-            S.beta[sg] = (r0r / old) * (S.alpha[sg] / om);
-        }
+__device__ __forceinline__ void seg_bicg_r0r(int nSeg, const BSeg &S, const double *res, int sg) {
+    if (!S.active[sg]) return;
+    const double old = S.r0r[sg], r0r = res[sg];
+    S.r0rOld[sg] = old;
+    S.r0r[sg] = r0r;
+    if (fabs(r0r) < 1e-300) { S.sing[sg] = 1; return; }
+    if (S.iter[sg] > 0 && !S.rst[sg]) {
+        const double om = S.omega[sg];
+        if (fabs(om) < 1e-300) { S.sing[sg] = 1; return; }
+        S.beta[sg] = (r0r / old) * (S.alpha[sg] / om);
     }
 }
-__global__ void k_b_bicg_alpha(int nSeg, BSeg S, const double *__restrict__ res) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg] || S.sing[sg]) continue;
-        S.alpha[sg] = S.r0r[sg] / res[sg];
-        S.rst[sg] = 0;
-    }
+__device__ __forceinline__ void seg_bicg_alpha(int nSeg, const BSeg &S, const double *res, int sg) {
+    if (!S.active[sg] || S.sing[sg]) return;
+    S.alpha[sg] = S.r0r[sg] / res[sg];
+    S.rst[sg] = 0;
 }
 // the half-step test on |s|; singular segments stop here
-__global__ void k_b_bicg_half(int nSeg, Ctl ctl, BSeg S, const double *__restrict__ res, int mixed) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg]) continue;
-        if (S.sing[sg]) {
-            S.active[sg] = 0;
-            continue;
-        }
-        const double fs = res[sg] / S.nf[sg];
-        if (bconv(ctl, fs, S.init[sg])) {
-            S.conv[sg] = 2;
-            S.repl[sg] = mixed ? 1 : 0;
-            if (!mixed) S.fin[sg] = fs;
-        }
+__device__ __forceinline__ void seg_bicg_half(int nSeg, const BSeg &S, const double *res, int sg, const Ctl &ctl, int mixed) {
+    if (!S.active[sg]) return;
+    if (S.sing[sg]) {
+        S.active[sg] = 0;
+        return;
+    }
+    const double fs = res[sg] / S.nf[sg];
+    if (bconv(ctl, fs, S.init[sg])) {
+        S.conv[sg] = 2;
+        S.repl[sg] = mixed ? 1 : 0;
+        if (!mixed) S.fin[sg] = fs;
     }
 }
 // after the half step: mixed precision stops or restarts from the FP64
 // residual of the replacement; FP64 stops (the plain solvers' early exit)
-__global__ void k_b_half_after(int nSeg, Ctl ctl, BSeg S, const double *__restrict__ res, int mixed) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg] || S.conv[sg] != 2) continue;
-        if (!mixed) {
-            S.iter[sg] += 1;
-            S.conv[sg] = 1;
-            S.active[sg] = 0;
-            continue;
-        }
-        const double fin = res[sg] / S.nf[sg];
-        S.fin[sg] = fin;
-        S.last[sg] = fin;
-        S.repl[sg] = 0;
-        const int it = S.iter[sg] + 1;
-        const bool c = bconv(ctl, fin, S.init[sg]);
-        if ((c && it >= ctl.minIter) || it >= ctl.maxIter || !isfinite(fin)) {
-            S.iter[sg] = it;
-            S.conv[sg] = c ? 1 : 0;
-            S.active[sg] = 0;
-        } else {
-            S.rst[sg] = 1;   // conv stays 2: the second half is skipped, the iteration counted
-        }
+__device__ __forceinline__ void seg_half_after(int nSeg, const BSeg &S, const double *res, int sg, const Ctl &ctl, int mixed) {
+    if (!S.active[sg] || S.conv[sg] != 2) return;
+    if (!mixed) {
+        S.iter[sg] += 1;
+        S.conv[sg] = 1;
+        S.active[sg] = 0;
+        return;
+    }
+    const double fin = res[sg] / S.nf[sg];
+    S.fin[sg] = fin;
+    S.last[sg] = fin;
+    S.repl[sg] = 0;
+    const int it = S.iter[sg] + 1;
+    const bool c = bconv(ctl, fin, S.init[sg]);
+    if ((c && it >= ctl.minIter) || it >= ctl.maxIter || !isfinite(fin)) {
+        S.iter[sg] = it;
+        S.conv[sg] = c ? 1 : 0;
+        S.active[sg] = 0;
+    } else {
+        S.rst[sg] = 1;   // conv stays 2: the second half is skipped, the iteration counted
     }
 }
-__global__ void k_b_bicg_omega(int nSeg, BSeg S, const double *__restrict__ res) {
-    for (int sg = threadIdx.x + blockIdx.x * blockDim.x; sg < nSeg; sg += blockDim.x * gridDim.x) {
-        if (!S.active[sg] || S.sing[sg] || S.conv[sg] == 2) continue;
-        S.omega[sg] = res[1 * nSeg + sg] / res[sg];
+__device__ __forceinline__ void seg_bicg_omega(int nSeg, const BSeg &S, const double *res, int sg) {
+    if (!S.active[sg] || S.sing[sg] || S.conv[sg] == 2) return;
+    S.omega[sg] = res[1 * nSeg + sg] / res[sg];
+}
+
+// partial[(slot * 6 + k) * nBlk + blk]; res[slot * nSeg + case * 8 + k]
+// The warp that has summed a segment's slots goes on with the scalar logic OP that
+// follows the reduction (a kernel of its own for it was 4 to 6 us of a 60 us
+// iteration of four small cases).
+enum SegOp { SEG_NONE, SEG_PCG_A, SEG_PCG_ALPHA, SEG_ITER, SEG_R0R, SEG_ALPHA, SEG_HALF, SEG_HALF_AFTER, SEG_OMEGA };
+template <int OP>
+__global__ void k_b_fin(int nSlots, unsigned vm, BTab t, const double *__restrict__ partial, double *res, BSeg S, Ctl ctl,
+                        int mixed, int skipHalf) {
+    const int cb = blockIdx.x, k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (k >= 6 || !((vm >> k) & 1u)) return;
+    const int b0 = t.caseBlk[cb], b1 = t.caseBlk[cb + 1];
+    const int nSeg = 8 * t.nCases;
+    for (int slot = 0; slot < nSlots; ++slot) {
+        double v = 0.0;
+        for (int i = b0 + lane; i < b1; i += 32) v += partial[(slot * 6 + k) * t.nBlk + i];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) res[slot * nSeg + cb * 8 + k] = v;
     }
+    if (lane != 0) return;
+    const int sg = cb * 8 + k;
+    if (OP == SEG_PCG_A) seg_pcg_a(nSeg, S, res, sg, mixed);
+    if (OP == SEG_PCG_ALPHA) seg_pcg_alpha(nSeg, S, res, sg);
+    if (OP == SEG_ITER) seg_iter_fin(nSeg, S, res, sg, ctl, skipHalf, mixed);
+    if (OP == SEG_R0R) seg_bicg_r0r(nSeg, S, res, sg);
+    if (OP == SEG_ALPHA) seg_bicg_alpha(nSeg, S, res, sg);
+    if (OP == SEG_HALF) seg_bicg_half(nSeg, S, res, sg, ctl, mixed);
+    if (OP == SEG_HALF_AFTER) seg_half_after(nSeg, S, res, sg, ctl, mixed);
+    if (OP == SEG_OMEGA) seg_bicg_omega(nSeg, S, res, sg);
 }
 
 // ---- level-scheduled sweeps over the union (cases without a 2-D layout) ---
@@ -1306,7 +1306,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_pcg_case(BTab t, BEll e, 
         }
         const double rho = case_total(acc_value(a0));
         const double wq = mixed ? case_total(acc_value(a1)) : 0.0;
-        if (tid == 0) {   // k_b_pcg_a
+        if (tid == 0) {   // seg_pcg_a
             const double aold = S.A[sg];
             S.Aold[sg] = aold;
             S.A[sg] = rho;
@@ -1370,7 +1370,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_pcg_case(BTab t, BEll e, 
             }
         }
         const double wApA = case_total(acc_value(aq));
-        if (tid == 0) {   // k_b_pcg_alpha
+        if (tid == 0) {   // seg_pcg_alpha
             if (fabs(wApA) / S.nf[sg] < 1e-300) {
                 S.sing[sg] = 1;
                 S.alpha[sg] = 0.0;
@@ -1416,7 +1416,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_pcg_case(BTab t, BEll e, 
             }
         }
         const double rs = case_total(acc_value(ar));
-        if (tid == 0) {   // k_b_iter_fin
+        if (tid == 0) {   // seg_iter_fin
             if (S.sing[sg]) {
                 S.active[sg] = 0;
             } else {
@@ -1673,7 +1673,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
                            });
             double v[3] = {acc_value(a[0]), acc_value(a[1]), acc_value(a[2])};
             case_totals(v);
-            if (tid == 0) {   // k_b_bicg_r0r
+            if (tid == 0) {   // seg_bicg_r0r
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     if (!((act >> k) & 1u)) continue;
@@ -1742,7 +1742,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
                            });
             double v[3] = {acc_value(a[0]), acc_value(a[1]), acc_value(a[2])};
             case_totals(v);
-            if (tid == 0)   // k_b_bicg_alpha
+            if (tid == 0)   // seg_bicg_alpha
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     if (!((live >> k) & 1u)) continue;
@@ -1776,7 +1776,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
                            });
             double v[3] = {acc_value(a[0]), acc_value(a[1]), acc_value(a[2])};
             case_totals(v);
-            if (tid == 0) {   // k_b_bicg_half
+            if (tid == 0) {   // seg_bicg_half
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const int sg = s0 + k;
@@ -1813,7 +1813,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
             }
             double tot[3];
             replace(mr, tot);
-            if (tid == 0) {   // k_b_half_after
+            if (tid == 0) {   // seg_half_after
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const int sg = s0 + k;
@@ -1875,7 +1875,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
 #pragma unroll
             for (int i = 0; i < 6; ++i) v[i] = acc_value(a[i]);
             case_totals(v);
-            if (tid == 0)   // k_b_bicg_omega
+            if (tid == 0)   // seg_bicg_omega
 #pragma unroll
                 for (int k = 0; k < 3; ++k)
                     if ((full >> k) & 1u) S.omega[s0 + k] = v[3 + k] / v[k];
@@ -1915,7 +1915,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
                            });
             double v[3] = {acc_value(a[0]), acc_value(a[1]), acc_value(a[2])};
             case_totals(v);
-            if (tid == 0) {   // k_b_iter_fin (skipHalf)
+            if (tid == 0) {   // seg_iter_fin (skipHalf)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const int sg = s0 + k;
@@ -2023,10 +2023,10 @@ struct BSolver {
     }
     static size_t vstride(int n) { return (6 * (size_t)n + 31) / 32 * 32; }
     V *v(int i) const { return vec + (size_t)i * vstride(N); }
-    int gridSeg() const { return (nSeg + 255) / 256; }
 
-    void fin(int nSlots, unsigned mask) {
-        k_b_fin<<<bt.n, 192, 0, st>>>(nSlots, mask, t, partial, res);
+    template <int OP = SEG_NONE>
+    void fin(int nSlots, unsigned mask, double *to = nullptr, int skipHalf = 0) {
+        k_b_fin<OP><<<bt.n, 192, 0, st>>>(nSlots, mask, t, partial, to ? to : res, S, ctl, mixed, skipHalf);
         RT_CHECK_LAUNCH();
     }
 
@@ -2081,19 +2081,21 @@ struct BSolver {
         RT_CHECK_LAUNCH();
         launch_count(ctx);
     }
+    template <int OP>
     void dot(const V *x, const V *y, const V *x2 = nullptr, const V *y2 = nullptr) {
         k_b_dot<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, S.active, x, y, x2, y2, partial);
         RT_CHECK_LAUNCH();
-        fin(x2 ? 2 : 1, vm);
+        fin<OP>(x2 ? 2 : 1, vm);
         launch_count(ctx, 2);
     }
     // residual replacement of the segments flagged in S.repl
+    template <int OP = SEG_NONE>
     void replace(V *x, V *r) {
         k_b_fold<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, bt.caseOf.p, S.repl, x, a.psi);
         k_b_true<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, e, vm, S.repl, a.diag, a.upper, a.lower, a.source, a.psi, r,
                                                   partial);
         RT_CHECK_LAUNCH();
-        fin(1, vm);
+        fin<OP>(1, vm);
         launch_count(ctx, 3);
     }
 
@@ -2102,7 +2104,7 @@ struct BSolver {
         double *xs = res + 2 * (size_t)nSeg;   // after the two result slots
         k_b_sumx<<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, a.psi, partial);
         RT_CHECK_LAUNCH();
-        k_b_fin<<<bt.n, 192, 0, st>>>(1, vm, t, partial, xs);
+        fin(1, vm, xs);
         k_b_init_res<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, e, vm, a.diag, a.upper, a.lower, a.source, a.psi, xs,
                                                       bt.cellStartD.p, r, x, partial);
         RT_CHECK_LAUNCH();
@@ -2120,53 +2122,42 @@ struct BSolver {
 
     void pcg_iteration(V *r, V *w, V *p, V *q, V *x) {
         precondition(r, w);
-        if (mixed) dot(w, r, w, q);   // q = A p of the previous iteration (unused on the first)
-        else dot(w, r);
-        k_b_pcg_a<<<gridSeg(), 256, 0, st>>>(nSeg, S, res, mixed);
+        if (mixed) dot<SEG_PCG_A>(w, r, w, q);   // q = A p of the previous iteration (unused on the first)
+        else dot<SEG_PCG_A>(w, r);
         k_b_pcg_p<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, bt.caseOf.p, S, w, p);
         amul(p, q);
-        dot(q, p);
-        k_b_pcg_alpha<<<gridSeg(), 256, 0, st>>>(nSeg, S, res);
+        dot<SEG_PCG_ALPHA>(q, p);
         k_b_pcg_update<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, S, p, q, x, r, partial);
         RT_CHECK_LAUNCH();
-        fin(1, vm);
-        k_b_iter_fin<<<gridSeg(), 256, 0, st>>>(nSeg, ctl, S, res, 0, mixed);
+        fin<SEG_ITER>(1, vm);
+        replace(x, r);
+        k_b_after<<<1, 1024, 0, st>>>(bt.n, ctl, S, res);
         RT_CHECK_LAUNCH();
+        launch_count(ctx, 4);
+    }
+
+    void bicg_iteration(V *r, V *r0, V *p, V *y, V *Ay, V *s, V *z, V *tt, V *x) {
+        dot<SEG_R0R>(r0, r);
+        k_b_bicg_p<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, bt.caseOf.p, S, r, Ay, p);
+        precondition(p, y);
+        amul(y, Ay);
+        dot<SEG_ALPHA>(r0, Ay);
+        k_b_bicg_s<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, S, r, Ay, s, partial);
+        RT_CHECK_LAUNCH();
+        fin<SEG_HALF>(1, vm);
+        k_b_axpy_half<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, bt.caseOf.p, S, y, x);
+        RT_CHECK_LAUNCH();
+        replace<SEG_HALF_AFTER>(x, r);
+        precondition(s, z);
+        amul(z, tt);
+        dot<SEG_OMEGA>(tt, tt, tt, s);
+        k_b_bicg_update<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, S, y, z, s, tt, x, r, partial);
+        RT_CHECK_LAUNCH();
+        fin<SEG_ITER>(1, vm, nullptr, 1);
         replace(x, r);
         k_b_after<<<1, 1024, 0, st>>>(bt.n, ctl, S, res);
         RT_CHECK_LAUNCH();
         launch_count(ctx, 7);
-    }
-
-    void bicg_iteration(V *r, V *r0, V *p, V *y, V *Ay, V *s, V *z, V *tt, V *x) {
-        dot(r0, r);
-        k_b_bicg_r0r<<<gridSeg(), 256, 0, st>>>(nSeg, S, res);
-        k_b_bicg_p<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, bt.caseOf.p, S, r, Ay, p);
-        precondition(p, y);
-        amul(y, Ay);
-        dot(r0, Ay);
-        k_b_bicg_alpha<<<gridSeg(), 256, 0, st>>>(nSeg, S, res);
-        k_b_bicg_s<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, S, r, Ay, s, partial);
-        RT_CHECK_LAUNCH();
-        fin(1, vm);
-        k_b_bicg_half<<<gridSeg(), 256, 0, st>>>(nSeg, ctl, S, res, mixed);
-        k_b_axpy_half<V><<<nblocks(N), RT_BLOCK, 0, st>>>(N, vm, bt.caseOf.p, S, y, x);
-        RT_CHECK_LAUNCH();
-        replace(x, r);
-        k_b_half_after<<<gridSeg(), 256, 0, st>>>(nSeg, ctl, S, res, mixed);
-        precondition(s, z);
-        amul(z, tt);
-        dot(tt, tt, tt, s);
-        k_b_bicg_omega<<<gridSeg(), 256, 0, st>>>(nSeg, S, res);
-        k_b_bicg_update<V><<<bt.nBlk, RT_BLOCK, 0, st>>>(t, vm, S, y, z, s, tt, x, r, partial);
-        RT_CHECK_LAUNCH();
-        fin(1, vm);
-        k_b_iter_fin<<<gridSeg(), 256, 0, st>>>(nSeg, ctl, S, res, 1, mixed);
-        RT_CHECK_LAUNCH();
-        replace(x, r);
-        k_b_after<<<1, 1024, 0, st>>>(bt.n, ctl, S, res);
-        RT_CHECK_LAUNCH();
-        launch_count(ctx, 12);
     }
 };
 
