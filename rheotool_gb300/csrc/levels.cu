@@ -204,6 +204,16 @@ __device__ void level_sweep(const LevelView &v, const int *start, Real *x, const
     }
 }
 
+// what lies in shared memory: the values (behind the starts), the levels' starts (all
+// but a chain of some 55,000 levels; those are read where they are)
+constexpr int kValuesIn = 1, kStartsIn = 2;
+__device__ __forceinline__ const int *level_starts(const LevelView &v, unsigned char *smem, int inSmem) {
+    if (!(inSmem & kStartsIn)) return v.start;
+    int *start = reinterpret_cast<int *>(smem);
+    for (int i = threadIdx.x; i <= v.nl; i += blockDim.x) start[i] = v.start[i];
+    return start;   // (the caller has a barrier before it reads them)
+}
+
 // w = M^-1 r of component blockIdx.x / CS of the masked ones, forward and
 // backward.  x holds the values by position: in shared memory (CS == 1 and
 // they fit) or in `scratch`.
@@ -212,16 +222,15 @@ __global__ void __launch_bounds__(kMaxThreads) k_level_apply(LevelView v, LevelC
                                                             int inSmem, const Real *r, Real *w, Real *scratch,
                                                             const unsigned *dmask) {
     extern __shared__ __align__(16) unsigned char smem[];
-    int *start = reinterpret_cast<int *>(smem);
     next_may_start();
-    for (int i = threadIdx.x; i <= v.nl; i += blockDim.x) start[i] = v.start[i];
+    const int *start = level_starts(v, smem, inSmem);
     wait_for_previous();
     const unsigned live = dmask ? mask & *dmask : mask;
     unsigned m = mask;
     for (int q = blockIdx.x / CS; q > 0; --q) m &= m - 1;
     const int comp = __ffs(m) - 1;
     if (!((live >> comp) & 1u)) return;   // (every CTA of the cluster alike)
-    Real *x = inSmem ? reinterpret_cast<Real *>(smem + ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16)
+    Real *x = inSmem & kValuesIn ? reinterpret_cast<Real *>(smem + ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16)
                      : scratch + (size_t)comp * v.N;
     r += (size_t)comp * v.N;
     w += (size_t)comp * v.N;
@@ -249,11 +258,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_level_factor(LevelView v, int w
                                                              double *__restrict__ rD) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
-    int *start = reinterpret_cast<int *>(smem);
-    double *x = inSmem ? reinterpret_cast<double *>(smem + ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16) : scratch;
+    const int *start = level_starts(v, smem, inSmem);
+    double *x = inSmem & kValuesIn ? reinterpret_cast<double *>(smem + ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16) : scratch;
     const int rank = CS > 1 ? blockIdx.x % CS : 0;
     const int all = CS * blockDim.x, tid = rank * blockDim.x + threadIdx.x;
-    for (int i = threadIdx.x; i <= v.nl; i += blockDim.x) start[i] = v.start[i];
     for (int p = tid; p < v.N; p += all) x[p] = diag[v.cell[p]];
     __syncthreads();
     if (CS > 1) level_barrier<CS>(0);
@@ -289,10 +297,9 @@ struct LevelLaunch {
 LevelLaunch plan(const LevelView &v, size_t real, int passes) {
     LevelLaunch q{};
     const size_t starts = ((size_t)(v.nl + 1) * 4 + 15) / 16 * 16, vals = (size_t)v.N * real;
-    RT_REQUIRE(starts <= kMaxSmem, RT_EINVAL, "too many levels");
     q.CS = v.width > passes * kMaxThreads ? 8 : 1;
-    q.inSmem = q.CS == 1 && starts + vals <= kMaxSmem;
-    q.smem = starts + (q.inSmem ? vals : 0);
+    q.inSmem = (q.CS == 1 && starts + vals <= kMaxSmem ? kValuesIn : 0) | (starts <= kMaxSmem ? kStartsIn : 0);
+    q.smem = (q.inSmem & kStartsIn ? starts : 0) + (q.inSmem & kValuesIn ? vals : 0);
     q.threads = kMaxThreads;
     q.walkers = std::min(kMaxThreads, (v.width + 31) / 32 * 32);
     return q;
@@ -324,7 +331,7 @@ void launch_levels(rt_ctx *ctx, void (*one)(A...), void (*eight)(A...), const Le
 
 template <class Real>
 Real *scratch(rt_ctx *ctx, const LevelLaunch &q, int ncomp) {
-    if (q.inSmem) return nullptr;
+    if (q.inSmem & kValuesIn) return nullptr;
     DBuf<double> &b = ctx->mesh.lev.scratch;
     const size_t need = ((size_t)ctx->mesh.N * ncomp * sizeof(Real) + 7) / 8;
     if (b.n < need) b.alloc(need);

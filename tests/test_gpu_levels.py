@@ -21,6 +21,7 @@ MESHES = {
     "global": lambda: channel_mesh(200, 190, 1),              # 38,000 cells: more than 220 KB in FP64
     "wide": lambda: channel_mesh(50, 44, 44),                 # levels of 1,900 cells: several passes
     "cluster": lambda: channel_mesh(66, 66, 66),              # levels of 3,270 cells: a cluster of eight
+    "chain": lambda: channel_mesh(60000, 1, 1),               # more levels than shared memory holds starts of
 }
 
 
