@@ -484,7 +484,6 @@ struct Prof {
 struct rt_ctx {
     int sweepMode = 0;           // 0 auto, 1 level-scheduled, 2 structured systolic
     int sweepTune = 0;           // 0 autotune the sweep schedule, k > 0: candidate k - 1
-    int sweepRing = 0;           // deepest plane ring of the systolic sweeps (steps; 0: the default cap)
     int device = 0;
     int numSMs = 0;
     cudaStream_t stream = nullptr;
@@ -508,7 +507,6 @@ struct rt_ctx {
     // persistent CTA per case (RT_OPT_BATCH_PERSISTENT; 0: the per-iteration
     // launch sequence)
     int batchPersistent = 1;
-    int sweepComponents = 1;   // RT_OPT_SWEEP_COMPONENTS
     std::vector<rt_step_perf> batchPerf;   // per case: the last step's solver records
     rt::DBuf<double> scal;       // device scalars of the Krylov loops [32 slots][8]
     rt::DBuf<double> stage;      // staging for AoS <-> SoA field transfers
