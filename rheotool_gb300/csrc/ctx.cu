@@ -89,8 +89,10 @@ void map_pages(void *h, size_t bytes) {
     auto map = [](uintptr_t a, uintptr_t b) {
         if (a < b) (void)madvise((void *)a, b - a, kPopulateWrite);
     };
-    const size_t cores = std::max(1u, std::thread::hardware_concurrency());
-    const size_t n = std::max<size_t>(1, std::min({(end - at) / kShare, cores, (size_t)8}));
+    if (at >= end) return;
+    size_t n = std::min<size_t>((end - at) / kShare, 8);
+    // (asked only where it matters: the answer may come from a file)
+    n = n > 1 ? std::min<size_t>(n, std::max(1u, std::thread::hardware_concurrency())) : 1;
     const size_t share = ((end - at) / page + n - 1) / n * page;
     std::vector<std::thread> others;
     try {
