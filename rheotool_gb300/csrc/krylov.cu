@@ -1303,12 +1303,13 @@ __global__ void k_bicg_arm(unsigned act, unsigned *m, double *S) {
     if (k < M_COUNT) m[k] = k == M_ACTIVE ? act : 0u;
 }
 
-// runs `iteration(LoopCtl)` until no component is left: the host launches
-// iterations ahead, at most two, and reads the mapped flag
+// runs `iteration(LoopCtl)` until no component is left, once at least (a component
+// that starts unconverged takes one iteration whatever its budget): the host
+// launches iterations ahead, at most two, and reads the mapped flag
 template <class It>
 void bicg_loop(rt_ctx *ctx, Solver &sv, const SolveArgs &a, It &&iteration) {
     Reduce &red = ctx->red;
-    const int maxIt = std::max(a.ctl.maxIter, a.ctl.minIter);
+    const int maxIt = std::max(1, std::max(a.ctl.maxIter, a.ctl.minIter));
     for (int it = 0; it < maxIt; ++it) {
         iteration(LoopCtl{a.ctl, red.active.p, red.devFlag, it});
         RT_CUDA(cudaEventRecord(red.poll[it & 1], sv.st));

@@ -1,0 +1,50 @@
+"""Solver controls at their limits: an iteration budget of zero, which every
+solver of OpenFOAM's do-while loops (PBiCGStab.C's do { ... } while) spends one
+iteration on when it starts unconverged."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from rheotool_gb300 import abi
+from rheotool_gb300.case import SolverControl, contraction_case
+from rheotool_gb300.mesh import contraction_mesh
+
+from test_gpu_parity import laplacian_system, rel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("structured", [True, False])
+@pytest.mark.parametrize("precision", [abi.RT_PREC_FP64, abi.RT_PREC_MIXED])
+def test_pbicgstab_without_a_budget_makes_one_iteration(ctx, structured, precision):
+    """maxIter 0: a component that starts converged takes none, the others one,
+    with the psi of maxIter 1; in FP64 the oracle's."""
+    from oracle.pyoracle import Oracle
+    mesh = contraction_mesh(12, 10, 30, 10, 6, 4.0, 4.0)
+    if not structured:
+        mesh = dataclasses.replace(mesh, shape=None, cellIJK=None)
+    rng = np.random.default_rng(61)
+    diag, upper, lower = laplacian_system(mesh, rng, asym=3.0)
+    b = rng.normal(size=(3, mesh.nCells)) * mesh.V
+    b[1] = 0.0
+    ctx.upload_mesh(mesh)
+    out = {}
+    try:
+        ctx.set_precision(precision)
+        for budget in (0, 1):
+            x = np.zeros_like(b)
+            ctl = SolverControl("PBiCGStab", "DILU", 1e-12, 0.0, 0, budget)
+            perf = ctx.ldu_solve(diag, upper, lower, b, x, ctl)
+            out[budget] = (x, [p.nIterations for p in perf], [p.finalResidual for p in perf])
+    finally:
+        ctx.set_precision(abi.RT_PREC_FP64)
+    assert out[0][1] == [1, 0, 1] and out[0][1:] == out[1][1:]
+    assert np.array_equal(out[0][0], out[1][0])
+    if precision == abi.RT_PREC_FP64:
+        orc = Oracle(contraction_case(mesh))
+        for k in range(3):
+            xo = np.zeros(mesh.nCells)
+            po = orc.ldu_solve(diag, upper, lower, b[k].copy(), xo, SolverControl("PBiCGStab", "DILU", 1e-12, 0.0, 0, 0))
+            assert po.nIterations == out[0][1][k]
+            assert rel(out[0][0][k], xo) < 1e-9
