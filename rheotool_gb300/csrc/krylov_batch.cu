@@ -2258,8 +2258,10 @@ rt_status run_batch(rt_ctx *ctx, const SolveArgs &a, rt_solver_perf *perf) {
         bt.sPending = true;
         active = 0;
     }
-    while (active && done < std::min(kEager, cap)) {
-        body();   // (the first one sets kernel attributes outside any capture)
+    // (once at least, whatever the budget; the first one sets kernel attributes
+    // outside any capture)
+    while (active && done < std::max(1, std::min(kEager, cap))) {
+        body();
         ++done;
         active = sv.poll();
     }

@@ -48,3 +48,26 @@ def test_pbicgstab_without_a_budget_makes_one_iteration(ctx, structured, precisi
             po = orc.ldu_solve(diag, upper, lower, b[k].copy(), xo, SolverControl("PBiCGStab", "DILU", 1e-12, 0.0, 0, 0))
             assert po.nIterations == out[0][1][k]
             assert rel(out[0][0][k], xo) < 1e-9
+
+
+@pytest.mark.parametrize("precision", [abi.RT_PREC_FP64, abi.RT_PREC_MIXED])
+@pytest.mark.parametrize("budget", [-2, -5])
+def test_batch_below_zero_budget_makes_one_iteration(precision, budget):
+    """A small batch (the launch path) with a negative maxIter: the step of maxIter 0."""
+    from rheotool_gb300.batch import BatchContext, cavity_sweep
+    out = {}
+    for n in (0, budget):
+        cases = cavity_sweep(n_cases=3, n_min=8, n_max=20, seed=7, dt=5e-3, precision=precision)
+        for c in cases:
+            for s in (c.solverP, c.solverU, c.solverTheta):
+                s.maxIter = n
+        bt = BatchContext(cases)
+        try:
+            bt.step(1)
+            f = bt.ctx.fields()
+            out[n] = ([(p.p.nIterations, p.U[0].nIterations, p.theta[0].nIterations) for p in bt.case_perf()], f)
+        finally:
+            bt.ctx.close()
+    assert out[budget][0] == out[0][0] == [(1, 1, 1)] * 3
+    for name in ("U", "p", "theta"):
+        assert np.array_equal(getattr(out[budget][1], name), getattr(out[0][1], name)), name
