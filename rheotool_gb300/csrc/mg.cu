@@ -269,7 +269,8 @@ __global__ void k_mg_smooth(MgLev L, int colour, unsigned m, const unsigned *dm)
                 (split(L.b, L, q, colour)[t] - nb_sum(c, n, split(L.x, L, q, 1 - colour))) / c[0];
 }
 
-// level 0's last half-sweep (red): every cell's x to w in cell order
+// level 0's last half-sweep (red): every cell's x to w in cell order (0 where the
+// diagonal is: such a cell of the matrix is outside the mesh to the cycle)
 template <class T>
 __global__ void k_mg_last(MgLev L, int colour, unsigned m, const int *__restrict__ cellAt, int N, T *__restrict__ w,
                           const unsigned *dm) {
@@ -290,7 +291,7 @@ __global__ void k_mg_last(MgLev L, int colour, unsigned m, const int *__restrict
         if ((m >> q) & 1u) {
             const float *x = split(L.x, L, q, 1 - colour);
             if (mine >= 0)
-                w[(size_t)q * N + mine] = (T)((split(L.b, L, q, colour)[t] - nb_sum(c, n, x)) / c[0]);
+                w[(size_t)q * N + mine] = c[0] != 0.0f ? (T)((split(L.b, L, q, colour)[t] - nb_sum(c, n, x)) / c[0]) : T(0);
             if (other >= 0) w[(size_t)q * N + other] = (T)x[t];
         }
 }
