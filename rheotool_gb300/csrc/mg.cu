@@ -196,7 +196,9 @@ __global__ void k_mg_coarsen(MgLev F, MgLev C, int sym) {
     }
 }
 
-// the split coefficients of a level, once its box-order ones are complete
+// the split coefficients of a level, once its box-order ones are complete, and x = 0
+// where the diagonal is zero: no pass writes x there, and it may hold that of an
+// earlier matrix in which the cell had one
 __global__ void k_mg_split(MgLev L) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= 2 * L.nh) return;
@@ -216,6 +218,9 @@ __global__ void k_mg_split(MgLev L) {
     }
 #pragma unroll
     for (int k = 0; k < 7; ++k) L.co[(2 * k + colour) * L.ns + t] = c[k];
+    if (c[0] == 0.0f)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) L.x[(2 * q + colour) * L.ns + t] = 0.0f;
 }
 
 __device__ __forceinline__ void coeffs(const MgLev &L, int colour, int t, float (&c)[7]) {

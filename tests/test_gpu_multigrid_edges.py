@@ -42,7 +42,7 @@ CELLS = {"red": (8, 12), "black": (8, 13)}   # (i, j): i + j even, odd
 
 
 @pytest.mark.parametrize("solver,pre,asym,nc", [("PCG", "DIC", 0.0, 1), ("PBiCGStab", "DILU", 0.3, 2)])
-@pytest.mark.parametrize("colour", ["red"])
+@pytest.mark.parametrize("colour", ["red", "black"])
 def test_zero_diagonal_in_fp32_leaves_the_cell_alone(ctx, colour, solver, pre, asym, nc):
     """A cell that the V-cycle cannot divide by keeps its psi, also where an
     earlier matrix of the same mesh moved it; the other cells get their solution."""
