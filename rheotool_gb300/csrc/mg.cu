@@ -751,8 +751,12 @@ int enqueue_vcycle(rt_ctx *ctx, const std::vector<MgLev> &L, unsigned m, const T
     }
     launch_tail(L, tf, m, dm, st);
     ++launches;
-    if (nL == 1) {   // a mesh no larger than the coarsest level: its x to w, as it is
-        launch_next(k_mg_last<T>, blocks(L[0].nh), kPassBlock, 0, st, L[0], 1, m, (const int *)s.cellAt.p, N, w, dm);
+    if (nL == 1) {
+        // a mesh no larger than the coarsest level: its x to w.  The sweeps ended on
+        // red, and the same half-sweep again changes nothing; one more on black would
+        // make the cycle unsymmetric, which PCG pays for (16 x 16 cells 18 iterations
+        // against 12, 128 x 4 91 against 71)
+        launch_next(k_mg_last<T>, blocks(L[0].nh), kPassBlock, 0, st, L[0], 0, m, (const int *)s.cellAt.p, N, w, dm);
         RT_CHECK_LAUNCH();
         return launches + 1;
     }

@@ -68,3 +68,70 @@ def test_zero_diagonal_in_fp32_leaves_the_cell_alone(ctx, colour, solver, pre, a
     x64[:, cell] = 0.75
     # (condition number below 1e4, residuals below 1e-12: see the box test of the V-cycle)
     assert np.linalg.norm(x - x64) <= 1e-8 * np.linalg.norm(x64)
+
+
+def one_level_pcg(mesh, diag, up, b, tol, budget):
+    """Iterations of flexible PCG with a one-level cycle in FP32: from x = 0 a red
+    half-sweep, then sixteen times black and red, which is symmetric."""
+    N = mesh.nCells
+    o, n = mesh.owner, mesh.neighbour
+    red = mesh.cellIJK.sum(axis=1) % 2 == 0
+    up32, d32 = up.astype(np.float32), diag.astype(np.float32)
+
+    def neighbours(x):
+        y = np.zeros(N, np.float32)
+        np.add.at(y, o, up32 * x[n])
+        np.add.at(y, n, up32 * x[o])
+        return y
+
+    def cycle(r):
+        r32, x = r.astype(np.float32), np.zeros(N, np.float32)
+        for colour in [red] + [~red, red] * 16:
+            x = np.where(colour, (r32 - neighbours(x)) / d32, x)
+        return x.astype(np.float64)
+
+    def amul(x):
+        y = diag * x
+        np.add.at(y, o, up * x[n])
+        np.add.at(y, n, up * x[o])
+        return y
+
+    nf = np.abs(b).sum() + 1e-20   # (psi starts from zero)
+    r, p, q, rho, alpha = b.copy(), None, None, 0.0, 0.0
+    for it in range(1, budget + 1):
+        w = cycle(r)
+        beta = 0.0 if p is None else -alpha * (w @ q) / rho
+        rho = w @ r
+        p = w if p is None else w + beta * p
+        q = amul(p)
+        alpha = rho / (p @ q)
+        r = r - alpha * q
+        if np.abs(r).sum() / nf < tol:
+            return it
+    return budget
+
+
+@pytest.mark.parametrize("dims", [(16, 16, 1), (22, 22, 1), (8, 8, 8), (128, 4, 1)])
+def test_one_level_cycle_is_symmetric(ctx, dims):
+    """A box of at most 512 cells is one level.  PCG needs a symmetric cycle: the
+    library takes no more iterations than the reference loop with such a cycle
+    (and two, for other roundings), on a Laplacian with one reference cell."""
+    nx, ny, nz = dims
+    mesh = cavity_mesh(nx, ny) if nz == 1 else channel_mesh(nx, ny, nz)
+    rng = np.random.default_rng(72)
+    N = mesh.nCells
+    up = -mesh.magSf * mesh.deltaCoeffs * (1.0 + rng.random(mesh.nFaces))
+    diag = -(np.bincount(mesh.owner, up, N) + np.bincount(mesh.neighbour, up, N))
+    diag[0] *= 2.0
+    b = rng.normal(size=N)
+    tol = 1e-8
+    want = one_level_pcg(mesh, diag, up, b, tol, 300)
+    ctx.upload_mesh(mesh)
+    try:
+        ctx.set_option(abi.RT_OPT_MIXED_TIGHTEN, 0)
+        x = np.zeros((1, N))
+        perf = solve(ctx, diag, up, up, b, x, SolverControl("PCG", "DIC", tol, 0.0, 0, 300))[0]
+    finally:
+        ctx.set_option(abi.RT_OPT_MIXED_TIGHTEN, 2)
+    assert perf.converged and want < 300
+    assert perf.nIterations <= want + 2, (perf.nIterations, want)
