@@ -68,6 +68,11 @@ void grad_scalar(rt_ctx *ctx, const double *x, const double *xb, double *g) {
 // ---------------------------------------------------------------------------
 // GaussDefCmpw
 // ---------------------------------------------------------------------------
+// below 2^959: sums of a few such values times a cell distance are finite
+__device__ __forceinline__ bool moderate_word(int hi) { return (unsigned)(hi & 0x7ff00000) < (unsigned)(1023 + 959) << 20; }
+__device__ __forceinline__ bool moderate(double x) { return moderate_word(__double2hiint(x)); }
+__device__ __forceinline__ bool moderate(const double *x) { return moderate_word(reinterpret_cast<const int *>(x)[1]); }
+
 // face pass: upwind coefficients and, per component, the deferred-correction
 // flux phi_f (psi_f^HR - psi_f^UD)
 template <int NC>
@@ -86,9 +91,10 @@ __global__ void k_defc_face(MeshView m, Lims L, int hr, const double *__restrict
     int o = m.owner[f], n = m.neighbour[f];
     double d0 = m.d[f], d1 = m.d[m.F + f], d2 = m.d[2 * m.F + f];
     // the terms of the upwind side alone: the weights u and 1 - u of the others are
-    // zero, which adds nothing to a finite sum
+    // zero, which adds nothing to a finite sum.  Where the other side may not be
+    // finite its term counts: zero times an infinity makes the flux no number
     const bool fromOwner = ph >= 0.0;
-    const int up = fromOwner ? o : n;
+    const int up = fromOwner ? o : n, down = fromOwner ? n : o;
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
         double g0 = g[((size_t)0 * NC + k) * N + up], g1 = g[((size_t)1 * NC + k) * N + up],
@@ -104,6 +110,12 @@ __global__ void k_defc_face(MeshView m, Lims L, int hr, const double *__restrict
         double am = a - 1.0;
         double far = __dmul_rn(1.0 - a - bb, fromOwner ? xn - 2.0 * gud : xo + 2.0 * gud);
         double tf = __fma_rn(fromOwner ? bb : am, xn, __fma_rn(fromOwner ? am : bb, xo, far));
+        const double *gd = g + (size_t)k * N + down;
+        const size_t row = (size_t)NC * N;
+        if (!(moderate(gd) && moderate(gd + row) && moderate(gd + 2 * row) && moderate(xo) && moderate(xn))) {
+            const double gdd = gd[0] * d0 + gd[row] * d1 + gd[2 * row] * d2;
+            tf += (1.0 - a - bb) * (fromOwner ? xo + 2.0 * gdd : xn - 2.0 * gdd) * 0.0;
+        }
         flux[(size_t)k * m.F + f] = tf * ph;
     }
 }
