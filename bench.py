@@ -695,7 +695,7 @@ def main():
                        "cells": N, "faces": F, "parallelism": f"replicas x{world} (independent cases)",
                        "l2": "inputs larger than L2: the step touches ~2 GB of fields and matrices per step",
                        "iterations_last_step": iters(perf),
-                       "sweep_schedule_autotuned": schedule},
+                       "sweep_schedule": schedule},
             "clocks": clocks, "gpu_launches": launches, "roofline": roof, "e2e": e2e, "cpu_baseline": cpu,
         }
         if second is not None:

@@ -498,9 +498,9 @@ rt_status rt_batch_case_setup(rt_ctx *ctx, const rt_bc_desc *bcs,
                               const int32_t *pRefCell, const double *pRefValue);
 rt_status rt_batch_step_perf(rt_ctx *ctx, rt_step_perf *perf);
 
-/* The sweep schedules in use: schedule[0..2] = candidate, P, NB of the FP64
- * one-component sweeps, schedule[3..5] of the FP32 ones (-1, 0, 0 before the
- * first application).  No reference counterpart. */
+/* The schedules of the last systolic sweeps: schedule[0..2] = candidate, P, NB
+ * of the FP64 sweeps, schedule[3..5] of the FP32 ones (-1, 0, 0 before the
+ * first application); the default depends on the number of components.  No reference counterpart. */
 rt_status rt_sweep_schedule(rt_ctx *ctx, int32_t *schedule);
 
 /* Device memory held by all contexts of this library in the process (bytes):

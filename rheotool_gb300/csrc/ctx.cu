@@ -1355,12 +1355,11 @@ rt_status rt_sweep_schedule(rt_ctx *ctx, int32_t *schedule) {
     return guarded(ctx, [&]() -> rt_status {
         RT_REQUIRE(schedule, RT_EINVAL, "null argument");
         const StructMesh &s = ctx->mesh.sm;
-        static const int P[5] = {8, 8, 16, 16, 4}, NB[5] = {3, 5, 3, 4, 6};
         for (int i = 0; i < 2; ++i) {
             const int k = s.tune[i];
             schedule[3 * i] = k;
-            schedule[3 * i + 1] = k >= 0 ? P[k] : 0;
-            schedule[3 * i + 2] = k >= 0 ? NB[k] : 0;
+            schedule[3 * i + 1] = k >= 0 ? kTuneP[k] : 0;
+            schedule[3 * i + 2] = k >= 0 ? kTuneNB[k] : 0;
         }
         return RT_OK;
     });

@@ -148,7 +148,7 @@ struct StructMesh {
     DBuf<int> faceLo, faceHi;  // 3*N: face to the (z, y, x) lower / upper neighbour, -1 if none
     DBuf<int> sync;            // tickets taken, error flag, tiles finished
     DBuf<unsigned long long> xfer[2];   // hand-off words between tiles (FP64, FP32)
-    int tune[2] = {-1, -1};    // schedule of the sweeps (FP64, FP32), -1 before the first application
+    int tune[2] = {-1, -1};    // schedule of the last application (FP64, FP32), -1 before the first
     DBuf<double> data;         // 12 + 6 + 6 arrays of nSkew doubles
     bool pendingCheck = false;
     // the box: the cell of each box position (-1 outside the mesh) and the
@@ -483,7 +483,7 @@ struct Prof {
 
 struct rt_ctx {
     int sweepMode = 0;           // 0 auto, 1 level-scheduled, 2 structured systolic
-    int sweepTune = 0;           // 0 autotune the sweep schedule, k > 0: candidate k - 1
+    int sweepTune = 0;           // the sweep schedule: 0 the default by size and components, k > 0: candidate k - 1
     int device = 0;
     int numSMs = 0;
     cudaStream_t stream = nullptr;

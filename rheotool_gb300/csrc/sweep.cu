@@ -681,22 +681,18 @@ void launch_one(rt_ctx *ctx, const TileRun<Real> &run) {
     launch_next(k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB>, groups * run.ncc, 32 * G::warps, shm, ctx->stream, run);
 }
 
-// Schedules of the sweeps: chunk size P (steps per staged block), staging depth
-// NB (blocks in flight) and with them the CTA's tiles: chunks of 16 steps leave
+// Schedules of the sweeps (sweep.h): chunk size P (steps per staged block), staging
+// depth NB (blocks in flight) and with them the CTA's tiles: chunks of 16 steps leave
 // an FP64 CTA room for two.  RT_OPT_SWEEP_TUNE takes one of them; the default is
 // two tiles and (16, 3), as fewer warps share the SM's issue slots (1M cells,
 // one component: FP64 235 us an application against 248 with four tiles and
 // (8, 5), FP32 132 against 154), but four when the groups of two would not all
 // run at once, one an SM (three components: FP64 258 us against 330, FP32 162
 // against 169).
-constexpr int kTuneN = 5;
-constexpr int kTuneP[kTuneN] = {8, 8, 16, 16, 4};
-constexpr int kTuneNB[kTuneN] = {3, 5, 3, 4, 6};
 constexpr int kNarrow = 2, kWide = 1;
 
 template <class Real, int MODE, int TJ>
-void launch_tuned(rt_ctx *ctx, const TileRun<Real> &run, int k) {
-    const bool all = (run.g.nTJ + 1) / 2 * run.g.nTK * run.ncc <= ctx->numSMs;   // groups of two tiles, one an SM
+void launch_tuned(rt_ctx *ctx, const TileRun<Real> &run, bool all, int k) {
     if constexpr (MODE == 2) {   // its two rings leave room for these
         if constexpr (TJ == 8) {
             if (!all) return launch_one<Real, MODE, TJ, 2, 2, 8, 3>(ctx, run);
@@ -704,7 +700,6 @@ void launch_tuned(rt_ctx *ctx, const TileRun<Real> &run, int k) {
         launch_one<Real, MODE, TJ, 2, 1, 16, 3>(ctx, run);
     } else {
         constexpr int WJ = TJ == 32 ? 4 : 2, WK = TJ == 32 ? 1 : 2;
-        if (k < 0) k = all ? kNarrow : kWide;
         switch (k) {
         case 0: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[0], kTuneNB[0]>(ctx, run); break;
         case 1: launch_one<Real, MODE, TJ, WJ, WK, kTuneP[1], kTuneNB[1]>(ctx, run); break;
@@ -720,8 +715,6 @@ template <class Real, int MODE>
 void launch_mode(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w) {
     StructMesh &s = ctx->mesh.sm;
     if (!mask) return;
-    const int k = ctx->sweepTune - 1;   // -1: the default
-    s.tune[sizeof(Real) == 4 ? 1 : 0] = k >= 0 ? k : kNarrow;
     TileRun<Real> run;
     run.g = g;
     run.mask = mask;
@@ -735,8 +728,11 @@ void launch_mode(rt_ctx *ctx, const SkewT<Real> &g, unsigned mask, Real *w) {
     run.maxSpin = std::max(64ll, ctx->waitLimit >> 3);
     run.stall = ctx->stallTest > 0 ? 1 : 0;
     if (run.stall) --ctx->stallTest;
-    if (s.TJ == 32) launch_tuned<Real, MODE, 32>(ctx, run, k);
-    else launch_tuned<Real, MODE, 8>(ctx, run, k);
+    const bool all = (s.nTJ + 1) / 2 * s.nTK * run.ncc <= ctx->numSMs;   // groups of two tiles, one an SM
+    const int k = ctx->sweepTune > 0 ? ctx->sweepTune - 1 : all ? kNarrow : kWide;
+    if (MODE != 2) s.tune[sizeof(Real) == 4 ? 1 : 0] = k;
+    if (s.TJ == 32) launch_tuned<Real, MODE, 32>(ctx, run, all, k);
+    else launch_tuned<Real, MODE, 8>(ctx, run, all, k);
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     s.pendingCheck = true;

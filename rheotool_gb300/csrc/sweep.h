@@ -5,6 +5,11 @@
 
 namespace rt {
 
+// the schedules that RT_OPT_SWEEP_TUNE chooses from: chunks of P steps, NB staged ahead
+constexpr int kTuneN = 5;
+constexpr int kTuneP[kTuneN] = {8, 8, 16, 16, 4};
+constexpr int kTuneNB[kTuneN] = {3, 5, 3, 4, 6};
+
 // per matrix: rD recurrence and the premultiplied sweep coefficients
 void skew_prepare(rt_ctx *ctx, const double *diag, const double *upper, const double *lower);
 // w = M^-1 r for the masked components (nc <= 6), forward then backward;

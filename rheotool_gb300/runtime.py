@@ -88,7 +88,7 @@ class Context:
         self.set_option(abi.RT_OPT_SWEEP, mode)
 
     def sweep_schedule(self) -> dict:
-        """The tuned schedules of the one-component systolic sweeps."""
+        """The schedules of the last systolic sweeps (chunk of P steps, NB chunks staged ahead)."""
         a = np.zeros(6, np.int32)
         self._check(self.lib.rt_sweep_schedule(self._ctx, abi.iptr(a)), "rt_sweep_schedule")
         return {"fp64": {"candidate": int(a[0]), "P": int(a[1]), "NB": int(a[2])},
