@@ -671,12 +671,9 @@ void launch_one(rt_ctx *ctx, const TileRun<Real> &run) {
     typedef Group<TJ, WJ, WK> G;
     constexpr int shm = group_smem<Real, G, MODE, P, NB>();
     static_assert(shm <= 226 * 1024, "one CTA's shared memory");
-    static bool opted = false;   // per instantiation
-    if (!opted) {
-        RT_CUDA(cudaFuncSetAttribute(k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
-        opted = true;
-    }
+    // (the current device's attribute: set at each launch, for contexts on any device)
+    RT_CUDA(cudaFuncSetAttribute(k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, shm));
     const int groups = (run.g.nTJ + WJ - 1) / WJ * ((run.g.nTK + WK - 1) / WK);
     launch_next(k_tile_sweep<Real, MODE, TJ, WJ, WK, P, NB>, groups * run.ncc, 32 * G::warps, shm, ctx->stream, run);
 }
