@@ -252,10 +252,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_level_apply(LevelView v, LevelC
 // reciprocal in cell order
 template <int CS>
 __global__ void __launch_bounds__(kMaxThreads) k_level_factor(LevelView v, int walkers, int inSmem,
-                                                             const double *__restrict__ diag,
-                                                             const double *__restrict__ upper,
-                                                             const double *__restrict__ lower, double *scratch,
-                                                             double *__restrict__ rD) {
+                                                             const double *diag, const double *upper,
+                                                             const double *lower, double *scratch, double *rD) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int *start = level_starts(v, smem, inSmem);
