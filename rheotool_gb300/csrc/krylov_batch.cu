@@ -1631,9 +1631,10 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
         case_mg_build(mg, cb, N, false, diag, upper, lower);
         case_mg_split(mg, cb, false, lev, reinterpret_cast<float *>(smem));
     }
-    auto vcycles = [&](const V *in, V *out) {
+    // (the components in m: a cycle each, so those that have stopped take none)
+    auto vcycles = [&](unsigned m, const V *in, V *out) {
         for (int k = 0; k < 3; ++k)
-            if ((vm >> k) & 1u) case_mg_apply<V>(mg, cb, lev, in + (size_t)k * N, out + (size_t)k * N);
+            if ((m >> k) & 1u) case_mg_apply<V>(mg, cb, lev, in + (size_t)k * N, out + (size_t)k * N);
     };
     // the segments (components) selected by a predicate on their state
     auto seg_mask = [&](auto pred) {
@@ -1723,7 +1724,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
         __syncthreads();
         // ---- y = M^-1 p, Ay = A y, alpha = r0r / r0.Ay
         if (useMg) {
-            vcycles(p, y);
+            vcycles(live, p, y);
         } else {
             case_precondition(g, cb, N, vm, p, y, err, maxSpin, ring, sProg, stageSmem);
             if (case_error(err)) break;
@@ -1845,7 +1846,7 @@ __global__ void __launch_bounds__(kCaseThreads, 1) k_b_bicg_case(BTab t, BEll e,
         const unsigned full = sMask[3];
         // ---- z = M^-1 s, tt = A z, omega = tt.s / tt.tt
         if (useMg) {
-            vcycles(sv, z);
+            vcycles(full, sv, z);
         } else {
             case_precondition(g, cb, N, vm, sv, z, err, maxSpin, ring, sProg, stageSmem);
             if (case_error(err)) break;
