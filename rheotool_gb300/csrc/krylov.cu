@@ -1463,14 +1463,19 @@ __global__ void k_mx_diag_apply(int N, unsigned mask, const float *__restrict__ 
         if ((mask >> k) & 1u) w[(size_t)k * N + c] = rD[c] * r[(size_t)k * N + c];
 }
 
-// FP64 <-> FP32 copies of the masked components
-__global__ void k_mx_d2f(int N, unsigned mask, const double *__restrict__ a, float *__restrict__ b) {
+// FP64 <-> FP32 copies of the masked components (dm: a device word of those still
+// iterating, or null)
+__global__ void k_mx_d2f(int N, unsigned mask, const double *__restrict__ a, float *__restrict__ b,
+                         const unsigned *__restrict__ dm) {
+    if (dm) mask &= *dm;
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
     for (int k = 0; k < 6; ++k)
         if ((mask >> k) & 1u) b[(size_t)k * N + c] = (float)a[(size_t)k * N + c];
 }
-__global__ void k_mx_f2d(int N, unsigned mask, const float *__restrict__ a, double *__restrict__ b) {
+__global__ void k_mx_f2d(int N, unsigned mask, const float *__restrict__ a, double *__restrict__ b,
+                         const unsigned *__restrict__ dm) {
+    if (dm) mask &= *dm;
     int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= N) return;
     for (int k = 0; k < 6; ++k)
@@ -1925,9 +1930,9 @@ struct Mixed : Solver {
             skew_precondition32d(ctx, a.nc, mask, r, w, dmask);
             return;
         }
-        k_mx_d2f<<<nblocks(N), RT_BLOCK, 0, st>>>(N, mask, r, r32);
-        precondition32(mask, r32, w32);
-        k_mx_f2d<<<nblocks(N), RT_BLOCK, 0, st>>>(N, mask, w32, w);
+        k_mx_d2f<<<nblocks(N), RT_BLOCK, 0, st>>>(N, mask, r, r32, dmask);
+        precondition32(mask, r32, w32, dmask);
+        k_mx_f2d<<<nblocks(N), RT_BLOCK, 0, st>>>(N, mask, w32, w, dmask);
         RT_CHECK_LAUNCH();
         launch_count(ctx, 2);
     }

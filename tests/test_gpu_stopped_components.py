@@ -1,11 +1,15 @@
 """Components and iterations that have stopped cost no preconditioner applications:
 device times of one solve against another of the same sizes, several times apart."""
+import dataclasses
+
 import numpy as np
 import pytest
 
 from rheotool_gb300 import abi
-from rheotool_gb300.case import cavity_case
-from rheotool_gb300.mesh import cavity_mesh
+from rheotool_gb300.case import SolverControl, cavity_case
+from rheotool_gb300.mesh import cavity_mesh, channel_mesh
+
+from test_gpu_parity import laplacian_system
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +42,33 @@ def test_batched_momentum_solve_skips_stopped_components():
         assert iters[0] > 5 and (iters[1] == 0 if kick == 0.0 else iters[1] > 5)
         ms[kick] = min(times)
     assert ms[0.0] < 0.85 * ms[0.1], ms
+
+
+@pytest.mark.parametrize("precision", [abi.RT_PREC_FP64, abi.RT_PREC_MIXED])
+def test_sweeps_launched_ahead_of_the_poll_return_at_once(ctx, precision):
+    """PCG on a mesh without box structure launches sixteen iterations before the
+    host can see that the first met the tolerance: the sweeps of the other
+    fifteen together take less than a half of sixteen that iterate (a tenth)."""
+    mesh = dataclasses.replace(channel_mesh(200, 190, 1), shape=None, cellIJK=None)
+    rng = np.random.default_rng(1)
+    system = laplacian_system(mesh, rng)
+    b = rng.normal(size=(1, mesh.nCells)) * mesh.V
+    ctx.upload_mesh(mesh)
+    scope = "dilu_precondition" if precision == abi.RT_PREC_FP64 else "dilu_precondition32"
+    ms = {}
+    try:
+        ctx.set_precision(precision)
+        # (the mixed form's tolerance is two decades tighter)
+        for n, tolerance, budget in ((16, 1e-300, 16), (1, 0.9 if precision == abi.RT_PREC_FP64 else 90.0, 1000)):
+            times = []
+            for _ in range(3):
+                ctx.profile(True)
+                p = ctx.ldu_solve(*system, b, np.zeros_like(b), SolverControl("PCG", "DIC", tolerance, 0.0, 0, budget))[0]
+                launches, t, _ = ctx.profile_report()[scope]
+                ctx.profile(False)
+                assert launches == 16 and p.nIterations == n
+                times.append(t)
+            ms[n] = min(times)
+    finally:
+        ctx.set_precision(abi.RT_PREC_FP64)
+    assert ms[1] < 0.5 * ms[16], ms
