@@ -1837,11 +1837,13 @@ struct Mixed : Solver {
         }
     }
 
-    // FP64 r -> FP32 preconditioner -> FP64 w (the structured sweeps round on
-    // the way in and out; otherwise through the FP32 vectors r32, w32)
+    // RT_OPT_MIXED_PRECOND's preconditioners are applied by precondition32d, in the PCG
+    // of one component (the pressure solve); PBiCGStab takes the exact sweeps
+    bool pcgOne() const { return a.ctl.solver == RT_SOLVER_PCG && a.nc == 1; }
+
     // the red-black DIC of the pressure solve (one component, structured mesh)
     bool redblack() const {
-        return ctx->mixedJacobi == -1 && a.nc == 1 && a.ctl.preconditioner == RT_PRECOND_DIC &&
+        return ctx->mixedJacobi == -1 && pcgOne() && a.ctl.preconditioner == RT_PRECOND_DIC &&
                ctx->mesh.colour.p != nullptr && !ctx->mesh.hasCoupled;
     }
     void redblack_apply(const double *r, double *w, const unsigned *dmask) {
@@ -1859,7 +1861,7 @@ struct Mixed : Solver {
     // the aggregation multigrid V-cycle of the pressure solve (one component,
     // a symmetric matrix, structured mesh without coupled faces)
     bool multigrid() const {
-        return ctx->mixedJacobi == -2 && a.nc == 1 && a.ctl.preconditioner == RT_PRECOND_DIC && mg_available(ctx);
+        return ctx->mixedJacobi == -2 && pcgOne() && a.ctl.preconditioner == RT_PRECOND_DIC && mg_available(ctx);
     }
     // the same V-cycle for the momentum solve (up to three components, a
     // non-symmetric matrix)
@@ -1871,7 +1873,7 @@ struct Mixed : Solver {
     // the Jacobi-swept DIC/DILU of the pressure solve (one component)
     bool jacobi() const {
         const int pre = a.ctl.preconditioner;
-        return ctx->mixedJacobi > 0 && a.nc == 1 && (pre == RT_PRECOND_DIC || pre == RT_PRECOND_DILU);
+        return ctx->mixedJacobi > 0 && pcgOne() && (pre == RT_PRECOND_DIC || pre == RT_PRECOND_DILU);
     }
     float *jrD() const { return ctx->jac.p; }
     float *jlo() const { return ctx->jac.p + N; }
@@ -1906,6 +1908,8 @@ struct Mixed : Solver {
         launch_count(ctx, 2 * sweeps);
     }
 
+    // FP64 r -> FP32 preconditioner -> FP64 w (the structured sweeps round on
+    // the way in and out; otherwise through the FP32 vectors r32, w32)
     void precondition32d(unsigned mask, const double *r, double *w, float *r32, float *w32,
                          const unsigned *dmask = nullptr) {
         if (multigrid()) {
