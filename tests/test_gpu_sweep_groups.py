@@ -53,3 +53,50 @@ def test_reported_schedule_is_the_one_that_ran(ctx, precision, ny, nz, nc, want)
     assert schedule == want
     _, _, schedule = solve(ctx, system, b, "PCG" if nc == 1 else "PBiCGStab", precision, 2, tune=5)
     assert schedule == {"candidate": 4, "P": 4, "NB": 6}
+
+
+SHAPES = {
+    "groups past the SMs": lambda: channel_mesh(6, 100, 100),       # four tiles by default
+    "one plane": lambda: cavity_mesh(21, 130),                      # tiles of 32 rows
+    "holes": lambda: contraction_mesh(12, 10, 30, 10, 11, 4.0, 4.0),
+    "odd edges": lambda: channel_mesh(17, 9, 5),                    # a row and a plane past the tiles
+}
+
+
+@pytest.mark.parametrize("nc", [1, 3, 6])
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_every_group_shape_gives_the_same_bits(ctx, name, nc):
+    """All schedules against the level-scheduled sweeps in FP64, and against each
+    other in FP32 (whose sweeps take the i term before the j term, as the level
+    sweeps do not)."""
+    mesh = SHAPES[name]()
+    rng = np.random.default_rng(82)
+    system = laplacian_system(mesh, rng, asym=3.0)
+    b = rng.normal(size=(nc, mesh.nCells)) * mesh.V
+    ctx.upload_mesh(mesh)
+    want, iters, _ = solve(ctx, system, b, "PBiCGStab", abi.RT_PREC_FP64, 6, sweep=abi.SWEEP_LEVELS)
+    want32 = None
+    for tune in range(6):
+        x, n, _ = solve(ctx, system, b, "PBiCGStab", abi.RT_PREC_FP64, 6, tune)
+        assert n == iters and np.array_equal(x, want), tune
+        x, n32, _ = solve(ctx, system, b, "PBiCGStab", abi.RT_PREC_MIXED, 6, tune)
+        if want32 is None:
+            want32, iters32 = x, n32
+        assert n32 == iters32 and np.array_equal(x, want32), tune
+
+
+@pytest.mark.parametrize("precision", [abi.RT_PREC_FP64, abi.RT_PREC_MIXED])
+def test_components_side_by_side_equal_one_by_one(ctx, precision):
+    """Three components in one launch (four tiles a CTA on 100 x 40 rows) and each
+    alone (two): the same bits."""
+    mesh = channel_mesh(6, 100, 40)
+    rng = np.random.default_rng(83)
+    system = laplacian_system(mesh, rng, asym=3.0)
+    b = rng.normal(size=(3, mesh.nCells)) * mesh.V
+    ctx.upload_mesh(mesh)
+    x, n, schedule = solve(ctx, system, b, "PBiCGStab", precision, 20)
+    assert schedule == WIDE
+    for k in range(3):
+        xk, nk, schedule = solve(ctx, system, b[k:k + 1].copy(), "PBiCGStab", precision, 20)
+        assert schedule == NARROW
+        assert nk[0] == n[k] and np.array_equal(xk[0], x[k])
