@@ -285,45 +285,6 @@ __global__ void k_sc_fin(unsigned mask, const double *res, double *S) {
     if (k < 6 && ((mask >> k) & 1u)) S[S_FIN * 8 + k] = res[k] / S[S_NF * 8 + k];
 }
 // --------------------------------------------------------------------------
-// vector update kernels
-// --------------------------------------------------------------------------
-// PCG: pA = wA (+ beta pA)
-__global__ void k_pcg_p(int N, unsigned mask, int first, const double *__restrict__ S,
-                        const double *__restrict__ wA, double *__restrict__ pA) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= N) return;
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        size_t i = (size_t)k * N + c;
-        if (first) pA[i] = wA[i];
-        else {
-            double beta = S[S_A * 8 + k] / S[S_AOLD * 8 + k];
-            pA[i] = wA[i] + beta * pA[i];
-        }
-    }
-}
-// PCG: psi += alpha pA; rA -= alpha wA; partial |rA| (slot 0)
-__global__ void k_pcg_update(int N, unsigned mask, const double *__restrict__ S,
-                             const double *__restrict__ pA, const double *__restrict__ wA,
-                             double *__restrict__ psi, double *__restrict__ rA, double *partial, int nB) {
-    for (int k = 0; k < 6; ++k) {
-        if (!((mask >> k) & 1u)) continue;
-        const bool sing = S[S_SING * 8 + k] != 0.0;
-        const double alpha = S[S_ALPHA * 8 + k];
-        double v = 0.0;
-        size_t o = (size_t)k * N;
-        #pragma unroll 4
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < N; c += gridDim.x * blockDim.x) {
-            if (!sing) {
-                psi[o + c] += alpha * pA[o + c];
-                rA[o + c] -= alpha * wA[o + c];
-            }
-            v += fabs(rA[o + c]);
-        }
-        store_partial(partial, nB, 0, k, v);
-    }
-}
-// --------------------------------------------------------------------------
 // host orchestration
 // --------------------------------------------------------------------------
 void reduce_init(rt_ctx *ctx) {
@@ -960,9 +921,7 @@ struct Solver {
 
     // finalize nSlots reduction slots of the masked comps into red.result
     void finalize(int nSlots, unsigned mask) {
-        // blocks beyond rblocks() left stale partials: zero them by using only
-        // the first rblocks() entries — the reduction kernels always launch
-        // exactly nB blocks, so all entries are written.
+        // (the reduction kernels launch exactly nB blocks: all nB entries are written)
         k_finalize<<<nSlots * 6, RT_BLOCK, 0, st>>>(nB, nSlots, mask, ctx->red.partial.p, ctx->red.result.p);
         RT_CHECK_LAUNCH();
         launch_count(ctx);
