@@ -308,8 +308,8 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
  * each running all the iterations of its case in one launch, or as a
  * per-iteration launch sequence replayed for all cases.  0: the launch
  * sequence; 1 (default): persistent when the batch holds at least half as
- * many cases as the GPU has SMs (a CTA per case leaves a small batch's SMs
- * idle); 2: persistent whatever the batch.  Both take the same scalar
+ * many cases as the GPU has SMs (below that it is faster alone, but not with
+ * several contexts stepping small batches side by side); 2: persistent whatever the batch.  Both take the same scalar
  * decisions; the persistent form sums each case's reductions in one pass of
  * its CTA, so the iterates agree to round-off, not bit for bit. */
 #define RT_OPT_BATCH_PERSISTENT 11
@@ -322,7 +322,7 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
  * structured meshes without coupled faces (and in the batched form's
  * persistent solver on structured 2-D cases), the aggregation multigrid
  * V-cycle of RT_OPT_MIXED_PRECOND -2 built from the non-symmetric momentum
- * matrix, its components in one cycle; elsewhere the exact DILU.  0: DILU
+ * matrix, its components in one cycle (batched: a cycle each); elsewhere the exact DILU.  0: DILU
  * with the exact triangular sweeps.  Both stop on the same FP64 residual
  * test; the FP64 plain form always uses the exact sweeps. */
 #define RT_OPT_MIXED_PRECOND_U 13

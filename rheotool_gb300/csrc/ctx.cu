@@ -474,6 +474,8 @@ rt_status rt_mesh_set_ijk(rt_ctx *ctx, int32_t nx, int32_t ny, int32_t nz, const
             for (MgGraph &g : s.mgGraph) g.reset();
             s.mgNext = 0;
         }
+        // (the limit of the former sweeps, eight 32-row warps a plane; the tiles have no
+        // such bound, and a larger box stays refused)
         RT_REQUIRE(ny <= 256, RT_EINVAL, "structured sweeps need ny <= 256");
         s.sync.alloc(SYNC_WORDS);
         for (auto &x : s.xfer) x.release();   // laid out anew on the next sweep

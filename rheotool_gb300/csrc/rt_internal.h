@@ -519,7 +519,7 @@ struct rt_ctx {
     void *noallocScratch = nullptr;
     // bounded waits of the systolic sweeps: spins before a wait gives up
     // (RT_OPT_WAIT_LIMIT); stallTest > 0: the next sweep launch's
-    // cluster-to-cluster consumers expect a tag no producer writes
+    // consumers take the hand-off words of other CTAs as never written
     // (RT_OPT_STALL_TEST, failure-detection tests)
     long long waitLimit = 1ll << 24;
     int stallTest = 0;
