@@ -1064,7 +1064,7 @@ rt_status pcg_device_loop(rt_ctx *ctx, Solver &sv, const SolveArgs &a, rt_solver
     RT_CHECK_LAUNCH();
     launch_count(ctx);
     red.hostFlag[0] = 1;
-    const int maxIt = std::max(a.ctl.maxIter, a.ctl.minIter);
+    const int maxIt = std::max(1, std::max(a.ctl.maxIter, a.ctl.minIter));   // (one at least, as in bicg_loop)
     const double fpc = (double)ctx->mesh.F / N;
     for (int it = 0; it < maxIt; ++it) {
         const int first = it == 0;

@@ -50,6 +50,35 @@ def test_pbicgstab_without_a_budget_makes_one_iteration(ctx, structured, precisi
             assert rel(out[0][0][k], xo) < 1e-9
 
 
+@pytest.mark.parametrize("structured", [True, False])
+@pytest.mark.parametrize("precision", [abi.RT_PREC_FP64, abi.RT_PREC_MIXED])
+def test_pcg_without_a_budget_makes_one_iteration(ctx, structured, precision):
+    """The same of PCG, whose batched form makes one too."""
+    from oracle.pyoracle import Oracle
+    mesh = contraction_mesh(12, 10, 30, 10, 6, 4.0, 4.0)
+    if not structured:
+        mesh = dataclasses.replace(mesh, shape=None, cellIJK=None)
+    rng = np.random.default_rng(63)
+    system = laplacian_system(mesh, rng)
+    b = rng.normal(size=(1, mesh.nCells)) * mesh.V
+    ctx.upload_mesh(mesh)
+    out = {}
+    try:
+        ctx.set_precision(precision)
+        for budget in (0, 1):
+            x = np.zeros_like(b)
+            perf = ctx.ldu_solve(*system, b, x, SolverControl("PCG", "DIC", 1e-12, 0.0, 0, budget))[0]
+            out[budget] = (x, perf.nIterations, perf.finalResidual)
+    finally:
+        ctx.set_precision(abi.RT_PREC_FP64)
+    assert out[0][1] == 1 and out[0][1:] == out[1][1:]
+    assert np.array_equal(out[0][0], out[1][0])
+    if precision == abi.RT_PREC_FP64:
+        xo = np.zeros(mesh.nCells)
+        po = Oracle(contraction_case(mesh)).ldu_solve(*system, b[0].copy(), xo, SolverControl("PCG", "DIC", 1e-12, 0.0, 0, 0))
+        assert po.nIterations == 1 and rel(out[0][0][0], xo) < 1e-9
+
+
 @pytest.mark.parametrize("precision", [abi.RT_PREC_FP64, abi.RT_PREC_MIXED])
 @pytest.mark.parametrize("budget", [-2, -5])
 def test_batch_below_zero_budget_makes_one_iteration(precision, budget):
