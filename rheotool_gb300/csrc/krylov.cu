@@ -1822,11 +1822,12 @@ struct Mixed : Solver {
     bool multigrid() const {
         return ctx->mixedJacobi == -2 && pcgOne() && a.ctl.preconditioner == RT_PRECOND_DIC && mg_available(ctx);
     }
-    // the same V-cycle for the momentum solve (up to three components, a
-    // non-symmetric matrix)
+    // the same V-cycle for the momentum solve (PBiCGStab, up to three components, a
+    // non-symmetric matrix).  What prepare() makes has to be what is applied: PCG's
+    // precondition32d would take the sweeps, or Jacobi's buffers, that nothing made
     bool multigridU() const {
-        return ctx->mixedPrecondU == -2 && a.nc <= 3 && (a.validMask & ~7u) == 0 &&
-               a.ctl.preconditioner == RT_PRECOND_DILU && mg_available(ctx);
+        return ctx->mixedPrecondU == -2 && a.ctl.solver == RT_SOLVER_PBICGSTAB && a.nc <= 3 &&
+               (a.validMask & ~7u) == 0 && a.ctl.preconditioner == RT_PRECOND_DILU && mg_available(ctx);
     }
 
     // the Jacobi-swept DIC/DILU of the pressure solve (one component)
